@@ -126,3 +126,20 @@ def test_casts():
     back = torch.empty(64 * 256, device="cuda")
     K.cast_bf16_to_f32(big[:, 1].contiguous().view(-1), back)
     assert torch.equal(back.view(64, 256), src.bfloat16().float())
+
+
+@pytest.mark.parametrize("rows,d", [(1, 8), (3, 40), (63, 1000), (700, 4104), (2048, 8192)])
+def test_rmsnorm_gain_gradient_at_odd_widths_and_few_rows(rows, d):
+    """Widths that are no multiple of the 32 columns a reducing CTA takes, fewer partial rows than its 32 warps and many
+    more. Tolerance: fp32 sums of `rows` products, so 1e-6 of the sum of their magnitudes."""
+    from ringattention_b200.ops import kernels as K
+
+    torch.manual_seed(rows)
+    x, dy = (torch.randn(rows, d, device="cuda").bfloat16() for _ in range(2))
+    w = torch.ones(d, device="cuda").bfloat16()
+    _, rstd = K.rmsnorm_fwd(x, w, 1e-6)
+    start = torch.randn(d, device="cuda")
+    dw = start.clone()
+    K.rmsnorm_bwd(dy, x, w, rstd, dw)
+    terms = dy.double() * x.double() * rstd.double()[:, None]
+    assert ((dw.double() - (start.double() + terms.sum(0))).abs() <= 1e-6 * (start.double().abs() + terms.abs().sum(0))).all()
