@@ -511,24 +511,88 @@ struct MergeParams {
   long long out_slot_o, out_slot_l, in_slot_o, in_slot_l;  // strides in floats
 };
 
-// One CTA per row = (b, h, i); D threads.
-__global__ void decode_merge_kernel(const MergeParams p) {
-  const int row = blockIdx.x, d = threadIdx.x;
-  const long long slot = p.step_ptr ? ((*p.step_ptr * p.slot_mul + p.slot_add) & 1) : 0;
-  const float* o_in = p.o_part + slot * p.in_slot_o;
-  const float* lp = p.lse_part + slot * p.in_slot_l + static_cast<long long>(row) * p.l_rs;
+// Merged value of column d and log-sum-exp of one row's partials; every thread walks all of them.
+__device__ __forceinline__ void merge_parts(const float* o_row, long long o_ps, const float* lp, long long l_ps, int nparts,
+                                            int d, float& o, float& lse) {
   float mx = -INFINITY;
-  for (int s = 0; s < p.nparts; ++s) mx = fmaxf(mx, lp[s * p.l_ps]);
-  float wsum = 0.f, o = 0.f;
+  for (int s = 0; s < nparts; ++s) mx = fmaxf(mx, lp[s * l_ps]);
+  float wsum = 0.f;
+  o = 0.f;
   if (mx != -INFINITY) {
-    for (int s = 0; s < p.nparts; ++s) {
-      const float w = __expf(lp[s * p.l_ps] - mx);
+    for (int s = 0; s < nparts; ++s) {
+      const float w = __expf(lp[s * l_ps] - mx);
       wsum += w;
-      o += w * o_in[static_cast<long long>(row) * p.o_rs + s * p.o_ps + d];
+      o += w * o_row[s * o_ps + d];
     }
     o /= wsum;
   }
-  const float lse = mx == -INFINITY ? -INFINITY : mx + __logf(wsum);
+  lse = mx == -INFINITY ? -INFINITY : mx + __logf(wsum);
+}
+
+// The same for rows with many partials, 32 columns a CTA: 32 warps of 32 columns take every 32nd partial each and meet in
+// shared memory in a fixed order. A decode call has few rows (batch x heads) and up to 512 partials of each: one CTA of D
+// threads a row is a chain of loads, 41 us for 32 rows of 256 partials; here a thread has eight loads, all in flight.
+// Valid in the threads of warp 0 (lane = column).
+constexpr int MERGE_WARPS = 32;
+constexpr int MERGE_MANY = 16;     // fewer partials: less than one for every second warp, and prefills have many rows of 2-8
+constexpr int MERGE_LSE = 1024;    // weights kept in shared memory
+__device__ __forceinline__ void merge_parts_wide(const float* o_col, long long o_ps, const float* lp, long long l_ps,
+                                                 int nparts, float& o, float& lse) {
+  __shared__ float weight[MERGE_LSE], red_o[MERGE_WARPS][33], red_w[MERGE_WARPS], red_m[MERGE_WARPS];
+  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  float mx = -INFINITY;
+  for (int s = threadIdx.x; s < nparts; s += 32 * MERGE_WARPS) {
+    const float v = lp[s * l_ps];
+    if (s < MERGE_LSE) weight[s] = v;
+    mx = fmaxf(mx, v);
+  }
+#pragma unroll
+  for (int i = 16; i > 0; i >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, i));
+  if (lane == 0) red_m[w] = mx;
+  __syncthreads();
+  mx = red_m[lane];
+#pragma unroll
+  for (int i = 16; i > 0; i >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, i));
+  float wsum = 0.f;
+  o = 0.f;
+  if (mx != -INFINITY) {
+#pragma unroll 8
+    for (int s = w; s < nparts; s += MERGE_WARPS) {
+      const float v = o_col[s * o_ps + lane];
+      const float e = __expf((s < MERGE_LSE ? weight[s] : lp[s * l_ps]) - mx);
+      wsum += e;
+      o += e * v;
+    }
+  }
+  red_o[w][lane] = o;
+  if (lane == 0) red_w[w] = wsum;
+  __syncthreads();
+  if (w == 0) {
+    o = wsum = 0.f;
+#pragma unroll
+    for (int i = 0; i < MERGE_WARPS; ++i) {
+      o += red_o[i][lane];
+      wsum += red_w[i];
+    }
+    if (mx != -INFINITY) o /= wsum;
+    lse = mx == -INFINITY ? -INFINITY : mx + __logf(wsum);
+  }
+}
+
+// One CTA per row = (b, h, i), D threads; WIDE: one per row and 32 columns.
+template <bool WIDE>
+__global__ void __launch_bounds__(WIDE ? 32 * MERGE_WARPS : 128) decode_merge_kernel(const MergeParams p) {
+  const int row = blockIdx.x, d = WIDE ? blockIdx.y * 32 + threadIdx.x : threadIdx.x;
+  const long long slot = p.step_ptr ? ((*p.step_ptr * p.slot_mul + p.slot_add) & 1) : 0;
+  const float* o_row = p.o_part + slot * p.in_slot_o + static_cast<long long>(row) * p.o_rs;
+  const float* lp = p.lse_part + slot * p.in_slot_l + static_cast<long long>(row) * p.l_rs;
+  float o, lse;
+  if (WIDE) {
+    merge_parts_wide(o_row + blockIdx.y * 32, p.o_ps, lp, p.l_ps, p.nparts, o, lse);
+    if (threadIdx.x >= 32) return;
+  } else {
+    merge_parts(o_row, p.o_ps, lp, p.l_ps, p.nparts, d, o, lse);
+  }
   if (p.inbox_o) {
     for (int r = 0; r < p.n_ranks; ++r) {
       p.inbox_o[r][slot * p.out_slot_o + (static_cast<long long>(row) * p.n_ranks + p.my_rank) * p.D + d] = o;
@@ -591,19 +655,9 @@ __global__ void decode_merge_exchange_kernel(const ExchangeParams e) {
   const uint32_t epoch = *reinterpret_cast<volatile uint32_t*>(e.epoch_ptr) + 1u;
   const long long slot = epoch & 1u;
   // ---- stage 1: this GPU's splits
-  const float* lp = p.lse_part + static_cast<long long>(row) * p.l_rs;
-  float mx = -INFINITY;
-  for (int s = 0; s < p.nparts; ++s) mx = fmaxf(mx, lp[s * p.l_ps]);
-  float wsum = 0.f, o = 0.f;
-  if (mx != -INFINITY) {
-    for (int s = 0; s < p.nparts; ++s) {
-      const float w = __expf(lp[s * p.l_ps] - mx);
-      wsum += w;
-      o += w * p.o_part[static_cast<long long>(row) * p.o_rs + s * p.o_ps + d];
-    }
-    o /= wsum;
-  }
-  const float lse = mx == -INFINITY ? -INFINITY : mx + __logf(wsum);
+  float o, lse;
+  merge_parts(p.o_part + static_cast<long long>(row) * p.o_rs, p.o_ps, p.lse_part + static_cast<long long>(row) * p.l_rs,
+              p.l_ps, p.nparts, d, o, lse);
   const long long slot_o = slot * e.slot_rows * n * p.D, slot_l = slot * e.slot_rows * n;
   for (int r = 0; r < n; ++r) {
     p.inbox_o[r][slot_o + (static_cast<long long>(row) * n + p.my_rank) * p.D + d] = o;
@@ -634,9 +688,9 @@ __global__ void decode_merge_exchange_kernel(const ExchangeParams e) {
   // ---- stage 2: the ranks' partials of this row (written by peers: read past L1)
   const float* il = e.inbox_l_local + slot_l + static_cast<long long>(row) * n;
   const float* io = e.inbox_o_local + slot_o + static_cast<long long>(row) * n * p.D;
-  mx = -INFINITY;
+  float mx = -INFINITY;
   for (int r = 0; r < n; ++r) mx = fmaxf(mx, __ldcg(il + r));
-  wsum = 0.f;
+  float wsum = 0.f;
   o = 0.f;
   if (mx != -INFINITY) {
     for (int r = 0; r < n; ++r) {
@@ -1230,7 +1284,9 @@ extern "C" int ra_decode_merge(const float* o_part, const float* lse_part, long 
   p.step_ptr = step_ptr;
   p.slot_mul = slot_mul; p.slot_add = slot_add;
   p.out_slot_o = out_slot_o; p.out_slot_l = out_slot_l; p.in_slot_o = in_slot_o; p.in_slot_l = in_slot_l;
-  decode_merge_kernel<<<rows, D, 0, static_cast<cudaStream_t>(stream)>>>(p);
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  if (nparts >= MERGE_MANY) decode_merge_kernel<true><<<dim3(rows, D / 32), 32 * MERGE_WARPS, 0, s>>>(p);
+  else decode_merge_kernel<false><<<rows, D, 0, s>>>(p);
   return check_launch("decode_merge_kernel");
 }
 

@@ -345,3 +345,29 @@ def test_streams_sharing_one_cached_context():
     shared._tok_buf.copy_(tok.to(torch.int32))
     eager = shared.decode_step(tok).argmax(dim=-1)
     assert eager.shape == (3,)
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("nparts", [1, 15, 16, 33, 512, 1100])
+def test_merge_of_few_and_many_partials(nparts, D):
+    """Both forms of the merge (from 16 partials on by 32 warps), with empty partials, a row without any and strided
+    inputs. Tolerance: fp32 weights by exp of a difference below 40, 4e-6 relative, times sums of up to 1100 terms."""
+    from ringattention_b200.ops import decode as Dk
+
+    torch.manual_seed(nparts)
+    B, H, QL = 2, 3, 2
+    rows = B * H * QL
+    o = torch.randn(rows, nparts, D, device="cuda")
+    lse = torch.randn(nparts, rows, device="cuda").t() * 5
+    if nparts > 1:
+        lse[:, nparts // 2] = -float("inf")
+    lse[3] = -float("inf")
+    out = torch.empty(B, QL, H, D, device="cuda")
+    lse_out = torch.empty(rows, device="cuda")
+    Dk.merge_partials(o, lse, H, QL, out=out, lse_out=lse_out)
+    w = torch.softmax(lse.double(), 1).nan_to_num(0.0)
+    want = (w[:, :, None] * o.double()).sum(1).view(B, H, QL, D).permute(0, 2, 1, 3)
+    want_l = torch.logsumexp(lse.double(), 1).view(B, H, QL).permute(0, 2, 1).reshape(-1)
+    assert (out.double() - want).abs().max() < 2e-5
+    fin = torch.isfinite(want_l)
+    assert torch.equal(torch.isfinite(lse_out), fin) and (lse_out.double() - want_l)[fin].abs().max() < 1e-5
