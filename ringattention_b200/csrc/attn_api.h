@@ -30,7 +30,7 @@ struct RaAttnBwdArgs {
 extern "C" int ra_attn_bwd(const RaAttnBwdArgs* a);
 extern "C" int ra_attn_bwd_prep(const void* o, long long o_sb, long long o_ss, long long o_sh,
                                 const void* d_o, long long do_sb, long long do_ss, long long do_sh,
-                                const float* lse, float* lse2, float* delta, int B, int H, int Sq,
+                                const float* lse, float* lse2, float* delta, float* dq_acc, int B, int H, int Sq,
                                 int Sq_pad, int D, void* stream);
 extern "C" int ra_cast_f32_bf16(const float* src, void* dst, long long rows, int d, long long src_ld,
                                 long long dst_ld, void* stream);

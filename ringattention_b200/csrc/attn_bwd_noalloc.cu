@@ -87,17 +87,10 @@ extern "C" int ra_attn_bwd_noalloc(const void* q, const void* k, const void* v, 
   float* dq_acc = scratch;
   float* lse2 = scratch + kNoAllocMaxDqElems;
   float* delta = lse2 + kNoAllocMaxRows;
-  cudaStream_t s = static_cast<cudaStream_t>(stream);
-
-  // The accumulator still holds the previous call's dQ: clear the part this call reduces into.
-  if (cudaMemsetAsync(dq_acc, 0, static_cast<size_t>(dq_elems) * sizeof(float), s) != cudaSuccess) {
-    set_error("ra_attn_bwd_noalloc: cudaMemsetAsync failed");
-    cudaGetLastError();
-    return kHostLaunchFail;
-  }
   const long long ss = static_cast<long long>(H) * D;  // contiguous (B, S, H, D)
   const long long sbq = ss * Sq, sbk = ss * Sk;
-  rc = ra_attn_bwd_prep(out, sbq, ss, D, dout, sbq, ss, D, lse, lse2, delta, B, H, Sq,
+  // (the accumulator still holds the previous call's dQ: this clears the part this call reduces into)
+  rc = ra_attn_bwd_prep(out, sbq, ss, D, dout, sbq, ss, D, lse, lse2, delta, dq_acc, B, H, Sq,
                         static_cast<int>(sq_pad), D, stream);
   if (rc != kHostOk) return rc;
 

@@ -108,8 +108,8 @@ def ring_backward(q, k, v, out, lse, dout, plan: RingPlan, symm_ring=None, dq=No
     """Returns ``(dq, dk, dv)`` bf16. ``dq/dk/dv`` may be given as (strided) destination views."""
     B, Sq, H, D = q.shape
     with phase("attn_bwd_prep"):
-        lse2, delta = flash.flash_bwd_prep(out, dout, lse)
-        dq_acc = torch.zeros(B, Sq, H, D, device=q.device, dtype=torch.float32)
+        dq_acc = torch.empty(B, Sq, H, D, device=q.device, dtype=torch.float32)
+        lse2, delta = flash.flash_bwd_prep(out, dout, lse, dq_acc)
     if dk is None:
         dk = torch.empty_like(k)
     if dv is None:

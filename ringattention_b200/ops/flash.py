@@ -223,19 +223,21 @@ DKV_STORE_FP32 = 1
 DKV_REDUCE_FP32 = 2
 
 
-def flash_bwd_prep(out, dout, lse):
+def flash_bwd_prep(out, dout, lse, dq_acc=None):
     """``delta = rowsum(dO*O)`` and ``lse*log2(e)`` in ``(B, H, Sq_pad)`` fp32 buffers (padded to a
-    multiple of 128 queries; padding and fully masked rows get ``+inf`` / 0)."""
+    multiple of 128 queries; padding and fully masked rows get ``+inf`` / 0). ``dq_acc`` (fp32, contiguous, ``out``'s
+    shape), when given, is zeroed in the same launch."""
     _check_bshd(out, "out"); _check_bshd(dout, "dout")
     B, Sq, H, D = out.shape
     sq_pad = (Sq + 127) // 128 * 128
     lse2 = torch.empty(B, H, sq_pad, device=out.device, dtype=torch.float32)
     delta = torch.empty(B, H, sq_pad, device=out.device, dtype=torch.float32)
     assert lse.dtype == torch.float32 and lse.is_contiguous() and lse.shape == (B, H, Sq)
+    assert dq_acc is None or (dq_acc.dtype == torch.float32 and dq_acc.is_contiguous() and dq_acc.shape == out.shape)
     _lib.call("ra_attn_bwd_prep", c_vp(out.data_ptr()), c_ll(out.stride(0)), c_ll(out.stride(1)),
               c_ll(out.stride(2)), c_vp(dout.data_ptr()), c_ll(dout.stride(0)), c_ll(dout.stride(1)),
               c_ll(dout.stride(2)), c_vp(lse.data_ptr()), c_vp(lse2.data_ptr()),
-              c_vp(delta.data_ptr()), B, H, Sq, sq_pad, D, _lib.stream_ptr())
+              c_vp(delta.data_ptr()), c_vp(_ptr(dq_acc)), B, H, Sq, sq_pad, D, _lib.stream_ptr())
     return lse2, delta
 
 

@@ -102,8 +102,8 @@ class RingInferenceAttention(torch.autograd.Function):
         B, ql, H, D = q.shape
         if dout.stride(3) != 1 or any(s % 8 for s in dout.stride()[:3]):
             dout = dout.contiguous()
-        lse2, delta = flash.flash_bwd_prep(out, dout, lse)
-        dq_acc = torch.zeros(B, ql, H, D, device=q.device, dtype=torch.float32)
+        dq_acc = torch.empty(B, ql, H, D, device=q.device, dtype=torch.float32)
+        lse2, delta = flash.flash_bwd_prep(out, dout, lse, dq_acc)
         dk, dv = torch.empty_like(k), torch.empty_like(v)
         flash.flash_bwd(q, k, v, dout, lse2, delta, ctx.ms, dq_acc, dk, dv, flash.DKV_STORE_BF16)
         if ctx.axis.size > 1:

@@ -117,3 +117,25 @@ def test_full_bias_is_served_by_the_torch_path():
     bias = torch.randn(1, 1, 64, 64, device="cuda")
     out = rab.ringattention(q, k, v, bias, None, None, None, True, dict(query_chunk_size=32, key_chunk_size=32))
     assert out.shape == q.shape and out.dtype == v.dtype
+
+
+@pytest.mark.parametrize("B,S,H,D", [(1, 1, 1, 64), (2, 130, 2, 128), (1, 257, 3, 64), (2, 128, 7, 128), (1, 1000, 9, 128), (1, 129, 16, 64)])
+@pytest.mark.parametrize("strided", [False, True])
+def test_backward_preparation(B, S, H, D, strided):
+    """delta, the scaled log-sum-exp and the zeroed accumulator at head counts around the eight of a CTA, at lengths around
+    a padded tile, and on views into a wider buffer. Tolerance: an fp32 sum of D products, 1e-6 of their magnitudes."""
+    from ringattention_b200.ops import flash
+
+    torch.manual_seed(S)
+    wide = torch.randn(2, B, S, H, 3, D, device="cuda").bfloat16()
+    out, dout = (w[:, :, :, 1] if strided else w[:, :, :, 1].contiguous() for w in wide)
+    lse = torch.randn(B, H, S, device="cuda")
+    lse[:, :, S // 2] = -float("inf")
+    acc = torch.full((B * S * H * D + 64,), 7.0, device="cuda")
+    lse2, delta = flash.flash_bwd_prep(out, dout, lse, acc[:-64].view(B, S, H, D))
+    terms = (out.double() * dout.double()).permute(0, 2, 1, 3)
+    assert ((delta[:, :, :S].double() - terms.sum(-1)).abs() <= 1e-6 * terms.abs().sum(-1) + 1e-12).all()
+    assert (delta[:, :, S:] == 0).all() and (lse2[:, :, S:] == -float("inf")).all()
+    want = torch.where(torch.isinf(lse), lse, -lse * 1.4426950408889634)
+    assert torch.allclose(lse2[:, :, :S], want, rtol=1e-6, atol=0)
+    assert (acc[:-64] == 0).all() and (acc[-64:] == 7).all()
