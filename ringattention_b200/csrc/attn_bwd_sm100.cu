@@ -38,6 +38,7 @@ static_assert(128 * BWD_REGS_PRODUCER + 256 * BWD_REGS_SOFTMAX + 128 * BWD_REGS_
 
 struct BwdParams {
   int B, H;
+  TileOrder order;  // of the 128-row kv tiles
   MaskParams mask;
   float scale;       // 1/sqrt(D)
   float scale_log2;  // log2(e)/sqrt(D)
@@ -157,11 +158,10 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constant
   const WaitCtx wc{abort_flag, p.status};
   const MaskParams& mk = p.mask;
 
-  const int nkt = (mk.Sk + 127) / 128;
   const int nqt = (mk.Sq + 127) / 128;
   const int idx = static_cast<int>(blockIdx.x) - p.copy_ctas;
-  const int bh = idx / nkt;
-  const int jt = idx - bh * nkt;  // kv tile; low tiles see the most queries under a causal mask
+  int bh, jt;
+  p.order(idx, jt, bh);  // kv tile; low tiles see the most queries under a causal mask
   const int h = bh % p.H;
   const int b = bh / p.H;
   const int k0 = jt * 128;
@@ -788,6 +788,9 @@ extern "C" int ra_attn_bwd(const RaAttnBwdArgs* a) {
   p.status = a->status;
   p.trace = a->trace;
   const int nkt = (a->Sk + 127) / 128;
+  // a head's Q, dO and the fp32 dQ that is reduced into in L2: 8 bytes an element
+  p.order = TileOrder{nkt, a->B * a->H,
+                      a->causal_block_size ? heads_together(nkt, a->B * a->H, 8ll * a->Sq * a->D, sm_count()) : 1};
   const long long grid = static_cast<long long>(nkt) * a->H * a->B + p.copy_ctas;
   cudaStream_t s = static_cast<cudaStream_t>(a->stream);
   if (a->D == 128) {

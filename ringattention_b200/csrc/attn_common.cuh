@@ -140,6 +140,34 @@ __device__ __forceinline__ unsigned int dropout_hash(unsigned int seed_lo, unsig
   return x;
 }
 
+// Order of the CTAs of a launch. A (batch, head) has n tiles of work; under a causal rule they differ in length and the grid's
+// last wave is as long as the longest tile that starts in it. So `group` heads are walked together, the longest tiles of
+// all of them first: unit idx -> tile rank (0 = longest) and (batch, head).
+struct TileOrder {
+  int n, bh, group;
+  __device__ __forceinline__ void operator()(int idx, int& rank, int& bh_idx) const {
+    const int per_group = n * group;
+    const int g = idx / per_group, r = idx - g * per_group;
+    const int in_group = min(group, bh - g * group);
+    rank = r / in_group;
+    bh_idx = g * group + (r - rank * in_group);
+  }
+};
+
+// How many heads walk together: enough that a group's total work keeps every SM busy for as long as its longest tile takes
+// (tile lengths 1 .. n: n (n + 1) / 2 units a head against n on each of `sms`), so that the tail of the launch is the
+// shortest tiles, but no more than what fits in about half of the L2, because the tiles of a head share its operands there.
+// Heads one after the other (group 1) left the last heads' longest tiles to the end: B1 S4096 H32 D128 forward 249 us where
+// the work is 125 us at the rate of long sequences.
+inline int heads_together(int n, int bh, long long head_bytes, int sms) {
+  long long g = (2ll * sms + n) / (n + 1);
+  const long long fit = (64ll << 20) / (head_bytes > 0 ? head_bytes : 1), roomy = (24ll << 20) / (head_bytes > 0 ? head_bytes : 1);
+  if (g < roomy) g = roomy;
+  if (g > fit) g = fit;
+  if (g > bh) g = bh;
+  return g < 1 ? 1 : static_cast<int>(g);
+}
+
 constexpr float kLog2e = 1.4426950408889634f;
 constexpr float kLn2 = 0.6931471805599453f;
 

@@ -32,6 +32,7 @@ static_assert(128 * FWD_REGS_PRODUCER + 256 * FWD_REGS_SOFTMAX <= FWD_THREADS * 
 
 struct FwdParams {
   int B, H;
+  TileOrder order;  // of the 256-row query pairs
   MaskParams mask;
   float scale_log2;  // log2(e) / sqrt(D)
   void* out;
@@ -141,12 +142,10 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constant
   const WaitCtx wc{abort_flag, p.status};
   const MaskParams& mk = p.mask;
 
-  // block -> (q pair, head, batch); heavy (late) q tiles first inside a head, heads outermost so
-  // that concurrently running CTAs share one head's K/V in L2.
-  const int n_qpairs = (mk.Sq + 255) / 256;
-  const int idx = static_cast<int>(blockIdx.x) - p.copy_ctas;
-  const int bh = idx / n_qpairs;
-  const int qp = n_qpairs - 1 - (idx - bh * n_qpairs);
+  // block -> (q pair, head, batch): heavy (late) q tiles first, a few heads at a time
+  int bh, qp;
+  p.order(static_cast<int>(blockIdx.x) - p.copy_ctas, qp, bh);
+  qp = p.order.n - 1 - qp;
   const int h = bh % p.H;
   const int b = bh / p.H;
   const int h_kv = EXT && p.kv_share > 1 ? h / p.kv_share : h;
@@ -735,7 +734,10 @@ extern "C" int ra_attn_fwd(const RaAttnFwdArgs* a) {
   p.gate = nullptr;
   p.gate_ld = 0;
   p.window = p.kv_share = p.k_row0 = p.k_rows = 0;
-  const long long grid = static_cast<long long>((a->Sq + 255) / 256) * a->H * a->B + p.copy_ctas;
+  const int n_qp = (a->Sq + 255) / 256;
+  p.order = TileOrder{n_qp, a->B * a->H,
+                      a->causal_block_size ? heads_together(n_qp, a->B * a->H, 4ll * a->Sk * a->D, sm_count()) : 1};
+  const long long grid = static_cast<long long>(n_qp) * a->H * a->B + p.copy_ctas;
   cudaStream_t s = static_cast<cudaStream_t>(a->stream);
   return a->D == 128 ? launch_fwd<2, 0, 128>(tq, tk, tv, tq, tk, p, grid, s)
                      : launch_fwd<1, 0, 64>(tq, tk, tv, tq, tk, p, grid, s);
@@ -798,7 +800,9 @@ extern "C" int ra_attn_two_part(const RaAttnTwoPartArgs* a) {
   p.sink = a->sink;
   p.gate = static_cast<const __nv_bfloat16*>(a->gate);
   p.gate_ld = a->gate_ld;
-  const long long grid = static_cast<long long>((a->Sq + 255) / 256) * a->H * a->B;
+  const int n_qp = (a->Sq + 255) / 256;
+  p.order = TileOrder{n_qp, a->B * a->H, 1};
+  const long long grid = static_cast<long long>(n_qp) * a->H * a->B;
   cudaStream_t s = static_cast<cudaStream_t>(a->stream);
   if (a->d1 > 64)
     return a->dv > 64 ? launch_fwd<2, 1, 128>(tq, tk, tv, tq2, tk2, p, grid, s)
@@ -868,7 +872,9 @@ extern "C" int ra_attn_window(const RaAttnWindowArgs* a) {
   p.kv_share = a->H / a->G;
   p.k_row0 = static_cast<int>(base % a->k_rows);
   p.k_rows = a->k_rows;
-  const long long grid = static_cast<long long>((a->Sq + 255) / 256) * a->H * a->B;
+  const int n_qp = (a->Sq + 255) / 256;
+  p.order = TileOrder{n_qp, a->B * a->H, 1};
+  const long long grid = static_cast<long long>(n_qp) * a->H * a->B;
   cudaStream_t s = static_cast<cudaStream_t>(a->stream);
   if (a->dk > 64)
     return a->dv > 64 ? launch_fwd<2, 0, 128, true>(tq, tk, tv, tq, tk, p, grid, s)
