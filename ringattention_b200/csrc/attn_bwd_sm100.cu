@@ -197,12 +197,20 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constant
   // which q tiles this kv tile is seen by
   uint32_t* sVis = reinterpret_cast<uint32_t*>(smem + SM::VIS_OFF);
   const bool use_vis = nqt <= 32 * VIS_WORDS;
+  // a tile of keys whose bias is -inf throughout (padding) is seen by no query
+  bool dead = false;
+  if (mk.bias) {
+    const int kj = k0 + static_cast<int>(threadIdx.x);
+    const float* bias = mk.bias + b * mk.bias_stride_b + h * mk.bias_stride_h;
+    dead = __syncthreads_and(threadIdx.x >= 128 || kj >= mk.Sk || bias[kj] * kLog2e == -INFINITY) != 0;
+  }
   if (use_vis)
     fill_visibility(sVis, nqt, static_cast<int>(threadIdx.x), BWD_THREADS,
-                    [&](int i) { return tile_visible(mk, b, i * 128, k0); });
+                    [&](int i) { return !dead && tile_visible(mk, b, i * 128, k0); });
   // next q tile at or after i that sees this kv tile, or nqt; every role walks the same mask
   auto next_vis = [&](int i) -> int {
     if (use_vis) return vis_next(sVis, i, nqt);
+    if (dead) return nqt;
     for (; i < nqt; ++i)
       if (tile_visible(mk, b, i * 128, k0)) break;
     return i;
@@ -364,6 +372,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constant
     const int swz = row & 7;
     const uint64_t scale2 = f2_pack(p.scale_log2, p.scale_log2);
     const uint64_t bias2 = f2_pack(my_bias2, my_bias2);
+    const bool biased = __any_sync(0xffffffffu, my_bias2 != 0.f);  // no row of this warp has one: nothing to add
 
     int it = 0;
     bool alive = true;
@@ -371,8 +380,8 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constant
       const int qi0 = i * 128;
       const int st = it & 1;
       const uint32_t par = it & 1;
-      const bool plain = tile_plain(mk, b, qi0, k0);
-      if (mk.seg_q) {
+      const int kind = tile_mask(mk, b, qi0, k0);
+      if (kind & kMaskSeg) {
         if (sm_tid < 128)
           sSegQ[st * 128 + sm_tid] =
               (qi0 + sm_tid) < mk.Sq ? mk.seg_q[static_cast<long long>(b) * mk.Sq + qi0 + sm_tid] : -2;
@@ -387,9 +396,10 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constant
       tc_fence_after();
       trace_event(p.trace, tr && sm_tid == 0, 1, it, 0);
 
-      // masked iff column (q index) c < lo: causal rule transposed; everything if the row is padding
+      // causal rule transposed: column (q index) c is hidden iff c < lo; all of them if the row is padding
+      const bool special = kind != 0 || biased;
       int lo = 0;
-      if (!plain) {
+      if (kind & kMaskEdge) {
         if (!row_valid) {
           lo = 128;
         } else if (mk.cbs) {
@@ -413,39 +423,37 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constant
           x[2 * g] = f2_fma(f2_pack_u(s[4 * g], s[4 * g + 1]), scale2, f2_pack(n.x, n.y));
           x[2 * g + 1] = f2_fma(f2_pack_u(s[4 * g + 2], s[4 * g + 3]), scale2, f2_pack(n.z, n.w));
         }
-        if (!plain) {
-          // keepw bit e: column (q index) base+e survives the causal rule, padding and dropout; the hash is a
-          // small rolled loop that only runs when dropout is on
+        if (special) {
+          // keepw bit e: column base + e survives. Gathered before the element loop, as in the forward, and the loop only
+          // runs for words with a hole; the dropout hash is a small rolled loop that only runs when dropout is on.
           const int base = half * 64 + c * 32;
           const int n = lo - base;
           uint32_t keepw = n <= 0 ? 0xffffffffu : (n >= 32 ? 0u : ~((1u << n) - 1u));
-          if (mk.keep && RA_IN_BOUNDS((qi0 + base) >> 5, 1, mk.keep_sr, kTagAttnMaskBits))
-            keepw &= mk.keep[b * mk.keep_sb + h * mk.keep_sh + static_cast<long long>(row_valid ? kj : mk.Sk - 1) * mk.keep_sr +
-                             ((qi0 + base) >> 5)];
-          if (mk.drop_threshold) {
-            uint32_t drop = 0;
+          if (kind & kMaskBits) {
+            if (mk.keep && RA_IN_BOUNDS((qi0 + base) >> 5, 1, mk.keep_sr, kTagAttnMaskBits))
+              keepw &= mk.keep[b * mk.keep_sb + h * mk.keep_sh + static_cast<long long>(row_valid ? kj : mk.Sk - 1) * mk.keep_sr +
+                               ((qi0 + base) >> 5)];
+            if (mk.drop_threshold) {
+              uint32_t drop = 0;
 #pragma unroll 1
-            for (int e = 0; e < 32; ++e)
-              drop |= static_cast<uint32_t>(dropout_hash(mk.seed_lo, mk.seed_hi, bh_u, qpos0 + base + e,
-                                                         static_cast<unsigned int>(kpos)) < mk.drop_threshold)
-                      << e;
-            keepw &= ~drop;
+              for (int e = 0; e < 32; ++e)
+                drop |= static_cast<uint32_t>(dropout_hash(mk.seed_lo, mk.seed_hi, bh_u, qpos0 + base + e,
+                                                           static_cast<unsigned int>(kpos)) < mk.drop_threshold)
+                        << e;
+              keepw &= ~drop;
+            }
           }
-          const bool has_seg = mk.seg_q != nullptr;
-          const int4* seg4 = reinterpret_cast<const int4*>(sSegQ + st * 128 + base);
+          if (kind & kMaskSeg) keep_segment<1>(&keepw, sSegQ + st * 128 + base, my_seg, lane);
+          if (biased) {
 #pragma unroll
-          for (int g = 0; g < 8; ++g) {
-            const int4 sg = has_seg ? seg4[g] : make_int4(my_seg, my_seg, my_seg, my_seg);
-            const int se[4] = {sg.x, sg.y, sg.z, sg.w};
+            for (int e = 0; e < 16; ++e) x[e] = f2_add(x[e], bias2);
+          }
+          if (!__all_sync(0xffffffffu, keepw == 0xffffffffu)) {
 #pragma unroll
-            for (int h2 = 0; h2 < 2; ++h2) {
-              const int e = 2 * g + h2;
-              x[e] = f2_add(x[e], bias2);
+            for (int e = 0; e < 16; ++e) {
               float x0, x1;
               f2_unpack(x[e], x0, x1);
-              const bool m0 = (((keepw >> (2 * e)) & 1u) == 0u) || (se[2 * h2] != my_seg);
-              const bool m1 = (((keepw >> (2 * e + 1)) & 1u) == 0u) || (se[2 * h2 + 1] != my_seg);
-              x[e] = f2_pack(m0 ? -INFINITY : x0, m1 ? -INFINITY : x1);
+              x[e] = f2_pack((keepw >> (2 * e)) & 1u ? x0 : -INFINITY, (keepw >> (2 * e + 1)) & 1u ? x1 : -INFINITY);
             }
           }
         }
@@ -645,7 +653,7 @@ __device__ __forceinline__ void load8(const __nv_bfloat16* src, float* f) {
 // A CTA takes 64 (q, h) rows, up to eight heads of consecutive queries, so that its reads of o and d_o and its zeros
 // are contiguous in a (B, S, H, D) tensor; D/8 lanes a row, all of a thread's loads issued before the first is used; the
 // results turn in shared memory so that they leave as runs along q. It is bound by memory: one warp a row, rows a whole
-// (H, D) line apart and 8 bytes a lane moved 2 TB/s (33 us at B1 S4096 H32 D128, beside 10 us for a fill kernel).
+// (H, D) line apart and 8 bytes a lane moved 2 TB/s (33 us at B1 S4096 H32 D128, beside 10 us for a fill kernel); this takes 29 us for both.
 constexpr int PREP_ROWS = 64;
 template <int D, bool ALIGNED>
 __global__ void __launch_bounds__(256) attn_bwd_prep_kernel(const __nv_bfloat16* __restrict__ o, long long o_sb, long long o_ss,

@@ -85,28 +85,51 @@ __device__ __forceinline__ int vis_next(const uint32_t* words, int t, int n) {
   return n;
 }
 
-// True when no entry of the tile needs element-wise masking or bias. With segment ids that is the case
-// when both tiles lie inside one and the same segment (per-tile min == max, equal on both sides), which
-// holds for most tiles of packed documents much longer than a tile.
-__device__ __forceinline__ bool tile_plain(const MaskParams& m, int b, int qi0, int k0) {
-  if (m.bias || m.drop_threshold || m.keep) return false;
-  if (k0 + 128 > m.Sk || qi0 + 128 > m.Sq) return false;
+// What may hide single entries of a visible tile; 0: nothing does. With segment ids the common case inside packed documents
+// much longer than a tile is that both tiles lie in one and the same segment (per-tile min == max, equal on both sides).
+enum TileMask : int { kMaskEdge = 1 /* causal rule or end of the keys */, kMaskSeg = 2, kMaskBits = 4 /* bitmap, dropout */ };
+__device__ __forceinline__ int tile_mask(const MaskParams& m, int b, int qi0, int k0) {
+  int kind = (m.drop_threshold || m.keep) ? kMaskBits : 0;
+  if (k0 + 128 > m.Sk) kind |= kMaskEdge;
   if (m.seg_q) {
-    if (!m.seg_q_mm) return false;
-    const int nqt = (m.Sq + 127) >> 7, nkt = (m.Sk + 127) >> 7;
-    const int* qm = m.seg_q_mm + (static_cast<long long>(b) * nqt + (qi0 >> 7)) * 2;
-    const int* km = m.seg_k_mm + (static_cast<long long>(b) * nkt + (k0 >> 7)) * 2;
-    const int q_lo = qm[0], k_lo = km[0];
-    if (q_lo != qm[1] || k_lo != km[1] || q_lo != k_lo) return false;
+    bool one = false;
+    if (m.seg_q_mm) {
+      const int nqt = (m.Sq + 127) >> 7, nkt = (m.Sk + 127) >> 7;
+      const int* qm = m.seg_q_mm + (static_cast<long long>(b) * nqt + (qi0 >> 7)) * 2;
+      const int* km = m.seg_k_mm + (static_cast<long long>(b) * nkt + (k0 >> 7)) * 2;
+      const int q_lo = qm[0], k_lo = km[0];
+      one = q_lo == qm[1] && k_lo == km[1] && q_lo == k_lo;
+    }
+    if (!one) kind |= kMaskSeg;
   }
   if (m.cbs == 1) {
-    if (m.qmap(qi0) < m.kmap(min(k0 + 127, m.Sk - 1))) return false;
+    if (m.qmap(qi0) < m.kmap(min(k0 + 127, m.Sk - 1))) kind |= kMaskEdge;
   } else if (m.cbs) {
     const int q_lo = m.qmap(qi0);
     const int k_hi = m.kmap(min(k0 + 127, m.Sk - 1));
-    if (q_lo / m.cbs < k_hi / m.cbs) return false;
+    if (q_lo / m.cbs < k_hi / m.cbs) kind |= kMaskEdge;
   }
-  return true;
+  return kind;
+}
+
+// keep[c] bit i &= (seg[32 c + i] == my_seg) for N words, by warp votes: the lanes of a warp have few different ids (rows of a
+// tile are neighbours in the sequence), and one vote per word answers for all lanes with the same one. Converged warps.
+template <int N>
+__device__ __forceinline__ void keep_segment(uint32_t* keep, const int* seg, int my_seg, int lane) {
+  int col[N];
+#pragma unroll
+  for (int c = 0; c < N; ++c) col[c] = seg[32 * c + lane];
+  uint32_t todo = 0xffffffffu;
+  while (todo) {
+    const int id = __shfl_sync(0xffffffffu, my_seg, __ffs(static_cast<int>(todo)) - 1);
+    const bool mine = id == my_seg;
+#pragma unroll
+    for (int c = 0; c < N; ++c) {
+      const uint32_t same = __ballot_sync(0xffffffffu, col[c] == id);
+      if (mine) keep[c] &= same;
+    }
+    todo &= ~__ballot_sync(0xffffffffu, mine);
+  }
 }
 
 // Number of leading columns of the k tile that the causal rule and the sequence end leave

@@ -81,7 +81,8 @@ struct FwdSmem {
   static constexpr int AUX_BYTES = 2 /*wg*/ * 2 /*buf*/ * 128 * 4 * 2 /*seg+bias*/;
   static constexpr int BAR_OFF = AUX_OFF + AUX_BYTES;
   static constexpr int VIS_OFF = BAR_OFF + 256;  // [2 q tiles][VIS_WORDS] visibility of the kv tiles
-  static constexpr int TOTAL = VIS_OFF + 2 * VIS_WORDS * 4 + 1024;
+  static constexpr int BIAS_OFF = VIS_OFF + 2 * VIS_WORDS * 4;  // [2][VIS_WORDS] kv tiles whose bias is not all 0, not all -inf
+  static constexpr int TOTAL = BIAS_OFF + 2 * VIS_WORDS * 4 + 1024;
 };
 
 // NQ: slabs of the query/key part that every head has of its own; NR: slabs of a second part (maps tma_q2, tma_k2) whose
@@ -191,11 +192,37 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constant
   // which kv tiles each of the two q tiles sees
   uint32_t* sVis = reinterpret_cast<uint32_t*>(smem + SM::VIS_OFF);
   const bool use_vis = nk <= 32 * VIS_WORDS;
+  // A key bias is mostly a padding mask: tiles whose bias is 0 throughout need no addition, tiles where it is -inf throughout
+  // (in the log2 domain, so the type's lowest value too) are not visited. One warp looks at a tile.
+  uint32_t* sAdd = reinterpret_cast<uint32_t*>(smem + SM::BIAS_OFF);
+  uint32_t* sLive = sAdd + VIS_WORDS;
+  if (use_vis && mk.bias) {
+    for (int t = threadIdx.x; t < VIS_WORDS; t += FWD_THREADS) sAdd[t] = sLive[t] = 0u;
+    __syncthreads();
+    const float* bias = mk.bias + b * mk.bias_stride_b + h * mk.bias_stride_h;
+    for (int j = warp; j < nk; j += FWD_THREADS / 32) {
+      bool add = false, live = false;
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+        const int kc = j * 128 + c * 32 + lane;
+        const float v = kc < mk.Sk ? bias[kc] * kLog2e : -INFINITY;
+        live |= v != -INFINITY;
+        add |= kc < mk.Sk && v != 0.f;
+      }
+      add = __any_sync(0xffffffffu, add);
+      live = __any_sync(0xffffffffu, live);
+      if (lane == 0) {
+        if (add) atomicOr(&sAdd[j >> 5], 1u << (j & 31));
+        if (live) atomicOr(&sLive[j >> 5], 1u << (j & 31));
+      }
+    }
+    __syncthreads();
+  }
   if (use_vis) {
 #pragma unroll
     for (int w = 0; w < 2; ++w)
       fill_visibility(sVis + w * VIS_WORDS, nk, static_cast<int>(threadIdx.x), FWD_THREADS,
-                      [&](int j) { return visible(w, j); });
+                      [&](int j) { return visible(w, j) && (!mk.bias || ((sLive[j >> 5] >> (j & 31)) & 1u)); });
   }
   // next kv tile at or after j that q tile w sees, or nk
   auto next_vis = [&](int w, int j) -> int {
@@ -365,14 +392,15 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constant
     // every role walks the same visibility mask, so skips stay consistent
     for (int j = next_vis(w, 0); j < nk && alive; j = next_vis(w, j + 1)) {
       const int k0 = j * 128;
-      const bool plain = tile_plain(mk, b, qi0, k0) && (!EXT || tile_window_plain(mk, p.window, qi0, k0));
-      if (!plain && (mk.seg_k || mk.bias)) {
-        const int buf = cnt & 1;
+      const int kind = tile_mask(mk, b, qi0, k0) | (EXT && !tile_window_plain(mk, p.window, qi0, k0) ? kMaskEdge : 0);
+      const bool biased = mk.bias && (!use_vis || ((sAdd[j >> 5] >> (j & 31)) & 1u));
+      const int buf = cnt & 1;
+      if ((kind & kMaskSeg) || biased) {
         const int kc = k0 + wg_tid;
-        if (mk.seg_k)
+        if (kind & kMaskSeg)
           sSeg[(w * 2 + buf) * 128 + wg_tid] =
               kc < mk.Sk ? mk.seg_k[static_cast<long long>(b) * mk.Sk + kc] : -1;
-        if (mk.bias)
+        if (biased)
           sBias[(w * 2 + buf) * 128 + wg_tid] =
               kc < mk.Sk ? mk.bias[b * mk.bias_stride_b + h * mk.bias_stride_h + kc] * kLog2e : 0.f;
         named_bar_sync(1 + w, 128);
@@ -388,8 +416,77 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constant
       tmem_ld_wait();
 
       float sc = p.scale_log2;  // multiplier still to be applied to sr[] inside the exp
-      float mx = -INFINITY;
-      if (plain) {
+      // Masked tiles differ from plain ones only in this block: what hides an entry is gathered into four words of bits per
+      // row first (segment ids by warp votes), a bias is added by a loop of its own, and only words with a hole are walked
+      // column by column. One loop over 128 columns that tested bits, ids and bias for each took 8.9 us a tile (D = 64) where a plain
+      // tile takes 1.2: far more instructions than the caches hold, refetched every time.
+      if (kind != 0 || biased) {
+        uint32_t keep[4] = {0xffffffffu, 0xffffffffu, 0xffffffffu, 0xffffffffu};
+        if (kind & kMaskEdge) {
+          const int limit = causal_col_limit(mk, qpos, k0);
+#pragma unroll
+          for (int c = 0; c < 4; ++c) {
+            const int n = limit - 32 * c;
+            keep[c] = n >= 32 ? 0xffffffffu : (n <= 0 ? 0u : ((1u << n) - 1u));
+          }
+          if (EXT && p.window) {
+            const int first = qpos - p.window + 1 - mk.kmap(k0);  // columns before it are too far away
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+              const int n = first - 32 * c;
+              keep[c] &= n >= 32 ? 0u : (n <= 0 ? 0xffffffffu : ~((1u << n) - 1u));
+            }
+          }
+        }
+        if (kind & kMaskBits) {
+          if (mk.keep) {
+            uint4 kb = make_uint4(0u, 0u, 0u, 0u);
+            if (RA_IN_BOUNDS((k0 >> 5), 4, mk.keep_sr, kTagAttnMaskBits))
+              kb = *reinterpret_cast<const uint4*>(
+                mk.keep + b * mk.keep_sb + h * mk.keep_sh + static_cast<long long>(row_valid ? qi : mk.Sq - 1) * mk.keep_sr +
+                (k0 >> 5));
+            keep[0] &= kb.x;
+            keep[1] &= kb.y;
+            keep[2] &= kb.z;
+            keep[3] &= kb.w;
+          }
+          if (mk.drop_threshold) {
+            const unsigned int kpos0 = static_cast<unsigned int>(mk.kmap(k0));
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+              uint32_t drop = 0;
+#pragma unroll 1
+              for (int i = 0; i < 32; ++i)
+                drop |= static_cast<uint32_t>(dropout_hash(mk.seed_lo, mk.seed_hi, bh_u, static_cast<unsigned int>(qpos),
+                                                           kpos0 + c * 32 + i) < mk.drop_threshold)
+                        << i;
+              keep[c] &= ~drop;
+            }
+          }
+        }
+        if (kind & kMaskSeg) keep_segment<4>(keep, sSeg + (w * 2 + buf) * 128, my_seg, lane);
+        if (biased) {
+          const float4* bias4 = reinterpret_cast<const float4*>(sBias + (w * 2 + buf) * 128);
+#pragma unroll
+          for (int g = 0; g < 32; ++g) {
+            const float4 bs = bias4[g];
+            sr[4 * g] = __float_as_uint(fmaf(__uint_as_float(sr[4 * g]), sc, bs.x));
+            sr[4 * g + 1] = __float_as_uint(fmaf(__uint_as_float(sr[4 * g + 1]), sc, bs.y));
+            sr[4 * g + 2] = __float_as_uint(fmaf(__uint_as_float(sr[4 * g + 2]), sc, bs.z));
+            sr[4 * g + 3] = __float_as_uint(fmaf(__uint_as_float(sr[4 * g + 3]), sc, bs.w));
+          }
+          sc = 1.0f;
+        }
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+          if (__all_sync(0xffffffffu, keep[c] == 0xffffffffu)) continue;
+#pragma unroll
+          for (int i = 0; i < 32; ++i)
+            if (!((keep[c] >> i) & 1u)) sr[32 * c + i] = 0xff800000u;  // -inf
+        }
+      }
+      float mx;
+      {
         float mc[4];
 #pragma unroll
         for (int c = 0; c < 4; ++c) mc[c] = fmaxf(__uint_as_float(sr[32 * c]), __uint_as_float(sr[32 * c + 1]));
@@ -400,71 +497,6 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constant
             mc[c] = max3(mc[c], __uint_as_float(sr[32 * c + i]), __uint_as_float(sr[32 * c + i + 1]));
         }
         mx = fmaxf(fmaxf(mc[0], mc[1]), fmaxf(mc[2], mc[3])) * sc;
-      } else {
-        // keep[c] bit i: column 32c+i survives the causal rule, the sequence end and dropout. Built apart
-        // from the element loop so that the (large) hash code is a small rolled loop that only runs when
-        // dropout is on; the element loop itself stays a handful of instructions per column.
-        const int limit = causal_col_limit(mk, qpos, k0);
-        uint32_t keep[4];
-#pragma unroll
-        for (int c = 0; c < 4; ++c) {
-          const int n = limit - 32 * c;
-          keep[c] = n >= 32 ? 0xffffffffu : (n <= 0 ? 0u : ((1u << n) - 1u));
-        }
-        if (EXT && p.window) {
-          const int first = qpos - p.window + 1 - mk.kmap(k0);  // columns before it are too far away
-#pragma unroll
-          for (int c = 0; c < 4; ++c) {
-            const int n = first - 32 * c;
-            keep[c] &= n >= 32 ? 0u : (n <= 0 ? 0xffffffffu : ~((1u << n) - 1u));
-          }
-        }
-        if (mk.keep) {
-          uint4 kb = make_uint4(0u, 0u, 0u, 0u);
-          if (RA_IN_BOUNDS((k0 >> 5), 4, mk.keep_sr, kTagAttnMaskBits))
-            kb = *reinterpret_cast<const uint4*>(
-              mk.keep + b * mk.keep_sb + h * mk.keep_sh + static_cast<long long>(row_valid ? qi : mk.Sq - 1) * mk.keep_sr +
-              (k0 >> 5));
-          keep[0] &= kb.x;
-          keep[1] &= kb.y;
-          keep[2] &= kb.z;
-          keep[3] &= kb.w;
-        }
-        if (mk.drop_threshold) {
-          const unsigned int kpos0 = static_cast<unsigned int>(mk.kmap(k0));
-#pragma unroll
-          for (int c = 0; c < 4; ++c) {
-            uint32_t drop = 0;
-#pragma unroll 1
-            for (int i = 0; i < 32; ++i)
-              drop |= static_cast<uint32_t>(dropout_hash(mk.seed_lo, mk.seed_hi, bh_u, static_cast<unsigned int>(qpos),
-                                                         kpos0 + c * 32 + i) < mk.drop_threshold)
-                      << i;
-            keep[c] &= ~drop;
-          }
-        }
-        const bool has_seg = mk.seg_k != nullptr, has_bias = mk.bias != nullptr;
-        const int4* seg4 = reinterpret_cast<const int4*>(sSeg + (w * 2 + (cnt & 1)) * 128);
-        const float4* bias4 = reinterpret_cast<const float4*>(sBias + (w * 2 + (cnt & 1)) * 128);
-        float mc[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
-#pragma unroll
-        for (int g = 0; g < 32; ++g) {
-          const int4 sg = has_seg ? seg4[g] : make_int4(my_seg, my_seg, my_seg, my_seg);
-          const float4 bs = has_bias ? bias4[g] : make_float4(0.f, 0.f, 0.f, 0.f);
-          const int se[4] = {sg.x, sg.y, sg.z, sg.w};
-          const float be[4] = {bs.x, bs.y, bs.z, bs.w};
-#pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            const int i = 4 * g + e;
-            float x = fmaf(__uint_as_float(sr[i]), sc, be[e]);
-            const bool masked = (((keep[i >> 5] >> (i & 31)) & 1u) == 0u) || (se[e] != my_seg);
-            x = masked ? -INFINITY : x;
-            sr[i] = __float_as_uint(x);
-            mc[e] = fmaxf(mc[e], x);
-          }
-        }
-        mx = fmaxf(fmaxf(mc[0], mc[1]), fmaxf(mc[2], mc[3]));
-        sc = 1.0f;
       }
 
       // ---- online softmax with lazy rescale of the accumulator

@@ -139,3 +139,77 @@ def test_backward_preparation(B, S, H, D, strided):
     want = torch.where(torch.isinf(lse), lse, -lse * 1.4426950408889634)
     assert torch.allclose(lse2[:, :, :S], want, rtol=1e-6, atol=0)
     assert (acc[:-64] == 0).all() and (acc[-64:] == 7).all()
+
+
+def _oracle(q, k, v, dout, hidden, bias=None):
+    """Dense attention and its gradients in 64 bits; rows without a visible key give zeros."""
+    q, k, v = (t.double().requires_grad_(True) for t in (q, k, v))
+    x = torch.einsum("bqhd,bkhd->bhqk", q, k) / q.shape[-1] ** 0.5
+    if bias is not None:
+        x = x + bias.double()
+    x = x.masked_fill(hidden | (x < -1e30), -float("inf"))
+    m = x.amax(-1, keepdim=True).clamp_min(-1e300)
+    e = torch.exp(x - m)
+    p = e / e.sum(-1, keepdim=True).clamp_min(1e-300)
+    out = torch.einsum("bhqk,bkhd->bqhd", p, v)
+    return (out.detach(), *torch.autograd.grad(out, (q, k, v), dout.double()))
+
+
+def _check_call(B, Sq, Sk, H, D, *, cbs=None, seg=None, bias=None, cache_idx=None, grad=True):
+    """``ringattention`` on one device against the oracle. bf16 keeps 8 bits: outputs within 1e-2 of the largest entry (P and
+    the result are rounded once each, 2^-8 apiece at worst), gradients within 2e-2 (dS is rounded as well)."""
+    import ringattention_b200 as rab
+
+    g = torch.Generator(device="cuda").manual_seed(Sq * 7 + Sk)
+    q, dout = (torch.randn(B, Sq, H, D, device="cuda", generator=g).bfloat16() for _ in range(2))
+    k, v = (torch.randn(B, Sk, H, D, device="cuda", generator=g).bfloat16() for _ in range(2))
+    hidden = torch.zeros(B, 1, Sq, Sk, dtype=torch.bool, device="cuda")
+    if cbs:
+        pos = torch.arange(Sq, device="cuda") + (cache_idx or 0)
+        hidden |= (pos[:, None] // cbs < torch.arange(Sk, device="cuda")[None] // cbs)
+    if seg is not None:
+        hidden |= (seg[:, :, None] != seg[:, None, :])[:, None]
+    want = _oracle(q, k, v, dout, hidden, bias)
+    kw = dict(causal_block_size=cbs, query_chunk_size=Sq, key_chunk_size=Sk)
+    q, k, v = (t.requires_grad_(grad) for t in (q, k, v))
+    out = rab.ringattention(q, k, v, bias, seg, cache_idx, None, True, kw)
+    got = [out.detach()] + (list(torch.autograd.grad(out, (q, k, v), dout)) if grad else [])
+    for i, (a, b) in enumerate(zip(got, want)):
+        assert torch.isfinite(a).all()
+        assert (a.double() - b).abs().max() <= (0.01 if i == 0 else 0.02) * b.abs().max() + 1e-3, i
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("S,pads", [(1371, (700, 1371, 256)), (513, (1, 128, 512)), (384, (129, 255, 383))])
+def test_padding_bias_hides_whole_and_partial_tiles(S, pads, D):
+    """The type's lowest value from a row's length on: tiles that are all padding are not visited, tiles without any are
+    plain, the one between is masked; causal and not."""
+    bias = torch.zeros(len(pads), 1, 1, S, device="cuda")
+    for b, n in enumerate(pads):
+        bias[b, 0, 0, n:] = torch.finfo(torch.float32).min
+    _check_call(len(pads), S, S, 2, D, cbs=1, bias=bias)
+    _check_call(len(pads), S, S, 2, D, bias=bias)
+
+
+@pytest.mark.parametrize("D", [64, 128])
+def test_finite_bias_in_some_tiles_and_per_head(D):
+    """A finite bias in one tile only, padding with -inf elsewhere, a row whose keys are all hidden, a bias per head."""
+    S, H = 640, 3
+    bias = torch.zeros(2, H, 1, S, device="cuda")
+    bias[0, 1, 0, 130:200] = torch.randn(70, device="cuda") * 3
+    bias[0, 2, 0, 256:384] = -float("inf")
+    bias[1, 0] = -float("inf")
+    bias[1, 2, 0, ::2] = -float("inf")
+    _check_call(2, S, S, H, D, bias=bias)
+    _check_call(2, S, S, H, D, cbs=1, bias=bias)
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("ids", ["per token", "runs", "one change", "alternating"])
+def test_segment_ids_of_every_kind(ids, D):
+    """Ids need not be sorted: every token its own, short runs that come back, one border inside a tile, two in turn."""
+    B, S = 2, 700
+    t = torch.arange(S, device="cuda")
+    seg = {"per token": t, "runs": t // 5 % 7, "one change": (t >= 333).int(), "alternating": t % 2}[ids].int()[None].expand(B, S).contiguous()
+    _check_call(B, S, S, 2, D, seg=seg)
+    _check_call(B, S, S, 2, D, cbs=1, seg=seg, bias=torch.randn(B, 1, 1, S, device="cuda"))
