@@ -17,7 +17,7 @@ template <int B_MN>
 int launch_gather(const CUtensorMap& ta, const TmaSet& set, const Params& p, const GatherParams& g,
                   cudaStream_t stream) {
   auto kern = gemm_bf16_kernel<0, B_MN, true>;
-  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES) != cudaSuccess) {
+  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Tile<BN>::SMEM_BYTES) != cudaSuccess) {
     set_error("gemm_gather: cudaFuncSetAttribute(MaxDynamicSharedMemorySize) failed");
     return kHostLaunchFail;
   }
@@ -25,7 +25,7 @@ int launch_gather(const CUtensorMap& ta, const TmaSet& set, const Params& p, con
   int compute = sm_count() - g.copy_ctas;  // every CTA of the grid must be resident at once
   if (compute < 1) compute = 1;
   if (tiles < compute) compute = tiles;
-  kern<<<compute + g.copy_ctas, THREADS, SMEM_BYTES, stream>>>(ta, set, p, g);
+  kern<<<compute + g.copy_ctas, THREADS, Tile<BN>::SMEM_BYTES, stream>>>(ta, set, p, g);
   return check_launch("gemm_bf16_kernel<gather>");
 }
 

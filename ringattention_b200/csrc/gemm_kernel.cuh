@@ -9,16 +9,22 @@ namespace ra {
 namespace gemm {
 
 constexpr int BM = 128;
-constexpr int BN = 256;
+constexpr int BN = 256;  // widest tile, and the only one of the gathering kernel
 constexpr int BK = 64;
-constexpr int STAGES = 4;
 constexpr int NUM_ACC = 2;
-constexpr int A_STAGE_BYTES = BM * BK * 2;  // 16 KiB
-constexpr int B_STAGE_BYTES = BN * BK * 2;  // 32 KiB
-constexpr int STAGE_TX_BYTES = A_STAGE_BYTES + B_STAGE_BYTES;
 constexpr int SLAB_BYTES = 64 * BK * 2;  // one 64-wide MN-major slab: 64 k-rows x 128 B
-constexpr int SMEM_BYTES = STAGES * STAGE_TX_BYTES + 1024 /*align*/ + 256 /*barriers*/;
 constexpr int THREADS = 192;
+
+// A tile of 128 rows and BN columns: the ring fills the same 192 KiB whatever BN is, two accumulators of BN columns.
+template <int BN_>
+struct Tile {
+  static constexpr int STAGES = BN_ == 256 ? 4 : (BN_ == 128 ? 6 : 8);
+  static constexpr int A_STAGE_BYTES = BM * BK * 2;  // 16 KiB
+  static constexpr int B_STAGE_BYTES = BN_ * BK * 2;
+  static constexpr int STAGE_TX_BYTES = A_STAGE_BYTES + B_STAGE_BYTES;
+  static constexpr int SMEM_BYTES = STAGES * STAGE_TX_BYTES + 1024 /*align*/ + 256 /*barriers*/;
+  static constexpr int TMEM_COLS = NUM_ACC * BN_;
+};
 
 struct Params {
   void* C;
@@ -30,8 +36,8 @@ struct Params {
   int group_m;  // m-tiles per rasterisation group (L2 reuse of B across the group)
   int* status;
   // SwiGLU epilogue (forward of a gate/up projection, B = W[2F][K] K-major with rows [gate | up]): every
-  // 256-column tile is made of gate columns [tn*128, tn*128+128) and the matching up columns (two 128-row
-  // TMA loads, tensor map 1), and the epilogue writes silu(gate) * up, F columns of bf16, instead of the
+  // tile of BN columns is made of BN/2 gate columns from tn*BN/2 on and the matching up columns (two
+  // TMA loads of BN/2 rows, tensor map 1), and the epilogue writes silu(gate) * up, F columns of bf16, instead of the
   // 2F pre-activations. gate and up are rounded to bf16 first, so the result equals the two-pass path.
   int swiglu_F;  // 0 = off
   // Plain K-major products only: squared-relu activation, and a tail of columns [n_split, N) (n_split a multiple of
@@ -99,10 +105,13 @@ __device__ __forceinline__ void tile_coords(int tile, int tiles_m, int tiles_n, 
   tn = r / gm;
 }
 
-template <int A_MN, int B_MN, bool GATHER>
+template <int A_MN, int B_MN, bool GATHER, int BN = gemm::BN>
 __global__ void __launch_bounds__(THREADS, 1)
 gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ TmaSet tma_bs,
                  const Params p, const GatherParams g) {
+  using T = Tile<BN>;
+  constexpr int STAGES = T::STAGES, A_STAGE_BYTES = T::A_STAGE_BYTES, B_STAGE_BYTES = T::B_STAGE_BYTES,
+                STAGE_TX_BYTES = T::STAGE_TX_BYTES;
   const int n_copy = GATHER ? g.copy_ctas : 0;
   if (GATHER && static_cast<int>(blockIdx.x) < n_copy) {
     // ---------------------------------------------------------------- gather CTAs
@@ -161,7 +170,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
     tma_prefetch_desc(&tma_bs.m[0]);
   }
   if (warp == 1) {
-    tmem_alloc(tmem_slot, 512);
+    tmem_alloc(tmem_slot, T::TMEM_COLS);
     tmem_relinquish();
   }
   tc_fence_before();
@@ -467,7 +476,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
   if (*abort_flag) bounded_drain_pause();
   if (warp == 1) {
     tc_fence_after();
-    tmem_dealloc(tmem_base, 512);
+    tmem_dealloc(tmem_base, T::TMEM_COLS);
   }
 }
 

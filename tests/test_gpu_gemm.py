@@ -60,3 +60,42 @@ def test_linear_fwd_dgrad_wgrad_match_autograd():
     assert (y.float() - (xf @ wf.t())).abs().max() <= 0.01 * (xf @ wf.t()).abs().max()
     assert (dx.float() - xf.grad).abs().max() <= 0.01 * xf.grad.abs().max()
     assert torch.allclose(dw, wf.grad, atol=2e-2, rtol=1e-3)
+
+
+@pytest.mark.parametrize("a_mn,b_mn", [(False, False), (False, True), (True, True)])
+@pytest.mark.parametrize("M,N,Kd", [(1, 8, 8), (128, 64, 640), (100, 72, 200), (257, 200, 1000), (2048, 1024, 328), (1100, 3000, 72), (4000, 1544, 136)])
+def test_gemm_at_every_tile_width(M, N, Kd, a_mn, b_mn):
+    """Products that get tiles of 64, 128 and 256 columns, ragged in every direction, with and without an fp32 addend. The
+    products of bf16 numbers are exact in fp32: tolerance 2e-6 of the sum of their magnitudes, plus bf16 rounding (2^-8)."""
+    from ringattention_b200.ops import _lib, kernels as K
+
+    if (a_mn and M % 8) or (b_mn and N % 8):
+        pytest.skip("a leading dimension that is no multiple of eight is refused")
+    g = torch.Generator(device="cuda").manual_seed(M + N)
+    a = torch.randn(M, Kd, device="cuda", generator=g).bfloat16()
+    b = torch.randn(N, Kd, device="cuda", generator=g).bfloat16()
+    A, B = (a.t().contiguous() if a_mn else a), (b.t().contiguous() if b_mn else b)
+    want = a.double() @ b.double().t()
+    slack = 2e-6 * (a.double().abs() @ b.double().abs().t())
+    wide = torch.full((M, N + 24), 3.0, device="cuda")
+    acc = wide[:, :N]
+    K.gemm(A, B, a_mn=a_mn, b_mn=b_mn, out=acc, residual=acc)
+    assert ((acc.double() - 3.0 - want).abs() <= slack + 1e-6).all() and (wide[:, N:] == 3.0).all()
+    c = K.gemm(A, B, a_mn=a_mn, b_mn=b_mn)
+    assert ((c.double() - want).abs() <= slack + 2**-8 * want.abs()).all()
+    _lib.check_status()
+
+
+@pytest.mark.parametrize("M,F,Kd", [(5, 8, 64), (128, 72, 200), (300, 1000, 1024), (2048, 2816, 512), (2100, 5504, 136)])
+def test_swiglu_epilogue_at_every_tile_width(M, F, Kd):
+    """Gate and up columns of a tile come from two places of the weight: ragged widths at each tile width. The result equals
+    the two-pass path, up to the last bit of a bf16 (2^-8) where a sum lies on a rounding border."""
+    from ringattention_b200.ops import kernels as K
+
+    g = torch.Generator(device="cuda").manual_seed(F)
+    x = torch.randn(M, Kd, device="cuda", generator=g).bfloat16()
+    w = (torch.randn(2 * F, Kd, device="cuda", generator=g) / Kd ** 0.5).bfloat16()
+    got = K.linear_swiglu(x, w)
+    gu = K.linear_fwd(x, w).float()
+    want = torch.nn.functional.silu(gu[:, :F]) * gu[:, F:]
+    assert ((got.float() - want).abs() <= 2**-7 * want.abs() + 1e-4).all()
