@@ -9,12 +9,20 @@
 // TMEM: S0 | S1 | O0 | O1 (4 x 128 columns). While one group runs its softmax the tensor core
 // works on the other tile, so MMA and exp overlap without a third party.
 //
+// HALVES: one CTA owns 128 query rows and its two softmax groups take every second visible KV tile each, with accumulators
+// of their own (O0, O1) that meet in the epilogue. The pipeline is the same (two tiles of scores in flight), a CTA's chain is half
+// as long and there are twice as many CTAs, at the price of loading K and V once per 128 rows. For launches with few
+// query tiles; see halves_pay(). Such a launch may also be split over the keys (`splits`): then every CTA takes its share of
+// the visible tiles, partial results go to fp32 buffers and attn_merge_kernel puts them together.
+//
 // The epilogue normalises O, optionally merges it with the carry (o_prev, lse_prev) of earlier
 // ring steps and writes fp32 (intermediate step) or bf16 (last step) plus the log-sum-exp.
 // Leading CTAs of the grid can be given a copy job: they pull the next ring step's KV block from
 // a peer GPU's memory into a local slab with plain 16-byte loads while the other CTAs compute.
 #include "attn_common.cuh"
 #include "common/host_util.h"
+
+#include <math.h>
 
 RA_BOUNDS_TRANSLATION_UNIT()
 
@@ -32,7 +40,9 @@ static_assert(128 * FWD_REGS_PRODUCER + 256 * FWD_REGS_SOFTMAX <= FWD_THREADS * 
 
 struct FwdParams {
   int B, H;
-  TileOrder order;  // of the 256-row query pairs
+  TileOrder order;  // of the 256-row query pairs (HALVES: 128-row tiles)
+  int splits;       // HALVES: CTAs per query tile, neighbours in the grid; `out` and `lse_out` of split s are s * split_o, s * split_l further
+  long long split_o, split_l;
   MaskParams mask;
   float scale_log2;  // log2(e) / sqrt(D)
   void* out;
@@ -88,7 +98,7 @@ struct FwdSmem {
 // NQ: slabs of the query/key part that every head has of its own; NR: slabs of a second part (maps tma_q2, tma_k2) whose
 // keys all heads share; DV: value width. EXT adds the options of an inference layer (see FwdParams); without it NR = 0 and
 // the head dim is 64 NQ = DV.
-template <int NQ, int NR, int DV, bool EXT>
+template <int NQ, int NR, int DV, bool EXT, bool HALVES>
 __global__ void __launch_bounds__(FWD_THREADS, 1)
 attn_fwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constant__ CUtensorMap tma_k,
                 const __grid_constant__ CUtensorMap tma_v, const __grid_constant__ CUtensorMap tma_q2,
@@ -144,13 +154,21 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constant
   const MaskParams& mk = p.mask;
 
   // block -> (q pair, head, batch): heavy (late) q tiles first, a few heads at a time
-  int bh, qp;
-  p.order(static_cast<int>(blockIdx.x) - p.copy_ctas, qp, bh);
-  qp = p.order.n - 1 - qp;
+  int bh, qp, split = 0;
+  {
+    int unit = static_cast<int>(blockIdx.x) - p.copy_ctas;
+    if (HALVES) {
+      split = unit % p.splits;
+      unit /= p.splits;
+    }
+    p.order(unit, qp, bh);
+    qp = p.order.n - 1 - qp;
+  }
   const int h = bh % p.H;
   const int b = bh / p.H;
   const int h_kv = EXT && p.kv_share > 1 ? h / p.kv_share : h;
-  const int q0 = qp * 256;
+  constexpr int NT = HALVES ? 1 : 2;  // q tiles
+  const int q0 = qp * (NT * 128);
   const int nk = (mk.Sk + 127) / 128;
   // row of a key tile (tiles never straddle the end of the ring)
   auto kv_row = [&](int k0) -> int {
@@ -220,7 +238,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constant
   }
   if (use_vis) {
 #pragma unroll
-    for (int w = 0; w < 2; ++w)
+    for (int w = 0; w < NT; ++w)
       fill_visibility(sVis + w * VIS_WORDS, nk, static_cast<int>(threadIdx.x), FWD_THREADS,
                       [&](int j) { return visible(w, j) && (!mk.bias || ((sLive[j >> 5] >> (j & 31)) & 1u)); });
   }
@@ -231,6 +249,29 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constant
       if (visible(w, j)) break;
     return j;
   };
+  if (HALVES && p.splits > 1) {  // keep this split's share of the visible tiles (the launcher sees to use_vis)
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      const int words = (nk + 31) >> 5;
+      int total = 0;
+      for (int i = 0; i < words; ++i) total += __popc(sVis[i]);
+      const int lo = static_cast<int>(static_cast<long long>(total) * split / p.splits);
+      const int hi = static_cast<int>(static_cast<long long>(total) * (split + 1) / p.splits);
+      int seen = 0;
+      for (int i = 0; i < words; ++i) {
+        uint32_t left = sVis[i], mine = 0;
+        const int n = __popc(left);
+        if (seen >= lo && seen + n <= hi) {
+          mine = left;
+        } else {
+          for (int at = seen; left; ++at, left &= left - 1)
+            if (at >= lo && at < hi) mine |= left & (~left + 1);
+        }
+        seen += n;
+        sVis[i] = mine;
+      }
+    }
+  }
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -242,16 +283,16 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constant
   if (warp == 0) {
     // ================================================================ TMA producer
     if (lane == 0) {
-      mbar_arrive_expect_tx(q_full, 2 * SM::Q_TILE_BYTES);
+      mbar_arrive_expect_tx(q_full, NT * SM::Q_TILE_BYTES);
 #pragma unroll
-      for (int w = 0; w < 2; ++w)
+      for (int w = 0; w < NT; ++w)
 #pragma unroll
         for (int s = 0; s < NSLAB; ++s)
           tma_load_4d(sQ + w * SM::Q_TILE_BYTES + s * SM::SLAB_BYTES, s < NQ ? &tma_q : &tma_q2, q_full,
                       (s < NQ ? s : s - NQ) * 64, h, q0 + w * 128, b);
       int it = 0;
-      for (int j = min(next_vis(0, 0), next_vis(1, 0)); j < nk;
-           j = min(next_vis(0, j + 1), next_vis(1, j + 1))) {
+      auto next_any = [&](int j) { return HALVES ? next_vis(0, j) : min(next_vis(0, j), next_vis(1, j)); };
+      for (int j = next_any(0); j < nk; j = next_any(j + 1)) {
         const int k0 = j * 128;
         const int st = it & 1;
         const uint32_t ph = (it >> 1) & 1;
@@ -290,7 +331,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constant
         for (int kk = 0; kk < NSLAB * 4; ++kk) {
           const uint32_t off = (kk >> 2) * SM::SLAB_BYTES + (kk & 3) * 32;
           if (leader)
-            umma_ss(tS[w], desc_advance(q_desc[w], off), desc_advance(k_desc[st], off), idesc_s,
+            umma_ss(tS[w], desc_advance(q_desc[HALVES ? 0 : w], off), desc_advance(k_desc[st], off), idesc_s,
                     kk != 0 ? 1u : 0u);
         }
         if (leader) umma_commit(&s_full[w]);
@@ -305,6 +346,35 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constant
         }
         if (leader) umma_commit(&o_done[w]);
       };
+      if constexpr (HALVES) {
+        // tile `it` of the walk belongs to group it & 1; its scores are issued two tiles ahead, behind the product of
+        // the probabilities they overwrite
+        bool ok = mbar_wait(q_full, 0, wc, kTimeoutSmemFull);
+        int js = next_vis(0, 0);  // next tile whose scores are to be issued
+        int n_s = 0;
+        auto next_scores = [&]() {
+          const int st = n_s % K_STAGES;
+          if (!mbar_wait(&k_full[st], (n_s / K_STAGES) & 1, wc, kTimeoutSmemFull)) return false;
+          tc_fence_after();
+          issue_s(n_s & 1, st);
+          if (leader) umma_commit(&k_empty[st]);
+          ++n_s;
+          js = next_vis(0, js + 1);
+          return true;
+        };
+        if (ok && js < nk) ok = next_scores();
+        if (ok && js < nk) ok = next_scores();
+        for (int it = 0; ok && it < n_s; ++it) {
+          const int w = it & 1, st = it & 1;
+          const uint32_t ph = (it >> 1) & 1;
+          if (!mbar_wait(&v_full[st], ph, wc, kTimeoutSmemFull)) break;
+          if (!mbar_wait(&p_full[w], ph, wc, kTimeoutTmemFull)) break;
+          tc_fence_after();
+          issue_pv(w, st, it > 1);
+          if (leader) umma_commit(&v_empty[st]);
+          if (js < nk) ok = next_scores();
+        }
+      } else {
       auto next_visible = [&](int j, bool& v0, bool& v1) {
         const int a = next_vis(0, j), c = next_vis(1, j);
         const int jj = min(a, c);
@@ -367,16 +437,18 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constant
         v1 = n1;
         ++it;
       }
+      }
     }
     __syncwarp();
   } else if (warp >= 4) {
     // ================================================================ softmax groups
     setmaxnreg_inc<FWD_REGS_SOFTMAX>();
-    const int w = (warp - 4) >> 2;  // q tile handled by this group
+    const int w = (warp - 4) >> 2;  // q tile handled by this group (HALVES: parity of its tiles in the walk)
+    const int wv = HALVES ? 0 : w;  // visibility mask it walks
     const int quad = warp & 3;
     const int row = quad * 32 + lane;
     const int wg_tid = quad * 32 + lane;
-    const int qi0 = q0 + w * 128;
+    const int qi0 = q0 + wv * 128;
     const int qi = qi0 + row;
     const bool row_valid = qi < mk.Sq;
     const int qpos = mk.qmap(row_valid ? qi : mk.Sq - 1);
@@ -390,7 +462,13 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constant
     bool alive = true;
 
     // every role walks the same visibility mask, so skips stay consistent
-    for (int j = next_vis(w, 0); j < nk && alive; j = next_vis(w, j + 1)) {
+    auto next_mine = [&](int j) {
+      j = next_vis(wv, j);
+      return HALVES && j < nk ? next_vis(wv, j + 1) : j;  // the other group takes the one between
+    };
+    int j = next_vis(wv, 0);
+    if (HALVES && w == 1 && j < nk) j = next_vis(wv, j + 1);
+    for (; j < nk && alive; j = next_mine(j + 1)) {
       const int k0 = j * 128;
       const int kind = tile_mask(mk, b, qi0, k0) | (EXT && !tile_window_plain(mk, p.window, qi0, k0) ? kMaskEdge : 0);
       const bool biased = mk.bias && (!use_vis || ((sAdd[j >> 5] >> (j & 31)) & 1u));
@@ -560,9 +638,46 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constant
     // ---- epilogue: normalise, merge with carry, store
     if (alive && cnt > 0) alive = mbar_wait(&o_done[w], (cnt - 1) & 1, wc, kTimeoutTmemFull);
     tc_fence_after();
+    // HALVES: this group finishes half of the columns of all rows. It hands the other half and its (reference, sum) to the
+    // other group through shared memory that held K and V: both groups have seen their last product complete, so no
+    // load and no MMA touches it any more. 16-byte pieces, XOR-swizzled by the row.
+    constexpr int HALF = DV / 2;               // columns
+    constexpr int PIECES = HALF / 4;
+    float own_mul = 1.f, other_mul = 0.f;      // factors of the two accumulators
+    float* const other_row = reinterpret_cast<float*>(sK) + ((1 - w) * 128 + row) * HALF;  // what the other group left for us
+    if (HALVES) {
+      float2* stat = reinterpret_cast<float2*>(sSeg);  // [group][128]: masks are done with
+      named_bar_sync(3, 256);
+      float* dst = reinterpret_cast<float*>(sK) + (w * 128 + row) * HALF;
+#pragma unroll 1
+      for (int c = 0; c < HALF / 32; ++c) {
+        uint32_t o[32];
+        if (cnt > 0) {
+          tmem_ld_x32(tO[w] + lane_base + (1 - w) * HALF + c * 32, o);
+          tmem_ld_wait();
+        } else {
+#pragma unroll
+          for (int i = 0; i < 32; ++i) o[i] = 0u;
+        }
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+          *reinterpret_cast<uint4*>(dst + (((c * 8 + i) ^ (row & (PIECES - 1))) << 2)) =
+              make_uint4(o[4 * i], o[4 * i + 1], o[4 * i + 2], o[4 * i + 3]);
+      }
+      stat[w * 128 + row] = make_float2(cnt > 0 ? m_ref : -INFINITY, l);
+      named_bar_sync(3, 256);
+      const float2 other = stat[(1 - w) * 128 + row];
+      const float m_own = cnt > 0 ? m_ref : -INFINITY;
+      const float m_all = fmaxf(m_own, other.x);
+      const float mu = m_all == -INFINITY ? 0.f : m_all;
+      own_mul = exp2_approx(m_own - mu);
+      other_mul = exp2_approx(other.x - mu);
+      l = l * own_mul + other.y * other_mul;
+      m_ref = m_all;
+    }
     float inv_l = 0.f;
     float lse = -INFINITY;
-    if (cnt > 0 && l > 0.f) {
+    if ((HALVES || cnt > 0) && l > 0.f) {
       inv_l = 1.0f / l;
       lse = (m_ref + log2f(l)) * kLn2;
     }
@@ -582,9 +697,9 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constant
         lse = mxl + __logf(tot);
       }
     }
-    if ((!EXT || p.lse_out) && row_valid &&
+    if ((!EXT || p.lse_out) && row_valid && (!HALVES || w == 0) &&
         RA_IN_BOUNDS(lse_idx, 1, static_cast<long long>(p.B) * p.H * mk.Sq, kTagAttnFwdLse))
-      p.lse_out[lse_idx] = lse;
+      p.lse_out[(HALVES ? split * p.split_l : 0) + lse_idx] = lse;
     float mul = inv_l * w_this;
     if (EXT && row_valid) {
       if (p.sink) mul /= 1.f + expf(p.sink[h] - lse);
@@ -593,9 +708,10 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constant
     }
     const float* oprev_row =
         p.o_prev ? p.o_prev + ((static_cast<long long>(b) * mk.Sq + qi) * p.H + h) * DV : nullptr;
-    const long long o_off = b * p.o_stride_b + static_cast<long long>(qi) * p.o_stride_s + h * p.o_stride_h;
+    const long long o_off = b * p.o_stride_b + static_cast<long long>(qi) * p.o_stride_s + h * p.o_stride_h +
+                            (HALVES ? split * p.split_o : 0);
 #pragma unroll 1
-    for (int c = 0; c < DV / 32; ++c) {
+    for (int c = HALVES ? w * (HALF / 32) : 0; c < (HALVES ? (w + 1) * (HALF / 32) : DV / 32); ++c) {
       uint32_t o[32];
       if (cnt > 0) {
         tmem_ld_x32(tO[w] + lane_base + c * 32, o);
@@ -606,8 +722,20 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constant
       }
       if (row_valid && RA_IN_BOUNDS(qi, 1, mk.Sq, kTagAttnFwdOut) && RA_IN_BOUNDS(c * 32, 32, DV, kTagAttnFwdOut)) {
         float f[32];
+        if (HALVES) {
 #pragma unroll
-        for (int i = 0; i < 32; ++i) f[i] = __uint_as_float(o[i]) * mul;
+          for (int i = 0; i < 8; ++i) {
+            const float4 x = *reinterpret_cast<const float4*>(
+                other_row + ((((c - w * (HALF / 32)) * 8 + i) ^ (row & (PIECES - 1))) << 2));
+            f[4 * i] = (__uint_as_float(o[4 * i]) * own_mul + x.x * other_mul) * mul;
+            f[4 * i + 1] = (__uint_as_float(o[4 * i + 1]) * own_mul + x.y * other_mul) * mul;
+            f[4 * i + 2] = (__uint_as_float(o[4 * i + 2]) * own_mul + x.z * other_mul) * mul;
+            f[4 * i + 3] = (__uint_as_float(o[4 * i + 3]) * own_mul + x.w * other_mul) * mul;
+          }
+        } else {
+#pragma unroll
+          for (int i = 0; i < 32; ++i) f[i] = __uint_as_float(o[i]) * mul;
+        }
         if (oprev_row) {
 #pragma unroll
           for (int i = 0; i < 8; ++i) {
@@ -651,6 +779,102 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constant
   }
 }
 
+// Puts the partial results of a launch split over the keys together: o (splits, B, Sq, H, D) and lse (splits, B, H, Sq) fp32 ->
+// out (bf16 or fp32 view) and lse_out (B, H, Sq). A warp per row; a split without a visible key has lse = -inf and its
+// (zero) row is not read.
+template <int D>
+__global__ void __launch_bounds__(256) attn_merge_kernel(const float* __restrict__ o, const float* __restrict__ lse, int splits,
+                                                         int B, int H, int Sq, void* out, int out_fp32, long long o_sb,
+                                                         long long o_ss, long long o_sh, float* __restrict__ lse_out) {
+  constexpr int PER = D / 32;
+  const long long rows = static_cast<long long>(B) * Sq * H;
+  const long long row = (static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
+  const int lane = threadIdx.x & 31;
+  if (row >= rows) return;
+  const int h = static_cast<int>(row % H), q = static_cast<int>(row / H % Sq), b = static_cast<int>(row / H / Sq);
+  const long long at = (static_cast<long long>(b) * H + h) * Sq + q;
+  float mx = -INFINITY;
+  for (int s = 0; s < splits; ++s) mx = fmaxf(mx, lse[s * rows + at]);
+  float acc[PER], sum = 0.f;
+#pragma unroll
+  for (int e = 0; e < PER; ++e) acc[e] = 0.f;
+  if (mx != -INFINITY) {
+#pragma unroll 4
+    for (int s = 0; s < splits; ++s) {
+      const float w = expf(lse[s * rows + at] - mx);
+      if (w == 0.f) continue;
+      const float* src = o + (s * rows + row) * D + lane * PER;
+      sum += w;
+#pragma unroll
+      for (int e = 0; e < PER; e += 2) {
+        const float2 v = *reinterpret_cast<const float2*>(src + e);
+        acc[e] += w * v.x;
+        acc[e + 1] += w * v.y;
+      }
+    }
+  }
+  const float inv = mx != -INFINITY ? 1.f / sum : 0.f;
+  if (lane == 0 && RA_IN_BOUNDS(at, 1, rows, kTagAttnFwdLse)) lse_out[at] = mx != -INFINITY ? mx + logf(sum) : -INFINITY;
+  const long long off = b * o_sb + static_cast<long long>(q) * o_ss + h * o_sh + lane * PER;
+#pragma unroll
+  for (int e = 0; e < PER; e += 2) {
+    if (out_fp32) {
+      *reinterpret_cast<float2*>(static_cast<float*>(out) + off + e) = make_float2(acc[e] * inv, acc[e + 1] * inv);
+    } else {
+      *reinterpret_cast<uint32_t*>(static_cast<__nv_bfloat16*>(out) + off + e) = pack_bf16x2(acc[e] * inv, acc[e + 1] * inv);
+    }
+  }
+}
+
+// How a launch is cut up. Lengths are in steps (two 128 x 128 tiles, what a CTA works on at a time); a CTA costs OVERHEAD steps
+// beside its tiles (start-up, first loads, epilogue), and the SMs are busy for at least the longest CTA and the
+// average load. Segment ids and bitmaps are not looked at: the causal rule alone gives the lengths.
+struct FwdShape {
+  bool halves;
+  int splits;
+};
+inline FwdShape fwd_shape(int B, int H, int Sq, int Sk, int cbs, long long q_off, long long k_off, bool one_run, bool may_split) {
+  constexpr double OVERHEAD = 2.5;
+  constexpr double MERGE = 3.0;  // steps: partial results out and in again, one more launch
+  const int nk = (Sk + 127) / 128, nq = (Sq + 127) / 128, sms = sm_count();
+  const long long bh = static_cast<long long>(B) * H;
+  FwdShape best{false, 1};
+  if (nq > 1024 || bh * nq > 64ll * sms) return best;  // plenty of work per SM: two query tiles share the loads of K and V
+  double len[1024];                                    // visible kv tiles of each query tile
+  for (int i = 0; i < nq; ++i) {
+    long long v = nk;
+    if (cbs && one_run) v = (q_off + i * 128ll + 127 - k_off) / 128 + 1;
+    len[i] = static_cast<double>(v < 0 ? 0 : (v > nk ? nk : v));
+  }
+  double sum = 0, top = 0;
+  for (int i = 0; i < nq; i += 2) {
+    const double l = (i + 1 < nq && len[i + 1] > len[i] ? len[i + 1] : len[i]) + OVERHEAD;
+    sum += l;
+    top = l > top ? l : top;
+  }
+  double t_best = sum * bh / sms > top ? sum * bh / sms : top;
+  const long long pairs = bh * ((nq + 1) / 2);
+  const double waves = static_cast<double>((pairs + sms - 1) / sms);
+  if (!cbs && waves * top > t_best) t_best = waves * top;  // equal lengths: whole waves
+  for (int s = 1; s <= (may_split ? 32 : 1); ++s) {
+    double hsum = 0, htop = 0;
+    for (int i = 0; i < nq; ++i) {
+      const double l = ceil(len[i] / (2 * s)) + OVERHEAD;
+      hsum += l;
+      htop = l > htop ? l : htop;
+    }
+    double t = hsum * bh * s / sms > htop ? hsum * bh * s / sms : htop;
+    const double w = static_cast<double>((bh * nq * s + sms - 1) / sms);
+    if ((!cbs || nq == 1) && w * htop > t) t = w * htop;
+    if (s > 1) t += MERGE;
+    if (t < 0.95 * t_best) {
+      t_best = t;
+      best = FwdShape{true, s};
+    }
+  }
+  return best;
+}
+
 }  // namespace attn
 }  // namespace ra
 
@@ -666,11 +890,11 @@ int make_bshd_map(CUtensorMap* m, const void* base, int B, int S, int H, int D, 
   return ra::make_tmap_bf16_sw128(m, base, 4, dims, str, box);
 }
 
-template <int NQ, int NR, int DV, bool EXT = (NR > 0)>
+template <int NQ, int NR, int DV, bool EXT = (NR > 0), bool HALVES = false>
 int launch_fwd(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const CUtensorMap& tq2,
                const CUtensorMap& tk2, const ra::attn::FwdParams& p, long long grid, cudaStream_t s) {
   using namespace ra::attn;
-  auto kern = attn_fwd_kernel<NQ, NR, DV, EXT>;
+  auto kern = attn_fwd_kernel<NQ, NR, DV, EXT, HALVES>;
   constexpr int smem = FwdSmem<NQ + NR, DV>::TOTAL;
   static_assert(smem <= 227 * 1024, "tile buffers do not fit in shared memory");
   if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) {
@@ -702,7 +926,25 @@ struct RaAttnFwdArgs {
   const void* copy_src; void* copy_dst; long long copy_bytes; int copy_ctas;
   int* status;
   void* stream;
+  // splits > 1 (as ra_attn_fwd_splits says, or any number up to 32): the keys are split over that many CTAs per query tile; ws
+  // holds splits * B * Sq * H * (D + 1) floats. Without o_prev and a copy job.
+  int splits;
+  float* ws;
 };
+
+namespace {
+ra::attn::FwdShape shape_of(const RaAttnFwdArgs* a, bool may_split) {
+  const bool one_run = a->q_half >= a->Sq && a->k_half >= a->Sk;
+  return ra::attn::fwd_shape(a->B, a->H, a->Sq, a->Sk, a->causal_block_size, a->q_off0, a->k_off0, one_run, may_split);
+}
+}  // namespace
+
+// Over how many CTAs per query tile ra_attn_fwd would like to split the keys of this launch (1: not at all).
+extern "C" int ra_attn_fwd_splits(const RaAttnFwdArgs* a) {
+  if (a->B <= 0 || a->H <= 0 || a->Sq <= 0 || a->Sk <= 0) return 1;
+  if (a->o_prev || a->copy_src || (a->Sk + 127) / 128 > 32 * ra::attn::VIS_WORDS) return 1;
+  return shape_of(a, true).splits;
+}
 
 extern "C" int ra_attn_fwd(const RaAttnFwdArgs* a) {
   using namespace ra;
@@ -714,6 +956,12 @@ extern "C" int ra_attn_fwd(const RaAttnFwdArgs* a) {
   if (a->B <= 0 || a->H <= 0 || a->Sq <= 0 || a->Sk <= 0 || (a->q_half < a->Sq && a->q_half % 128) ||
       (a->k_half < a->Sk && a->k_half % 128) || (a->copy_bytes % 16)) {
     set_error("ra_attn_fwd: bad shape");
+    return kHostBadArg;
+  }
+  const int splits = a->splits > 1 ? a->splits : 1;
+  if (splits > 1 && (splits > 32 || !a->ws || (reinterpret_cast<uintptr_t>(a->ws) & 15) || a->o_prev || a->copy_src ||
+                     !a->lse_out || (a->Sk + 127) / 128 > 32 * VIS_WORDS)) {
+    set_error("ra_attn_fwd: a launch split over the keys takes a workspace, at most 32 splits, no carry and no copy job");
     return kHostBadArg;
   }
   CUtensorMap tq, tk, tv;
@@ -766,13 +1014,35 @@ extern "C" int ra_attn_fwd(const RaAttnFwdArgs* a) {
   p.gate = nullptr;
   p.gate_ld = 0;
   p.window = p.kv_share = p.k_row0 = p.k_rows = 0;
-  const int n_qp = (a->Sq + 255) / 256;
-  p.order = TileOrder{n_qp, a->B * a->H,
-                      a->causal_block_size ? heads_together(n_qp, a->B * a->H, 4ll * a->Sk * a->D, sm_count()) : 1};
-  const long long grid = static_cast<long long>(n_qp) * a->H * a->B + p.copy_ctas;
+  const bool halves = splits > 1 || shape_of(a, false).halves;
+  const int n_q = halves ? (a->Sq + 127) / 128 : (a->Sq + 255) / 256;
+  p.order = TileOrder{n_q, a->B * a->H,
+                      a->causal_block_size ? heads_together(n_q, a->B * a->H, 4ll * a->Sk * a->D, sm_count()) : 1};
+  p.splits = splits;
+  p.split_l = static_cast<long long>(a->B) * a->H * a->Sq;
+  p.split_o = p.split_l * a->D;
+  if (splits > 1) {
+    p.out = a->ws;
+    p.out_fp32 = 1;
+    p.o_stride_h = a->D;
+    p.o_stride_s = static_cast<long long>(a->H) * a->D;
+    p.o_stride_b = p.o_stride_s * a->Sq;
+    p.lse_out = a->ws + splits * p.split_o;
+  }
+  const long long grid = static_cast<long long>(n_q) * a->H * a->B * splits + p.copy_ctas;
   cudaStream_t s = static_cast<cudaStream_t>(a->stream);
-  return a->D == 128 ? launch_fwd<2, 0, 128>(tq, tk, tv, tq, tk, p, grid, s)
+  if (halves)
+    rc = a->D == 128 ? launch_fwd<2, 0, 128, false, true>(tq, tk, tv, tq, tk, p, grid, s)
+                     : launch_fwd<1, 0, 64, false, true>(tq, tk, tv, tq, tk, p, grid, s);
+  else
+    rc = a->D == 128 ? launch_fwd<2, 0, 128>(tq, tk, tv, tq, tk, p, grid, s)
                      : launch_fwd<1, 0, 64>(tq, tk, tv, tq, tk, p, grid, s);
+  if (rc || splits == 1) return rc;
+  const unsigned blocks = static_cast<unsigned>((p.split_l + 7) / 8);
+  auto merge = a->D == 128 ? attn_merge_kernel<128> : attn_merge_kernel<64>;
+  merge<<<blocks, 256, 0, s>>>(static_cast<const float*>(p.out), p.lse_out, splits, a->B, a->H, a->Sq, a->out, a->out_fp32, a->o_sb,
+                               a->o_ss, a->o_sh, a->lse_out);
+  return check_launch("attn_merge_kernel");
 }
 
 // Causal attention with two-part queries and keys: score = (q1 . k1 + q2 . k2) * scale, where k2 is shared by all heads.

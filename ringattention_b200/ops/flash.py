@@ -92,6 +92,7 @@ class _FwdArgs(ctypes.Structure):
         ("copy_src", c_vp), ("copy_dst", c_vp), ("copy_bytes", c_ll), ("copy_ctas", ctypes.c_int),
         ("status", c_vp),
         ("stream", c_vp),
+        ("splits", ctypes.c_int), ("ws", c_vp),
     ]
 
 
@@ -182,7 +183,11 @@ def flash_fwd(q, k, v, mask: MaskSpec, *, o_prev=None, lse_prev=None, out_fp32=F
     a.copy_src, a.copy_dst, a.copy_bytes, a.copy_ctas = copy_src, copy_dst, copy_bytes, copy_ctas
     a.status = _lib.status_tensor(dev).data_ptr()
     a.stream = torch.cuda.current_stream().cuda_stream
-    _lib.call("ra_attn_fwd", ctypes.byref(a))
+    splits = _lib.lib().ra_attn_fwd_splits(ctypes.byref(a))
+    if splits > 1:  # few query tiles: the keys are split over several CTAs, partial results meet in a second launch
+        ws = torch.empty(splits * B * Sq * H * (D + 1), device=dev, dtype=torch.float32)
+        a.splits, a.ws = splits, ws.data_ptr()
+    _lib.call("ra_attn_fwd", ctypes.byref(a), n_kernels=2 if splits > 1 else 1)
     return out, lse_out
 
 

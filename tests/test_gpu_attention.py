@@ -213,3 +213,16 @@ def test_segment_ids_of_every_kind(ids, D):
     seg = {"per token": t, "runs": t // 5 % 7, "one change": (t >= 333).int(), "alternating": t % 2}[ids].int()[None].expand(B, S).contiguous()
     _check_call(B, S, S, 2, D, seg=seg)
     _check_call(B, S, S, 2, D, cbs=1, seg=seg, bias=torch.randn(B, 1, 1, S, device="cuda"))
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("B,Sq,Sk,H,cbs,cache_idx", [
+    (1, 1, 1, 1, 1, None), (1, 128, 128, 1, 1, None), (1, 129, 129, 2, 1, None), (2, 300, 300, 3, 64, None),   # one tile or two
+    (1, 512, 512, 8, None, None), (1, 2048, 2048, 4, 1, None), (1, 1300, 1300, 2, None, None),                 # tiles shared by two groups
+    (1, 16, 20000, 2, 1, 19984), (1, 200, 9000, 4, 1, 8000), (2, 100, 8200, 1, None, None), (1, 130, 4100, 2, 32, 3970),  # keys split
+    (1, 128, 40000, 1, 1, 100),                                                                                # most keys in the future
+    (1, 2048, 2048, 40, 1, None), (1, 700, 700, 64, None, None),                                               # many tiles: two query tiles a CTA
+])
+def test_every_way_a_forward_is_cut_up(B, Sq, Sk, H, cbs, cache_idx, D):
+    """Sizes on both sides of the rule that gives a CTA two query tiles or one, and splits the keys of a few query tiles."""
+    _check_call(B, Sq, Sk, H, D, cbs=cbs, cache_idx=cache_idx, grad=Sq * Sk * B * H < 3e8)
