@@ -19,6 +19,7 @@ struct RaAttnBwdArgs {
   const float* bias; long long bias_sb, bias_sh;
   unsigned long long seed; unsigned int drop_threshold;
   const unsigned int* keep; long long keep_sb, keep_sh, keep_sr;  // boolean mask bitmap by kv row, or null
+  const unsigned char* keep_tiles; long long keep_tiles_sb, keep_tiles_sh;  // kinds of its tiles [q][k], or null
   const void* copy_src; void* copy_dst; long long copy_bytes; int copy_ctas;
   int* status;
   void* stream;

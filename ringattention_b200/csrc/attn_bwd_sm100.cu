@@ -206,13 +206,13 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constant
   }
   if (use_vis)
     fill_visibility(sVis, nqt, static_cast<int>(threadIdx.x), BWD_THREADS,
-                    [&](int i) { return !dead && tile_visible(mk, b, i * 128, k0); });
+                    [&](int i) { return !dead && tile_visible(mk, b, h, i * 128, k0); });
   // next q tile at or after i that sees this kv tile, or nqt; every role walks the same mask
   auto next_vis = [&](int i) -> int {
     if (use_vis) return vis_next(sVis, i, nqt);
     if (dead) return nqt;
     for (; i < nqt; ++i)
-      if (tile_visible(mk, b, i * 128, k0)) break;
+      if (tile_visible(mk, b, h, i * 128, k0)) break;
     return i;
   };
   tc_fence_before();
@@ -380,7 +380,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constant
       const int qi0 = i * 128;
       const int st = it & 1;
       const uint32_t par = it & 1;
-      const int kind = tile_mask(mk, b, qi0, k0);
+      const int kind = tile_mask(mk, b, h, qi0, k0);
       if (kind & kMaskSeg) {
         if (sm_tid < 128)
           sSegQ[st * 128 + sm_tid] =
@@ -777,6 +777,9 @@ extern "C" int ra_attn_bwd(const RaAttnBwdArgs* a) {
   p.mask.keep_sb = a->keep_sb;
   p.mask.keep_sh = a->keep_sh;
   p.mask.keep_sr = a->keep_sr;
+  p.mask.keep_tiles = a->keep_tiles;
+  p.mask.keep_tiles_sb = a->keep_tiles_sb;
+  p.mask.keep_tiles_sh = a->keep_tiles_sh;
   p.scale = a->softmax_scale;
   p.scale_log2 = a->softmax_scale * kLog2e;
   p.lse2 = a->lse2;

@@ -34,12 +34,22 @@ struct MaskParams {
   // of row k: queries 32w..32w+31); strides in 32-bit words, row stride a multiple of 4.
   const uint32_t* keep;
   long long keep_sb, keep_sh, keep_sr;
+  // kind of the bitmap's 128 x 128 tiles [b][h][q tile][k tile]: 0 no bit set, 1 all set, 2 some; or null
+  const uint8_t* keep_tiles;
+  long long keep_tiles_sb, keep_tiles_sh;
 };
 
+// Kind of a tile of the bitmap (2 where it is not known, or there is none).
+__device__ __forceinline__ int bitmap_tile(const MaskParams& m, int b, int h, int qi0, int k0) {
+  if (!m.keep_tiles) return 2;
+  return m.keep_tiles[b * m.keep_tiles_sb + h * m.keep_tiles_sh + static_cast<long long>(qi0 >> 7) * ((m.Sk + 127) >> 7) + (k0 >> 7)];
+}
+
 // False when every entry of the (128 q x 128 k) tile is masked by the causal rule or because the
-// segment-id ranges of the two tiles are disjoint. qi0/k0 are local start indices.
-__device__ __forceinline__ bool tile_visible(const MaskParams& m, int b, int qi0, int k0) {
+// segment-id ranges of the two tiles are disjoint, or by the bitmap. qi0/k0 are local start indices.
+__device__ __forceinline__ bool tile_visible(const MaskParams& m, int b, int h, int qi0, int k0) {
   if (qi0 >= m.Sq || k0 >= m.Sk) return false;
+  if (m.keep_tiles && bitmap_tile(m, b, h, qi0, k0) == 0) return false;
   if (m.cbs == 1) {  // plain causal: no divisions on the hot path
     if (m.qmap(min(qi0 + 127, m.Sq - 1)) < m.kmap(k0)) return false;
   } else if (m.cbs) {
@@ -88,8 +98,8 @@ __device__ __forceinline__ int vis_next(const uint32_t* words, int t, int n) {
 // What may hide single entries of a visible tile; 0: nothing does. With segment ids the common case inside packed documents
 // much longer than a tile is that both tiles lie in one and the same segment (per-tile min == max, equal on both sides).
 enum TileMask : int { kMaskEdge = 1 /* causal rule or end of the keys */, kMaskSeg = 2, kMaskBits = 4 /* bitmap, dropout */ };
-__device__ __forceinline__ int tile_mask(const MaskParams& m, int b, int qi0, int k0) {
-  int kind = (m.drop_threshold || m.keep) ? kMaskBits : 0;
+__device__ __forceinline__ int tile_mask(const MaskParams& m, int b, int h, int qi0, int k0) {
+  int kind = (m.drop_threshold || (m.keep && bitmap_tile(m, b, h, qi0, k0) != 1)) ? kMaskBits : 0;
   if (k0 + 128 > m.Sk) kind |= kMaskEdge;
   if (m.seg_q) {
     bool one = false;

@@ -177,7 +177,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constant
     return r >= p.k_rows ? r - p.k_rows : r;
   };
   auto visible = [&](int w, int j) -> bool {
-    return tile_visible(mk, b, q0 + w * 128, j * 128) && (!EXT || tile_in_window(mk, p.window, q0 + w * 128, j * 128));
+    return tile_visible(mk, b, h, q0 + w * 128, j * 128) && (!EXT || tile_in_window(mk, p.window, q0 + w * 128, j * 128));
   };
 
   if (threadIdx.x == 0) {
@@ -470,7 +470,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constant
     if (HALVES && w == 1 && j < nk) j = next_vis(wv, j + 1);
     for (; j < nk && alive; j = next_mine(j + 1)) {
       const int k0 = j * 128;
-      const int kind = tile_mask(mk, b, qi0, k0) | (EXT && !tile_window_plain(mk, p.window, qi0, k0) ? kMaskEdge : 0);
+      const int kind = tile_mask(mk, b, h, qi0, k0) | (EXT && !tile_window_plain(mk, p.window, qi0, k0) ? kMaskEdge : 0);
       const bool biased = mk.bias && (!use_vis || ((sAdd[j >> 5] >> (j & 31)) & 1u));
       const int buf = cnt & 1;
       if ((kind & kMaskSeg) || biased) {
@@ -923,6 +923,7 @@ struct RaAttnFwdArgs {
   const float* bias; long long bias_sb, bias_sh;
   unsigned long long seed; unsigned int drop_threshold;
   const unsigned int* keep; long long keep_sb, keep_sh, keep_sr;  // boolean mask bitmap by query row, or null
+  const unsigned char* keep_tiles; long long keep_tiles_sb, keep_tiles_sh;  // kinds of its tiles, or null
   const void* copy_src; void* copy_dst; long long copy_bytes; int copy_ctas;
   int* status;
   void* stream;
@@ -991,6 +992,9 @@ extern "C" int ra_attn_fwd(const RaAttnFwdArgs* a) {
   p.mask.keep_sb = a->keep_sb;
   p.mask.keep_sh = a->keep_sh;
   p.mask.keep_sr = a->keep_sr;
+  p.mask.keep_tiles = a->keep_tiles;
+  p.mask.keep_tiles_sb = a->keep_tiles_sb;
+  p.mask.keep_tiles_sh = a->keep_tiles_sh;
   if (a->keep && ((a->keep_sr % 4) || (a->keep_sb % 4) || (a->keep_sh % 4) || (reinterpret_cast<uintptr_t>(a->keep) & 15))) {
     set_error("ra_attn_fwd: mask bitmap rows must be 16-byte aligned");
     return kHostBadArg;

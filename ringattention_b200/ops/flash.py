@@ -57,6 +57,7 @@ class MaskSpec:
     pdrop: float = 0.0
     keep_q: Optional[torch.Tensor] = None  # (B, 1|H, Sq, 4*ceil(Sk/128)) int32 bitmap by query row (forward)
     keep_k: Optional[torch.Tensor] = None  # (B, 1|H, Sk, 4*ceil(Sq/128)) int32 bitmap by kv row (backward)
+    keep_tiles: Optional[torch.Tensor] = None  # (B, 1|H, ceil(Sq/128), ceil(Sk/128)) uint8 of the bitmap's tiles: 0 empty, 1 full, 2 mixed
 
 
 def seg_tile_minmax(seg: torch.Tensor) -> torch.Tensor:
@@ -89,6 +90,7 @@ class _FwdArgs(ctypes.Structure):
         ("bias", c_vp), ("bias_sb", c_ll), ("bias_sh", c_ll),
         ("seed", ctypes.c_ulonglong), ("drop_threshold", ctypes.c_uint),
         ("keep", c_vp), ("keep_sb", c_ll), ("keep_sh", c_ll), ("keep_sr", c_ll),
+        ("keep_tiles", c_vp), ("keep_tiles_sb", c_ll), ("keep_tiles_sh", c_ll),
         ("copy_src", c_vp), ("copy_dst", c_vp), ("copy_bytes", c_ll), ("copy_ctas", ctypes.c_int),
         ("status", c_vp),
         ("stream", c_vp),
@@ -107,21 +109,27 @@ def _ptr(t):
     return 0 if t is None else t.data_ptr()
 
 
-def pack_mask(mask: torch.Tensor, want_q: bool = True, want_k: bool = True):
-    """Pack a boolean ``(B, 1|H, 1|Sq, Sk)`` mask (True = attend) into the two bitmaps the kernels read:
-    by query row for the forward, by kv row for the backward (``MaskSpec.keep_q`` / ``keep_k``). A mask
-    without query rows (a key-padding mask) must be expanded by the caller to the query length first."""
+def mask_bitmaps(mask: torch.Tensor, want_q: bool = True, want_k: bool = True):
+    """Pack a boolean ``(B, 1|H, 1|Sq, Sk)`` mask (True = attend) into what the kernels read: the bitmaps by query row
+    for the forward and by kv row for the backward (``MaskSpec.keep_q`` / ``keep_k``), and the kind of every tile
+    (``keep_tiles``). A mask without query rows (a key-padding mask) must be expanded by the caller to the query length first."""
     assert mask.dim() == 4 and mask.is_cuda
-    m = mask.to(torch.uint8)
+    m = mask.view(torch.uint8) if mask.dtype == torch.bool else mask.to(torch.uint8)  # a bool is a byte of 0 or 1
     if m.stride(3) != 1:
         m = m.contiguous()
     B, Hm, Sq, Sk = m.shape
-    Wk, Wq = 4 * ((Sk + 127) // 128), 4 * ((Sq + 127) // 128)
-    by_q = torch.zeros(B, Hm, Sq, Wk, device=m.device, dtype=torch.int32) if want_q else None
-    by_k = torch.zeros(B, Hm, Sk, Wq, device=m.device, dtype=torch.int32) if want_k else None
+    nq, nk = (Sq + 127) // 128, (Sk + 127) // 128
+    by_q = torch.empty(B, Hm, Sq, 4 * nk, device=m.device, dtype=torch.int32) if want_q else None
+    by_k = torch.empty(B, Hm, Sk, 4 * nq, device=m.device, dtype=torch.int32) if want_k else None
+    tiles = torch.empty(B, Hm, nq, nk, device=m.device, dtype=torch.uint8)
     _lib.call("ra_pack_mask", c_vp(m.data_ptr()), c_ll(m.stride(0)), c_ll(m.stride(1)), c_ll(m.stride(2)),
-              c_vp(_ptr(by_q)), c_vp(_ptr(by_k)), B, Hm, Sq, Sk, _lib.stream_ptr())
-    return by_q, by_k
+              c_vp(_ptr(by_q)), c_vp(_ptr(by_k)), c_vp(tiles.data_ptr()), B, Hm, Sq, Sk, _lib.stream_ptr())
+    return by_q, by_k, tiles
+
+
+def pack_mask(mask: torch.Tensor, want_q: bool = True, want_k: bool = True):
+    """The two bitmaps of :func:`mask_bitmaps`."""
+    return mask_bitmaps(mask, want_q, want_k)[:2]
 
 
 def _fill_mask(a, mask: MaskSpec, H: int, by_k: bool = False):
@@ -134,6 +142,10 @@ def _fill_mask(a, mask: MaskSpec, H: int, by_k: bool = False):
         a.keep_sb = keep.stride(0)
         a.keep_sh = keep.stride(1) if keep.shape[1] == H else 0
         a.keep_sr = keep.stride(2)
+        tiles = mask.keep_tiles
+        if tiles is not None:
+            assert tiles.dtype == torch.uint8 and tiles.is_contiguous() and tiles.shape[:2] == keep.shape[:2]
+            a.keep_tiles, a.keep_tiles_sb, a.keep_tiles_sh = tiles.data_ptr(), tiles.stride(0), tiles.stride(1) if tiles.shape[1] == H else 0
     a.causal_block_size = int(mask.causal_block_size or 0)
     a.q_off0, a.q_off1, a.q_half = mask.q_pos.off0, mask.q_pos.off1, mask.q_pos.half
     a.k_off0, a.k_off1, a.k_half = mask.k_pos.off0, mask.k_pos.off1, mask.k_pos.half
@@ -212,6 +224,7 @@ class _BwdArgs(ctypes.Structure):
         ("bias", c_vp), ("bias_sb", c_ll), ("bias_sh", c_ll),
         ("seed", ctypes.c_ulonglong), ("drop_threshold", ctypes.c_uint),
         ("keep", c_vp), ("keep_sb", c_ll), ("keep_sh", c_ll), ("keep_sr", c_ll),
+        ("keep_tiles", c_vp), ("keep_tiles_sb", c_ll), ("keep_tiles_sh", c_ll),
         ("copy_src", c_vp), ("copy_dst", c_vp), ("copy_bytes", c_ll), ("copy_ctas", ctypes.c_int),
         ("status", c_vp),
         ("stream", c_vp),

@@ -80,11 +80,11 @@ class RingInferenceAttention(torch.autograd.Function):
     ringattention_inference.py:64)."""
 
     @staticmethod
-    def forward(ctx, q, k, v, mask_local, axis, symm_ring):
+    def forward(ctx, q, k, v, mask_local, axis, symm_ring, need_grad):
         B, ql, H, D = q.shape
         ms = MaskSpec(causal_block_size=0, q_pos=Positions(0), k_pos=Positions(0))
         if mask_local is not None:
-            ms.keep_q, ms.keep_k = flash.pack_mask(mask_local)
+            ms.keep_q, ms.keep_k, ms.keep_tiles = flash.mask_bitmaps(mask_local, want_k=need_grad)
         if axis.size == 1:
             out, lse = flash.flash_fwd(q, k, v, ms)
         else:
@@ -111,7 +111,7 @@ class RingInferenceAttention(torch.autograd.Function):
             dist.all_reduce(dq_acc, group=ctx.axis.group)
         dq = torch.empty_like(q)
         K.cast_f32_to_bf16(dq_acc.view(B * ql, H * D), dq.view(B * ql, H * D))
-        return dq, dk, dv, None, None, None
+        return dq, dk, dv, None, None, None, None
 
 
 def ring_inference_attention(q, k, v, attn_mask, axis, symm_ring=None):
@@ -128,4 +128,4 @@ def ring_inference_attention(q, k, v, attn_mask, axis, symm_ring=None):
         return t.stride(3) == 1 and not any(s % 8 for s in t.stride()[:3]) and t.data_ptr() % 16 == 0
 
     qq, kk, vv = (t if ok(t) else t.contiguous() for t in (q, k, v))
-    return RingInferenceAttention.apply(qq, kk, vv, m, axis, symm_ring)
+    return RingInferenceAttention.apply(qq, kk, vv, m, axis, symm_ring, need_grad)

@@ -371,3 +371,58 @@ def test_merge_of_few_and_many_partials(nparts, D):
     assert (out.double() - want).abs().max() < 2e-5
     fin = torch.isfinite(want_l)
     assert torch.equal(torch.isfinite(lse_out), fin) and (lse_out.double() - want_l)[fin].abs().max() < 1e-5
+
+
+def test_kinds_of_mask_tiles():
+    from ringattention_b200.ops import flash
+
+    m = torch.zeros(1, 2, 300, 333, dtype=torch.bool, device="cuda")
+    m[0, 0] = True                       # full, the ragged tiles too
+    m[0, 1, :128, 128:256] = True
+    m[0, 1, 299, 332] = True
+    m[0, 1, 130:200, 5:90] = True
+    _, _, tiles = flash.mask_bitmaps(m, want_k=False)
+    assert tiles[0, 0].unique().tolist() == [1]
+    assert tiles[0, 1].tolist() == [[0, 1, 0], [2, 0, 0], [0, 0, 2]]
+    every = torch.ones(1, 1, 300, 333, dtype=torch.bool, device="cuda")
+    every[0, 0, 299, 332] = False
+    assert flash.mask_bitmaps(every)[2][0, 0].tolist() == [[1, 1, 1], [1, 1, 1], [1, 1, 2]]
+
+
+@pytest.mark.parametrize("need_grad", [False, True])
+@pytest.mark.parametrize("B,ql,S,H,D,kind", [(1, 9, 3000, 2, 64, "causal"), (1, 500, 4096, 4, 128, "causal"), (2, 130, 2049, 3, 64, "holes"),
+                                             (1, 300, 1000, 5, 128, "per head"), (2, 64, 5000, 2, 128, "padding"), (1, 16, 9000, 1, 64, "nothing")])
+def test_masked_prompt_chunks(B, ql, S, H, D, kind, need_grad):
+    """Chunks of a prompt against a longer cache, with masks whose tiles are full, empty and mixed, at sizes where the keys are
+    split over several CTAs and where they are not. bf16 in and out: 1e-2 of the largest entry, gradients 2e-2."""
+    import ringattention_b200 as rab
+
+    g = torch.Generator(device="cuda").manual_seed(S)
+    q, dout = (torch.randn(B, ql, H, D, device="cuda", generator=g).bfloat16() for _ in range(2))
+    k, v = (torch.randn(B, S, H, D, device="cuda", generator=g).bfloat16() for _ in range(2))
+    at = torch.arange(S, device="cuda")
+    if kind == "causal":
+        mask = (at[None] <= torch.arange(S - ql, S, device="cuda")[:, None])[None, None]
+    elif kind == "holes":
+        mask = torch.rand(B, 1, ql, S, device="cuda", generator=g) < 0.5
+        mask[:, :, :, 256:512] = False
+    elif kind == "per head":
+        mask = (torch.rand(1, H, ql, S, device="cuda", generator=g) < 0.9) & (at < 700)
+        mask[0, 1] = True
+        mask[0, 2, 5] = False
+    elif kind == "padding":
+        mask = (at[None] < torch.tensor([S, 1300], device="cuda")[:, None])[:, None, None]
+    else:
+        mask = torch.zeros(1, 1, ql, S, dtype=torch.bool, device="cuda")
+        mask[..., 3, 8000] = True
+    qd, kd, vd = (t.double().requires_grad_() for t in (q, k, v))
+    x = (torch.einsum("bqhd,bkhd->bhqk", qd, kd) / D ** 0.5).masked_fill(~mask, -float("inf"))
+    e = torch.exp(x - x.amax(-1, keepdim=True).clamp_min(-1e300))
+    want = torch.einsum("bhqk,bkhd->bqhd", e / e.sum(-1, keepdim=True).clamp_min(1e-300), vd)
+    q, k, v = (t.requires_grad_(need_grad) for t in (q, k, v))
+    out = rab.ringattention_inference(q, k, v, mask)
+    assert (out.double() - want).abs().max() <= 0.01 * want.abs().max() + 1e-3
+    if need_grad:
+        got = torch.autograd.grad(out, (q, k, v), dout)
+        for a, b in zip(got, torch.autograd.grad(want, (qd, kd, vd), dout.double())):
+            assert (a.double() - b).abs().max() <= 0.02 * b.abs().max() + 1e-3
