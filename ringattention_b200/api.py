@@ -87,12 +87,12 @@ def ringattention(q, k, v, attn_bias=None, segment_ids=None, cache_idx=None, axi
         raise ValueError("q must be (B,Sq,H,D) and k, v (B,Sk,H,D) with matching B, H, D")
     if _fused_ok(q, attn_bias):
         from .ops import attention as A
+        from .ops.flash import tma_ready
 
         B, Sq, H, D = q.shape
         plan = A.make_plan(axis.rank, axis.size, B, Sq, k.shape[1], H, kw, segment_ids=segment_ids,
                            attn_bias=attn_bias, cache_idx=cache_idx, device=q.device)
-        qq, kk, vv = (t if (t.stride(3) == 1 and not any(s % 8 for s in t.stride()[:3])
-                             and t.data_ptr() % 16 == 0) else t.contiguous() for t in (q, k, v))
+        qq, kk, vv = (t if tma_ready(t) else t.contiguous() for t in (q, k, v))
         return A.RingFlashAttention.apply(qq, kk, vv, plan, _symm_ring_for(axis, q.device))
     _warn_fallback(q, _fallback_reason(q, attn_bias))
     return R.RingAttentionRef.apply(q, k, v, attn_bias, segment_ids, cache_idx, axis.comm,

@@ -105,6 +105,7 @@ int check_launch(const char* what) {
 }  // namespace ra
 
 extern "C" const char* ra_last_error() { return ra::g_err; }
+extern "C" int ra_sm_count() { return ra::sm_count(); }
 
 // ---- checked build: sum of the per-translation-unit violation records (see common/bounds.cuh)
 #ifdef RA_BOUNDS_CHECK

@@ -756,3 +756,44 @@ extern "C" int ra_pack_mask(const void* mask, long long sb, long long sh, long l
       static_cast<uint8_t*>(tiles), Hm, Sq, Sk, Wk, Wq);
   return check_launch("pack_mask");
 }
+
+
+// ---------------------------------------------------------------------------------------------------
+// Segment ids of a shard: dst (B, n) <- the shard's positions of src (B, ld): position i lies at off0 + i, from `half` on at
+// off1 + (i - half); mm (B, ceil(n / 128), 2) <- smallest and largest id of each 128 tokens. One warp per tile, one launch where
+// position arithmetic, gathers and reductions in PyTorch took ten for each side of a block.
+namespace ra {
+namespace ew {
+__global__ void __launch_bounds__(128) segment_tiles_kernel(const int* __restrict__ src, long long ld, int off0, int off1, int half,
+                                                            int n, int tiles, int* __restrict__ dst, int* __restrict__ mm) {
+  const int lane = threadIdx.x & 31, t = blockIdx.x * 4 + (threadIdx.x >> 5), b = blockIdx.y;
+  if (t >= tiles) return;
+  int lo = 0x7fffffff, hi = static_cast<int>(0x80000000u);
+#pragma unroll
+  for (int c = 0; c < 4; ++c) {
+    const int i = t * 128 + 32 * c + lane;
+    if (i < n) {
+      const int id = src[b * ld + (i < half ? off0 + i : off1 + (i - half))];
+      lo = min(lo, id);
+      hi = max(hi, id);
+      dst[static_cast<long long>(b) * n + i] = id;
+    }
+  }
+  lo = __reduce_min_sync(0xffffffffu, lo);
+  hi = __reduce_max_sync(0xffffffffu, hi);
+  if (lane == 0) *reinterpret_cast<int2*>(mm + (static_cast<long long>(b) * tiles + t) * 2) = make_int2(lo, hi);
+}
+}  // namespace ew
+}  // namespace ra
+
+extern "C" int ra_segment_tiles(const int* src, long long ld, int off0, int off1, int half, int B, int n, int* dst, int* mm, void* stream) {
+  using namespace ra;
+  if (B < 1 || B > 65535 || n < 1 || off0 < 0 || off1 < 0 || (reinterpret_cast<uintptr_t>(mm) & 7)) {
+    set_error("ra_segment_tiles: bad shape");
+    return kHostBadArg;
+  }
+  const int tiles = (n + 127) / 128;
+  ew::segment_tiles_kernel<<<dim3((tiles + 3) / 4, B), 128, 0, static_cast<cudaStream_t>(stream)>>>(src, ld, off0, off1, half, n, tiles,
+                                                                                                   dst, mm);
+  return check_launch("segment_tiles");
+}

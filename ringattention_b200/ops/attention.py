@@ -67,8 +67,7 @@ def make_plan(rank: int, world: int, B: int, Sq: int, Sk: int, H: int, kw: Block
     seg_q = seg_q_mm = None
     if segment_ids is not None:
         seg32 = segment_ids.to(device=device, dtype=torch.int32)
-        seg_q = seg32.index_select(1, q_pos.tensor(Sq, device)).contiguous()
-        seg_q_mm = flash.seg_tile_minmax(seg_q)
+        seg_q, seg_q_mm = flash.segment_shard(seg32, q_pos, Sq)
     if attn_bias is not None:
         if attn_bias.dim() != 4 or attn_bias.shape[-2] != 1:
             raise NotImplementedError(
@@ -83,10 +82,10 @@ def make_plan(rank: int, world: int, B: int, Sq: int, Sk: int, H: int, kw: Block
         ms = MaskSpec(causal_block_size=cbs, q_pos=q_pos, k_pos=k_pos, seed=seed, pdrop=pdrop)
         if segment_ids is not None:
             ms.seg_q, ms.seg_q_mm = seg_q, seg_q_mm
-            ms.seg_k = seg32.index_select(1, k_pos.tensor(Sk, device)).contiguous()
-            ms.seg_k_mm = flash.seg_tile_minmax(ms.seg_k)
+            same = k_pos == q_pos and Sk == Sq
+            ms.seg_k, ms.seg_k_mm = (seg_q, seg_q_mm) if same else flash.segment_shard(seg32, k_pos, Sk)
         if attn_bias is not None:
-            ms.bias = bias_f.index_select(2, k_pos.tensor(Sk, device)).contiguous()
+            ms.bias = flash.take_positions(bias_f, 2, k_pos, Sk)
         plan.steps.append(RingStep(block=j, mask=ms, needed=_block_needed(q_segs, k_segs, cbs)))
     return plan
 

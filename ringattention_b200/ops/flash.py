@@ -71,6 +71,37 @@ def seg_tile_minmax(seg: torch.Tensor) -> torch.Tensor:
     return torch.stack([t.amin(dim=2), t.amax(dim=2)], dim=2).to(torch.int32).contiguous()
 
 
+def _check_runs(pos: Positions, n: int, total: int) -> None:
+    runs = [(pos.off0, min(n, pos.half))] + ([(pos.off1, n - pos.half)] if n > pos.half else [])
+    if any(off < 0 or off + m > total for off, m in runs):
+        raise IndexError(f"positions {runs} reach past the {total} given ones")
+
+
+def take_positions(x: torch.Tensor, dim: int, pos: Positions, n: int) -> torch.Tensor:
+    """The ``n`` positions of a shard along ``dim`` of a global tensor, as a contiguous copy."""
+    _check_runs(pos, n, x.shape[dim])
+    if n <= pos.half:
+        return x.narrow(dim, pos.off0, n).clone(memory_format=torch.contiguous_format)
+    return torch.cat([x.narrow(dim, pos.off0, pos.half), x.narrow(dim, pos.off1, n - pos.half)], dim=dim).contiguous()
+
+
+def segment_shard(seg: torch.Tensor, pos: Positions, n: int):
+    """``(ids, minmax)`` of a shard's ``n`` positions out of the global int32 ids ``(B, S_total)``: a contiguous copy and
+    what :func:`seg_tile_minmax` gives for it, in one launch (any device but CUDA, and batches past a grid's limit: PyTorch)."""
+    B = seg.shape[0]
+    if not seg.is_cuda or B > 65535:
+        ids = take_positions(seg, 1, pos, n)
+        return ids, seg_tile_minmax(ids)
+    _check_runs(pos, n, seg.shape[1])
+    if seg.stride(1) != 1:
+        seg = seg.contiguous()
+    ids = torch.empty(B, n, device=seg.device, dtype=torch.int32)
+    mm = torch.empty(B, (n + 127) // 128, 2, device=seg.device, dtype=torch.int32)
+    _lib.call("ra_segment_tiles", c_vp(seg.data_ptr()), c_ll(seg.stride(0)), pos.off0, pos.off1, min(pos.half, 1 << 30), B, n,
+              c_vp(ids.data_ptr()), c_vp(mm.data_ptr()), _lib.stream_ptr())
+    return ids, mm
+
+
 class _FwdArgs(ctypes.Structure):
     _fields_ = [
         ("q", c_vp), ("k", c_vp), ("v", c_vp),
@@ -98,10 +129,16 @@ class _FwdArgs(ctypes.Structure):
     ]
 
 
+def tma_ready(t: torch.Tensor) -> bool:
+    """Whether the kernels take a ``(B, S, H, D)`` view as it is: contiguous ``D``, strides and base of whole 16 bytes."""
+    sb, ss, sh, sd = t.stride()
+    return sd == 1 and not (sb | ss | sh) & 7 and not t.data_ptr() & 15
+
+
 def _check_bshd(t: torch.Tensor, name: str) -> None:
     if t.dim() != 4 or t.dtype != torch.bfloat16 or not t.is_cuda or t.stride(3) != 1:
         raise ValueError(f"{name} must be a CUDA bf16 (B, S, H, D) view with contiguous D")
-    if any(s % 8 for s in t.stride()[:3]) or t.data_ptr() % 16:
+    if not tma_ready(t):
         raise ValueError(f"{name}: strides must be multiples of 8 elements and base 16-byte aligned")
 
 
@@ -132,36 +169,30 @@ def pack_mask(mask: torch.Tensor, want_q: bool = True, want_k: bool = True):
     return mask_bitmaps(mask, want_q, want_k)[:2]
 
 
-def _fill_mask(a, mask: MaskSpec, H: int, by_k: bool = False):
+def _mask_fields(mask: MaskSpec, H: int, by_k: bool = False) -> tuple:
+    """The mask's fields of the launch arguments, in their order from ``causal_block_size`` to ``keep_tiles_sh``."""
     keep = mask.keep_k if by_k else mask.keep_q
     if (mask.keep_q is not None or mask.keep_k is not None) and keep is None:
         raise ValueError("the mask bitmap for this pass is missing (pack_mask builds both)")
+    kp = (0, 0, 0, 0, 0, 0, 0)
     if keep is not None:
         assert keep.dtype == torch.int32 and keep.dim() == 4 and keep.is_contiguous()
-        a.keep = keep.data_ptr()
-        a.keep_sb = keep.stride(0)
-        a.keep_sh = keep.stride(1) if keep.shape[1] == H else 0
-        a.keep_sr = keep.stride(2)
+        per_head = keep.shape[1] == H
+        kp = (keep.data_ptr(), keep.stride(0), keep.stride(1) if per_head else 0, keep.stride(2), 0, 0, 0)
         tiles = mask.keep_tiles
         if tiles is not None:
             assert tiles.dtype == torch.uint8 and tiles.is_contiguous() and tiles.shape[:2] == keep.shape[:2]
-            a.keep_tiles, a.keep_tiles_sb, a.keep_tiles_sh = tiles.data_ptr(), tiles.stride(0), tiles.stride(1) if tiles.shape[1] == H else 0
-    a.causal_block_size = int(mask.causal_block_size or 0)
-    a.q_off0, a.q_off1, a.q_half = mask.q_pos.off0, mask.q_pos.off1, mask.q_pos.half
-    a.k_off0, a.k_off1, a.k_half = mask.k_pos.off0, mask.k_pos.off1, mask.k_pos.half
-    a.seg_q, a.seg_k = _ptr(mask.seg_q), _ptr(mask.seg_k)
-    a.seg_q_mm, a.seg_k_mm = _ptr(mask.seg_q_mm), _ptr(mask.seg_k_mm)
+            kp = kp[:4] + (tiles.data_ptr(), tiles.stride(0), tiles.stride(1) if per_head else 0)
+    bias = (0, 0, 0)
     if mask.bias is not None:
-        bias = mask.bias
-        assert bias.dtype == torch.float32 and bias.dim() == 3 and bias.stride(2) == 1
-        a.bias = bias.data_ptr()
-        a.bias_sb = bias.stride(0)
-        a.bias_sh = bias.stride(1) if bias.shape[1] == H else 0
-    a.seed = int(mask.seed) & (2**64 - 1)
-    if mask.pdrop > 0.0:
-        a.drop_threshold = max(1, min(int(mask.pdrop * 4294967296.0), 0xFFFFFFFF))
-    else:
-        a.drop_threshold = 0
+        bm = mask.bias
+        assert bm.dtype == torch.float32 and bm.dim() == 3 and bm.stride(2) == 1
+        bias = (bm.data_ptr(), bm.stride(0), bm.stride(1) if bm.shape[1] == H else 0)
+    drop = max(1, min(int(mask.pdrop * 4294967296.0), 0xFFFFFFFF)) if mask.pdrop > 0.0 else 0
+    qp, kv = mask.q_pos, mask.k_pos
+    return (int(mask.causal_block_size or 0), qp.off0, qp.off1, qp.half, kv.off0, kv.off1, kv.half,
+            _ptr(mask.seg_q), _ptr(mask.seg_k), _ptr(mask.seg_q_mm), _ptr(mask.seg_k_mm), *bias,
+            int(mask.seed) & (2**64 - 1), drop, *kp)
 
 
 def flash_fwd(q, k, v, mask: MaskSpec, *, o_prev=None, lse_prev=None, out_fp32=False,
@@ -179,22 +210,10 @@ def flash_fwd(q, k, v, mask: MaskSpec, *, o_prev=None, lse_prev=None, out_fp32=F
         lse_out = torch.empty(B, H, Sq, device=dev, dtype=torch.float32)
     if o_prev is not None:
         assert o_prev.dtype == torch.float32 and o_prev.is_contiguous() and lse_prev is not None
-    a = _FwdArgs()
-    a.q, a.k, a.v = q.data_ptr(), k.data_ptr(), v.data_ptr()
-    a.q_sb, a.q_ss, a.q_sh = q.stride(0), q.stride(1), q.stride(2)
-    a.k_sb, a.k_ss, a.k_sh = k.stride(0), k.stride(1), k.stride(2)
-    a.v_sb, a.v_ss, a.v_sh = v.stride(0), v.stride(1), v.stride(2)
-    a.out = out.data_ptr()
-    a.o_sb, a.o_ss, a.o_sh = out.stride(0), out.stride(1), out.stride(2)
-    a.out_fp32 = 1 if out.dtype == torch.float32 else 0
-    a.lse_out = lse_out.data_ptr()
-    a.o_prev, a.lse_prev = _ptr(o_prev), _ptr(lse_prev)
-    a.B, a.H, a.Sq, a.Sk, a.D = B, H, Sq, Sk, D
-    a.softmax_scale = 1.0 / math.sqrt(D)
-    _fill_mask(a, mask, H)
-    a.copy_src, a.copy_dst, a.copy_bytes, a.copy_ctas = copy_src, copy_dst, copy_bytes, copy_ctas
-    a.status = _lib.status_tensor(dev).data_ptr()
-    a.stream = torch.cuda.current_stream().cuda_stream
+    a = _FwdArgs(q.data_ptr(), k.data_ptr(), v.data_ptr(), *q.stride()[:3], *k.stride()[:3], *v.stride()[:3],
+                 out.data_ptr(), *out.stride()[:3], int(out.dtype == torch.float32), lse_out.data_ptr(),
+                 _ptr(o_prev), _ptr(lse_prev), B, H, Sq, Sk, D, 1.0 / math.sqrt(D), *_mask_fields(mask, H),
+                 copy_src, copy_dst, copy_bytes, copy_ctas, _lib.status_tensor(dev).data_ptr(), _lib.stream_handle(), 0, 0)
     splits = _lib.lib().ra_attn_fwd_splits(ctypes.byref(a))
     if splits > 1:  # few query tiles: the keys are split over several CTAs, partial results meet in a second launch
         ws = torch.empty(splits * B * Sq * H * (D + 1), device=dev, dtype=torch.float32)
@@ -272,23 +291,10 @@ def flash_bwd(q, k, v, dout, lse2, delta, mask: MaskSpec, dq_acc, dk, dv, dkv_mo
     assert dk.shape == k.shape and dv.shape == k.shape and dk.stride() == dv.stride()
     want = torch.bfloat16 if dkv_mode == DKV_STORE_BF16 else torch.float32
     assert dk.dtype == want and dv.dtype == want and dk.stride(3) == 1
-    a = _BwdArgs()
-    a.q, a.k, a.v, a.d_o = q.data_ptr(), k.data_ptr(), v.data_ptr(), dout.data_ptr()
-    a.q_sb, a.q_ss, a.q_sh = q.stride(0), q.stride(1), q.stride(2)
-    a.k_sb, a.k_ss, a.k_sh = k.stride(0), k.stride(1), k.stride(2)
-    a.v_sb, a.v_ss, a.v_sh = v.stride(0), v.stride(1), v.stride(2)
-    a.do_sb, a.do_ss, a.do_sh = dout.stride(0), dout.stride(1), dout.stride(2)
-    a.lse2, a.delta, a.Sq_pad = lse2.data_ptr(), delta.data_ptr(), lse2.shape[2]
-    a.dq_acc = dq_acc.data_ptr()
-    a.dk, a.dv = dk.data_ptr(), dv.data_ptr()
-    a.dkv_sb, a.dkv_ss, a.dkv_sh = dk.stride(0), dk.stride(1), dk.stride(2)
-    a.dkv_mode = dkv_mode
-    a.B, a.H, a.Sq, a.Sk, a.D = B, H, Sq, Sk, D
-    a.softmax_scale = 1.0 / math.sqrt(D)
-    _fill_mask(a, mask, H, by_k=True)
-    a.copy_src, a.copy_dst, a.copy_bytes, a.copy_ctas = copy_src, copy_dst, copy_bytes, copy_ctas
-    a.status = _lib.status_tensor(dev).data_ptr()
-    a.stream = torch.cuda.current_stream().cuda_stream
     tb = BWD_TRACE_BUFFERS.get(dev.index if dev.index is not None else torch.cuda.current_device())
-    a.trace = 0 if tb is None else tb.data_ptr()
+    a = _BwdArgs(q.data_ptr(), k.data_ptr(), v.data_ptr(), dout.data_ptr(), *q.stride()[:3], *k.stride()[:3],
+                 *v.stride()[:3], *dout.stride()[:3], lse2.data_ptr(), delta.data_ptr(), lse2.shape[2],
+                 dq_acc.data_ptr(), dk.data_ptr(), dv.data_ptr(), *dk.stride()[:3], dkv_mode, B, H, Sq, Sk, D,
+                 1.0 / math.sqrt(D), *_mask_fields(mask, H, by_k=True), copy_src, copy_dst, copy_bytes, copy_ctas,
+                 _lib.status_tensor(dev).data_ptr(), _lib.stream_handle(), 0 if tb is None else tb.data_ptr())
     _lib.call("ra_attn_bwd", ctypes.byref(a))

@@ -124,8 +124,5 @@ def ring_inference_attention(q, k, v, attn_mask, axis, symm_ring=None):
     S_loc = k.shape[1]
     m = _local_mask(attn_mask, axis.rank, S_loc, B, H, ql)
 
-    def ok(t):
-        return t.stride(3) == 1 and not any(s % 8 for s in t.stride()[:3]) and t.data_ptr() % 16 == 0
-
-    qq, kk, vv = (t if ok(t) else t.contiguous() for t in (q, k, v))
+    qq, kk, vv = (t if flash.tma_ready(t) else t.contiguous() for t in (q, k, v))
     return RingInferenceAttention.apply(qq, kk, vv, m, axis, symm_ring, need_grad)

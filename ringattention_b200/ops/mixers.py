@@ -198,7 +198,7 @@ def two_part_attention(q, k1, k2, v, out, *, scale: float, q_pos0: int, sink=Non
     a.B, a.H, a.Sq, a.Sk = B, H, Sq, k1.shape[1]
     a.d1, a.d2, a.dv = k1.shape[3], k2.shape[2], v.shape[3]
     a.scale, a.q_pos0 = scale, q_pos0
-    a.status, a.stream = _lib.status_tensor(q.device).data_ptr(), torch.cuda.current_stream().cuda_stream
+    a.status, a.stream = _lib.status_tensor(q.device).data_ptr(), _lib.stream_handle()
     _lib.call("ra_attn_two_part", ctypes.byref(a))
 
 
@@ -254,7 +254,7 @@ def window_attention(q, k_ring, v_ring, out, *, scale: float, q_pos0: int, windo
     a.out, (a.o_sb, a.o_ss, a.o_sh) = _p(out), out.stride()[:3]
     a.sink, a.B, a.H, a.G, a.Sq, a.dk, a.dv = _p(sink), B, H, k_ring.shape[1], Sq, dk, v_ring.shape[3]
     a.window, a.k_rows, a.scale, a.q_pos0 = window, k_ring.shape[2], scale, q_pos0
-    a.status, a.stream = _lib.status_tensor(q.device).data_ptr(), torch.cuda.current_stream().cuda_stream
+    a.status, a.stream = _lib.status_tensor(q.device).data_ptr(), _lib.stream_handle()
     _lib.call("ra_attn_window", ctypes.byref(a))
 
 

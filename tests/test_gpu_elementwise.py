@@ -143,3 +143,21 @@ def test_rmsnorm_gain_gradient_at_odd_widths_and_few_rows(rows, d):
     K.rmsnorm_bwd(dy, x, w, rstd, dw)
     terms = dy.double() * x.double() * rstd.double()[:, None]
     assert ((dw.double() - (start.double() + terms.sum(0))).abs() <= 1e-6 * (start.double().abs() + terms.abs().sum(0))).all()
+
+
+@pytest.mark.parametrize("B,total,n,pos", [(1, 1, 1, (0,)), (2, 700, 700, (0,)), (3, 1000, 129, (871,)), (1, 4096, 512, (256, 3328, 256)), (2, 2048, 1024, (512, 0, 512))])
+@pytest.mark.parametrize("strided", [False, True])
+def test_segment_shards(B, total, n, pos, strided):
+    """Ids of one run and of two, at ragged lengths, out of a view: equal to gathering and reducing in PyTorch."""
+    from ringattention_b200.ops import flash
+
+    g = torch.Generator(device="cuda").manual_seed(total)
+    ids = torch.randint(-5, 2**31 - 1, (B, total + 3), device="cuda", generator=g, dtype=torch.int32)
+    ids = ids[:, 3:] if strided else ids[:, 3:].contiguous()
+    p = flash.Positions(*pos)
+    got, mm = flash.segment_shard(ids, p, n)
+    want = ids.index_select(1, p.tensor(n, "cuda"))
+    assert torch.equal(got, want) and torch.equal(mm, flash.seg_tile_minmax(want)) and got.data_ptr() != ids.data_ptr()
+    assert torch.equal(flash.take_positions(ids[:, None].float(), 2, p, n), want[:, None].float())
+    with pytest.raises(IndexError):
+        flash.segment_shard(ids, flash.Positions(total - n + 1), n)
