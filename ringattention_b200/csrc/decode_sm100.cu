@@ -84,6 +84,29 @@ __device__ __forceinline__ uint4 pack8(const float* f) {
 
 constexpr int DEC_UNROLL = 4;  // cache rows per thread and loop trip
 
+// Which rows [r0, r1) of a CTA's range some query row attends to under the mask, as bits in shared memory, so that
+// rows nobody sees are not loaded: a batch of unequal lengths otherwise streams its padding too (eight rows of the batch, half to
+// all of 4000 cached rows each, 32 heads: 98 us where the visible rows take 75). Ranges too long for the bits (`seen` past the end)
+// count as seen. Returns whether any row is; call with all threads of the CTA.
+constexpr int SEEN_ROWS = 8192;
+__device__ __forceinline__ bool mark_seen(uint32_t* seen, const uint8_t* mask, long long m_sq, int QL, int r0, int r1) {
+  const int n = r1 - r0;
+  if (n > SEEN_ROWS) return true;
+  bool any = false;
+  for (int t = threadIdx.x; t < ((n + 31) & ~31); t += THREADS) {  // a warp's 32 rows are one word: uniform trip count
+    bool on = false;
+    if (t < n)
+      for (int i = 0; i < QL; ++i) on |= mask[i * m_sq + r0 + t] != 0;
+    const uint32_t bits = __ballot_sync(0xffffffffu, on);
+    if ((threadIdx.x & 31) == 0) seen[t >> 5] = bits;
+    any |= bits != 0;
+  }
+  return __syncthreads_or(any) != 0;
+}
+__device__ __forceinline__ bool row_seen(const uint32_t* seen, int r, int r0, int r1) {
+  return r1 - r0 > SEEN_ROWS || ((seen[(r - r0) >> 5] >> ((r - r0) & 31)) & 1u);
+}
+
 // D = head dim (64 or 128), QL = query rows held per CTA, ST = stages of the asynchronous-copy ring (0: the rows
 // of a trip are loaded straight into registers). With ST > 0 every thread copies the rows of trip i + ST - 1 into
 // its own shared-memory slots (cp.async, no registers held while the data is in flight) before it works on trip
@@ -132,10 +155,13 @@ __global__ void __launch_bounds__(THREADS) decode_splitkv_kernel(const SplitPara
     if (rows_per_split < 1) rows_per_split = 1;
   }
   const int r0 = split * rows_per_split;
-  const int r1 = min(S, r0 + rows_per_split);
+  int r1 = min(S, r0 + rows_per_split);
   const __nv_bfloat16* kb = p.k + b * p.k_sb + h * p.k_sh + dl * 8;
   const __nv_bfloat16* vb = p.v + b * p.v_sb + h * p.v_sh + dl * 8;
   const int step = WARPS * RPW;
+  __shared__ uint32_t seen[SEEN_ROWS / 32];
+  const uint8_t* mask = p.mask ? p.mask + b * p.m_sb + h * p.m_sh : nullptr;
+  if (mask && r0 < r1 && !mark_seen(seen, mask, p.m_sq, QL, r0, r1)) r1 = r0;  // nothing to see here
 
   // The trip count is the same for every lane of a warp (the loop variable ignores `sub`), so the
   // full-mask shuffles below always see all 32 lanes; rows past the end are merely masked out.
@@ -144,7 +170,7 @@ __global__ void __launch_bounds__(THREADS) decode_splitkv_kernel(const SplitPara
 #pragma unroll
     for (int u = 0; u < UNROLL; ++u) {
       const int r = base_w + sub + u * step;
-      const bool in = r < r1;
+      const bool in = r < r1 && (!mask || row_seen(seen, r, r0, r1));
       const long long rr = in ? r : r0;  // r0 < r1 whenever the loop runs: a valid address, never read when !in
       uint4* dst = stage_buf + ((slot * UNROLL + u) * 2) * THREADS + threadIdx.x;
       cp_async16(dst, kb + rr * p.k_ss, in ? 16 : 0);
@@ -173,7 +199,7 @@ __global__ void __launch_bounds__(THREADS) decode_splitkv_kernel(const SplitPara
       cp_async_wait<(ST > 0 ? ST - 1 : 0)>();  // all but the newest ST - 1 groups are complete: this trip's rows are in
 #pragma unroll
       for (int u = 0; u < UNROLL; ++u) {
-        ok[u] = base + u * step < r1;
+        ok[u] = base + u * step < r1 && (!mask || row_seen(seen, base + u * step, r0, r1));
         const uint4* src = stage_buf + ((slot_out * UNROLL + u) * 2) * THREADS + threadIdx.x;
         ku[u] = src[0];
         vu[u] = src[THREADS];
@@ -183,7 +209,7 @@ __global__ void __launch_bounds__(THREADS) decode_splitkv_kernel(const SplitPara
 #pragma unroll
       for (int u = 0; u < UNROLL; ++u) {
         const int r = base + u * step;
-        ok[u] = r < r1;
+        ok[u] = r < r1 && (!mask || row_seen(seen, r, r0, r1));
         if (ok[u]) {
           ku[u] = *reinterpret_cast<const uint4*>(kb + static_cast<long long>(r) * p.k_ss);
           vu[u] = *reinterpret_cast<const uint4*>(vb + static_cast<long long>(r) * p.v_ss);
@@ -208,8 +234,7 @@ __global__ void __launch_bounds__(THREADS) decode_splitkv_kernel(const SplitPara
         for (int o = LPR / 2; o > 0; o >>= 1) d += __shfl_xor_sync(0xffffffffu, d, o);
         bool vis = ok[u];
         if (q_pos0 >= 0) vis = vis && (p.k_pos0 + r <= q_pos0 + i);
-        if (p.mask && vis)
-          vis = p.mask[b * p.m_sb + h * p.m_sh + i * p.m_sq + r] != 0;
+        if (mask && vis && (QL > 1 || r1 - r0 > SEEN_ROWS)) vis = mask[i * p.m_sq + r] != 0;
         s[u][i] = vis ? d : -INFINITY;
       }
     }
@@ -327,7 +352,10 @@ __global__ void __launch_bounds__(THREADS) decode_splitkv_mma_kernel(const Split
     if (rows_per_split < 1) rows_per_split = 1;
   }
   const int r0 = split * rows_per_split;
-  const int r1 = min(S, r0 + rows_per_split);
+  int r1 = min(S, r0 + rows_per_split);
+  __shared__ uint32_t seen[SEEN_ROWS / 32];
+  const uint8_t* mask = p.mask ? p.mask + b * p.m_sb + h * p.m_sh : nullptr;
+  if (mask && r0 < r1 && !mark_seen(seen, mask, p.m_sq, QL, r0, r1)) r1 = r0;  // nothing to see here
   const __nv_bfloat16* kb = p.k + b * p.k_sb + h * p.k_sh;
   const __nv_bfloat16* vb = p.v + b * p.v_sb + h * p.v_sh;
 
@@ -358,7 +386,7 @@ __global__ void __launch_bounds__(THREADS) decode_splitkv_mma_kernel(const Split
       const int piece = lane + 32 * j;
       const int row = piece / PPR, ch = piece % PPR;
       const int r = base + row;
-      const bool in = r < r1;
+      const bool in = r < r1 && (!mask || row_seen(seen, r, r0, r1));
       const long long rr = in ? r : r0;  // a valid address; not read when !in (the piece is zero-filled)
       const int off = row * RB + ((ch ^ (row & 7)) << 4);
       cp_async16(kt + off, kb + rr * p.k_ss + ch * 8, in ? 16 : 0);
@@ -411,7 +439,7 @@ __global__ void __launch_bounds__(THREADS) decode_splitkv_mma_kernel(const Split
         const int r = base + 8 * nt + 2 * t + e;
         bool vis = r < r1 && g < QL;
         if (q_pos0 >= 0) vis = vis && (p.k_pos0 + r <= q_pos0 + g);
-        if (p.mask && vis) vis = p.mask[b * p.m_sb + h * p.m_sh + g * p.m_sq + r] != 0;
+        if (mask && vis) vis = mask[g * p.m_sq + r] != 0;
         x[nt][e] = vis ? s[nt][e] * p.scale_log2 : -INFINITY;
         mx = fmaxf(mx, x[nt][e]);
       }

@@ -66,7 +66,7 @@ def default_splits(S: int, B: int, H: int, mma: bool = False) -> int:
     ring 64 to 512 splits are within 3 % of each other (6.83 to 7.02 TB/s). At least 512 cache rows per CTA.
     The tensor-core kernel (``mma``) has two CTAs of four warps per SM and likes half as many, longer ranges: four
     query rows, 128 / 256 / 512 splits: 0.315 / 0.332 / 0.408 ms."""
-    sms = torch.cuda.get_device_properties(torch.cuda.current_device()).multi_processor_count
+    sms = _lib.lib().ra_sm_count()
     per_sm, rows = (32, 1024) if mma else (64, 512)
     want = max(1, (per_sm * sms) // max(1, B * H))
     return max(1, min(want, (S + rows - 1) // rows, 512))
@@ -100,7 +100,7 @@ def decode_partial(q, k, v, *, n_valid: Optional[int] = None, q_pos0: int = -1, 
     a.pos_ptr = pos_ptr
     # striped cache (with pos_ptr): (ranks, rank, prefilled rows per rank, prefilled positions)
     a.stripe_n, a.stripe_rank, a.stripe_base, a.stripe_len0 = stripe if stripe is not None else (0, 0, 0, 0)
-    a.stream = torch.cuda.current_stream().cuda_stream
+    a.stream = _lib.stream_handle()
     a.stages = STAGES
     a.mma = int(QL >= MMA_MIN_ROWS)
     _lib.call("ra_decode_splitkv", ctypes.byref(a))
@@ -178,7 +178,9 @@ def ring_decode_attention(q, k, v, attn_mask, axis, symm_ring=None, *, n_valid: 
         if m.shape[2] not in (1, QL):
             pad = torch.zeros(*m.shape[:2], QL - m.shape[2], m.shape[3], dtype=m.dtype, device=m.device)
             m = torch.cat([m, pad], dim=2)
-        mask_u8 = m.to(torch.uint8).contiguous()
+        mask_u8 = m.view(torch.uint8) if m.dtype == torch.bool else m.to(torch.uint8)  # a bool is a byte of 0 or 1
+        if mask_u8.stride(3) != 1:
+            mask_u8 = mask_u8.contiguous()
     if k_pos0 is None:
         k_pos0 = rank * S_loc
     pos_ptr = 0 if state is None else state.data_ptr()

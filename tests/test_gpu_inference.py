@@ -426,3 +426,41 @@ def test_masked_prompt_chunks(B, ql, S, H, D, kind, need_grad):
         got = torch.autograd.grad(out, (q, k, v), dout)
         for a, b in zip(got, torch.autograd.grad(want, (qd, kd, vd), dout.double())):
             assert (a.double() - b).abs().max() <= 0.02 * b.abs().max() + 1e-3
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("ql", [1, 2, 5, 8])
+@pytest.mark.parametrize("S,kind", [(37, "valid"), (700, "valid"), (5000, "valid"), (9000, "holes"), (300000, "valid"), (513, "per row"), (1000, "nothing")])
+def test_decode_skips_rows_nobody_sees(S, kind, ql, D):
+    """Cached rows that the mask hides from all query rows hold infinities: they are not read. Ranges longer and shorter than
+    the bits a CTA keeps, masks by query row and head, a batch row that sees nothing. bf16 in and out: 1e-2 of the largest entry."""
+    import ringattention_b200 as rab
+
+    B, H = (2, 3) if S < 100000 else (16, 8)
+    if S >= 100000 and (D, ql) not in ((64, 1), (64, 2)):
+        pytest.skip("the long range once for each kernel")
+    if S >= 100000:
+        S = 40000  # 16 x 8 (row, head) pairs: ranges of more than 8192 rows
+    g = torch.Generator(device="cuda").manual_seed(S + ql)
+    q = torch.randn(B, ql, H, D, device="cuda", generator=g).bfloat16()
+    k, v = (torch.randn(B, S, H, D, device="cuda", generator=g).bfloat16() for _ in range(2))
+    at = torch.arange(S, device="cuda")
+    if kind == "valid":
+        mask = (at[None] < torch.randint(S // 2, S, (B, 1), device="cuda", generator=g))[:, None, None]
+    elif kind == "holes":
+        mask = (torch.rand(B, 1, 1, S, device="cuda", generator=g) < 0.3) & (at < 4000)
+    elif kind == "per row":
+        mask = torch.rand(1, H, ql, S, device="cuda", generator=g) < 0.05
+    else:
+        mask = torch.ones(B, 1, 1, S, dtype=torch.bool, device="cuda")
+        mask[1] = False
+    seen = mask.any(2).any(1)  # (B|1, S)
+    x = (torch.einsum("bqhd,bkhd->bhqk", q.double(), k.double()) / D ** 0.5).masked_fill(~mask, -float("inf"))
+    e = torch.exp(x - x.amax(-1, keepdim=True).clamp_min(-1e300))
+    want = torch.einsum("bhqk,bkhd->bqhd", e / e.sum(-1, keepdim=True).clamp_min(1e-300), v.double())
+    if kind != "per row":  # rows that some other head sees are read there
+        hidden = (~seen).expand(B, S)
+        k[hidden], v[hidden] = float("inf"), float("nan")
+    with torch.no_grad():
+        out = rab.ringattention_inference(q, k, v, mask)
+    assert (out.double() - want).abs().max() <= 0.01 * want.abs().max() + 1e-3
