@@ -84,27 +84,74 @@ __device__ __forceinline__ uint4 pack8(const float* f) {
 
 constexpr int DEC_UNROLL = 4;  // cache rows per thread and loop trip
 
-// Which rows [r0, r1) of a CTA's range some query row attends to under the mask, as bits in shared memory, so that
-// rows nobody sees are not loaded: a batch of unequal lengths otherwise streams its padding too (eight rows of the batch, half to
-// all of 4000 cached rows each, 32 heads: 98 us where the visible rows take 75). Ranges too long for the bits (`seen` past the end)
-// count as seen. Returns whether any row is; call with all threads of the CTA.
-constexpr int SEEN_ROWS = 8192;
+// Which rows [r0, r1) of a CTA's range each query row attends to under the mask, as bits in shared memory (seen[i][r - r0] of
+// query row i, and of any of them behind the last), so that rows nobody sees are not loaded and the loop over the rows asks no
+// global memory: a batch of unequal lengths otherwise streams its padding too (eight rows of the batch, half to all of 4000 cached
+// rows each, 32 heads: 98 us where the visible rows take 75). Ranges too long for the bits count as seen. Returns whether
+// any row is; call with all threads of the CTA. The bits share the space of the CTA's partial results: a KB more of shared memory
+// would leave one CTA of the tensor-core kernel per SM instead of two (65536 rows, four query rows, 32 heads: 283 instead of 190 us).
+constexpr int SEEN_ROWS = 4096, SEEN_WORDS = SEEN_ROWS / 32;
+template <int MAXQ>
 __device__ __forceinline__ bool mark_seen(uint32_t* seen, const uint8_t* mask, long long m_sq, int QL, int r0, int r1) {
   const int n = r1 - r0;
   if (n > SEEN_ROWS) return true;
   bool any = false;
-  for (int t = threadIdx.x; t < ((n + 31) & ~31); t += THREADS) {  // a warp's 32 rows are one word: uniform trip count
-    bool on = false;
-    if (t < n)
-      for (int i = 0; i < QL; ++i) on |= mask[i * m_sq + r0 + t] != 0;
-    const uint32_t bits = __ballot_sync(0xffffffffu, on);
-    if ((threadIdx.x & 31) == 0) seen[t >> 5] = bits;
-    any |= bits != 0;
+  const uint8_t* m = mask + r0;
+  if (((reinterpret_cast<uintptr_t>(m) | static_cast<uintptr_t>(m_sq)) & 3) == 0) {
+    // four rows a thread and load, a word of bits from eight threads (uniform trip count)
+    for (int t = threadIdx.x * 4; t < ((n + 127) & ~127); t += THREADS * 4) {
+      uint32_t v[MAXQ];
+#pragma unroll
+      for (int i = 0; i < MAXQ; ++i) {
+        v[i] = 0u;
+        if (i < QL && t + 4 <= n) {
+          v[i] = *reinterpret_cast<const uint32_t*>(m + i * m_sq + t);
+        } else if (i < QL) {
+          for (int e = 0; t + e < n; ++e) v[i] |= static_cast<uint32_t>(m[i * m_sq + t + e]) << (8 * e);
+        }
+      }
+      uint32_t all = 0u;
+#pragma unroll
+      for (int i = 0; i < MAXQ; ++i) {
+        if (i >= QL) break;
+        uint32_t bits = 0u;
+#pragma unroll
+        for (int e = 0; e < 4; ++e) bits |= ((v[i] >> (8 * e)) & 0xffu) ? 1u << e : 0u;
+        bits <<= 4 * (threadIdx.x & 7);
+#pragma unroll
+        for (int o = 1; o < 8; o <<= 1) bits |= __shfl_xor_sync(0xffffffffu, bits, o);
+        if ((threadIdx.x & 7) == 0) seen[i * SEEN_WORDS + (t >> 5)] = bits;
+        all |= bits;
+      }
+      if (MAXQ > 1 && (threadIdx.x & 7) == 0) seen[QL * SEEN_WORDS + (t >> 5)] = all;
+      any |= all != 0;
+    }
+  } else {
+    for (int t = threadIdx.x; t < ((n + 31) & ~31); t += THREADS) {  // a warp's 32 rows are one word
+      bool on[MAXQ];
+#pragma unroll
+      for (int i = 0; i < MAXQ; ++i) on[i] = i < QL && t < n && m[i * m_sq + t] != 0;
+      uint32_t all = 0u;
+#pragma unroll
+      for (int i = 0; i < MAXQ; ++i) {
+        if (i >= QL) break;
+        const uint32_t bits = __ballot_sync(0xffffffffu, on[i]);
+        if ((threadIdx.x & 31) == 0) seen[i * SEEN_WORDS + (t >> 5)] = bits;
+        all |= bits;
+      }
+      if (MAXQ > 1 && (threadIdx.x & 31) == 0) seen[QL * SEEN_WORDS + (t >> 5)] = all;
+      any |= all != 0;
+    }
   }
   return __syncthreads_or(any) != 0;
 }
 __device__ __forceinline__ bool row_seen(const uint32_t* seen, int r, int r0, int r1) {
   return r1 - r0 > SEEN_ROWS || ((seen[(r - r0) >> 5] >> ((r - r0) & 31)) & 1u);
+}
+// query row i sees cache row r
+__device__ __forceinline__ bool pair_seen(const uint32_t* seen, const uint8_t* mask, long long m_sq, int i, int r, int r0, int r1) {
+  if (r1 - r0 > SEEN_ROWS) return mask[i * m_sq + r] != 0;
+  return (seen[i * SEEN_WORDS + ((r - r0) >> 5)] >> ((r - r0) & 31)) & 1u;
 }
 
 // D = head dim (64 or 128), QL = query rows held per CTA, ST = stages of the asynchronous-copy ring (0: the rows
@@ -159,9 +206,13 @@ __global__ void __launch_bounds__(THREADS) decode_splitkv_kernel(const SplitPara
   const __nv_bfloat16* kb = p.k + b * p.k_sb + h * p.k_sh + dl * 8;
   const __nv_bfloat16* vb = p.v + b * p.v_sb + h * p.v_sh + dl * 8;
   const int step = WARPS * RPW;
-  __shared__ uint32_t seen[SEEN_ROWS / 32];
+  __shared__ float sm_m[WARPS][QL], sm_l[WARPS][QL];
+  __shared__ float sm_o[WARPS][QL][D];
+  uint32_t* const seen = reinterpret_cast<uint32_t*>(&sm_o[0][0][0]);
+  static_assert((QL > 1 ? QL + 1 : 1) * SEEN_WORDS * 4 <= static_cast<int>(sizeof(sm_o)), "bits of the mask do not fit");
+  const uint32_t* const seen_any = seen + (QL > 1 ? QL : 0) * SEEN_WORDS;
   const uint8_t* mask = p.mask ? p.mask + b * p.m_sb + h * p.m_sh : nullptr;
-  if (mask && r0 < r1 && !mark_seen(seen, mask, p.m_sq, QL, r0, r1)) r1 = r0;  // nothing to see here
+  if (mask && r0 < r1 && !mark_seen<QL>(seen, mask, p.m_sq, QL, r0, r1)) r1 = r0;  // nothing to see here
 
   // The trip count is the same for every lane of a warp (the loop variable ignores `sub`), so the
   // full-mask shuffles below always see all 32 lanes; rows past the end are merely masked out.
@@ -170,7 +221,7 @@ __global__ void __launch_bounds__(THREADS) decode_splitkv_kernel(const SplitPara
 #pragma unroll
     for (int u = 0; u < UNROLL; ++u) {
       const int r = base_w + sub + u * step;
-      const bool in = r < r1 && (!mask || row_seen(seen, r, r0, r1));
+      const bool in = r < r1 && (!mask || row_seen(seen_any, r, r0, r1));
       const long long rr = in ? r : r0;  // r0 < r1 whenever the loop runs: a valid address, never read when !in
       uint4* dst = stage_buf + ((slot * UNROLL + u) * 2) * THREADS + threadIdx.x;
       cp_async16(dst, kb + rr * p.k_ss, in ? 16 : 0);
@@ -199,7 +250,7 @@ __global__ void __launch_bounds__(THREADS) decode_splitkv_kernel(const SplitPara
       cp_async_wait<(ST > 0 ? ST - 1 : 0)>();  // all but the newest ST - 1 groups are complete: this trip's rows are in
 #pragma unroll
       for (int u = 0; u < UNROLL; ++u) {
-        ok[u] = base + u * step < r1 && (!mask || row_seen(seen, base + u * step, r0, r1));
+        ok[u] = base + u * step < r1 && (!mask || row_seen(seen_any, base + u * step, r0, r1));
         const uint4* src = stage_buf + ((slot_out * UNROLL + u) * 2) * THREADS + threadIdx.x;
         ku[u] = src[0];
         vu[u] = src[THREADS];
@@ -209,7 +260,7 @@ __global__ void __launch_bounds__(THREADS) decode_splitkv_kernel(const SplitPara
 #pragma unroll
       for (int u = 0; u < UNROLL; ++u) {
         const int r = base + u * step;
-        ok[u] = r < r1 && (!mask || row_seen(seen, r, r0, r1));
+        ok[u] = r < r1 && (!mask || row_seen(seen_any, r, r0, r1));
         if (ok[u]) {
           ku[u] = *reinterpret_cast<const uint4*>(kb + static_cast<long long>(r) * p.k_ss);
           vu[u] = *reinterpret_cast<const uint4*>(vb + static_cast<long long>(r) * p.v_ss);
@@ -234,7 +285,7 @@ __global__ void __launch_bounds__(THREADS) decode_splitkv_kernel(const SplitPara
         for (int o = LPR / 2; o > 0; o >>= 1) d += __shfl_xor_sync(0xffffffffu, d, o);
         bool vis = ok[u];
         if (q_pos0 >= 0) vis = vis && (p.k_pos0 + r <= q_pos0 + i);
-        if (mask && vis && (QL > 1 || r1 - r0 > SEEN_ROWS)) vis = mask[i * p.m_sq + r] != 0;
+        if (mask && vis && (QL > 1 || r1 - r0 > SEEN_ROWS)) vis = pair_seen(seen, mask, p.m_sq, i, r, r0, r1);
         s[u][i] = vis ? d : -INFINITY;
       }
     }
@@ -262,9 +313,8 @@ __global__ void __launch_bounds__(THREADS) decode_splitkv_kernel(const SplitPara
   }
 
   if (ST > 0) cp_async_wait<0>();  // only empty groups can be left; nothing is in flight when the CTA ends
+  if (mask) __syncthreads();        // the bits of the mask give way to the partial results
   // ---- combine the row groups of a warp, then the warps of the CTA
-  __shared__ float sm_m[WARPS][QL], sm_l[WARPS][QL];
-  __shared__ float sm_o[WARPS][QL][D];
 #pragma unroll
   for (int i = 0; i < QL; ++i) {
 #pragma unroll
@@ -353,9 +403,13 @@ __global__ void __launch_bounds__(THREADS) decode_splitkv_mma_kernel(const Split
   }
   const int r0 = split * rows_per_split;
   int r1 = min(S, r0 + rows_per_split);
-  __shared__ uint32_t seen[SEEN_ROWS / 32];
+  __shared__ float sm_m[WARPS][8], sm_l[WARPS][8];
+  __shared__ float sm_o[WARPS][8][D];
+  uint32_t* const seen = reinterpret_cast<uint32_t*>(&sm_o[0][0][0]);
+  static_assert(9 * SEEN_WORDS * 4 <= static_cast<int>(sizeof(sm_o)), "bits of the mask do not fit");
+  const uint32_t* const seen_any = seen + QL * SEEN_WORDS;
   const uint8_t* mask = p.mask ? p.mask + b * p.m_sb + h * p.m_sh : nullptr;
-  if (mask && r0 < r1 && !mark_seen(seen, mask, p.m_sq, QL, r0, r1)) r1 = r0;  // nothing to see here
+  if (mask && r0 < r1 && !mark_seen<8>(seen, mask, p.m_sq, QL, r0, r1)) r1 = r0;  // nothing to see here
   const __nv_bfloat16* kb = p.k + b * p.k_sb + h * p.k_sh;
   const __nv_bfloat16* vb = p.v + b * p.v_sb + h * p.v_sh;
 
@@ -386,7 +440,7 @@ __global__ void __launch_bounds__(THREADS) decode_splitkv_mma_kernel(const Split
       const int piece = lane + 32 * j;
       const int row = piece / PPR, ch = piece % PPR;
       const int r = base + row;
-      const bool in = r < r1 && (!mask || row_seen(seen, r, r0, r1));
+      const bool in = r < r1 && (!mask || row_seen(seen_any, r, r0, r1));
       const long long rr = in ? r : r0;  // a valid address; not read when !in (the piece is zero-filled)
       const int off = row * RB + ((ch ^ (row & 7)) << 4);
       cp_async16(kt + off, kb + rr * p.k_ss + ch * 8, in ? 16 : 0);
@@ -439,7 +493,7 @@ __global__ void __launch_bounds__(THREADS) decode_splitkv_mma_kernel(const Split
         const int r = base + 8 * nt + 2 * t + e;
         bool vis = r < r1 && g < QL;
         if (q_pos0 >= 0) vis = vis && (p.k_pos0 + r <= q_pos0 + g);
-        if (mask && vis) vis = mask[g * p.m_sq + r] != 0;
+        if (mask && vis) vis = pair_seen(seen, mask, p.m_sq, g, r, r0, r1);
         x[nt][e] = vis ? s[nt][e] * p.scale_log2 : -INFINITY;
         mx = fmaxf(mx, x[nt][e]);
       }
@@ -487,8 +541,7 @@ __global__ void __launch_bounds__(THREADS) decode_splitkv_mma_kernel(const Split
   // ---- the row sum over the four lanes of a row, then the warps of the CTA (as in the kernel above)
   l += __shfl_xor_sync(0xffffffffu, l, 1);
   l += __shfl_xor_sync(0xffffffffu, l, 2);
-  __shared__ float sm_m[WARPS][8], sm_l[WARPS][8];
-  __shared__ float sm_o[WARPS][8][D];
+  if (mask) __syncthreads();  // the bits of the mask give way to the partial results
   if (t == 0) {
     sm_m[warp][g] = m;
     sm_l[warp][g] = l;
@@ -563,6 +616,7 @@ __device__ __forceinline__ void merge_parts(const float* o_row, long long o_ps, 
 // Valid in the threads of warp 0 (lane = column).
 constexpr int MERGE_WARPS = 32;
 constexpr int MERGE_MANY = 16;     // fewer partials: less than one for every second warp, and prefills have many rows of 2-8
+constexpr int MERGE_SOME = 4;      // from here on if all CTAs run at once (16 rows of 15 partials of a decode step: 3 us less)
 constexpr int MERGE_LSE = 1024;    // weights kept in shared memory
 __device__ __forceinline__ void merge_parts_wide(const float* o_col, long long o_ps, const float* lp, long long l_ps,
                                                  int nparts, float& o, float& lse) {
@@ -1313,7 +1367,7 @@ extern "C" int ra_decode_merge(const float* o_part, const float* lse_part, long 
   p.slot_mul = slot_mul; p.slot_add = slot_add;
   p.out_slot_o = out_slot_o; p.out_slot_l = out_slot_l; p.in_slot_o = in_slot_o; p.in_slot_l = in_slot_l;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  if (nparts >= MERGE_MANY) decode_merge_kernel<true><<<dim3(rows, D / 32), 32 * MERGE_WARPS, 0, s>>>(p);
+  if (nparts >= MERGE_MANY || (nparts >= MERGE_SOME && rows * (D / 32) <= 2 * sm_count())) decode_merge_kernel<true><<<dim3(rows, D / 32), 32 * MERGE_WARPS, 0, s>>>(p);
   else decode_merge_kernel<false><<<rows, D, 0, s>>>(p);
   return check_launch("decode_merge_kernel");
 }

@@ -65,11 +65,17 @@ def default_splits(S: int, B: int, H: int, mma: bool = False) -> int:
     4.57 TB/s, 74 splits 4.65 (a ragged last wave), 256 splits 5.19 with register loads; with the asynchronous-copy
     ring 64 to 512 splits are within 3 % of each other (6.83 to 7.02 TB/s). At least 512 cache rows per CTA.
     The tensor-core kernel (``mma``) has two CTAs of four warps per SM and likes half as many, longer ranges: four
-    query rows, 128 / 256 / 512 splits: 0.315 / 0.332 / 0.408 ms."""
+    query rows, 128 / 256 / 512 splits: 0.315 / 0.332 / 0.408 ms.
+    Short caches: ranges down to 128 rows while four CTAs (two of ``mma``) per SM are not there yet. 16 heads x 2176 rows, 5 / 17
+    splits: 15.9 / 10.5 us with the merge; 8 heads x 4000 rows, 8 / 32 splits: 18.9 / 10.7 us; four query rows, 16 heads x 2176, 3 / 17
+    splits: 19.2 / 12.7 us. Beyond that short ranges only cost (8 x 32 heads x 4000 rows, 8 / 16 splits: 96.9 / 101.8 us)."""
     sms = _lib.lib().ra_sm_count()
-    per_sm, rows = (32, 1024) if mma else (64, 512)
-    want = max(1, (per_sm * sms) // max(1, B * H))
-    return max(1, min(want, (S + rows - 1) // rows, 512))
+    per_sm, rows, resident = (32, 1024, 2) if mma else (64, 512, 4)
+    pairs = max(1, B * H)
+    want = max(1, (per_sm * sms) // pairs)
+    full = min(want, (S + rows - 1) // rows)
+    fill = min(resident * sms // pairs, (S + 127) // 128)
+    return max(1, min(max(full, fill), 512))
 
 
 def decode_partial(q, k, v, *, n_valid: Optional[int] = None, q_pos0: int = -1, k_pos0: int = 0,

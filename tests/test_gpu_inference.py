@@ -432,15 +432,14 @@ def test_masked_prompt_chunks(B, ql, S, H, D, kind, need_grad):
 @pytest.mark.parametrize("ql", [1, 2, 5, 8])
 @pytest.mark.parametrize("S,kind", [(37, "valid"), (700, "valid"), (5000, "valid"), (9000, "holes"), (300000, "valid"), (513, "per row"), (1000, "nothing")])
 def test_decode_skips_rows_nobody_sees(S, kind, ql, D):
-    """Cached rows that the mask hides from all query rows hold infinities: they are not read. Ranges longer and shorter than
-    the bits a CTA keeps, masks by query row and head, a batch row that sees nothing. bf16 in and out: 1e-2 of the largest entry."""
+    """Cached rows that the mask hides from all query rows hold infinities: they are not read. Masks by query row and head, a batch row that sees nothing. bf16 in and out: 1e-2 of the largest entry."""
     import ringattention_b200 as rab
 
     B, H = (2, 3) if S < 100000 else (16, 8)
     if S >= 100000 and (D, ql) not in ((64, 1), (64, 2)):
         pytest.skip("the long range once for each kernel")
     if S >= 100000:
-        S = 40000  # 16 x 8 (row, head) pairs: ranges of more than 8192 rows
+        S = 40000  # 16 x 8 (row, head) pairs
     g = torch.Generator(device="cuda").manual_seed(S + ql)
     q = torch.randn(B, ql, H, D, device="cuda", generator=g).bfloat16()
     k, v = (torch.randn(B, S, H, D, device="cuda", generator=g).bfloat16() for _ in range(2))
@@ -463,4 +462,26 @@ def test_decode_skips_rows_nobody_sees(S, kind, ql, D):
         k[hidden], v[hidden] = float("inf"), float("nan")
     with torch.no_grad():
         out = rab.ringattention_inference(q, k, v, mask)
+    assert (out.double() - want).abs().max() <= 0.01 * want.abs().max() + 1e-3
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("ql", [1, 2, 8])
+@pytest.mark.parametrize("S,off", [(4096, 0), (4097, 0), (4500, 1), (130, 3), (31, 2)])
+def test_decode_mask_bits_at_the_edges_of_a_range(S, off, ql, D):
+    """One range for all rows: as many as a CTA keeps bits for, one more (the mask is read as it is then), and mask rows that do
+    not start at multiples of four bytes. bf16 inputs, probabilities in bf16 at most: 1e-2 of the largest entry."""
+    from ringattention_b200.ops import decode as Dk
+
+    g = torch.Generator(device="cuda").manual_seed(S + ql + D)
+    H = 2
+    q = torch.randn(1, ql, H, D, device="cuda", generator=g).bfloat16()
+    k, v = (torch.randn(1, S, H, D, device="cuda", generator=g).bfloat16() for _ in range(2))
+    m = (torch.rand(1, H, ql, S + 4, device="cuda", generator=g) < 0.3)[..., off:off + S]
+    m[0, 0, 0, :] = False
+    o, lse = Dk.decode_partial(q, k, v, mask=m.view(torch.uint8), splits=1)
+    out = torch.empty(1, ql, H, D, device="cuda")
+    Dk.merge_partials(o, lse, H, ql, out=out)
+    x = (torch.einsum("bqhd,bkhd->bhqk", q.double(), k.double()) / D ** 0.5).masked_fill(~m, -float("inf"))
+    want = torch.einsum("bhqk,bkhd->bqhd", torch.softmax(x, -1).nan_to_num(0.0), v.double())
     assert (out.double() - want).abs().max() <= 0.01 * want.abs().max() + 1e-3
