@@ -160,7 +160,9 @@ __device__ __forceinline__ bool pair_seen(const uint32_t* seen, const uint8_t* m
 // i, so memory requests are outstanding during the arithmetic too; a thread only ever reads what it copied itself,
 // hence cp.async.wait_group is all the synchronisation needed. Dynamic shared memory: ST * 4 rows * 32 bytes per
 // thread.
-template <int D, int QL, int ST>
+// MASKED: there is a mask. A variant of its own, because the tests for hidden rows in the copies and the loop cost a call without a mask
+// 4 to 10 % (eight query rows, 65536 cached rows, 32 heads: 187 -> 209 us).
+template <int D, int QL, int ST, bool MASKED>
 __global__ void __launch_bounds__(THREADS) decode_splitkv_kernel(const SplitParams p) {
   constexpr int LPR = D / 8;        // lanes per cache row (16 bytes per lane)
   constexpr int RPW = 32 / LPR;     // rows per warp step
@@ -211,8 +213,8 @@ __global__ void __launch_bounds__(THREADS) decode_splitkv_kernel(const SplitPara
   uint32_t* const seen = reinterpret_cast<uint32_t*>(&sm_o[0][0][0]);
   static_assert((QL > 1 ? QL + 1 : 1) * SEEN_WORDS * 4 <= static_cast<int>(sizeof(sm_o)), "bits of the mask do not fit");
   const uint32_t* const seen_any = seen + (QL > 1 ? QL : 0) * SEEN_WORDS;
-  const uint8_t* mask = p.mask ? p.mask + b * p.m_sb + h * p.m_sh : nullptr;
-  if (mask && r0 < r1 && !mark_seen<QL>(seen, mask, p.m_sq, QL, r0, r1)) r1 = r0;  // nothing to see here
+  const uint8_t* mask = MASKED ? p.mask + b * p.m_sb + h * p.m_sh : nullptr;
+  if (MASKED && r0 < r1 && !mark_seen<QL>(seen, mask, p.m_sq, QL, r0, r1)) r1 = r0;  // nothing to see here
 
   // The trip count is the same for every lane of a warp (the loop variable ignores `sub`), so the
   // full-mask shuffles below always see all 32 lanes; rows past the end are merely masked out.
@@ -221,7 +223,7 @@ __global__ void __launch_bounds__(THREADS) decode_splitkv_kernel(const SplitPara
 #pragma unroll
     for (int u = 0; u < UNROLL; ++u) {
       const int r = base_w + sub + u * step;
-      const bool in = r < r1 && (!mask || row_seen(seen_any, r, r0, r1));
+      const bool in = r < r1 && (!MASKED || row_seen(seen_any, r, r0, r1));
       const long long rr = in ? r : r0;  // r0 < r1 whenever the loop runs: a valid address, never read when !in
       uint4* dst = stage_buf + ((slot * UNROLL + u) * 2) * THREADS + threadIdx.x;
       cp_async16(dst, kb + rr * p.k_ss, in ? 16 : 0);
@@ -250,7 +252,7 @@ __global__ void __launch_bounds__(THREADS) decode_splitkv_kernel(const SplitPara
       cp_async_wait<(ST > 0 ? ST - 1 : 0)>();  // all but the newest ST - 1 groups are complete: this trip's rows are in
 #pragma unroll
       for (int u = 0; u < UNROLL; ++u) {
-        ok[u] = base + u * step < r1 && (!mask || row_seen(seen_any, base + u * step, r0, r1));
+        ok[u] = base + u * step < r1 && (!MASKED || row_seen(seen_any, base + u * step, r0, r1));
         const uint4* src = stage_buf + ((slot_out * UNROLL + u) * 2) * THREADS + threadIdx.x;
         ku[u] = src[0];
         vu[u] = src[THREADS];
@@ -260,7 +262,7 @@ __global__ void __launch_bounds__(THREADS) decode_splitkv_kernel(const SplitPara
 #pragma unroll
       for (int u = 0; u < UNROLL; ++u) {
         const int r = base + u * step;
-        ok[u] = r < r1 && (!mask || row_seen(seen_any, r, r0, r1));
+        ok[u] = r < r1 && (!MASKED || row_seen(seen_any, r, r0, r1));
         if (ok[u]) {
           ku[u] = *reinterpret_cast<const uint4*>(kb + static_cast<long long>(r) * p.k_ss);
           vu[u] = *reinterpret_cast<const uint4*>(vb + static_cast<long long>(r) * p.v_ss);
@@ -285,7 +287,7 @@ __global__ void __launch_bounds__(THREADS) decode_splitkv_kernel(const SplitPara
         for (int o = LPR / 2; o > 0; o >>= 1) d += __shfl_xor_sync(0xffffffffu, d, o);
         bool vis = ok[u];
         if (q_pos0 >= 0) vis = vis && (p.k_pos0 + r <= q_pos0 + i);
-        if (mask && vis && (QL > 1 || r1 - r0 > SEEN_ROWS)) vis = pair_seen(seen, mask, p.m_sq, i, r, r0, r1);
+        if (MASKED && vis && (QL > 1 || r1 - r0 > SEEN_ROWS)) vis = pair_seen(seen, mask, p.m_sq, i, r, r0, r1);
         s[u][i] = vis ? d : -INFINITY;
       }
     }
@@ -313,7 +315,7 @@ __global__ void __launch_bounds__(THREADS) decode_splitkv_kernel(const SplitPara
   }
 
   if (ST > 0) cp_async_wait<0>();  // only empty groups can be left; nothing is in flight when the CTA ends
-  if (mask) __syncthreads();        // the bits of the mask give way to the partial results
+  if (MASKED) __syncthreads();        // the bits of the mask give way to the partial results
   // ---- combine the row groups of a warp, then the warps of the CTA
 #pragma unroll
   for (int i = 0; i < QL; ++i) {
@@ -376,7 +378,7 @@ __global__ void __launch_bounds__(THREADS) decode_splitkv_kernel(const SplitPara
 constexpr int MMA_ST = 3;       // stages of a warp's ring
 constexpr int MMA_ROWS = 16;    // cache rows per chunk
 
-template <int D>
+template <int D, bool MASKED>
 __global__ void __launch_bounds__(THREADS) decode_splitkv_mma_kernel(const SplitParams p, int QL) {
   constexpr int RB = D * 2;                 // bytes per cache row
   constexpr int PPR = D / 8;                // 16-byte pieces per row
@@ -408,8 +410,8 @@ __global__ void __launch_bounds__(THREADS) decode_splitkv_mma_kernel(const Split
   uint32_t* const seen = reinterpret_cast<uint32_t*>(&sm_o[0][0][0]);
   static_assert(9 * SEEN_WORDS * 4 <= static_cast<int>(sizeof(sm_o)), "bits of the mask do not fit");
   const uint32_t* const seen_any = seen + QL * SEEN_WORDS;
-  const uint8_t* mask = p.mask ? p.mask + b * p.m_sb + h * p.m_sh : nullptr;
-  if (mask && r0 < r1 && !mark_seen<8>(seen, mask, p.m_sq, QL, r0, r1)) r1 = r0;  // nothing to see here
+  const uint8_t* mask = MASKED ? p.mask + b * p.m_sb + h * p.m_sh : nullptr;
+  if (MASKED && r0 < r1 && !mark_seen<8>(seen, mask, p.m_sq, QL, r0, r1)) r1 = r0;  // nothing to see here
   const __nv_bfloat16* kb = p.k + b * p.k_sb + h * p.k_sh;
   const __nv_bfloat16* vb = p.v + b * p.v_sb + h * p.v_sh;
 
@@ -440,7 +442,7 @@ __global__ void __launch_bounds__(THREADS) decode_splitkv_mma_kernel(const Split
       const int piece = lane + 32 * j;
       const int row = piece / PPR, ch = piece % PPR;
       const int r = base + row;
-      const bool in = r < r1 && (!mask || row_seen(seen_any, r, r0, r1));
+      const bool in = r < r1 && (!MASKED || row_seen(seen_any, r, r0, r1));
       const long long rr = in ? r : r0;  // a valid address; not read when !in (the piece is zero-filled)
       const int off = row * RB + ((ch ^ (row & 7)) << 4);
       cp_async16(kt + off, kb + rr * p.k_ss + ch * 8, in ? 16 : 0);
@@ -493,7 +495,7 @@ __global__ void __launch_bounds__(THREADS) decode_splitkv_mma_kernel(const Split
         const int r = base + 8 * nt + 2 * t + e;
         bool vis = r < r1 && g < QL;
         if (q_pos0 >= 0) vis = vis && (p.k_pos0 + r <= q_pos0 + g);
-        if (mask && vis) vis = pair_seen(seen, mask, p.m_sq, g, r, r0, r1);
+        if (MASKED && vis) vis = pair_seen(seen, mask, p.m_sq, g, r, r0, r1);
         x[nt][e] = vis ? s[nt][e] * p.scale_log2 : -INFINITY;
         mx = fmaxf(mx, x[nt][e]);
       }
@@ -541,7 +543,7 @@ __global__ void __launch_bounds__(THREADS) decode_splitkv_mma_kernel(const Split
   // ---- the row sum over the four lanes of a row, then the warps of the CTA (as in the kernel above)
   l += __shfl_xor_sync(0xffffffffu, l, 1);
   l += __shfl_xor_sync(0xffffffffu, l, 2);
-  if (mask) __syncthreads();  // the bits of the mask give way to the partial results
+  if (MASKED) __syncthreads();  // the bits of the mask give way to the partial results
   if (t == 0) {
     sm_m[warp][g] = m;
     sm_l[warp][g] = l;
@@ -610,14 +612,15 @@ __device__ __forceinline__ void merge_parts(const float* o_row, long long o_ps, 
   lse = mx == -INFINITY ? -INFINITY : mx + __logf(wsum);
 }
 
-// The same for rows with many partials, 32 columns a CTA: 32 warps of 32 columns take every 32nd partial each and meet in
-// shared memory in a fixed order. A decode call has few rows (batch x heads) and up to 512 partials of each: one CTA of D
+// The same for rows with many partials, 32 columns a CTA: MERGE_WARPS warps of 32 columns take every MERGE_WARPS-th partial each and
+// meet in shared memory in a fixed order. A decode call has few rows (batch x heads) and up to 512 partials of each: one CTA of D
 // threads a row is a chain of loads, 41 us for 32 rows of 256 partials; here a thread has eight loads, all in flight.
 // Valid in the threads of warp 0 (lane = column).
-constexpr int MERGE_WARPS = 32;
-constexpr int MERGE_MANY = 16;     // fewer partials: less than one for every second warp, and prefills have many rows of 2-8
+constexpr int MERGE_MANY = 32;     // fewer partials of many rows: a CTA of D threads a row (prefills have 2-8; 1024 rows of 20: 6 us less)
+constexpr int MERGE_TOP = 64;      // more: 32 warps, otherwise 8 (1024 rows of 20 partials: 4096 CTAs of 32 warps would take 13 waves)
 constexpr int MERGE_SOME = 4;      // from here on if all CTAs run at once (16 rows of 15 partials of a decode step: 3 us less)
 constexpr int MERGE_LSE = 1024;    // weights kept in shared memory
+template <int MERGE_WARPS>
 __device__ __forceinline__ void merge_parts_wide(const float* o_col, long long o_ps, const float* lp, long long l_ps,
                                                  int nparts, float& o, float& lse) {
   __shared__ float weight[MERGE_LSE], red_o[MERGE_WARPS][33], red_w[MERGE_WARPS], red_m[MERGE_WARPS];
@@ -632,7 +635,7 @@ __device__ __forceinline__ void merge_parts_wide(const float* o_col, long long o
   for (int i = 16; i > 0; i >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, i));
   if (lane == 0) red_m[w] = mx;
   __syncthreads();
-  mx = red_m[lane];
+  mx = red_m[lane & (MERGE_WARPS - 1)];
 #pragma unroll
   for (int i = 16; i > 0; i >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, i));
   float wsum = 0.f;
@@ -661,16 +664,16 @@ __device__ __forceinline__ void merge_parts_wide(const float* o_col, long long o
   }
 }
 
-// One CTA per row = (b, h, i), D threads; WIDE: one per row and 32 columns.
-template <bool WIDE>
-__global__ void __launch_bounds__(WIDE ? 32 * MERGE_WARPS : 128) decode_merge_kernel(const MergeParams p) {
-  const int row = blockIdx.x, d = WIDE ? blockIdx.y * 32 + threadIdx.x : threadIdx.x;
+// One CTA per row = (b, h, i), D threads; W > 0: one of W warps per row and 32 columns.
+template <int W>
+__global__ void __launch_bounds__(W ? 32 * W : 128) decode_merge_kernel(const MergeParams p) {
+  const int row = blockIdx.x, d = W ? blockIdx.y * 32 + threadIdx.x : threadIdx.x;
   const long long slot = p.step_ptr ? ((*p.step_ptr * p.slot_mul + p.slot_add) & 1) : 0;
   const float* o_row = p.o_part + slot * p.in_slot_o + static_cast<long long>(row) * p.o_rs;
   const float* lp = p.lse_part + slot * p.in_slot_l + static_cast<long long>(row) * p.l_rs;
   float o, lse;
-  if (WIDE) {
-    merge_parts_wide(o_row + blockIdx.y * 32, p.o_ps, lp, p.l_ps, p.nparts, o, lse);
+  if (W) {
+    merge_parts_wide<(W ? W : 1)>(o_row + blockIdx.y * 32, p.o_ps, lp, p.l_ps, p.nparts, o, lse);
     if (threadIdx.x >= 32) return;
   } else {
     merge_parts(o_row, p.o_ps, lp, p.l_ps, p.nparts, d, o, lse);
@@ -1186,7 +1189,9 @@ __global__ void __launch_bounds__(LM_THREADS) small_m_linear_mma_kernel(const Lm
 
 // One decode token per sequence: rotate the q and k heads of the (B, 1, 3, H, D) qkv buffer in place (RoPE at the
 // position in *pos_ptr) and append the rotated K and the V to the cache shard when this rank owns the position
-// (same ownership rule and cache views as kv_append_kernel). One launch instead of two per layer and token.
+// (same ownership rule and cache views as kv_append_kernel). One launch instead of two per layer and token. Four values a thread
+// and as many CTAs as that takes: the sines of a token are a chain of some hundred instructions each, and one CTA a token with
+// sixteen values a thread took 3.2 us for 16 heads.
 template <int D>
 __global__ void rope_append_kernel(__nv_bfloat16* __restrict__ qkv, __nv_bfloat16* __restrict__ kc,
                                    __nv_bfloat16* __restrict__ vc, long long sb, long long ss, long long sh,
@@ -1201,36 +1206,36 @@ __global__ void rope_append_kernel(__nv_bfloat16* __restrict__ qkv, __nv_bfloat1
   }
   const bool mine = r >= 0 && r < S_max;
   const int b = blockIdx.x;
-  constexpr int hd2 = D / 2, VPH = hd2 / 8;  // 16-byte vectors per half head
+  const int first = blockIdx.y * blockDim.x + threadIdx.x, stride = gridDim.y * blockDim.x;
+  constexpr int hd2 = D / 2, PPH = hd2 / 2;  // a thread turns two neighbouring pairs (e, e + D/2) at a time
   __nv_bfloat16* base = qkv + static_cast<long long>(b) * 3 * H * D;
-  // q and k heads: 2H heads x VPH vector pairs
-  for (int i = threadIdx.x; i < 2 * H * VPH; i += blockDim.x) {
-    const int hh = i / VPH, v = i - hh * VPH;  // hh in [0, 2H): q heads then k heads
-    __nv_bfloat16* p = base + static_cast<long long>(hh) * D + v * 8;
-    float a[8], c[8];
-    unpack8(*reinterpret_cast<const uint4*>(p), a);
-    unpack8(*reinterpret_cast<const uint4*>(p + hd2), c);
+  for (int i = first; i < 2 * H * PPH; i += stride) {  // q heads then k heads
+    const int hh = i / PPH, v = i - hh * PPH;
+    __nv_bfloat16* p = base + static_cast<long long>(hh) * D + v * 2;
+    const float2 a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(p));
+    const float2 c = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(p + hd2));
+    const float af[2] = {a.x, a.y}, cf[2] = {c.x, c.y};
+    float a2[2], c2[2];
 #pragma unroll
-    for (int e = 0; e < 8; ++e) {
-      const float inv_freq = exp2f(-log2_theta * (2.0f * (v * 8 + e) / D));
+    for (int e = 0; e < 2; ++e) {
+      const float inv_freq = exp2f(-log2_theta * (2.0f * (v * 2 + e) / D));
       float sn, cs;
       sincosf(static_cast<int>(pos) * inv_freq, &sn, &cs);  // same arithmetic as the stand-alone RoPE kernel
-      const float a2 = a[e] * cs - c[e] * sn, c2 = c[e] * cs + a[e] * sn;
-      a[e] = a2;
-      c[e] = c2;
+      a2[e] = af[e] * cs - cf[e] * sn;
+      c2[e] = cf[e] * cs + af[e] * sn;
     }
-    const uint4 lo = pack8(a), hi = pack8(c);
-    *reinterpret_cast<uint4*>(p) = lo;
-    *reinterpret_cast<uint4*>(p + hd2) = hi;
+    const __nv_bfloat162 lo = __floats2bfloat162_rn(a2[0], a2[1]), hi = __floats2bfloat162_rn(c2[0], c2[1]);
+    *reinterpret_cast<__nv_bfloat162*>(p) = lo;
+    *reinterpret_cast<__nv_bfloat162*>(p + hd2) = hi;
     if (mine && hh >= H && RA_IN_BOUNDS(r, 1, S_max, kTagDecodeCacheRow)) {
-      const long long off = b * sb + r * ss + (hh - H) * sh + v * 8;
-      *reinterpret_cast<uint4*>(kc + off) = lo;
-      *reinterpret_cast<uint4*>(kc + off + hd2) = hi;
+      const long long off = b * sb + r * ss + (hh - H) * sh + v * 2;
+      *reinterpret_cast<__nv_bfloat162*>(kc + off) = lo;
+      *reinterpret_cast<__nv_bfloat162*>(kc + off + hd2) = hi;
     }
   }
   if (mine) {
     const uint4* src_v = reinterpret_cast<const uint4*>(base + 2ll * H * D);
-    for (int i = threadIdx.x; i < H * D / 8; i += blockDim.x) {
+    for (int i = first; i < H * D / 8; i += stride) {
       const int h = i / (D / 8), cidx = i - h * (D / 8);
       *reinterpret_cast<uint4*>(vc + b * sb + r * ss + h * sh + cidx * 8) = src_v[i];
     }
@@ -1298,14 +1303,15 @@ extern "C" int ra_decode_splitkv(const RaDecodeArgs* a) {
     int dev = 0;
     cudaGetDevice(&dev);
     if (dev < 64 && !attr_done[dev]) {  // with the static arrays the 128-wide variant needs more than 48 KB
-      cudaFuncSetAttribute(decode_splitkv_mma_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, kRing128);
-      cudaFuncSetAttribute(decode_splitkv_mma_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, kRing64);
+      cudaFuncSetAttribute(decode_splitkv_mma_kernel<128, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kRing128);
+      cudaFuncSetAttribute(decode_splitkv_mma_kernel<128, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kRing128);
+      cudaFuncSetAttribute(decode_splitkv_mma_kernel<64, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kRing64);
+      cudaFuncSetAttribute(decode_splitkv_mma_kernel<64, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kRing64);
       attr_done[dev] = true;
     }
-    if (a->D == 128)
-      decode_splitkv_mma_kernel<128><<<grid, THREADS, kRing128, s>>>(p, a->QL);
-    else
-      decode_splitkv_mma_kernel<64><<<grid, THREADS, kRing64, s>>>(p, a->QL);
+    auto kern = a->D == 128 ? (a->mask ? decode_splitkv_mma_kernel<128, true> : decode_splitkv_mma_kernel<128, false>)
+                            : (a->mask ? decode_splitkv_mma_kernel<64, true> : decode_splitkv_mma_kernel<64, false>);
+    kern<<<grid, THREADS, a->D == 128 ? kRing128 : kRing64, s>>>(p, a->QL);
     return check_launch("decode_splitkv_mma_kernel");
   }
   if (a->stages != 0 && a->stages != 3 && a->stages != 4) {
@@ -1320,10 +1326,12 @@ extern "C" int ra_decode_splitkv(const RaDecodeArgs* a) {
     int dev = 0;                                                                                            \
     cudaGetDevice(&dev);                                                                                    \
     if (smem > 0 && dev < 64 && !attr_done[dev]) {                                                          \
-      cudaFuncSetAttribute(decode_splitkv_kernel<DD, QQ, SS>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem); \
+      cudaFuncSetAttribute(decode_splitkv_kernel<DD, QQ, SS, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem); \
+      cudaFuncSetAttribute(decode_splitkv_kernel<DD, QQ, SS, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem); \
       attr_done[dev] = true;                                                                                \
     }                                                                                                       \
-    decode_splitkv_kernel<DD, QQ, SS><<<grid, THREADS, smem, s>>>(p);                                       \
+    if (a->mask) decode_splitkv_kernel<DD, QQ, SS, true><<<grid, THREADS, smem, s>>>(p);                    \
+    else decode_splitkv_kernel<DD, QQ, SS, false><<<grid, THREADS, smem, s>>>(p);                           \
   } while (0)
 #define RA_LAUNCH_DEC(DD, QQ)                                                                               \
   do {                                                                                                      \
@@ -1367,8 +1375,10 @@ extern "C" int ra_decode_merge(const float* o_part, const float* lse_part, long 
   p.slot_mul = slot_mul; p.slot_add = slot_add;
   p.out_slot_o = out_slot_o; p.out_slot_l = out_slot_l; p.in_slot_o = in_slot_o; p.in_slot_l = in_slot_l;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  if (nparts >= MERGE_MANY || (nparts >= MERGE_SOME && rows * (D / 32) <= 2 * sm_count())) decode_merge_kernel<true><<<dim3(rows, D / 32), 32 * MERGE_WARPS, 0, s>>>(p);
-  else decode_merge_kernel<false><<<rows, D, 0, s>>>(p);
+  if (nparts > MERGE_TOP) decode_merge_kernel<32><<<dim3(rows, D / 32), 1024, 0, s>>>(p);
+  else if (nparts >= MERGE_MANY || (nparts >= MERGE_SOME && rows * (D / 32) <= 4 * sm_count()))
+    decode_merge_kernel<8><<<dim3(rows, D / 32), 256, 0, s>>>(p);
+  else decode_merge_kernel<0><<<rows, D, 0, s>>>(p);
   return check_launch("decode_merge_kernel");
 }
 
@@ -1605,10 +1615,10 @@ extern "C" int ra_rope_append(void* qkv, void* k_cache, void* v_cache, long long
   __nv_bfloat16 *q = static_cast<__nv_bfloat16*>(qkv), *kc = static_cast<__nv_bfloat16*>(k_cache),
                 *vc = static_cast<__nv_bfloat16*>(v_cache);
   if (D == 128)
-    rope_append_kernel<128><<<B, 256, 0, s>>>(q, kc, vc, sb, ss, sh, pos_ptr, log2f(theta), k0, S_max, H, stripe_n,
+    rope_append_kernel<128><<<dim3(B, (H * D / 2 + 127) / 128), 128, 0, s>>>(q, kc, vc, sb, ss, sh, pos_ptr, log2f(theta), k0, S_max, H, stripe_n,
                                               stripe_rank, stripe_base, stripe_len0);
   else
-    rope_append_kernel<64><<<B, 256, 0, s>>>(q, kc, vc, sb, ss, sh, pos_ptr, log2f(theta), k0, S_max, H, stripe_n,
+    rope_append_kernel<64><<<dim3(B, (H * D / 2 + 127) / 128), 128, 0, s>>>(q, kc, vc, sb, ss, sh, pos_ptr, log2f(theta), k0, S_max, H, stripe_n,
                                              stripe_rank, stripe_base, stripe_len0);
   return check_launch("rope_append_kernel");
 }
