@@ -19,6 +19,7 @@ class InferenceEngine:
         # [position, step] on the device: lets one recorded CUDA graph serve every decode step
         self.state = torch.zeros(2, dtype=torch.int64, device=self.device)
         self._graph = None
+        self._old_graph = None                      # the one recorded before reset(): the next one takes over its buffers
         self._tok_buf = torch.zeros(token_rows, dtype=torch.int32, device=self.device)
 
     # ------------------------------------------------------------------ supplied by the engine
@@ -63,22 +64,43 @@ class InferenceEngine:
         self._check_room(1)
         if self._graph is None:
             self.state[0] = self.length
-            torch.cuda.synchronize()
-            g = torch.cuda.CUDAGraph()
-            with torch.cuda.graph(g):
-                logits = self._decode_body(self._tok_buf)
-                self._tok_buf.copy_(self.sample(logits).to(torch.int32))
-            self._graph = g
+            self._graph = self._record(self._greedy_step)
         self._graph.replay()
         self.length += 1
         return self._tok_buf
+
+    def _greedy_step(self) -> None:
+        logits = self._decode_body(self._tok_buf)
+        self._tok_buf.copy_(self.sample(logits).to(torch.int32))
+
+    def _record(self, body) -> torch.cuda.CUDAGraph:
+        """Record ``body`` as ``torch.cuda.graph`` does, but leave the allocator's cached blocks and Python's garbage alone:
+        emptying the cache before every prompt's recording made the next prompt's prefill allocate all of its
+        buffers from the driver again. The buffers of the graph recorded before are taken over (it is dropped here)."""
+        torch.cuda.synchronize()
+        g = torch.cuda.CUDAGraph()
+        side = torch.cuda.Stream(self.device)
+        side.wait_stream(torch.cuda.current_stream())
+        with torch.cuda.stream(side):
+            if self._old_graph is None:
+                g.capture_begin()
+            else:
+                g.capture_begin(pool=self._old_graph.pool())
+            try:
+                body()
+            finally:
+                g.capture_end()
+        torch.cuda.current_stream().wait_stream(side)
+        self._old_graph = None
+        return g
 
     def reset(self) -> None:
         """Forget the cached context (the cache memory is kept). The recorded decode graph is dropped
         too: it may hold properties of the prefilled context as launch constants."""
         self.length = 0
         self.state.zero_()
-        self._graph = None
+        if self._graph is not None:
+            self._graph, self._old_graph = None, self._graph
         self._clear_cache()
 
     # ------------------------------------------------------------------ generation
