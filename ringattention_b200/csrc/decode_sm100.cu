@@ -1024,6 +1024,175 @@ __global__ void __launch_bounds__(256) small_m_linear_pro_kernel(const __nv_bflo
   }
 }
 
+// One row: y[N] = f(x) W^T (+ res), the product that a single sequence's decode step consists of. What bounds it is how soon and how
+// evenly the weights stream in, so nothing stands before the first weight load: the eight warps of a CTA share K (piece
+// c * 256 + warp * 32 + lane of 16 bytes), so a thread needs only its own few pieces of f(x), which it keeps in registers, and needs
+// no barrier and no shared memory for them; the norm's factor is applied to the finished sum. A CTA takes tiles of eight
+// columns, eight loads of 16 bytes a thread in flight and the next eight issued before they are used; the warps' sums
+// meet in shared memory once a tile. us a call on B200, a warp per column (small_m_linear_pro_kernel) -> here:
+//   6144 x 2048 8.2 -> 6.8, 2048 x 2048 4.8 -> 3.8, 32000 x 2048 24.7 -> 22.7, 22016 x 4096 32.0 -> 31.3, 4096 x 4096 9.0 -> 7.9,
+//   with SwiGLU ahead of it 2048 x 5504 10.5 -> 8.9, 4096 x 11008 25.9 -> 23.1
+// f(x) is rounded to bf16 as in the kernels above.
+enum { PRO_NONE = 0 };
+constexpr int ROW_COLS = 8, ROW_WARPS = 8, ROW_MAX_CHUNKS = 6;  // K up to 6 * 256 * 8
+
+__device__ __forceinline__ uint4 ld_stream(const uint4* p) {
+  uint4 v;
+  asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+  return v;
+}
+
+// NC: chunks of K, 1 or an even number (the last may be empty). GATED: w = [gate | up] of N rows each, a tile is four gate columns and the
+// matching up columns, and y = silu(gate) * up of the two rounded to bf16 (as the activation kernels take them): the next product's
+// CTAs need not each repeat the activation of the whole row (2048 x 5504: 8.9 us with it, 6.5 without; 4096 x 11008: 23.1 and 18.1).
+template <int PRO, int NC, bool GATED>
+__global__ void __launch_bounds__(32 * ROW_WARPS, 2) row_linear_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ w,
+                                                                       __nv_bfloat16* __restrict__ y, const __nv_bfloat16* __restrict__ res,
+                                                                       const __nv_bfloat16* __restrict__ gain, float eps, int N, int K) {
+  static_assert(NC == 1 || NC % 2 == 0, "the two sets of loads alternate by chunk, or by tile when there is one chunk");
+  __shared__ float red[2][ROW_WARPS][ROW_COLS];
+  __shared__ float red_ss[ROW_WARPS];
+  __shared__ uint4 fx_s[NC > 2 ? NC : 1][32 * ROW_WARPS];  // a thread's own pieces; registers hold no more than two
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  constexpr int OUT = GATED ? ROW_COLS / 2 : ROW_COLS;  // columns of y a tile gives
+  const int n16 = K / 8, tiles = (N + OUT - 1) / OUT, stride = static_cast<int>(gridDim.x);
+  const uint4* wv = reinterpret_cast<const uint4*>(w);
+  auto load = [&](int tile, int c, uint4* to) {
+    const int piece = c * 32 * ROW_WARPS + threadIdx.x;
+    if (tile < tiles && (NC == 1 || piece < n16)) {
+      const uint4* src = wv + (NC == 1 ? min(piece, n16 - 1) : piece);
+#pragma unroll
+      for (int j = 0; j < ROW_COLS; ++j) {  // columns past the end repeat the last one: their sums are not stored
+        const int col = GATED ? min(tile * (ROW_COLS / 2) + (j & 3), N - 1) + (j & 4 ? N : 0) : min(tile * ROW_COLS + j, N - 1);
+        to[j] = ld_stream(src + static_cast<long long>(col) * n16);
+      }
+    }
+  };
+  uint4 wa[ROW_COLS] = {}, wb[ROW_COLS] = {};
+  const int tile0 = blockIdx.x;
+  load(tile0, 0, wa);
+  load(NC == 1 ? tile0 + stride : tile0, NC == 1 ? 0 : 1, wb);
+  // ---- this thread's pieces of f(x); pieces past the end are zero
+  uint4 fx[NC > 2 ? 1 : NC];
+  float ss = 0.f;
+#pragma unroll
+  for (int c = 0; c < NC; ++c) {
+    const int piece = c * 32 * ROW_WARPS + threadIdx.x;
+    uint4 f = make_uint4(0u, 0u, 0u, 0u);
+    if (piece < n16) {
+      f = reinterpret_cast<const uint4*>(x)[piece];
+      if (PRO != PRO_NONE) {
+        float xf[8], of[8];
+        unpack8(f, xf);
+        unpack8(PRO == PRO_SWIGLU ? reinterpret_cast<const uint4*>(x)[piece + n16] : reinterpret_cast<const uint4*>(gain)[piece], of);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) {
+          if (PRO == PRO_RMSNORM) {
+            ss = fmaf(xf[e], xf[e], ss);
+            xf[e] *= of[e];
+          } else {
+            xf[e] = xf[e] / (1.f + __expf(-xf[e])) * of[e];
+          }
+        }
+        f = pack8(xf);
+      }
+    }
+    if (NC > 2) fx_s[c][threadIdx.x] = f;
+    else fx[NC > 2 ? 0 : c] = f;
+  }
+  if (PRO == PRO_RMSNORM) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+    if (lane == 0) red_ss[warp] = ss;
+  }
+  float rstd = 1.f;
+  int buf = 0;
+  float acc[ROW_COLS];
+  auto consume = [&](int c, const uint4* from) {
+    if (c * 32 * ROW_WARPS + static_cast<int>(threadIdx.x) < n16) {
+      float xf[8];
+      unpack8(NC > 2 ? fx_s[c][threadIdx.x] : fx[NC > 2 ? 0 : c], xf);
+#pragma unroll
+      for (int j = 0; j < ROW_COLS; ++j) {
+        float wf[8];
+        unpack8(from[j], wf);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) acc[j] = fmaf(wf[e], xf[e], acc[j]);
+      }
+    }
+  };
+  auto finish = [&](int tile) {
+    // ---- columns over the lanes: lane l ends with the warp's sum of column (l >> 2)
+    static_assert(ROW_COLS == 8, "the exchange below is written for eight columns");
+    const bool up16 = lane & 16, up8 = lane & 8, up4 = lane & 4;
+    float a4[4], a2[2], a1;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const float mine = up16 ? acc[j + 4] : acc[j], theirs = up16 ? acc[j] : acc[j + 4];
+      a4[j] = mine + __shfl_xor_sync(0xffffffffu, theirs, 16);
+    }
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      const float mine = up8 ? a4[j + 2] : a4[j], theirs = up8 ? a4[j] : a4[j + 2];
+      a2[j] = mine + __shfl_xor_sync(0xffffffffu, theirs, 8);
+    }
+    a1 = (up4 ? a2[1] : a2[0]) + __shfl_xor_sync(0xffffffffu, up4 ? a2[0] : a2[1], 4);
+    a1 += __shfl_xor_sync(0xffffffffu, a1, 2);
+    a1 += __shfl_xor_sync(0xffffffffu, a1, 1);
+    if ((lane & 3) == 0) red[buf][warp][lane >> 2] = a1;
+    __syncthreads();  // (two buffers: the next tile's sums go to the other one, and this one is free again behind its barrier)
+    if (warp == 0 && lane < ROW_COLS) {
+      if (PRO == PRO_RMSNORM && tile == tile0) {
+        float t = 0.f;
+#pragma unroll
+        for (int i = 0; i < ROW_WARPS; ++i) t += red_ss[i];
+        rstd = rsqrtf(t / K + eps);
+      }
+      float v = 0.f;
+#pragma unroll
+      for (int i = 0; i < ROW_WARPS; ++i) v += red[buf][i][lane];
+      v *= rstd;
+      if (GATED) {
+        const float gv = __bfloat162float(__float2bfloat16(v));
+        const float uv = __shfl_down_sync(0xffu, gv, 4);
+        v = gv / (1.f + __expf(-gv)) * uv;
+      }
+      const int col = tile * OUT + lane;
+      if (lane < OUT && col < N) {
+        if (!GATED && res) v += __bfloat162float(res[col]);
+        if (RA_IN_BOUNDS(col, 1, N, kTagSmallMLinear)) y[col] = __float2bfloat16(v);
+      }
+    }
+    buf ^= 1;
+#pragma unroll
+    for (int j = 0; j < ROW_COLS; ++j) acc[j] = 0.f;
+  };
+#pragma unroll
+  for (int j = 0; j < ROW_COLS; ++j) acc[j] = 0.f;
+  if (NC == 1) {
+    for (int tile = tile0; tile < tiles; tile += 2 * stride) {
+      consume(0, wa);
+      load(tile + 2 * stride, 0, wa);
+      finish(tile);
+      if (tile + stride >= tiles) break;
+      consume(0, wb);
+      load(tile + 3 * stride, 0, wb);
+      finish(tile + stride);
+    }
+  } else {
+    for (int tile = tile0; tile < tiles; tile += stride) {
+#pragma unroll
+      for (int c = 0; c < NC; c += 2) {
+        consume(c, wa);
+        load(c + 2 < NC ? tile : tile + stride, c + 2 < NC ? c + 2 : 0, wa);
+        consume(c + 1, wb);
+        load(c + 3 < NC ? tile : tile + stride, c + 3 < NC ? c + 3 : 1, wb);
+      }
+      finish(tile);
+    }
+  }
+}
+
 // The same product on the tensor cores, for 2..8 rows (several decode streams): with M rows the kernels above spend
 // M times the FMAs per weight and become bound by their instruction stream (M = 8: 189 us against 34 us for M = 1 on
 // 22016 x 4096). Built like decode_splitkv_mma_kernel: the rows of x are the M side of a 16 x 8 x 16 MMA (rows >= M are
@@ -1444,6 +1613,34 @@ extern "C" int ra_decode_advance(long long* state, void* stream) {
   return check_launch("decode_advance_kernel");
 }
 
+namespace {
+// One row with K up to ROW_MAX_CHUNKS * 2048: two CTAs per SM walk the tiles, as many rounds for each.
+int launch_row_linear(int pro, bool gated, const void* x, const void* w, void* y, const void* res, const void* gain, float eps, int N, int K,
+                      cudaStream_t s) {
+  using namespace ra::decode;
+  const int out = gated ? ROW_COLS / 2 : ROW_COLS;
+  const int tiles = (N + out - 1) / out, most = 2 * sm_count(), rounds = (tiles + most - 1) / most;
+  const int grid = (tiles + rounds - 1) / rounds, nc = (K / 8 + 32 * ROW_WARPS - 1) / (32 * ROW_WARPS);
+  auto go = [&](auto kern) {
+    kern<<<grid, 32 * ROW_WARPS, 0, s>>>(static_cast<const __nv_bfloat16*>(x), static_cast<const __nv_bfloat16*>(w), static_cast<__nv_bfloat16*>(y),
+                                         static_cast<const __nv_bfloat16*>(res), static_cast<const __nv_bfloat16*>(gain), eps, N, K);
+  };
+#define RA_ROW_CASE(CC)                                                        \
+  case CC:                                                                     \
+    if (gated) go(row_linear_kernel<PRO_RMSNORM, CC, true>);                   \
+    else if (pro == PRO_RMSNORM) go(row_linear_kernel<PRO_RMSNORM, CC, false>); \
+    else if (pro == PRO_SWIGLU) go(row_linear_kernel<PRO_SWIGLU, CC, false>);  \
+    else go(row_linear_kernel<PRO_NONE, CC, false>);                           \
+    break;
+  switch (nc == 1 ? 1 : (nc + 1) / 2 * 2) {
+    RA_ROW_CASE(1) RA_ROW_CASE(2) RA_ROW_CASE(4) RA_ROW_CASE(6)
+  }
+#undef RA_ROW_CASE
+  return check_launch("row_linear_kernel");
+}
+bool row_linear_takes(int M, int K) { return M == 1 && K >= 8 && K <= ra::decode::ROW_MAX_CHUNKS * 256 * ra::decode::ROW_WARPS; }
+}  // namespace
+
 extern "C" int ra_small_m_linear(const void* x, const void* w, void* y, const void* res, int M, int N,
                                  int K, void* stream) {
   using namespace ra::decode;
@@ -1451,8 +1648,9 @@ extern "C" int ra_small_m_linear(const void* x, const void* w, void* y, const vo
     set_error("ra_small_m_linear: need 1 <= M <= 8 and K % 8 == 0");
     return kHostBadArg;
   }
-  const int blocks = (N * 32 + 255) / 256;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
+  if (row_linear_takes(M, K)) return launch_row_linear(PRO_NONE, false, x, w, y, res, nullptr, 0.f, N, K, s);
+  const int blocks = (N * 32 + 255) / 256;
   const __nv_bfloat16* xx = static_cast<const __nv_bfloat16*>(x);
   const __nv_bfloat16* ww = static_cast<const __nv_bfloat16*>(w);
   __nv_bfloat16* yy = static_cast<__nv_bfloat16*>(y);
@@ -1470,6 +1668,17 @@ extern "C" int ra_small_m_linear(const void* x, const void* w, void* y, const vo
   return check_launch("small_m_linear_kernel");
 }
 
+// One row: y (F) = silu(n Wg^T) * (n Wu^T) for n = rmsnorm(x) * gain and w = [Wg | Wu] (2 F, K).
+extern "C" int ra_row_norm_gated(const void* x, const void* w, void* y, const void* gain, float eps, int F, int K, void* stream) {
+  using namespace ra::decode;
+  if (K % 8 || F < 1 || !gain || !row_linear_takes(1, K)) {
+    set_error("ra_row_norm_gated: need K % 8 == 0, a gain and K up to ra_row_linear_max_k()");
+    return kHostBadArg;
+  }
+  return launch_row_linear(PRO_RMSNORM, true, x, w, y, nullptr, gain, eps, F, K, static_cast<cudaStream_t>(stream));
+}
+extern "C" int ra_row_linear_max_k() { return ra::decode::ROW_MAX_CHUNKS * 256 * ra::decode::ROW_WARPS; }
+
 // Shared memory the prologue variant needs: M * K bf16. The Python side falls back to two launches above this.
 extern "C" int ra_small_m_linear_fused_max_smem() { return 48 * 1024; }
 
@@ -1483,6 +1692,7 @@ extern "C" int ra_small_m_linear_fused(const void* x, const void* w, void* y, co
               "with a gain) or 2 (SwiGLU)");
     return kHostBadArg;
   }
+  if (row_linear_takes(M, K)) return launch_row_linear(prologue, false, x, w, y, res, gain, eps, N, K, static_cast<cudaStream_t>(stream));
   // columns per warp: the whole grid resident at once (four CTAs of 256 threads per SM)
   const int resident = sm_count() * 4;
   int cpw = (N + 8 * resident - 1) / (8 * resident);

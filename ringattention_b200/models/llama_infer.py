@@ -197,7 +197,8 @@ class LlamaInference(InferenceEngine):
         x = K.embedding_fwd(tokens, P.w("embed"))
         for l in range(cfg.n_layers):
             # RMSNorm runs in the prologue of the projection, RoPE and the cache append share a launch, and
-            # SwiGLU runs in the prologue of the down projection: 7 launches per layer instead of 11 (13 on a ring)
+            # SwiGLU runs behind the gate/up projection (one sequence) or in the prologue of the down projection: 7 launches
+            # per layer instead of 11 (13 on a ring)
             qkv = K.norm_linear(x, P.w(f"l{l}.n1"), cfg.rms_eps, P.w(f"l{l}.wqkv"))
             q = qkv.view(B, 1, 3, H, D)[:, :, 0]
             if self.streams:  # shared prefix: the new K/V go to the streams' private tails
@@ -212,8 +213,7 @@ class LlamaInference(InferenceEngine):
                                                 None, self.axis, self.symm_ring, k_pos0=0, state=self.state,
                                                 exchange=l, exchanges_per_step=cfg.n_layers, stripe=stripe)
             x = K.linear_auto(attn.reshape(B, d), P.w(f"l{l}.wo"), residual=x)
-            gu = K.norm_linear(x, P.w(f"l{l}.n2"), cfg.rms_eps, P.w(f"l{l}.wgu"))
-            x = K.swiglu_linear(gu, P.w(f"l{l}.wd"), residual=x)
+            x = K.norm_swiglu_linear(x, P.w(f"l{l}.n2"), cfg.rms_eps, P.w(f"l{l}.wgu"), P.w(f"l{l}.wd"), residual=x)
         logits = K.norm_linear(x, P.w("nf"), cfg.rms_eps, P.w("lm_head")).float()
         K.decode_advance(self.state)
         return logits

@@ -410,6 +410,18 @@ def swiglu_linear(gu, w, residual=None, out=None):
     return linear_auto(swiglu_fwd(gu), w, out=out, residual=residual)
 
 
+def norm_swiglu_linear(x, gain, eps: float, wgu, wd, residual=None):
+    """``(silu(g) * u) Wd^T (+ residual)`` for ``[g | u] = rmsnorm(x) [Wg ; Wu]^T``: the feed-forward half of a decoder layer. One
+    row takes two launches with the activation behind the first; several rows :func:`norm_linear` and :func:`swiglu_linear`."""
+    F = wd.shape[1]
+    assert wgu.shape == (2 * F, x.shape[1])
+    if _fused_small_m_ok(x, wgu) and x.shape[0] == 1 and x.shape[1] <= _lib.lib().ra_row_linear_max_k():
+        h = torch.empty(1, F, device=x.device, dtype=torch.bfloat16)
+        _lib.call("ra_row_norm_gated", ptr(x), ptr(wgu), ptr(h), ptr(gain), c_f(eps), F, x.shape[1], stream_ptr())
+        return linear_auto(h, wd, residual=residual)
+    return swiglu_linear(norm_linear(x, gain, eps, wgu), wd, residual=residual)
+
+
 def rope_append(qkv, k_cache, v_cache, pos_state, theta: float, k0: int = 0, stripe=None):
     """RoPE of the q and k heads of a one-token ``(B, 1, 3, H, D)`` qkv buffer, in place, at the position in
     ``pos_state[0]``, and the cache append of :func:`kv_append` (rotated K, V), in one launch."""

@@ -485,3 +485,32 @@ def test_decode_mask_bits_at_the_edges_of_a_range(S, off, ql, D):
     x = (torch.einsum("bqhd,bkhd->bhqk", q.double(), k.double()) / D ** 0.5).masked_fill(~m, -float("inf"))
     want = torch.einsum("bhqk,bkhd->bqhd", torch.softmax(x, -1).nan_to_num(0.0), v.double())
     assert (out.double() - want).abs().max() <= 0.01 * want.abs().max() + 1e-3
+
+
+@pytest.mark.parametrize("N,K", [(1, 8), (7, 2040), (8, 2048), (2371, 2056), (4740, 64), (4096, 4096), (130, 5504), (64, 12288), (64, 12296)])
+def test_row_products_at_the_edges_of_their_tiles(N, K):
+    """One row against few and many columns, K in one, two, four and six chunks, none of them full, and past the last. Sums are fp32
+    and the output is rounded to bf16, 2^-8 of the value; f(x) is rounded to bf16 before the product: term i is off by at most
+    a_i = 2^-9 |f_i w_i|, the sum by 7 sqrt(sum a_i^2) but once in 10^10 (Hoeffding)."""
+    from ringattention_b200.ops import kernels as Kn
+
+    g = torch.Generator(device="cuda").manual_seed(N + K)
+    rnd = lambda *s: torch.randn(*s, device="cuda", generator=g).bfloat16()
+    x, w, r, gain, x2 = rnd(1, K), rnd(N, K), rnd(1, N), rnd(K), rnd(1, 2 * K)
+
+    def close(got, f, w, r=0.0, rounded=7 * 2.0 ** -9):
+        want = f @ w.double().t() + r
+        off = rounded * (f.square() @ w.double().square().t()).sqrt() + 2 ** -8 * want.abs() + 1e-5 * K ** 0.5
+        assert bool(((got.double() - want).abs() <= off).all())
+
+    close(Kn.linear_auto(x, w, residual=r), x.double(), w, r.double(), rounded=0.0)
+    n = x.double() * torch.rsqrt(x.double().square().mean() + 1e-5) * gain.double()
+    close(Kn.norm_linear(x, gain, 1e-5, w), n, w)
+    close(Kn.swiglu_linear(x2, w, residual=r), torch.nn.functional.silu(x2[:, :K].double()) * x2[:, K:].double(), w, r.double())
+    # the gated pair: gate and up are rounded as the two-launch form rounds them; where a sum's order puts one across a rounding
+    # border, h moves by 2^-8 of its value: twice the error of one rounding
+    F = max(8, N // 8 * 8)
+    wgu, wd, r = (rnd(2 * F, K).double() * K ** -0.5).bfloat16(), rnd(40, F), rnd(1, 40)
+    gu = Kn.norm_linear(x, gain, 1e-5, wgu).double()
+    h = torch.nn.functional.silu(gu[:, :F]) * gu[:, F:]
+    close(Kn.norm_swiglu_linear(x, gain, 1e-5, wgu, wd, residual=r), h, wd, r.double(), rounded=7 * 3 * 2.0 ** -9)
