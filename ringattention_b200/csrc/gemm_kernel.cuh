@@ -50,6 +50,7 @@ struct Params {
   // entries rounded up to a multiple of 32; null: neither)
   const float* bias;
   float alpha;
+  int r_fp32;  // the addend is fp32 although C is bf16 (the last part of a sum that is kept in fp32)
 };
 
 constexpr int MAX_SHARDS = 8;
@@ -332,7 +333,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
       const int n0 = tn * BN;
       // The fp32 addend is loaded one chunk of 32 columns ahead, the first while the tile's products still run: with a
       // short K the epilogue would otherwise be a chain of memory round trips longer than the main loop.
-      const bool add32 = p.c_fp32 && p.R && row < p.M;
+      const bool add32 = (p.c_fp32 || p.r_fp32) && p.R && row < p.M;
       float4 ahead[8];
       auto load_addend = [&](int c) {
         const float* src = reinterpret_cast<const float*>(p.R) + static_cast<long long>(row) * p.ldr + n0 + c * 32;
@@ -401,7 +402,18 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
               r[e] = __float_as_uint(v * v);
             }
           }
-          if (p.C2 && col0 >= p.n_split) {
+          const bool tail = p.C2 && col0 >= p.n_split;
+          if (add32 && !tail) {
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+              r[4 * j] = __float_as_uint(__uint_as_float(r[4 * j]) + ahead[j].x);
+              r[4 * j + 1] = __float_as_uint(__uint_as_float(r[4 * j + 1]) + ahead[j].y);
+              r[4 * j + 2] = __float_as_uint(__uint_as_float(r[4 * j + 2]) + ahead[j].z);
+              r[4 * j + 3] = __float_as_uint(__uint_as_float(r[4 * j + 3]) + ahead[j].w);
+            }
+            if (c + 1 < BN / 32) load_addend(c + 1);
+          }
+          if (tail) {
             float* dst = p.C2 + static_cast<long long>(row) * p.ldc2 + (col0 - p.n_split);
 #pragma unroll
             for (int j = 0; j < 8; ++j)
@@ -411,20 +423,11 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
                                 __uint_as_float(r[4 * j + 3]));
           } else if (p.c_fp32) {
             float* dst = reinterpret_cast<float*>(p.C) + static_cast<long long>(row) * p.ldc + col0;
-            float4 now[8];
-            if (add32) {
-#pragma unroll
-              for (int j = 0; j < 8; ++j) now[j] = ahead[j];
-              if (c + 1 < BN / 32) load_addend(c + 1);
-            }
 #pragma unroll
             for (int j = 0; j < 8; ++j) {
               if (col0 + j * 4 < p.N) {
-                float4 v = make_float4(__uint_as_float(r[4 * j]), __uint_as_float(r[4 * j + 1]),
-                                       __uint_as_float(r[4 * j + 2]), __uint_as_float(r[4 * j + 3]));
-                if (add32) {
-                  v.x += now[j].x; v.y += now[j].y; v.z += now[j].z; v.w += now[j].w;
-                }
+                const float4 v = make_float4(__uint_as_float(r[4 * j]), __uint_as_float(r[4 * j + 1]),
+                                             __uint_as_float(r[4 * j + 2]), __uint_as_float(r[4 * j + 3]));
                 if (RA_IN_BOUNDS(row, 1, p.M, kTagGemmStore) && RA_IN_BOUNDS(col0 + 4 * j, 4, p.N, kTagGemmStore))
                   *reinterpret_cast<float4*>(dst + 4 * j) = v;
               }
@@ -438,7 +441,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
                 float f[8];
 #pragma unroll
                 for (int e = 0; e < 8; ++e) f[e] = __uint_as_float(r[8 * j + e]);
-                if (p.R) {
+                if (p.R && !p.r_fp32) {
                   const uint4 o = *reinterpret_cast<const uint4*>(
                       reinterpret_cast<const __nv_bfloat16*>(p.R) + static_cast<long long>(row) * p.ldr + col0 + 8 * j);
                   const __nv_bfloat162* ob = reinterpret_cast<const __nv_bfloat162*>(&o);

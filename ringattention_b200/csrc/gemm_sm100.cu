@@ -78,7 +78,7 @@ int launch_bn(const Operands& o, const Params& p, cudaStream_t stream) {
 
 template <int A_MN, int B_MN>
 int launch(const Operands& o, const Params& p, cudaStream_t stream) {
-  const int bn = choose_bn((p.M + BM - 1) / BM, p.N, (p.K + BK - 1) / BK, p.c_fp32 && p.R);
+  const int bn = choose_bn((p.M + BM - 1) / BM, p.N, (p.K + BK - 1) / BK, (p.c_fp32 || p.r_fp32) && p.R);
   if (bn == 256) return launch_bn<A_MN, B_MN, 256>(o, p, stream);
   if (bn == 128) return launch_bn<A_MN, B_MN, 128>(o, p, stream);
   return launch_bn<A_MN, B_MN, 64>(o, p, stream);
@@ -90,14 +90,14 @@ int launch(const Operands& o, const Params& p, cudaStream_t stream) {
 
 // C[M,N] (ldc) = A * B^T (+ R). a_mn = 0: A is [M][lda] (K contiguous); 1: A is [K][lda] (M
 // contiguous). b_mn = 0: B is [N][ldb]; 1: B is [K][ldb]. All leading dimensions in elements and
-// multiples of 8; base pointers 16-byte aligned. c_fp32 selects the type of C and R. R is an
-// optional addend (residual or running gradient) and may alias C for in-place accumulation.
+// multiples of 8; base pointers 16-byte aligned. c_fp32 selects the type of C and R (1: fp32, 0: bf16, 2: C bf16 and R fp32). R is
+// an optional addend (residual or running gradient) and may alias C for in-place accumulation where their types agree.
 extern "C" int ra_gemm_bf16(const void* A, const void* B, void* C, const void* R, int M, int N,
                             int K, long long lda, long long ldb, long long ldc, long long ldr,
                             int a_mn, int b_mn, int c_fp32, int group_m, int* status,
                             void* stream) {
   using namespace ra;
-  if (M <= 0 || N <= 0 || K <= 0 || (lda % 8) || (ldb % 8) || (ldc % (c_fp32 ? 4 : 8)) ||
+  if (M <= 0 || N <= 0 || K <= 0 || (lda % 8) || (ldb % 8) || (ldc % (c_fp32 == 1 ? 4 : 8)) ||
       (reinterpret_cast<uintptr_t>(A) & 15) || (reinterpret_cast<uintptr_t>(B) & 15) ||
       (reinterpret_cast<uintptr_t>(C) & 15) || (reinterpret_cast<uintptr_t>(R) & 15) ||
       (R && (ldr % (c_fp32 ? 4 : 8)))) {
@@ -105,7 +105,8 @@ extern "C" int ra_gemm_bf16(const void* A, const void* B, void* C, const void* R
     return kHostBadArg;
   }
   const gemm::Operands o{A, B, lda, ldb};
-  gemm::Params p{C, ldc, M, N, K, c_fp32, R, ldr, group_m > 0 ? group_m : 8, status, 0};
+  gemm::Params p{C, ldc, M, N, K, c_fp32 == 1, R, ldr, group_m > 0 ? group_m : 8, status, 0};
+  p.r_fp32 = c_fp32 == 2;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   if (!a_mn && !b_mn) return gemm::launch<0, 0>(o, p, s);
   if (!a_mn && b_mn) return gemm::launch<0, 1>(o, p, s);

@@ -26,12 +26,32 @@ from ..config import POLICY_NOTHING_SAVEABLE, _policy_name
 from . import kernels as K
 
 
-class DenseLinears:
-    """The four products of the feed-forward on plain ``(N, K)`` bf16 weight tensors."""
+class WeightGrad:
+    """Gradient of one ``(N, K)`` bf16 weight, summed over ``parts`` products ``dy^T x``: fp32 between them, and the last one leaves in the
+    weight's type, so that nothing is zeroed first or cast afterwards (d 4096, F 11008: 205 of 7200 us; d 1024, one part: four
+    of thirteen launches)."""
 
-    def __init__(self, wgu: torch.Tensor, wd: torch.Tensor, dwgu: Optional[torch.Tensor] = None,
-                 dwd: Optional[torch.Tensor] = None):
-        self.wgu, self.wd, self.dwgu, self.dwd = wgu, wd, dwgu, dwd
+    def __init__(self, w: torch.Tensor, parts: int):
+        self.w, self.left, self.acc, self.grad = w, parts, None, None
+
+    def add(self, dy, x):
+        self.left -= 1
+        if self.left == 0:
+            self.grad = K.gemm(dy, x, a_mn=True, b_mn=True, out=torch.empty(self.w.shape, device=self.w.device, dtype=self.w.dtype),
+                               residual=self.acc)
+            self.acc = None
+        elif self.acc is None:
+            self.acc = K.gemm(dy, x, a_mn=True, b_mn=True, out_dtype=torch.float32)
+        else:
+            K.linear_wgrad(dy, x, self.acc)
+
+
+class DenseLinears:
+    """The four products of the feed-forward on plain ``(N, K)`` bf16 weight tensors; ``parts``: chunks of a backward pass."""
+
+    def __init__(self, wgu: torch.Tensor, wd: torch.Tensor, parts: int = 0):
+        self.wgu, self.wd = wgu, wd
+        self.dwgu, self.dwd = WeightGrad(wgu, parts), WeightGrad(wd, parts)
 
     def gate_up(self, x):                      # (rows, 2F) pre-activations
         return K.linear_fwd(x, self.wgu)
@@ -46,10 +66,10 @@ class DenseLinears:
         return K.linear_dgrad(dy, self.wd)
 
     def down_wgrad(self, dy, a):
-        K.linear_wgrad(dy, a, self.dwd)
+        self.dwd.add(dy, a)
 
     def gate_up_wgrad(self, dgu, x):
-        K.linear_wgrad(dgu, x, self.dwgu)
+        self.dwgu.add(dgu, x)
 
     def gate_up_dgrad(self, dgu, out):
         return K.linear_dgrad(dgu, self.wgu, out=out)
@@ -105,11 +125,10 @@ class _BlockwiseSwiGLU(torch.autograd.Function):
     def backward(ctx, dy):
         x2, wgu, wd = ctx.saved_tensors
         dy = dy.contiguous()
-        dwgu = torch.zeros(wgu.shape, device=wgu.device, dtype=torch.float32)
-        dwd = torch.zeros(wd.shape, device=wd.device, dtype=torch.float32)
-        dx = ffn_backward(DenseLinears(wgu, wd, dwgu, dwd), x2, dy, ctx.chunk, kept=ctx.kept)
+        lin = DenseLinears(wgu, wd, -(-x2.shape[0] // min(ctx.chunk, x2.shape[0])))
+        dx = ffn_backward(lin, x2, dy, ctx.chunk, kept=ctx.kept)
         ctx.kept = None
-        return dx, dwgu.to(wgu.dtype), dwd.to(wd.dtype), None, None
+        return dx, lin.dwgu.grad, lin.dwd.grad, None, None
 
 
 class FusedSwiGLU(torch.nn.Module):

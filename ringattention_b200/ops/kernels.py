@@ -32,7 +32,7 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
 
     ``a`` is ``(M, K)`` (``a_mn=False``) or ``(K, M)`` (``a_mn=True``); ``b`` is ``(N, K)`` or
     ``(K, N)``. Both are 2-D bf16 with a contiguous last dim. ``residual`` has C's dtype and may be
-    ``out`` itself (in-place accumulation, used for fp32 weight-gradient accumulation).
+    ``out`` itself (in-place accumulation, used for fp32 weight-gradient accumulation), or is fp32 where C is bf16.
     """
     assert a.dtype == torch.bfloat16 and b.dtype == torch.bfloat16 and a.dim() == 2 and b.dim() == 2
     assert a.stride(1) == 1 and b.stride(1) == 1
@@ -50,7 +50,10 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
     assert out.shape == (M, N) and out.stride(1) == 1
     c_fp32 = 1 if out.dtype == torch.float32 else 0
     if residual is not None:
-        assert residual.dtype == out.dtype and residual.shape == out.shape and residual.stride(1) == 1
+        assert residual.shape == out.shape and residual.stride(1) == 1
+        assert residual.dtype == out.dtype or (residual.dtype, out.dtype) == (torch.float32, torch.bfloat16)
+        if residual.dtype != out.dtype:
+            c_fp32 = 2
     _lib.call("ra_gemm_bf16", ptr(a), ptr(b), ptr(out), ptr(residual), M, N, K,
               c_ll(a.stride(0)), c_ll(b.stride(0)), c_ll(out.stride(0)),
               c_ll(residual.stride(0) if residual is not None else 0),

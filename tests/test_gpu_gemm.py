@@ -99,3 +99,20 @@ def test_swiglu_epilogue_at_every_tile_width(M, F, Kd):
     gu = K.linear_fwd(x, w).float()
     want = torch.nn.functional.silu(gu[:, :F]) * gu[:, F:]
     assert ((got.float() - want).abs() <= 2**-7 * want.abs() + 1e-4).all()
+
+
+@pytest.mark.parametrize("a_mn,b_mn", [(False, False), (True, True)])
+@pytest.mark.parametrize("M,N,Kd", [(8, 8, 8), (104, 72, 200), (2048, 1024, 328), (4000, 1544, 136)])
+def test_gemm_fp32_addend_bf16_result(M, N, Kd, a_mn, b_mn):
+    """The last part of a sum kept in fp32, at tiles of 64, 128 and 256 columns: one rounding to bf16 (2^-8 of the value at most)
+    beside 2e-6 of the sum of the magnitudes."""
+    from ringattention_b200.ops import kernels as K
+
+    g = torch.Generator(device="cuda").manual_seed(M + N)
+    a, b = torch.randn(M, Kd, device="cuda", generator=g).bfloat16(), torch.randn(N, Kd, device="cuda", generator=g).bfloat16()
+    r = torch.randn(M, N + 12, device="cuda", generator=g)[:, :N]
+    A, B = (a.t().contiguous() if a_mn else a), (b.t().contiguous() if b_mn else b)
+    got = K.gemm(A, B, a_mn=a_mn, b_mn=b_mn, out=torch.empty(M, N, device="cuda", dtype=torch.bfloat16), residual=r)
+    want = a.double() @ b.double().t() + r.double()
+    slack = 2e-6 * (a.double().abs() @ b.double().abs().t() + r.double().abs())
+    assert ((got.double() - want).abs() <= slack + 2**-8 * want.abs()).all()
