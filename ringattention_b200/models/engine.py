@@ -19,7 +19,10 @@ class InferenceEngine:
         # [position, step] on the device: lets one recorded CUDA graph serve every decode step
         self.state = torch.zeros(2, dtype=torch.int64, device=self.device)
         self._graph = None
-        self._old_graph = None                      # the one recorded before reset(): the next one takes over its buffers
+        self._old_graph = None                      # one that no longer serves: the next one takes over its buffers
+        self._recorded = None                       # launch constants of the recorded step
+        self._reset_since = False                   # reset() since it was recorded
+        self._state_at = 0                          # position in `state`
         self._tok_buf = torch.zeros(token_rows, dtype=torch.int32, device=self.device)
 
     # ------------------------------------------------------------------ supplied by the engine
@@ -53,21 +56,40 @@ class InferenceEngine:
         self.state[0] = self.length
         logits = self._decode_body(tokens.to(self.device, torch.int32).reshape(-1).contiguous())
         self.length += 1
+        self._state_at = self.length
         return logits
 
     @torch.no_grad()
     def decode_step_graph(self) -> torch.Tensor:
-        """Greedy step on the token in ``self._tok_buf`` through a CUDA graph recorded on first use:
+        """Greedy step on the token in ``self._tok_buf`` through a CUDA graph recorded on first use (see :meth:`launch_constants`):
         one replay per token instead of a handful of launches per layer. Writes the next token back into
         ``self._tok_buf`` and returns it. Call :meth:`decode_step` at least once before (buffers and
         kernels must exist before capture)."""
         self._check_room(1)
-        if self._graph is None:
+        if self._state_at != self.length:
             self.state[0] = self.length
+        if not self._graph_serves():
+            self._graph, self._old_graph = None, self._graph or self._old_graph
             self._graph = self._record(self._greedy_step)
+            self._recorded = self.launch_constants()
         self._graph.replay()
         self.length += 1
+        self._state_at = self.length
         return self._tok_buf
+
+    def launch_constants(self):
+        """What a recorded decode step holds beside the engine's own buffers, integers and objects: it is replayed for as long as these are
+        the same (None: a property of the context, record again after every reset)."""
+        return None
+
+    def _graph_serves(self) -> bool:
+        if self._graph is None:
+            return False
+        now = self.launch_constants()
+        if now is None or self._recorded is None:
+            return not self._reset_since
+        return len(now) == len(self._recorded) and all(
+            a is b or (isinstance(a, int) and isinstance(b, int) and a == b) for a, b in zip(now, self._recorded))
 
     def _greedy_step(self) -> None:
         logits = self._decode_body(self._tok_buf)
@@ -92,15 +114,16 @@ class InferenceEngine:
                 g.capture_end()
         torch.cuda.current_stream().wait_stream(side)
         self._old_graph = None
+        self._reset_since = False
         return g
 
     def reset(self) -> None:
-        """Forget the cached context (the cache memory is kept). The recorded decode graph is dropped
-        too: it may hold properties of the prefilled context as launch constants."""
+        """Forget the cached context (the cache memory is kept). The recorded decode graph stays for as long as its launch
+        constants do."""
         self.length = 0
         self.state.zero_()
-        if self._graph is not None:
-            self._graph, self._old_graph = None, self._graph
+        self._state_at = 0
+        self._reset_since = True
         self._clear_cache()
 
     # ------------------------------------------------------------------ generation
@@ -121,12 +144,13 @@ class InferenceEngine:
         out: List[torch.Tensor] = []
         lat: List[float] = []
         nxt = self.first_tokens(logits)
+        eager = 0 if self._graph_serves() else 2    # buffers and kernels must exist before a step is recorded
         for i in range(new_tokens):
             out.append(nxt.clone())
             e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
             e0.record()
-            if use_graph and i >= 2:
-                if i == 2:
+            if use_graph and i >= eager:
+                if i == eager:
                     self._tok_buf.copy_(nxt.to(torch.int32))
                 nxt = self.decode_step_graph()
             else:

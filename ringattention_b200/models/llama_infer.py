@@ -192,7 +192,8 @@ class LlamaInference(InferenceEngine):
         slot, barrier count) is read from device memory, so the sequence can be graph-captured."""
         cfg, P = self.cfg, self.params
         B, H, D, d = (self.streams or self.B), self.H, self.D, self.d
-        stripe = (self.world, self.rank, self.n_rows, self.prefill_len)
+        # one rank: rows are positions, and the recorded step holds nothing of the prompt
+        stripe = (self.world, self.rank, self.n_rows, self.prefill_len) if self.world > 1 or self.streams else None
         tail_stripe = (self.world, self.rank, 0, self.prefill_len)
         x = K.embedding_fwd(tokens, P.w("embed"))
         for l in range(cfg.n_layers):
@@ -217,6 +218,10 @@ class LlamaInference(InferenceEngine):
         logits = K.norm_linear(x, P.w("nf"), cfg.rms_eps, P.w("lm_head")).float()
         K.decode_advance(self.state)
         return logits
+
+    def launch_constants(self):
+        held = (self.params, self.params.p16_shard, self.params.p16_rep, *self.k_cache, *self.v_cache)
+        return held + (self.n_rows, self.prefill_len) if self.world > 1 or self.streams else held
 
     def _clear_cache(self) -> None:
         self.n_rows = self.prefill_len = 0

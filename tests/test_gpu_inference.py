@@ -514,3 +514,26 @@ def test_row_products_at_the_edges_of_their_tiles(N, K):
     gu = Kn.norm_linear(x, gain, 1e-5, wgu).double()
     h = torch.nn.functional.silu(gu[:, :F]) * gu[:, F:]
     close(Kn.norm_swiglu_linear(x, gain, 1e-5, wgu, wd, residual=r), h, wd, r.double(), rounded=7 * 3 * 2.0 ** -9)
+
+
+def test_recorded_step_is_kept_over_prompts_and_dropped_with_the_weights():
+    from ringattention_b200.config import LlamaConfig
+    from ringattention_b200.models.llama_infer import LlamaInference
+
+    cfg = LlamaConfig.named("llama-tiny")
+    torch.manual_seed(6)
+    prompts = [torch.randint(0, cfg.vocab_size, (2, n), device="cuda") for n in (256, 128, 384)]
+    fresh = lambda seed, p: LlamaInference(cfg, max_context=1024, batch=2, seed=seed).generate(p, 7)[0]
+    eng = LlamaInference(cfg, max_context=1024, batch=2, seed=9)
+    assert torch.equal(eng.generate(prompts[0], 7)[0], fresh(9, prompts[0]))
+    graph = eng._graph
+    assert torch.equal(eng.generate(prompts[1], 7)[0], fresh(9, prompts[1])) and eng._graph is graph
+    eng.decode_step(torch.zeros(2, dtype=torch.int64, device="cuda"))  # an eager step between replays
+    eng.reset()
+    other = LlamaInference(cfg, max_context=1024, batch=2, seed=5).params
+    eng.params = other
+    assert torch.equal(eng.generate(prompts[2], 7)[0], fresh(5, prompts[2])) and eng._graph is not graph
+    graph = eng._graph
+    eng.params.p16_rep.mul_(1.5)  # in place: the recorded step reads what is there
+    want = LlamaInference(cfg, max_context=1024, batch=2, params=other).generate(prompts[0], 7)[0]
+    assert torch.equal(eng.generate(prompts[0], 7)[0], want) and eng._graph is graph
