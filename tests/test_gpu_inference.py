@@ -350,7 +350,7 @@ def test_streams_sharing_one_cached_context():
 @pytest.mark.parametrize("D", [64, 128])
 @pytest.mark.parametrize("nparts", [1, 15, 16, 33, 512, 1100])
 def test_merge_of_few_and_many_partials(nparts, D):
-    """Both forms of the merge (from 16 partials on by 32 warps), with empty partials, a row without any and strided
+    """All forms of the merge (a thread per column, 8 and 32 warps), with empty partials, a row without any and strided
     inputs. Tolerance: fp32 weights by exp of a difference below 40, 4e-6 relative, times sums of up to 1100 terms."""
     from ringattention_b200.ops import decode as Dk
 
@@ -537,3 +537,30 @@ def test_recorded_step_is_kept_over_prompts_and_dropped_with_the_weights():
     eng.params.p16_rep.mul_(1.5)  # in place: the recorded step reads what is there
     want = LlamaInference(cfg, max_context=1024, batch=2, params=other).generate(prompts[0], 7)[0]
     assert torch.equal(eng.generate(prompts[0], 7)[0], want) and eng._graph is graph
+
+
+@pytest.mark.parametrize("Sq,Sk", [(1, 16), (4, 144), (130, 272), (300, 4096), (33, 500), (2, 2040)])
+def test_mask_rows_at_multiples_of_sixteen_bytes(Sq, Sk):
+    """The bitmaps and kinds of tiles of a mask do not depend on where its rows start: rows at multiples of 16 bytes (whole and ragged
+    ends), rows that are not, a row shared by all queries, and bytes of any value."""
+    from ringattention_b200.ops import flash
+
+    g = torch.Generator(device="cuda").manual_seed(Sq + Sk)
+    B, H, ld = 2, 3, (Sk + 15) // 16 * 16 + 16
+    m = torch.randint(0, 256, (B, H, Sq, Sk), device="cuda", generator=g, dtype=torch.uint8)
+    m *= torch.rand(B, H, Sq, Sk, device="cuda", generator=g) < 0.4
+    m[0, 0], m[0, 1] = 0, 128
+    room = torch.full((B, H, Sq, ld + 1), 7, device="cuda", dtype=torch.uint8)
+    at16 = torch.full((B, H, Sq, ld), 9, device="cuda", dtype=torch.uint8)
+    odd = room[..., 1:1 + Sk]
+    odd.copy_(m)
+    at16[..., :Sk].copy_(m)
+    for a, b in zip(flash.mask_bitmaps(at16[..., :Sk]), flash.mask_bitmaps(odd)):
+        assert torch.equal(a, b)
+    want = torch.zeros(B, H, Sq, 128 * ((Sk + 127) // 128), device="cuda", dtype=torch.int64)
+    want[..., :Sk] = m != 0
+    words = (want.view(B, H, Sq, -1, 32) << torch.arange(32, device="cuda")).sum(-1)
+    assert torch.equal(flash.mask_bitmaps(at16[..., :Sk])[0].long() & 0xffffffff, words)
+    one = at16[:, :, :1, :Sk].expand(B, H, Sq, Sk)
+    for a, b in zip(flash.mask_bitmaps(one), flash.mask_bitmaps(odd[:, :, :1].expand(B, H, Sq, Sk))):
+        assert torch.equal(a, b)
