@@ -200,27 +200,28 @@ __global__ void __launch_bounds__(256, 2) rmsnorm_bwd_kernel(const __nv_bfloat16
   }
 }
 
-// dw[c] += sum over the `parts` partial rows. A CTA takes 32 columns, its 32 warps every 32nd partial row (128 coalesced
-// bytes a load, four in flight), and the warps' sums meet in shared memory in a fixed order. What bounds it is the latency
-// of the chain of loads: with one thread per column walking all ~590 rows it took 85 us at any width (4 CTAs of 256 threads
-// at d = 1024), an eighth of a small decoder's training step; 19 rows a thread take 5 us.
-constexpr int DW_ROWS = 32;
-__global__ void __launch_bounds__(32 * DW_ROWS) rmsnorm_dw_reduce_kernel(const float* __restrict__ dw_part,
-                                                                         float* __restrict__ dw, int parts, int d) {
-  __shared__ float sums[DW_ROWS][33];
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const int c = blockIdx.x * 32 + lane;
+// dw[c] += sum over the `parts` partial rows (2368 for 4096 rows of x). A CTA takes eight columns, 128 groups of eight threads every 128th
+// partial row (a 32-byte sector a load, eight in flight), and their sums meet in shared memory in a fixed order. What bounds it is
+// the latency of the chains of loads and how many SMs take part: one thread per column walking all rows took 85 us at any width, an
+// eighth of a small decoder's training step; 32 columns a CTA (32 CTAs at d = 1024) 9.4 us, eight 4.5 us.
+constexpr int DW_COLS = 8, DW_ROWS = 128;
+__global__ void __launch_bounds__(DW_COLS * DW_ROWS) rmsnorm_dw_reduce_kernel(const float* __restrict__ dw_part,
+                                                                              float* __restrict__ dw, int parts, int d) {
+  __shared__ float sums[DW_ROWS][DW_COLS + 1];
+  const int r = threadIdx.x / DW_COLS, c = blockIdx.x * DW_COLS + threadIdx.x % DW_COLS;  // d is a multiple of DW_COLS
   float acc = 0.f;
-  if (c < d) {
-#pragma unroll 4
-    for (int p = w; p < parts; p += DW_ROWS) acc += dw_part[static_cast<long long>(p) * d + c];
-  }
-  sums[w][lane] = acc;
+#pragma unroll 8
+  for (int p = r; p < parts; p += DW_ROWS) acc += dw_part[static_cast<long long>(p) * d + c];
+  sums[r][threadIdx.x % DW_COLS] = acc;
   __syncthreads();
-  // warp w sums column w of the 32: one row's partial sum per lane
-  acc = warp_sum(sums[lane][w]);
-  const int col = blockIdx.x * 32 + w;
-  if (lane == 0 && col < d && RA_IN_BOUNDS(col, 1, d, kTagRmsnorm)) dw[col] += acc;
+  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (w >= DW_COLS) return;  // warp w sums column w
+  acc = 0.f;
+#pragma unroll
+  for (int i = 0; i < DW_ROWS; i += 32) acc += sums[i + lane][w];
+  acc = warp_sum(acc);
+  const int col = blockIdx.x * DW_COLS + w;
+  if (lane == 0 && RA_IN_BOUNDS(col, 1, d, kTagRmsnorm)) dw[col] += acc;
 }
 
 // ---------------------------------------------------------------------------------- RoPE
@@ -558,7 +559,7 @@ extern "C" int ra_rmsnorm_bwd(const void* dy, const void* x, const void* w, cons
   else rmsnorm_bwd_kernel<8><<<grid, 256, 0, s>>>(gp, xp, wp, rstd, rp, op, dw_part, rows, d);
   int rc = check_launch("rmsnorm_bwd");
   if (rc != kHostOk) return rc;
-  rmsnorm_dw_reduce_kernel<<<(d + 31) / 32, 32 * DW_ROWS, 0, s>>>(dw_part, dw, parts, d);
+  rmsnorm_dw_reduce_kernel<<<d / DW_COLS, DW_COLS * DW_ROWS, 0, s>>>(dw_part, dw, parts, d);
   return check_launch("rmsnorm_dw_reduce");
 }
 
