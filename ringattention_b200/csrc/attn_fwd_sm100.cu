@@ -645,6 +645,10 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constant
     constexpr int PIECES = HALF / 4;
     float own_mul = 1.f, other_mul = 0.f;      // factors of the two accumulators
     float* const other_row = reinterpret_cast<float*>(sK) + ((1 - w) * 128 + row) * HALF;  // what the other group left for us
+    // The carry's log-sum-exp. lse_out may be the same tensor (a ring accumulates in place), and with HALVES both groups need the value
+    // that one of them overwrites: so it is read here, ahead of the barriers below, and the store comes behind them.
+    const long long lse_idx = (static_cast<long long>(b) * p.H + h) * mk.Sq + qi;
+    const float lse_carry = p.o_prev && row_valid ? p.lse_prev[lse_idx] : -INFINITY;
     if (HALVES) {
       float2* stat = reinterpret_cast<float2*>(sSeg);  // [group][128]: masks are done with
       named_bar_sync(3, 256);
@@ -682,15 +686,13 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constant
       lse = (m_ref + log2f(l)) * kLn2;
     }
     float w_prev = 0.f, w_this = 1.f;
-    const long long lse_idx = (static_cast<long long>(b) * p.H + h) * mk.Sq + qi;
     if (p.o_prev && row_valid) {
-      const float lp = p.lse_prev[lse_idx];
-      const float mxl = fmaxf(lp, lse);
+      const float mxl = fmaxf(lse_carry, lse);
       if (mxl == -INFINITY) {
         w_prev = 0.f;
         w_this = 0.f;
       } else {
-        const float ep = __expf(lp - mxl), et = __expf(lse - mxl);
+        const float ep = __expf(lse_carry - mxl), et = __expf(lse - mxl);
         const float tot = ep + et;
         w_prev = ep / tot;
         w_this = et / tot;

@@ -226,3 +226,33 @@ def test_segment_ids_of_every_kind(ids, D):
 def test_every_way_a_forward_is_cut_up(B, Sq, Sk, H, cbs, cache_idx, D):
     """Sizes on both sides of the rule that gives a CTA two query tiles or one, and splits the keys of a few query tiles."""
     _check_call(B, Sq, Sk, H, D, cbs=cbs, cache_idx=cache_idx, grad=Sq * Sk * B * H < 3e8)
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("S,H,q_pos,k_pos", [
+    (512, 8, (0,), (0,)),                     # four query tiles a head: two groups on one tile
+    (2048, 4, (2048,), (0,)),                 # a block of earlier positions: every tile visible
+    (1000, 8, (0, 7168, 512), (512, 6656, 512)),  # two runs of positions a shard, a ragged last tile
+    (2048, 40, (0,), (0,)),                   # two query tiles a CTA
+])
+def test_carry_merged_in_place(S, H, q_pos, k_pos, D):
+    """A ring step gives the accumulator and the log-sum-exp of the steps before and has them overwritten by the merged ones:
+    the same bits as with tensors of their own, every time."""
+    from ringattention_b200.ops import flash
+
+    g = torch.Generator(device="cuda").manual_seed(S + H)
+    q, k, v = (torch.randn(1, S, H, D, device="cuda", generator=g).bfloat16() for _ in range(3))
+    ms = flash.MaskSpec(causal_block_size=1, q_pos=flash.Positions(*q_pos), k_pos=flash.Positions(*k_pos))
+    o_prev, lse_prev = torch.randn(1, S, H, D, device="cuda", generator=g), 6 + torch.randn(1, H, S, device="cuda", generator=g)
+    lse_prev[0, 0, 3] = -float("inf")  # no key seen yet
+    out, lse = flash.flash_fwd(q, k, v, ms, o_prev=o_prev, lse_prev=lse_prev, out_fp32=True)
+    alone, lse_alone = flash.flash_fwd(q, k, v, ms, out_fp32=True)
+    both = torch.logaddexp(lse_prev.double(), lse_alone.double())
+    w = [torch.exp(x.double() - both).nan_to_num(0.0).permute(0, 2, 1)[..., None] for x in (lse_prev, lse_alone)]
+    # the launch without a carry may be cut up otherwise: probabilities are rounded to bf16 (2^-9 of each) in both
+    assert (out.double() - w[0] * o_prev.double() - w[1] * alone.double()).abs().max() < 2 ** -8 * v.abs().max()
+    assert (lse.double() - both)[torch.isfinite(both)].abs().max() < 1e-5
+    for _ in range(300):
+        o, l = o_prev.clone(), lse_prev.clone()
+        flash.flash_fwd(q, k, v, ms, o_prev=o, lse_prev=l, out=o, lse_out=l)
+        assert torch.equal(o, out) and torch.equal(l, lse)
