@@ -21,7 +21,7 @@ class InferenceEngine:
         self._graph = None
         self._old_graph = None                      # one that no longer serves: the next one takes over its buffers
         self._recorded = None                       # launch constants of the recorded step
-        self._reset_since = False                   # reset() since it was recorded
+        self._reset_since = False                   # reset() since it was recorded or found to serve
         self._state_at = 0                          # position in `state`
         self._tok_buf = torch.zeros(token_rows, dtype=torch.int32, device=self.device)
 
@@ -71,25 +71,29 @@ class InferenceEngine:
         if not self._graph_serves():
             self._graph, self._old_graph = None, self._graph or self._old_graph
             self._graph = self._record(self._greedy_step)
-            self._recorded = self.launch_constants()
+            self._recorded = self._constants()
+        self._reset_since = False
         self._graph.replay()
         self.length += 1
         self._state_at = self.length
         return self._tok_buf
 
     def launch_constants(self):
-        """What a recorded decode step holds beside the engine's own buffers, integers and objects: it is replayed for as long as these are
-        the same (None: a property of the context, record again after every reset)."""
+        """Everything that a recorded decode step holds and that may be another thing for the next prompt, as plain values that compare by
+        ``==`` (addresses and layouts of the weights and caches, the configuration): after a :meth:`reset` the step is replayed if these are
+        still the same. None: record again after every reset (the default; also for a step with addresses in it that others
+        may free, as of buffers that are shared with peers or with other engines)."""
         return None
 
+    def _constants(self):
+        # a sampler of the caller's own may hold anything
+        return self.launch_constants() if self.sample is InferenceEngine.sample else None
+
     def _graph_serves(self) -> bool:
-        if self._graph is None:
-            return False
-        now = self.launch_constants()
-        if now is None or self._recorded is None:
-            return not self._reset_since
-        return len(now) == len(self._recorded) and all(
-            a is b or (isinstance(a, int) and isinstance(b, int) and a == b) for a, b in zip(now, self._recorded))
+        if self._graph is None or not self._reset_since:
+            return self._graph is not None
+        now = self._constants()
+        return now is not None and now == self._recorded
 
     def _greedy_step(self) -> None:
         logits = self._decode_body(self._tok_buf)
@@ -114,12 +118,10 @@ class InferenceEngine:
                 g.capture_end()
         torch.cuda.current_stream().wait_stream(side)
         self._old_graph = None
-        self._reset_since = False
         return g
 
     def reset(self) -> None:
-        """Forget the cached context (the cache memory is kept). The recorded decode graph stays for as long as its launch
-        constants do."""
+        """Forget the cached context (the cache memory is kept). The recorded decode graph stays if its launch constants do."""
         self.length = 0
         self.state.zero_()
         self._state_at = 0

@@ -21,6 +21,7 @@ of the chunk being prefilled are masked causally at their true positions.
 from __future__ import annotations
 
 import ctypes
+import dataclasses
 from typing import Optional
 
 import torch
@@ -220,8 +221,14 @@ class LlamaInference(InferenceEngine):
         return logits
 
     def launch_constants(self):
-        held = (self.params, self.params.p16_shard, self.params.p16_rep, *self.k_cache, *self.v_cache)
-        return held + (self.n_rows, self.prefill_len) if self.world > 1 or self.streams else held
+        # A ring's step holds addresses of symmetric buffers that grow, and are freed, at the call of anything else on the ring; a step of
+        # shared-prefix streams the prefix's length and the tails; a subclass's step what it likes. All of those are recorded per prompt.
+        if self.world > 1 or self.streams or getattr(self._decode_body, "__func__", None) is not LlamaInference._decode_body:
+            return None
+        P = self.params
+        held = (P.p16_shard, P.p16_rep, *self.k_cache, *self.v_cache)
+        return (dataclasses.astuple(self.cfg), tuple(P.mat.items()), tuple(P.rep.items()),
+                tuple((t.data_ptr(), t.shape, t.stride()) for t in held))
 
     def _clear_cache(self) -> None:
         self.n_rows = self.prefill_len = 0
