@@ -49,11 +49,14 @@ class InferenceEngine:
         return logits.argmax(dim=-1)
 
     # ------------------------------------------------------------------ decode
+    def _set_position(self) -> None:
+        self.state[0] = self._state_at = self.length
+
     @torch.no_grad()
     def decode_step(self, tokens: torch.Tensor) -> torch.Tensor:
         """One token per sequence: ``tokens (B,)`` -> logits ``(B, vocab)`` fp32 (same on all ranks)."""
         self._check_room(1)
-        self.state[0] = self.length
+        self._set_position()
         logits = self._decode_body(tokens.to(self.device, torch.int32).reshape(-1).contiguous())
         self.length += 1
         self._state_at = self.length
@@ -67,7 +70,7 @@ class InferenceEngine:
         kernels must exist before capture)."""
         self._check_room(1)
         if self._state_at != self.length:
-            self.state[0] = self.length
+            self._set_position()
         if not self._graph_serves():
             self._graph, self._old_graph = None, self._graph or self._old_graph
             self._graph = self._record(self._greedy_step)

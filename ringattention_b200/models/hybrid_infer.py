@@ -162,7 +162,7 @@ class HybridInference(InferenceEngine):
             raise ValueError("want names a place outside the step")
         if self.cut and T > self.max_step:
             return self._long_step(tokens, want, taps)
-        self.state[0] = self.length
+        self._set_position()
         idx = None
         if want is not None:
             idx = torch.tensor([b * T + w for b in range(B) for w in want], dtype=torch.int32, device=self.device)

@@ -135,3 +135,29 @@ def test_default_is_to_record_after_every_reset():
     for _ in range(3):
         _prompt(eng)
     assert len(n) == 3
+
+
+def test_a_replayed_step_stands_behind_the_tokens_of_a_step_before_it():
+    """The position on the device is written again whenever something else than a replay has moved it, also when the tokens between
+    lead back to the place of the last replay."""
+    from ringattention_b200.models import registry
+    from ringattention_b200.models.hybrid_infer import HybridInference
+
+    eng = HybridInference(registry.load_config("kalonex-tiny"), max_context=64, device="cpu")
+    eng._forward = lambda *a, **k: None
+    at = []
+
+    class Graph:  # a recorded step advances the position itself
+        def replay(self):
+            at.append(int(eng.state[0]))
+            eng.state[0] += 1
+
+    eng._record = lambda body: Graph()
+    tok = torch.zeros(1, 4, dtype=torch.int64)
+    eng.step(tok)
+    eng.decode_step_graph()
+    eng.decode_step_graph()
+    eng.length = 2
+    eng.step(tok)
+    eng.decode_step_graph()
+    assert at == [4, 5, 6] and eng.length == 7
