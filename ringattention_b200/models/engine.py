@@ -10,6 +10,12 @@ from typing import List
 
 import torch
 
+# Free memory of the device below which the allocator gives its cached blocks back before a step is recorded. While a capture is under way it
+# cannot, and the private pool of a capture takes none of them: the recording would run out of memory beside gigabytes of cached blocks, or
+# leave the driver nothing to upload the graph with. A step's own buffers are megabytes (the partial results of 512 splits of 64 heads 17, the
+# logits of eight sequences 1.5); a graph of 60 launches took 70.
+RECORD_ROOM = 1 << 30
+
 
 class InferenceEngine:
     def __init__(self, batch: int, device, token_rows: int):
@@ -103,10 +109,25 @@ class InferenceEngine:
         self._tok_buf.copy_(self.sample(logits).to(torch.int32))
 
     def _record(self, body) -> torch.cuda.CUDAGraph:
-        """Record ``body`` as ``torch.cuda.graph`` does, but leave the allocator's cached blocks and Python's garbage alone:
-        emptying the cache before every prompt's recording made the next prompt's prefill allocate all of its
-        buffers from the driver again. The buffers of the graph recorded before are taken over (it is dropped here)."""
+        """Record ``body`` as ``torch.cuda.graph`` does, but leave the allocator's cached blocks alone while the device has room
+        (:data:`RECORD_ROOM`): emptying the cache before every prompt's recording made the next prompt's prefill allocate all of
+        its buffers from the driver again. A step that needs more than there was is recorded again without the cache. The buffers of
+        the graph recorded before are taken over (it is dropped here)."""
         torch.cuda.synchronize()
+        low = torch.cuda.mem_get_info(self.device)[0] < RECORD_ROOM
+        for again in (False, True):
+            if low or again:
+                torch.cuda.empty_cache()
+            try:
+                graph = self._capture(body)
+                break
+            except torch.OutOfMemoryError:
+                if again:
+                    raise
+        self._old_graph = None
+        return graph
+
+    def _capture(self, body) -> torch.cuda.CUDAGraph:
         g = torch.cuda.CUDAGraph()
         side = torch.cuda.Stream(self.device)
         side.wait_stream(torch.cuda.current_stream())
@@ -120,7 +141,6 @@ class InferenceEngine:
             finally:
                 g.capture_end()
         torch.cuda.current_stream().wait_stream(side)
-        self._old_graph = None
         return g
 
     def reset(self) -> None:

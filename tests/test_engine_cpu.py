@@ -161,3 +161,28 @@ def test_a_replayed_step_stands_behind_the_tokens_of_a_step_before_it():
     eng.step(tok)
     eng.decode_step_graph()
     assert at == [4, 5, 6] and eng.length == 7
+
+
+@pytest.mark.parametrize("free,fails,emptied", [(1 << 30, 0, 0), ((1 << 30) - 1, 0, 1), (1 << 34, 1, 1), (0, 1, 2), (1 << 34, 2, 1)])
+def test_the_allocators_cache_is_emptied_when_a_recording_is_short_of_memory(free, fails, emptied, monkeypatch):
+    """A capture cannot make the allocator give its cached blocks back: with too little free memory that happens ahead of it, and after
+    one that ran out of memory; a second failure is the caller's."""
+    eng, log = InferenceEngine(1, "cpu", 1), []
+    monkeypatch.setattr(torch.cuda, "synchronize", lambda *a: None)
+    monkeypatch.setattr(torch.cuda, "mem_get_info", lambda device=None: (free, 1 << 37))
+    monkeypatch.setattr(torch.cuda, "empty_cache", lambda: log.append("empty"))
+
+    def capture(body):
+        log.append("capture")
+        if log.count("capture") <= fails:
+            raise torch.OutOfMemoryError("no memory")
+        return _Graph()
+
+    eng._capture, eng._old_graph = capture, _Graph()
+    if fails == 2:
+        with pytest.raises(torch.OutOfMemoryError):
+            eng._record(None)
+    else:
+        assert isinstance(eng._record(None), _Graph) and eng._old_graph is None
+    assert log.count("empty") == emptied and log.count("capture") == 1 + min(fails, 1)
+    assert log[0] == ("empty" if free < 1 << 30 else "capture")
