@@ -684,6 +684,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constant
     if ((HALVES || cnt > 0) && l > 0.f) {
       inv_l = 1.0f / l;
       lse = (m_ref + log2f(l)) * kLn2;
+    } else if (HALVES && p.splits > 1 && l != l) {
+      lse = l;  // tells attn_merge_kernel that the row is no number, not that this split sees none of its keys
     }
     float w_prev = 0.f, w_this = 1.f;
     if (p.o_prev && row_valid) {
@@ -782,8 +784,9 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constant
 }
 
 // Puts the partial results of a launch split over the keys together: o (splits, B, Sq, H, D) and lse (splits, B, H, Sq) fp32 ->
-// out (bf16 or fp32 view) and lse_out (B, H, Sq). A warp per row; a split without a visible key has lse = -inf and its
-// (zero) row is not read.
+// out (bf16 or fp32 view) and lse_out (B, H, Sq). A warp per row. Every split's row is read and multiplied, by a weight of 0 where the
+// split sees no key (lse = -inf) or its keys weigh nothing beside the others': NaN and infinities then come out as they do of a launch that is
+// not split, where a probability of 0 meets them in the product with V. lse is NaN where a split's sum is.
 template <int D>
 __global__ void __launch_bounds__(256) attn_merge_kernel(const float* __restrict__ o, const float* __restrict__ lse, int splits,
                                                          int B, int H, int Sq, void* out, int out_fp32, long long o_sb,
@@ -796,27 +799,25 @@ __global__ void __launch_bounds__(256) attn_merge_kernel(const float* __restrict
   const int h = static_cast<int>(row % H), q = static_cast<int>(row / H % Sq), b = static_cast<int>(row / H / Sq);
   const long long at = (static_cast<long long>(b) * H + h) * Sq + q;
   float mx = -INFINITY;
-  for (int s = 0; s < splits; ++s) mx = fmaxf(mx, lse[s * rows + at]);
+  for (int s = 0; s < splits; ++s) mx = fmaxf(mx, lse[s * rows + at]);  // (of the numbers among them)
   float acc[PER], sum = 0.f;
 #pragma unroll
   for (int e = 0; e < PER; ++e) acc[e] = 0.f;
-  if (mx != -INFINITY) {
 #pragma unroll 4
-    for (int s = 0; s < splits; ++s) {
-      const float w = expf(lse[s * rows + at] - mx);
-      if (w == 0.f) continue;
-      const float* src = o + (s * rows + row) * D + lane * PER;
-      sum += w;
+  for (int s = 0; s < splits; ++s) {
+    const float l = lse[s * rows + at];
+    const float w = l == -INFINITY ? 0.f : expf(l - mx);
+    const float* src = o + (s * rows + row) * D + lane * PER;
+    sum += w;
 #pragma unroll
-      for (int e = 0; e < PER; e += 2) {
-        const float2 v = *reinterpret_cast<const float2*>(src + e);
-        acc[e] += w * v.x;
-        acc[e + 1] += w * v.y;
-      }
+    for (int e = 0; e < PER; e += 2) {
+      const float2 v = *reinterpret_cast<const float2*>(src + e);
+      acc[e] += w * v.x;
+      acc[e + 1] += w * v.y;
     }
   }
-  const float inv = mx != -INFINITY ? 1.f / sum : 0.f;
-  if (lane == 0 && RA_IN_BOUNDS(at, 1, rows, kTagAttnFwdLse)) lse_out[at] = mx != -INFINITY ? mx + logf(sum) : -INFINITY;
+  const float inv = sum == 0.f ? 0.f : 1.f / sum;
+  if (lane == 0 && RA_IN_BOUNDS(at, 1, rows, kTagAttnFwdLse)) lse_out[at] = sum > 0.f ? mx + logf(sum) : -INFINITY;
   const long long off = b * o_sb + static_cast<long long>(q) * o_ss + h * o_sh + lane * PER;
 #pragma unroll
   for (int e = 0; e < PER; e += 2) {

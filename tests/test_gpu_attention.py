@@ -256,3 +256,63 @@ def test_carry_merged_in_place(S, H, q_pos, k_pos, D):
         o, l = o_prev.clone(), lse_prev.clone()
         flash.flash_fwd(q, k, v, ms, o_prev=o, lse_prev=l, out=o, lse_out=l)
         assert torch.equal(o, out) and torch.equal(l, lse)
+
+
+def _strange(where, q, k, v):
+    """One entry or row that is no ordinary number; key and value 4000 lie in the middle of the cache."""
+    if where == "query":
+        q[0, 7, 0, 3] = float("nan")
+    elif where == "key":
+        k[0, 4000, :, 3] = float("nan")
+    elif where == "infinite key":  # scores of +inf or -inf, by the query's sign
+        k[0, 4000, :, 3] = float("inf")
+    elif where == "value":
+        v[0, 4000, :, 5] = float("nan")
+    elif where == "infinite value":
+        v[0, 4000, :, 5] = -float("inf")
+    else:  # every key
+        k[0, :, 0, 3] = float("nan")
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("masked", [False, True])
+@pytest.mark.parametrize("where", ["query", "key", "infinite key", "value", "infinite value", "every key"])
+def test_what_is_no_number_passes_through_a_launch_split_over_the_keys(where, masked, D, monkeypatch):
+    """A launch split over the keys gives NaN and infinities, and a log-sum-exp without a number, where one that is not split does, and the
+    same numbers elsewhere (probabilities and results are rounded to bf16 on both sides, 2^-8 of the largest entry each). Without a mask also where dense
+    attention in 64 bits does. The mask hides key 4000 from some rows, and all keys from one."""
+    from ringattention_b200.ops import _lib, flash
+
+    B, Sq, Sk, H = 1, 130, 8000, 2
+    g = torch.Generator(device="cuda").manual_seed(D)
+    q = torch.randn(B, Sq, H, D, device="cuda", generator=g).bfloat16()
+    k, v = (torch.randn(B, Sk, H, D, device="cuda", generator=g).bfloat16() for _ in range(2))
+    _strange(where, q, k, v)
+    ms = flash.MaskSpec(causal_block_size=0, q_pos=flash.Positions(0), k_pos=flash.Positions(0))
+    if masked:
+        m = torch.rand(B, 1, Sq, Sk, device="cuda", generator=g) < 0.5
+        m[0, 0, 9] = False
+        ms.keep_q, ms.keep_k, ms.keep_tiles = flash.mask_bitmaps(m)
+    rule, chosen = _lib.lib().ra_attn_fwd_splits, []
+
+    def spy(a):
+        chosen.append(rule(a))
+        return chosen[-1]
+
+    monkeypatch.setattr(_lib.lib(), "ra_attn_fwd_splits", spy)
+    out, lse = flash.flash_fwd(q, k, v, ms)
+    assert chosen[0] > 1
+    monkeypatch.setattr(_lib.lib(), "ra_attn_fwd_splits", lambda a: 1)
+    want, want_lse = flash.flash_fwd(q, k, v, ms)
+    out, want = out.float(), want.float()
+    for a, b in ((out, want), (lse, want_lse)):
+        fin = torch.isfinite(b)
+        assert torch.equal(torch.isfinite(a), fin) and torch.equal(a.isnan(), b.isnan()) and torch.equal(a == float("inf"), b == float("inf"))
+        assert not fin.any() or bool(((a - b)[fin].abs() <= 2 ** -6 * b[fin].abs().max() + 1e-6).all())
+    if not masked:
+        x = torch.einsum("bqhd,bkhd->bhqk", q.double(), k.double())
+        if where == "infinite key":  # the kernel's score is what fp32 gives
+            x = torch.einsum("bqhd,bkhd->bhqk", q.float(), k.float()).double()
+        dense = torch.einsum("bhqk,bkhd->bqhd", torch.softmax(x / D ** 0.5, -1), v.double())
+        assert torch.equal(out.isnan(), dense.isnan()) and torch.equal(out.isinf(), dense.isinf())
+        assert not torch.isfinite(out).all()
