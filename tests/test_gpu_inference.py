@@ -564,3 +564,35 @@ def test_mask_rows_at_multiples_of_sixteen_bytes(Sq, Sk):
     one = at16[:, :, :1, :Sk].expand(B, H, Sq, Sk)
     for a, b in zip(flash.mask_bitmaps(one), flash.mask_bitmaps(odd[:, :, :1].expand(B, H, Sq, Sk))):
         assert torch.equal(a, b)
+
+
+def test_recording_a_step_when_memory_is_short(monkeypatch):
+    """With little free memory the allocator's cached blocks are given back before a step is recorded, with enough they stay; a
+    recording that runs out of memory all the same is made again without them."""
+    from ringattention_b200.config import LlamaConfig
+    from ringattention_b200.models import engine
+    from ringattention_b200.models.llama_infer import LlamaInference
+
+    cfg = LlamaConfig.named("llama-tiny")
+    prompt = torch.randint(0, cfg.vocab_size, (2, 128), device="cuda", generator=torch.Generator(device="cuda").manual_seed(3))
+    want = LlamaInference(cfg, max_context=512, batch=2, seed=4).generate(prompt, 6, use_graph=False)[0]
+    cached = 256 << 20
+    for room, fails in ((1 << 60, 0), (0, 0), (0, 1)):
+        monkeypatch.setattr(engine, "RECORD_ROOM", room)
+        eng = LlamaInference(cfg, max_context=512, batch=2, seed=4)
+        step, calls = eng._greedy_step, []
+
+        def body():
+            calls.append(torch.empty(8 << 20, dtype=torch.uint8, device="cuda").numel())  # out of the recording's pool
+            if len(calls) <= fails:
+                raise torch.OutOfMemoryError("no memory")
+            step()
+
+        eng._greedy_step = body
+        eng.generate(prompt, 3, use_graph=False)  # buffers and kernels exist
+        block = torch.empty(cached, dtype=torch.uint8, device="cuda")
+        del block
+        held = torch.cuda.memory_reserved()
+        assert torch.equal(eng.generate(prompt, 6)[0], want) and len(calls) == 1 + fails
+        given_back = torch.cuda.memory_reserved() < held - cached // 2
+        assert given_back == (room > 0 or fails > 0)
