@@ -801,7 +801,7 @@ extern "C" int ra_attn_bwd(const RaAttnBwdArgs* a) {
   const int nkt = (a->Sk + 127) / 128;
   // a head's Q, dO and the fp32 dQ that is reduced into in L2: 8 bytes an element
   p.order = TileOrder{nkt, a->B * a->H,
-                      a->causal_block_size ? heads_together(nkt, a->B * a->H, 8ll * a->Sq * a->D, sm_count()) : 1};
+                      a->causal_block_size ? head_groups(nkt, a->B * a->H, 8ll * a->Sq * a->D, sm_count()) : a->B * a->H};
   const long long grid = static_cast<long long>(nkt) * a->H * a->B + p.copy_ctas;
   cudaStream_t s = static_cast<cudaStream_t>(a->stream);
   if (a->D == 128) {

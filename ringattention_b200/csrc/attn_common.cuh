@@ -174,31 +174,41 @@ __device__ __forceinline__ unsigned int dropout_hash(unsigned int seed_lo, unsig
 }
 
 // Order of the CTAs of a launch. A (batch, head) has n tiles of work; under a causal rule they differ in length and the grid's
-// last wave is as long as the longest tile that starts in it. So `group` heads are walked together, the longest tiles of
-// all of them first: unit idx -> tile rank (0 = longest) and (batch, head).
+// last wave is as long as the longest tile that starts in it. So the heads are walked in `groups` of as good as equal size, the longest
+// tiles of a group's heads first: unit idx -> tile rank (0 = longest) and (batch, head).
 struct TileOrder {
-  int n, bh, group;
+  int n, bh, groups;
   __device__ __forceinline__ void operator()(int idx, int& rank, int& bh_idx) const {
-    const int per_group = n * group;
-    const int g = idx / per_group, r = idx - g * per_group;
-    const int in_group = min(group, bh - g * group);
-    rank = r / in_group;
-    bh_idx = g * group + (r - rank * in_group);
+    const int base = bh / groups, larger = bh - base * groups;  // the first `larger` groups have a head more
+    int size = base + 1, first = 0;
+    if (idx >= larger * n * size) {
+      idx -= larger * n * size;
+      first = larger * size;
+      size = base;
+    }
+    const int g = idx / (n * size), r = idx - g * n * size;
+    rank = r / size;
+    bh_idx = first + g * size + r - rank * size;
   }
 };
 
-// How many heads walk together: enough that a group's total work keeps every SM busy for as long as its longest tile takes
-// (tile lengths 1 .. n: n (n + 1) / 2 units a head against n on each of `sms`), so that the tail of the launch is the
-// shortest tiles, but no more than what fits in about half of the L2, because the tiles of a head share its operands there.
-// Heads one after the other (group 1) left the last heads' longest tiles to the end: B1 S4096 H32 D128 forward 249 us where
-// the work is 125 us at the rate of long sequences.
-inline int heads_together(int n, int bh, long long head_bytes, int sms) {
-  long long g = (2ll * sms + n) / (n + 1);
-  const long long fit = (64ll << 20) / (head_bytes > 0 ? head_bytes : 1), roomy = (24ll << 20) / (head_bytes > 0 ? head_bytes : 1);
-  if (g < roomy) g = roomy;
-  if (g > fit) g = fit;
-  if (g > bh) g = bh;
-  return g < 1 ? 1 : static_cast<int>(g);
+// Into how many groups. A group of `need` heads keeps every SM busy for as long as its longest tile takes (tile lengths 1 .. n:
+// n (n + 1) / 2 units a head against n on each of `sms`), so that the tail of the launch is the shortest tiles; heads whose operands take
+// no more than 24 MB together lose nothing by sharing the L2 and are walked together anyway; and above 64 MB, about half of the L2, the
+// tiles of a head no longer find its operands there. The groups are of equal size: with groups of `need` heads and a rest, 16 heads as
+// 3 + 3 + 3 + 3 + 3 + 1, the long tiles of the last head run alone at the end. us on B200, causal, D 128: heads one after the other / need and a rest / this:
+//   backward 16 x 16384 3294 / 3434 / 3187, 16 x 8192 869 / 914 / 761, 8 x 8192 476 / 443 / 385, 32 x 4096 492 / 452 / 440, 16 x 2048 98 / 68 / 68
+//   forward 4 x 32768 1036 / 1134 / 979, 8 x 16384 618 / 541 / 490, 16 x 8192 366 / 272 / 264, 32 x 4096 238 / 158 / 161, 32 x 2048 95 / 54 / 54
+inline int head_groups(int n, int bh, long long head_bytes, int sms) {
+  const long long bytes = head_bytes > 0 ? head_bytes : 1;
+  const long long fit = (64ll << 20) / bytes, roomy = (24ll << 20) / bytes;
+  long long need = (2ll * sms + n) / (n + 1);
+  if (need < roomy) need = roomy;
+  if (need > fit) need = fit;
+  if (need > bh) need = bh;
+  if (need < 1) need = 1;
+  const long long most = bh / need, least = fit > 0 ? (bh + fit - 1) / fit : bh;
+  return static_cast<int>(most > least ? most : least);
 }
 
 constexpr float kLog2e = 1.4426950408889634f;

@@ -1024,7 +1024,7 @@ extern "C" int ra_attn_fwd(const RaAttnFwdArgs* a) {
   const bool halves = splits > 1 || shape_of(a, false).halves;
   const int n_q = halves ? (a->Sq + 127) / 128 : (a->Sq + 255) / 256;
   p.order = TileOrder{n_q, a->B * a->H,
-                      a->causal_block_size ? heads_together(n_q, a->B * a->H, 4ll * a->Sk * a->D, sm_count()) : 1};
+                      a->causal_block_size ? head_groups(n_q, a->B * a->H, 4ll * a->Sk * a->D, sm_count()) : a->B * a->H};
   p.splits = splits;
   p.split_l = static_cast<long long>(a->B) * a->H * a->Sq;
   p.split_o = p.split_l * a->D;
@@ -1110,7 +1110,7 @@ extern "C" int ra_attn_two_part(const RaAttnTwoPartArgs* a) {
   p.gate = static_cast<const __nv_bfloat16*>(a->gate);
   p.gate_ld = a->gate_ld;
   const int n_qp = (a->Sq + 255) / 256;
-  p.order = TileOrder{n_qp, a->B * a->H, 1};
+  p.order = TileOrder{n_qp, a->B * a->H, a->B * a->H};
   const long long grid = static_cast<long long>(n_qp) * a->H * a->B;
   cudaStream_t s = static_cast<cudaStream_t>(a->stream);
   if (a->d1 > 64)
@@ -1182,7 +1182,7 @@ extern "C" int ra_attn_window(const RaAttnWindowArgs* a) {
   p.k_row0 = static_cast<int>(base % a->k_rows);
   p.k_rows = a->k_rows;
   const int n_qp = (a->Sq + 255) / 256;
-  p.order = TileOrder{n_qp, a->B * a->H, 1};
+  p.order = TileOrder{n_qp, a->B * a->H, a->B * a->H};
   const long long grid = static_cast<long long>(n_qp) * a->H * a->B;
   cudaStream_t s = static_cast<cudaStream_t>(a->stream);
   if (a->dk > 64)

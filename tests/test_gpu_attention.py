@@ -222,6 +222,7 @@ def test_segment_ids_of_every_kind(ids, D):
     (1, 16, 20000, 2, 1, 19984), (1, 200, 9000, 4, 1, 8000), (2, 100, 8200, 1, None, None), (1, 130, 4100, 2, 32, 3970),  # keys split
     (1, 128, 40000, 1, 1, 100),                                                                                # most keys in the future
     (1, 2048, 2048, 40, 1, None), (1, 700, 700, 64, None, None),                                               # many tiles: two query tiles a CTA
+    (1, 2048, 2048, 67, 1, None),                                                                              # groups of unequal numbers of heads
 ])
 def test_every_way_a_forward_is_cut_up(B, Sq, Sk, H, cbs, cache_idx, D):
     """Sizes on both sides of the rule that gives a CTA two query tiles or one, and splits the keys of a few query tiles."""
