@@ -177,9 +177,10 @@ __device__ __forceinline__ unsigned int dropout_hash(unsigned int seed_lo, unsig
 // last wave is as long as the longest tile that starts in it. So the heads are walked in `groups` of as good as equal size, the longest
 // tiles of a group's heads first: unit idx -> tile rank (0 = longest) and (batch, head).
 struct TileOrder {
-  int n, bh, groups;
+  int n, base, larger;  // tiles of a head; heads of a group, the first `larger` groups have one more
+  TileOrder() = default;
+  TileOrder(int n_, int bh, int groups) : n(n_), base(bh / groups), larger(bh % groups) {}
   __device__ __forceinline__ void operator()(int idx, int& rank, int& bh_idx) const {
-    const int base = bh / groups, larger = bh - base * groups;  // the first `larger` groups have a head more
     int size = base + 1, first = 0;
     if (idx >= larger * n * size) {
       idx -= larger * n * size;
@@ -196,7 +197,8 @@ struct TileOrder {
 // n (n + 1) / 2 units a head against n on each of `sms`), so that the tail of the launch is the shortest tiles; heads whose operands take
 // no more than 24 MB together lose nothing by sharing the L2 and are walked together anyway; and above 64 MB, about half of the L2, the
 // tiles of a head no longer find its operands there. The groups are of equal size: with groups of `need` heads and a rest, 16 heads as
-// 3 + 3 + 3 + 3 + 3 + 1, the long tiles of the last head run alone at the end. us on B200, causal, D 128: heads one after the other / need and a rest / this:
+// 3 + 3 + 3 + 3 + 3 + 1, the long tiles of the last head run alone at the end. us on B200, causal, D 128, a build that walks the heads one
+// after the other / groups of `need` and a rest / this:
 //   backward 16 x 16384 3294 / 3434 / 3187, 16 x 8192 869 / 914 / 761, 8 x 8192 476 / 443 / 385, 32 x 4096 492 / 452 / 440, 16 x 2048 98 / 68 / 68
 //   forward 4 x 32768 1036 / 1134 / 979, 8 x 16384 618 / 541 / 490, 16 x 8192 366 / 272 / 264, 32 x 4096 238 / 158 / 161, 32 x 2048 95 / 54 / 54
 inline int head_groups(int n, int bh, long long head_bytes, int sms) {

@@ -22,8 +22,6 @@
 #include "attn_common.cuh"
 #include "common/host_util.h"
 
-#include <math.h>
-
 RA_BOUNDS_TRANSLATION_UNIT()
 
 namespace ra {
@@ -829,48 +827,57 @@ __global__ void __launch_bounds__(256) attn_merge_kernel(const float* __restrict
   }
 }
 
-// How a launch is cut up. Lengths are in steps (two 128 x 128 tiles, what a CTA works on at a time); a CTA costs OVERHEAD steps
-// beside its tiles (start-up, first loads, epilogue), and the SMs are busy for at least the longest CTA and the
-// average load. Segment ids and bitmaps are not looked at: the causal rule alone gives the lengths.
+// How a launch is cut up: two query tiles a CTA ("pairs"), one (HALVES), or one and its keys over several CTAs. The estimate is the time of
+// the launch in hundredths of a step of pairs (two 128 x 128 tiles; 1.82 us at D 128, 1.77 at D 64): a CTA takes its steps and a
+// fixed cost (start-up, first loads, epilogue), and the CTAs, longest first, go to whichever SM is free: the SMs are busy for the average load at
+// least, and the k-th CTA of an SM is no shorter than the longest that starts behind k - 1 full rounds. Segment ids and bitmaps are not
+// looked at: the causal rule alone gives the lengths.
+// The constants are fitted to 120 launches of both head dims timed in every form on B200 (300 to 32768 query rows, 2 to 32 heads, causal or not, up to
+// 65536 keys): the choice is the fastest form or within 3 % of it. A step of HALVES loads K and V for one query tile only, so at D 128 it takes
+// 15 % longer; its CTA ends sooner. us, pairs / HALVES / keys over 2 / over 4 CTAs, D 128, * the choice:
+//   32 heads x 512, not causal 18.3 / 13.8* / 35.9 / -       32 x 4096, not causal 286* / 317 / - / -     32 x 4096, causal 158* / 196 / - / -
+//   4 x 4096, causal 70.6 / 42.8* / 49.2 / 70.1              16 x 2048, not causal 41.6* / 51.3 / - / -   16 x 500 on 16384 keys 256 / 158 / 96* / 113
+//   32 x 1000 on 16384 keys 261* / 320 / 369 / 399           32 x 128 on 4096 keys 62 / 44 / 33 / 26*
+// With equal steps, a fixed cost of 2.5 steps and whole rounds for launches that are not causal only, 32 heads x 4096, not causal, went to HALVES
+// and 16 x 500 causal rows on 16384 keys to three CTAs each (136 us).
 struct FwdShape {
   bool halves;
   int splits;
 };
-inline FwdShape fwd_shape(int B, int H, int Sq, int Sk, int cbs, long long q_off, long long k_off, bool one_run, bool may_split) {
-  constexpr double OVERHEAD = 2.5;
-  constexpr double MERGE = 3.0;  // steps: partial results out and in again, one more launch
+inline FwdShape fwd_shape(int B, int H, int Sq, int Sk, int D, int cbs, long long q_off, long long k_off, bool one_run, bool may_split) {
+  const int step = D == 128 ? 115 : 96, cta = D == 128 ? 490 : 400, cta_pair = D == 128 ? 650 : 430;  // of HALVES, HALVES, pairs
+  constexpr int step_pair = 100, merge = 500;  // merge: partial results out and in again, one more launch
   const int nk = (Sk + 127) / 128, nq = (Sq + 127) / 128, sms = sm_count();
   const long long bh = static_cast<long long>(B) * H;
   FwdShape best{false, 1};
   if (nq > 1024 || bh * nq > 64ll * sms) return best;  // plenty of work per SM: two query tiles share the loads of K and V
-  double len[1024];                                    // visible kv tiles of each query tile
-  for (int i = 0; i < nq; ++i) {
-    long long v = nk;
-    if (cbs && one_run) v = (q_off + i * 128ll + 127 - k_off) / 128 + 1;
-    len[i] = static_cast<double>(v < 0 ? 0 : (v > nk ? nk : v));
-  }
-  double sum = 0, top = 0;
-  for (int i = 0; i < nq; i += 2) {
-    const double l = (i + 1 < nq && len[i + 1] > len[i] ? len[i + 1] : len[i]) + OVERHEAD;
-    sum += l;
-    top = l > top ? l : top;
-  }
-  double t_best = sum * bh / sms > top ? sum * bh / sms : top;
-  const long long pairs = bh * ((nq + 1) / 2);
-  const double waves = static_cast<double>((pairs + sms - 1) / sms);
-  if (!cbs && waves * top > t_best) t_best = waves * top;  // equal lengths: whole waves
-  for (int s = 1; s <= (may_split ? 32 : 1); ++s) {
-    double hsum = 0, htop = 0;
-    for (int i = 0; i < nq; ++i) {
-      const double l = ceil(len[i] / (2 * s)) + OVERHEAD;
-      hsum += l;
-      htop = l > htop ? l : htop;
+  auto tiles = [&](int i) -> long long {  // visible kv tiles of query tile i; no fewer than of the tile before
+    const long long v = cbs && one_run ? (q_off + i * 128ll + 127 - k_off) / 128 + 1 : nk;
+    return v < 0 ? 0 : (v > nk ? nk : v);
+  };
+  // `each` CTAs of each of n lengths, cost(0) the longest
+  auto makespan = [&](int n, long long each, auto cost) -> long long {
+    long long sum = 0;
+    for (int i = 0; i < n; ++i) sum += cost(i);
+    long long t = sum * each / sms;
+    for (long long k = 1, at = 0; at < n * each; ++k, at += sms) {
+      const long long c = k * cost(static_cast<int>(at / each));
+      if (c > t) t = c;
     }
-    double t = hsum * bh * s / sms > htop ? hsum * bh * s / sms : htop;
-    const double w = static_cast<double>((bh * nq * s + sms - 1) / sms);
-    if ((!cbs || nq == 1) && w * htop > t) t = w * htop;
-    if (s > 1) t += MERGE;
-    if (t < 0.95 * t_best) {
+    return t;
+  };
+  long long t_best = makespan((nq + 1) / 2, bh, [&](int i) {
+    const int later = 2 * ((nq + 1) / 2 - 1 - i) + 1;  // second tile of the i-th pair from the end
+    return tiles(later < nq ? later : nq - 1) * step_pair + cta_pair;
+  });
+  long long all = 0;
+  for (int i = 0; i < nq; ++i) all += tiles(i);
+  for (int s = 1; s <= (may_split ? 32 : 1) && s <= nk; ++s) {
+    const long long extra = s > 1 ? merge : 0;
+    // more CTAs only add to the average load: no larger s is worth a look
+    if (((all * step / 2 + static_cast<long long>(s) * nq * cta) * bh / sms + extra) * 100 >= t_best * 97) break;
+    const long long t = extra + makespan(nq, bh * s, [&](int i) { return (tiles(nq - 1 - i) + 2 * s - 1) / (2 * s) * step + cta; });
+    if (t * 100 < t_best * 97) {
       t_best = t;
       best = FwdShape{true, s};
     }
@@ -939,7 +946,7 @@ struct RaAttnFwdArgs {
 namespace {
 ra::attn::FwdShape shape_of(const RaAttnFwdArgs* a, bool may_split) {
   const bool one_run = a->q_half >= a->Sq && a->k_half >= a->Sk;
-  return ra::attn::fwd_shape(a->B, a->H, a->Sq, a->Sk, a->causal_block_size, a->q_off0, a->k_off0, one_run, may_split);
+  return ra::attn::fwd_shape(a->B, a->H, a->Sq, a->Sk, a->D, a->causal_block_size, a->q_off0, a->k_off0, one_run, may_split);
 }
 }  // namespace
 
