@@ -60,7 +60,7 @@ def _pad_q(q: torch.Tensor):
     return q.contiguous(), ql, tgt
 
 
-def default_splits(S: int, B: int, H: int, mma: bool = False) -> int:
+def default_splits(S: int, B: int, H: int, mma: bool = False, exchange: bool = False) -> int:
     """Many small CTAs: measured on a 128K-row, 32-head shard, 18 splits (4 CTAs per SM in total) gave
     4.57 TB/s, 74 splits 4.65 (a ragged last wave), 256 splits 5.19 with register loads; with the asynchronous-copy
     ring 64 to 512 splits are within 3 % of each other (6.83 to 7.02 TB/s). At least 512 cache rows per CTA.
@@ -68,13 +68,17 @@ def default_splits(S: int, B: int, H: int, mma: bool = False) -> int:
     query rows, 128 / 256 / 512 splits: 0.315 / 0.332 / 0.408 ms.
     Short caches: ranges down to 128 rows while four CTAs (two of ``mma``) per SM are not there yet. 16 heads x 2176 rows, 5 / 17
     splits: 15.9 / 10.5 us with the merge; 8 heads x 4000 rows, 8 / 32 splits: 18.9 / 10.7 us; four query rows, 16 heads x 2176, 3 / 17
-    splits: 19.2 / 12.7 us. Beyond that short ranges only cost (8 x 32 heads x 4000 rows, 8 / 16 splits: 96.9 / 101.8 us)."""
+    splits: 19.2 / 12.7 us. Beyond that short ranges only cost (8 x 32 heads x 4000 rows, 8 / 16 splits: 96.9 / 101.8 us).
+    ``exchange``: the partials go to :func:`merge_exchange`, where one thread per column walks them, and many of them cost more there than
+    short ranges save above 4096 rows. Split-KV and exchange on one device with the other rank's rows in place, without / with the
+    short ranges: 16 heads x 2176 rows 30.0 / 26.7 us, 3000 31.3 / 28.3, 4000 31.4 / 31.4, 8192 35.6 / 37.6, 16384 42.8 / 46.4; 8 heads x 3000
+    24.2 / 19.8, 8192 25.2 / 27.0, 16384 29.6 / 33.8; four query rows, 16 heads x 4000 33.7 / 31.9, 8192 34.4 / 36.5."""
     sms = _lib.lib().ra_sm_count()
     per_sm, rows, resident = (32, 1024, 2) if mma else (64, 512, 4)
     pairs = max(1, B * H)
     want = max(1, (per_sm * sms) // pairs)
     full = min(want, (S + rows - 1) // rows)
-    fill = min(resident * sms // pairs, (S + 127) // 128)
+    fill = 0 if exchange and S > 4096 else min(resident * sms // pairs, (S + 127) // 128)
     return max(1, min(max(full, fill), 512))
 
 
@@ -191,16 +195,18 @@ def ring_decode_attention(q, k, v, attn_mask, axis, symm_ring=None, *, n_valid: 
         k_pos0 = rank * S_loc
     pos_ptr = 0 if state is None else state.data_ptr()
     step_ptr = 0 if state is None else state.data_ptr() + 8
+    rows = B * H * QL
+    exchanged = world > 1 and exchange_fits(rows)
+    splits = default_splits(S_loc if n_valid is None else int(n_valid), B, H, mma=QL >= MMA_MIN_ROWS, exchange=exchanged)
     o_part, lse_part = decode_partial(qp, k, v, n_valid=n_valid, q_pos0=q_pos0, k_pos0=k_pos0, mask=mask_u8,
-                                      pos_ptr=pos_ptr, stripe=stripe)
+                                      pos_ptr=pos_ptr, stripe=stripe, splits=splits)
     out = torch.empty(B, QL, H, D, device=q.device, dtype=v.dtype)
     if world == 1:
         merge_partials(o_part, lse_part, H, QL, out=out)
         return out[:, :ql]
     if symm_ring is None:
         raise RuntimeError("multi-rank decode needs a symmetric-memory ring")
-    rows = B * H * QL
-    if exchange_fits(rows):
+    if exchanged:
         merge_exchange(o_part, lse_part, H, QL, out, symm_ring)
         return out[:, :ql]
     # too many rows for the one-launch exchange: merge into the inboxes, barrier, merge the ranks

@@ -254,3 +254,17 @@ def test_memory_planner_scales_linearly_with_the_ring_size():
     assert inf[8] > 1_048_576 and 7 * inf[1] < inf[8] < 9 * inf[1]
     # sharding the weights over fsdp frees optimizer memory
     assert M.bytes_per_gpu(cfg, 32768, sp=4, fsdp=2)["optimizer"] < M.bytes_per_gpu(cfg, 32768, sp=4)["optimizer"]
+
+
+def test_short_ranges_of_a_cache_stop_where_the_exchange_of_a_ring_pays_for_them():
+    """Up to 4096 rows a shard is split alike on one device and on a ring; beyond, the ring's merge (a thread per column walks the
+    partials) gets no more of them than 512 rows a range (1024 on the tensor cores) give."""
+    from ringattention_b200.ops import decode as Dk
+
+    for B, H in ((1, 8), (1, 16), (1, 32), (4, 16)):
+        for mma, rows in ((False, 512), (True, 1024)):
+            for S in (100, 2176, 4096):
+                assert Dk.default_splits(S, B, H, mma, exchange=True) == Dk.default_splits(S, B, H, mma)
+            for S in (4097, 8192, 16384, 65536):
+                n = Dk.default_splits(S, B, H, mma, exchange=True)
+                assert n <= -(-S // rows) and n <= Dk.default_splits(S, B, H, mma)
