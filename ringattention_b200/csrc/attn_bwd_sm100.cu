@@ -374,13 +374,18 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constant
     const uint64_t bias2 = f2_pack(my_bias2, my_bias2);
     const bool biased = __any_sync(0xffffffffu, my_bias2 != 0.f);  // no row of this warp has one: nothing to add
 
+    // kinds of this kv tile's bitmap tiles, as in the forward
+    const int kinds_row = (mk.Sk + 127) >> 7;
+    const uint8_t* tile_kinds = mk.keep_tiles && !mk.drop_threshold
+                                    ? mk.keep_tiles + b * mk.keep_tiles_sb + h * mk.keep_tiles_sh + (k0 >> 7) : nullptr;
+    const bool bits = mk.drop_threshold || mk.keep;
     int it = 0;
     bool alive = true;
     for (int i = next_vis(0); i < nqt && alive; i = next_vis(i + 1)) {
       const int qi0 = i * 128;
       const int st = it & 1;
       const uint32_t par = it & 1;
-      const int kind = tile_mask(mk, b, h, qi0, k0);
+      const int kind = tile_mask(mk, b, tile_kinds ? tile_kinds[static_cast<long long>(i) * kinds_row] != 1 : bits, qi0, k0);
       if (kind & kMaskSeg) {
         if (sm_tid < 128)
           sSegQ[st * 128 + sm_tid] =

@@ -97,9 +97,10 @@ __device__ __forceinline__ int vis_next(const uint32_t* words, int t, int n) {
 
 // What may hide single entries of a visible tile; 0: nothing does. With segment ids the common case inside packed documents
 // much longer than a tile is that both tiles lie in one and the same segment (per-tile min == max, equal on both sides).
+// bits: the bitmap has a hole in this tile, or there is dropout.
 enum TileMask : int { kMaskEdge = 1 /* causal rule or end of the keys */, kMaskSeg = 2, kMaskBits = 4 /* bitmap, dropout */ };
-__device__ __forceinline__ int tile_mask(const MaskParams& m, int b, int h, int qi0, int k0) {
-  int kind = (m.drop_threshold || (m.keep && bitmap_tile(m, b, h, qi0, k0) != 1)) ? kMaskBits : 0;
+__device__ __forceinline__ int tile_mask(const MaskParams& m, int b, bool bits, int qi0, int k0) {
+  int kind = bits ? kMaskBits : 0;
   if (k0 + 128 > m.Sk) kind |= kMaskEdge;
   if (m.seg_q) {
     bool one = false;

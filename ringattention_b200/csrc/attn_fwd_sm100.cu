@@ -459,6 +459,13 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constant
     int cnt = 0;
     bool alive = true;
 
+    // Kinds of this query tile's bitmap tiles; without them every tile's bits are looked at, if there are any. A pointer for the whole
+    // walk: asked for per tile out of the launch's parameters they cost every launch, those without a bitmap too (2 x 32 heads x 512, not
+    // causal, 19.2 -> 18.5 us; the backward's 16 x 2048 118.6 -> 116.3).
+    const uint8_t* tile_kinds = mk.keep_tiles && !mk.drop_threshold
+                                    ? mk.keep_tiles + b * mk.keep_tiles_sb + h * mk.keep_tiles_sh + static_cast<long long>(qi0 >> 7) * nk
+                                    : nullptr;
+    const bool bits = mk.drop_threshold || mk.keep;
     // every role walks the same visibility mask, so skips stay consistent
     auto next_mine = [&](int j) {
       j = next_vis(wv, j);
@@ -468,7 +475,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constant
     if (HALVES && w == 1 && j < nk) j = next_vis(wv, j + 1);
     for (; j < nk && alive; j = next_mine(j + 1)) {
       const int k0 = j * 128;
-      const int kind = tile_mask(mk, b, h, qi0, k0) | (EXT && !tile_window_plain(mk, p.window, qi0, k0) ? kMaskEdge : 0);
+      const int kind = tile_mask(mk, b, tile_kinds ? tile_kinds[j] != 1 : bits, qi0, k0) | (EXT && !tile_window_plain(mk, p.window, qi0, k0) ? kMaskEdge : 0);
       const bool biased = mk.bias && (!use_vis || ((sAdd[j >> 5] >> (j & 31)) & 1u));
       const int buf = cnt & 1;
       if ((kind & kMaskSeg) || biased) {
