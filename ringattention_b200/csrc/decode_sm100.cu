@@ -1034,7 +1034,9 @@ __global__ void __launch_bounds__(256) small_m_linear_pro_kernel(const __nv_bflo
 //   with SwiGLU ahead of it 2048 x 5504 10.5 -> 8.9, 4096 x 11008 25.9 -> 23.1
 // f(x) is rounded to bf16 as in the kernels above.
 enum { PRO_NONE = 0 };
-constexpr int ROW_COLS = 8, ROW_WARPS = 8, ROW_MAX_CHUNKS = 6;  // K up to 6 * 256 * 8
+// The chunks of K are unrolled, so there is a last one: K up to 6 * 256 * 8 = 12288; longer rows (a d_ff of 13824 or 28672) take
+// small_m_linear_kernel, a warp per column.
+constexpr int ROW_COLS = 8, ROW_WARPS = 8, ROW_MAX_CHUNKS = 6;
 
 __device__ __forceinline__ uint4 ld_stream(const uint4* p) {
   uint4 v;

@@ -41,7 +41,7 @@ inline int choose_bn(int tiles_m, int n, int num_kb, bool addend32) {
   return best;
 }
 
-// Operands and the rows of B a tile of `bn` columns loads at a time; for SwiGLU products `tb` covers half a tile.
+// The operands' bases and leading dimensions in elements; launch_bn makes their tensor maps, whose boxes depend on the tile's width.
 struct Operands {
   const void *a, *b;
   long long lda, ldb;

@@ -128,10 +128,10 @@ def test_casts():
     assert torch.equal(back.view(64, 256), src.bfloat16().float())
 
 
-@pytest.mark.parametrize("rows,d", [(1, 8), (3, 40), (63, 1000), (700, 4104), (2048, 8192)])
+@pytest.mark.parametrize("rows,d", [(1, 8), (3, 40), (63, 1000), (126, 40), (128, 40), (130, 1000), (700, 4104), (2048, 8192)])
 def test_rmsnorm_gain_gradient_at_odd_widths_and_few_rows(rows, d):
-    """Widths that are no multiple of the 32 columns a reducing CTA takes, fewer partial rows than its 32 warps and many
-    more. Tolerance: fp32 sums of `rows` products, so 1e-6 of the sum of their magnitudes."""
+    """From the eight columns that a reducing CTA takes to the widest; fewer partial rows (the rows, rounded up to an even number) than its 128
+    groups of threads, as many, two more, and many more. Tolerance: fp32 sums of `rows` products, so 1e-6 of the sum of their magnitudes."""
     from ringattention_b200.ops import kernels as K
 
     torch.manual_seed(rows)
