@@ -12,7 +12,7 @@
 // HALVES: one CTA owns 128 query rows and its two softmax groups take every second visible KV tile each, with accumulators
 // of their own (O0, O1) that meet in the epilogue. The pipeline is the same (two tiles of scores in flight), a CTA's chain is half
 // as long and there are twice as many CTAs, at the price of loading K and V once per 128 rows. For launches with few
-// query tiles; see halves_pay(). Such a launch may also be split over the keys (`splits`): then every CTA takes its share of
+// query tiles; see fwd_shape(). Such a launch may also be split over the keys (`splits`): then every CTA takes its share of
 // the visible tiles, partial results go to fp32 buffers and attn_merge_kernel puts them together.
 //
 // The epilogue normalises O, optionally merges it with the carry (o_prev, lse_prev) of earlier

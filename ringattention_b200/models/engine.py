@@ -13,7 +13,7 @@ import torch
 # Free memory of the device below which the allocator gives its cached blocks back before a step is recorded. While a capture is under way it
 # cannot, and the private pool of a capture takes none of them: the recording would run out of memory beside gigabytes of cached blocks, or
 # leave the driver nothing to upload the graph with. A step's own buffers are megabytes (the partial results of 512 splits of 64 heads 17, the
-# logits of eight sequences 1.5); a graph of 60 launches took 70.
+# logits of eight sequences 1.5); the first capture of a process took 72 from the driver.
 RECORD_ROOM = 1 << 30
 
 
