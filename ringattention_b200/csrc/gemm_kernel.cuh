@@ -106,6 +106,145 @@ __device__ __forceinline__ void tile_coords(int tile, int tiles_m, int tiles_n, 
   tn = r / gm;
 }
 
+// Epilogue of the columns [32 c_begin, 32 c_end) of a tile for one row (an even number of such pieces with the SwiGLU epilogue): from the
+// accumulator at t_row to C. `wait` returns once the accumulator is complete, or false.
+template <int BN, typename Wait>
+__device__ __forceinline__ bool epilogue(const Params& p, uint32_t t_row, int row, int tn, int c_begin, int c_end, Wait wait) {
+  const int n0 = tn * BN;
+  // The fp32 addend is loaded one chunk of 32 columns ahead, the first while the tile's products still run: with a
+  // short K the epilogue would otherwise be a chain of memory round trips longer than the main loop.
+  const bool add32 = (p.c_fp32 || p.r_fp32) && p.R && row < p.M;
+  float4 ahead[8];
+  auto load_addend = [&](int c) {
+    const float* src = reinterpret_cast<const float*>(p.R) + static_cast<long long>(row) * p.ldr + n0 + c * 32;
+#pragma unroll
+    for (int j = 0; j < 8; ++j)
+      if (n0 + c * 32 + j * 4 < p.N) ahead[j] = *reinterpret_cast<const float4*>(src + 4 * j);
+  };
+  if (add32) load_addend(c_begin);
+  if (!wait()) return false;
+  tc_fence_after();
+  if (p.swiglu_F) {
+#pragma unroll 1
+    for (int c = c_begin / 2; c < c_end / 2; ++c) {
+      uint32_t rg[32], ru[32];
+      tmem_ld_x32(t_row + c * 32, rg);
+      tmem_ld_x32(t_row + BN / 2 + c * 32, ru);
+      tmem_ld_wait();
+      const int col0 = tn * (BN / 2) + c * 32;
+      if (row < p.M && col0 < p.swiglu_F) {
+        __nv_bfloat16* dst = reinterpret_cast<__nv_bfloat16*>(p.C) + static_cast<long long>(row) * p.ldc + col0;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          if (col0 + j * 8 < p.swiglu_F) {
+            float f[8];
+#pragma unroll
+            for (int e = 0; e < 8; ++e) {
+              const float gv = __bfloat162float(__float2bfloat16(__uint_as_float(rg[8 * j + e])));
+              const float uv = __bfloat162float(__float2bfloat16(__uint_as_float(ru[8 * j + e])));
+              f[e] = gv / (1.f + __expf(-gv)) * uv;
+            }
+            uint4 v;
+            v.x = pack_bf16x2(f[0], f[1]);
+            v.y = pack_bf16x2(f[2], f[3]);
+            v.z = pack_bf16x2(f[4], f[5]);
+            v.w = pack_bf16x2(f[6], f[7]);
+            if (RA_IN_BOUNDS(row, 1, p.M, kTagGemmStore) && RA_IN_BOUNDS(col0 + 8 * j, 8, p.swiglu_F, kTagGemmStore))
+              *reinterpret_cast<uint4*>(dst + 8 * j) = v;
+          }
+        }
+      }
+    }
+  } else
+#pragma unroll 1
+  for (int c = c_begin; c < c_end; ++c) {
+    uint32_t r[32];
+    tmem_ld_x32(t_row + c * 32, r);
+    tmem_ld_wait();
+    const int col0 = n0 + c * 32;
+    if (row < p.M && col0 < p.N) {
+      if (p.bias) {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          const float4 bv = *reinterpret_cast<const float4*>(p.bias + col0 + 4 * j);
+          r[4 * j] = __float_as_uint(fmaf(__uint_as_float(r[4 * j]), p.alpha, bv.x));
+          r[4 * j + 1] = __float_as_uint(fmaf(__uint_as_float(r[4 * j + 1]), p.alpha, bv.y));
+          r[4 * j + 2] = __float_as_uint(fmaf(__uint_as_float(r[4 * j + 2]), p.alpha, bv.z));
+          r[4 * j + 3] = __float_as_uint(fmaf(__uint_as_float(r[4 * j + 3]), p.alpha, bv.w));
+        }
+      }
+      if (p.relu2) {
+#pragma unroll
+        for (int e = 0; e < 32; ++e) {
+          const float v = fmaxf(__uint_as_float(r[e]), 0.f);
+          r[e] = __float_as_uint(v * v);
+        }
+      }
+      const bool tail = p.C2 && col0 >= p.n_split;
+      if (add32 && !tail) {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          r[4 * j] = __float_as_uint(__uint_as_float(r[4 * j]) + ahead[j].x);
+          r[4 * j + 1] = __float_as_uint(__uint_as_float(r[4 * j + 1]) + ahead[j].y);
+          r[4 * j + 2] = __float_as_uint(__uint_as_float(r[4 * j + 2]) + ahead[j].z);
+          r[4 * j + 3] = __float_as_uint(__uint_as_float(r[4 * j + 3]) + ahead[j].w);
+        }
+        if (c + 1 < c_end) load_addend(c + 1);
+      }
+      if (tail) {
+        float* dst = p.C2 + static_cast<long long>(row) * p.ldc2 + (col0 - p.n_split);
+#pragma unroll
+        for (int j = 0; j < 8; ++j)
+          if (col0 + j * 4 < p.N && RA_IN_BOUNDS(col0 - p.n_split + 4 * j, 4, p.ldc2, kTagGemmStore))
+            *reinterpret_cast<float4*>(dst + 4 * j) =
+                make_float4(__uint_as_float(r[4 * j]), __uint_as_float(r[4 * j + 1]), __uint_as_float(r[4 * j + 2]),
+                            __uint_as_float(r[4 * j + 3]));
+      } else if (p.c_fp32) {
+        float* dst = reinterpret_cast<float*>(p.C) + static_cast<long long>(row) * p.ldc + col0;
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          if (col0 + j * 4 < p.N) {
+            const float4 v = make_float4(__uint_as_float(r[4 * j]), __uint_as_float(r[4 * j + 1]),
+                                         __uint_as_float(r[4 * j + 2]), __uint_as_float(r[4 * j + 3]));
+            if (RA_IN_BOUNDS(row, 1, p.M, kTagGemmStore) && RA_IN_BOUNDS(col0 + 4 * j, 4, p.N, kTagGemmStore))
+              *reinterpret_cast<float4*>(dst + 4 * j) = v;
+          }
+        }
+      } else {
+        __nv_bfloat16* dst =
+            reinterpret_cast<__nv_bfloat16*>(p.C) + static_cast<long long>(row) * p.ldc + col0;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          if (col0 + j * 8 < p.N) {
+            float f[8];
+#pragma unroll
+            for (int e = 0; e < 8; ++e) f[e] = __uint_as_float(r[8 * j + e]);
+            if (p.R && !p.r_fp32) {
+              const uint4 o = *reinterpret_cast<const uint4*>(
+                  reinterpret_cast<const __nv_bfloat16*>(p.R) + static_cast<long long>(row) * p.ldr + col0 + 8 * j);
+              const __nv_bfloat162* ob = reinterpret_cast<const __nv_bfloat162*>(&o);
+#pragma unroll
+              for (int e = 0; e < 4; ++e) {
+                const float2 of = __bfloat1622float2(ob[e]);
+                f[2 * e] += of.x;
+                f[2 * e + 1] += of.y;
+              }
+            }
+            uint4 v;
+            v.x = pack_bf16x2(f[0], f[1]);
+            v.y = pack_bf16x2(f[2], f[3]);
+            v.z = pack_bf16x2(f[4], f[5]);
+            v.w = pack_bf16x2(f[6], f[7]);
+            if (RA_IN_BOUNDS(row, 1, p.M, kTagGemmStore) && RA_IN_BOUNDS(col0 + 8 * j, 8, p.N, kTagGemmStore))
+              *reinterpret_cast<uint4*>(dst + 8 * j) = v;
+          }
+        }
+      }
+    }
+  }
+  return true;
+}
+
 template <int A_MN, int B_MN, bool GATHER, int BN = gemm::BN>
 __global__ void __launch_bounds__(THREADS, 1)
 gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ TmaSet tma_bs,
@@ -329,141 +468,10 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
       int tm, tn;
       tile_coords(tile, tiles_m, tiles_n, p.group_m, tm, tn);
       tn = (tn + tn_rot) % tiles_n;
-      const int row = tm * BM + quad * 32 + lane;
-      const int n0 = tn * BN;
-      // The fp32 addend is loaded one chunk of 32 columns ahead, the first while the tile's products still run: with a
-      // short K the epilogue would otherwise be a chain of memory round trips longer than the main loop.
-      const bool add32 = (p.c_fp32 || p.r_fp32) && p.R && row < p.M;
-      float4 ahead[8];
-      auto load_addend = [&](int c) {
-        const float* src = reinterpret_cast<const float*>(p.R) + static_cast<long long>(row) * p.ldr + n0 + c * 32;
-#pragma unroll
-        for (int j = 0; j < 8; ++j)
-          if (n0 + c * 32 + j * 4 < p.N) ahead[j] = *reinterpret_cast<const float4*>(src + 4 * j);
-      };
-      if (add32) load_addend(0);
-      if (!mbar_wait(&tfull[acc], acc_phase, wc, kTimeoutTmemFull)) break;
-      tc_fence_after();
-      const uint32_t t_row = tmem_base + (static_cast<uint32_t>(quad * 32) << 16) +
-                             static_cast<uint32_t>(acc * BN);
-      if (p.swiglu_F) {
-#pragma unroll 1
-        for (int c = 0; c < BN / 64; ++c) {
-          uint32_t rg[32], ru[32];
-          tmem_ld_x32(t_row + c * 32, rg);
-          tmem_ld_x32(t_row + BN / 2 + c * 32, ru);
-          tmem_ld_wait();
-          const int col0 = tn * (BN / 2) + c * 32;
-          if (row < p.M && col0 < p.swiglu_F) {
-            __nv_bfloat16* dst = reinterpret_cast<__nv_bfloat16*>(p.C) + static_cast<long long>(row) * p.ldc + col0;
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-              if (col0 + j * 8 < p.swiglu_F) {
-                float f[8];
-#pragma unroll
-                for (int e = 0; e < 8; ++e) {
-                  const float gv = __bfloat162float(__float2bfloat16(__uint_as_float(rg[8 * j + e])));
-                  const float uv = __bfloat162float(__float2bfloat16(__uint_as_float(ru[8 * j + e])));
-                  f[e] = gv / (1.f + __expf(-gv)) * uv;
-                }
-                uint4 v;
-                v.x = pack_bf16x2(f[0], f[1]);
-                v.y = pack_bf16x2(f[2], f[3]);
-                v.z = pack_bf16x2(f[4], f[5]);
-                v.w = pack_bf16x2(f[6], f[7]);
-                if (RA_IN_BOUNDS(row, 1, p.M, kTagGemmStore) && RA_IN_BOUNDS(col0 + 8 * j, 8, p.swiglu_F, kTagGemmStore))
-                  *reinterpret_cast<uint4*>(dst + 8 * j) = v;
-              }
-            }
-          }
-        }
-      } else
-#pragma unroll 1
-      for (int c = 0; c < BN / 32; ++c) {
-        uint32_t r[32];
-        tmem_ld_x32(t_row + c * 32, r);
-        tmem_ld_wait();
-        const int col0 = n0 + c * 32;
-        if (row < p.M && col0 < p.N) {
-          if (p.bias) {
-#pragma unroll
-            for (int j = 0; j < 8; ++j) {
-              const float4 bv = *reinterpret_cast<const float4*>(p.bias + col0 + 4 * j);
-              r[4 * j] = __float_as_uint(fmaf(__uint_as_float(r[4 * j]), p.alpha, bv.x));
-              r[4 * j + 1] = __float_as_uint(fmaf(__uint_as_float(r[4 * j + 1]), p.alpha, bv.y));
-              r[4 * j + 2] = __float_as_uint(fmaf(__uint_as_float(r[4 * j + 2]), p.alpha, bv.z));
-              r[4 * j + 3] = __float_as_uint(fmaf(__uint_as_float(r[4 * j + 3]), p.alpha, bv.w));
-            }
-          }
-          if (p.relu2) {
-#pragma unroll
-            for (int e = 0; e < 32; ++e) {
-              const float v = fmaxf(__uint_as_float(r[e]), 0.f);
-              r[e] = __float_as_uint(v * v);
-            }
-          }
-          const bool tail = p.C2 && col0 >= p.n_split;
-          if (add32 && !tail) {
-#pragma unroll
-            for (int j = 0; j < 8; ++j) {
-              r[4 * j] = __float_as_uint(__uint_as_float(r[4 * j]) + ahead[j].x);
-              r[4 * j + 1] = __float_as_uint(__uint_as_float(r[4 * j + 1]) + ahead[j].y);
-              r[4 * j + 2] = __float_as_uint(__uint_as_float(r[4 * j + 2]) + ahead[j].z);
-              r[4 * j + 3] = __float_as_uint(__uint_as_float(r[4 * j + 3]) + ahead[j].w);
-            }
-            if (c + 1 < BN / 32) load_addend(c + 1);
-          }
-          if (tail) {
-            float* dst = p.C2 + static_cast<long long>(row) * p.ldc2 + (col0 - p.n_split);
-#pragma unroll
-            for (int j = 0; j < 8; ++j)
-              if (col0 + j * 4 < p.N && RA_IN_BOUNDS(col0 - p.n_split + 4 * j, 4, p.ldc2, kTagGemmStore))
-                *reinterpret_cast<float4*>(dst + 4 * j) =
-                    make_float4(__uint_as_float(r[4 * j]), __uint_as_float(r[4 * j + 1]), __uint_as_float(r[4 * j + 2]),
-                                __uint_as_float(r[4 * j + 3]));
-          } else if (p.c_fp32) {
-            float* dst = reinterpret_cast<float*>(p.C) + static_cast<long long>(row) * p.ldc + col0;
-#pragma unroll
-            for (int j = 0; j < 8; ++j) {
-              if (col0 + j * 4 < p.N) {
-                const float4 v = make_float4(__uint_as_float(r[4 * j]), __uint_as_float(r[4 * j + 1]),
-                                             __uint_as_float(r[4 * j + 2]), __uint_as_float(r[4 * j + 3]));
-                if (RA_IN_BOUNDS(row, 1, p.M, kTagGemmStore) && RA_IN_BOUNDS(col0 + 4 * j, 4, p.N, kTagGemmStore))
-                  *reinterpret_cast<float4*>(dst + 4 * j) = v;
-              }
-            }
-          } else {
-            __nv_bfloat16* dst =
-                reinterpret_cast<__nv_bfloat16*>(p.C) + static_cast<long long>(row) * p.ldc + col0;
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-              if (col0 + j * 8 < p.N) {
-                float f[8];
-#pragma unroll
-                for (int e = 0; e < 8; ++e) f[e] = __uint_as_float(r[8 * j + e]);
-                if (p.R && !p.r_fp32) {
-                  const uint4 o = *reinterpret_cast<const uint4*>(
-                      reinterpret_cast<const __nv_bfloat16*>(p.R) + static_cast<long long>(row) * p.ldr + col0 + 8 * j);
-                  const __nv_bfloat162* ob = reinterpret_cast<const __nv_bfloat162*>(&o);
-#pragma unroll
-                  for (int e = 0; e < 4; ++e) {
-                    const float2 of = __bfloat1622float2(ob[e]);
-                    f[2 * e] += of.x;
-                    f[2 * e + 1] += of.y;
-                  }
-                }
-                uint4 v;
-                v.x = pack_bf16x2(f[0], f[1]);
-                v.y = pack_bf16x2(f[2], f[3]);
-                v.z = pack_bf16x2(f[4], f[5]);
-                v.w = pack_bf16x2(f[6], f[7]);
-                if (RA_IN_BOUNDS(row, 1, p.M, kTagGemmStore) && RA_IN_BOUNDS(col0 + 8 * j, 8, p.N, kTagGemmStore))
-                  *reinterpret_cast<uint4*>(dst + 8 * j) = v;
-              }
-            }
-          }
-        }
-      }
+      const uint32_t t_row = tmem_base + (static_cast<uint32_t>(quad * 32) << 16) + static_cast<uint32_t>(acc * BN);
+      if (!epilogue<BN>(p, t_row, tm * BM + quad * 32 + lane, tn, 0, BN / 32,
+                        [&] { return mbar_wait(&tfull[acc], acc_phase, wc, kTimeoutTmemFull); }))
+        break;
       tc_fence_before();
       mbar_arrive(&tempty[acc]);
       if (++acc == NUM_ACC) {

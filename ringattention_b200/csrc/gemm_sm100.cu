@@ -4,41 +4,58 @@
 //   warp 1      tcgen05.mma issuer (one thread), two 128xBN fp32 accumulators in TMEM
 //   warps 2..5  epilogue: tcgen05.ld -> bf16/fp32 -> global, overlapped with the next tile's MMAs
 //
+// or the same on pairs of CTAs with tiles of 256 rows (gemm_pair.cuh); choose_form() says which.
+//
 // Each operand is either K-major (contiguous along the reduction dim) or MN-major (contiguous
 // along M resp. N); both are loaded with 128-byte-swizzled TMA boxes and described to the tensor
 // core by shared-memory descriptors, so the forward (x W^T), dgrad (dy W) and wgrad (dy^T x)
 // products of a linear layer all run through this one kernel without any transposes in memory.
 #include "gemm_kernel.cuh"
+#include "gemm_pair.cuh"
 
 RA_BOUNDS_TRANSLATION_UNIT()
 
 namespace ra {
 namespace gemm {
 
-// Width of the tiles for a product of tiles_m row tiles, n columns (of the accumulator) and num_kb k-blocks: the one with the
-// shortest estimated time. Wide tiles move the fewest bytes per column, which decides once every SM has several of them;
-// below that a launch takes as long as one SM's tiles, and narrower ones spread over more SMs and have a shorter epilogue.
-// Clocks per k-block, per 32 columns of epilogue (more with an fp32 addend) and per tile were fitted to 130 products with 128
-// to 4096 rows timed on B200 at each width; the choice is within 5 % of the best of the three for all of them, 0.2 % on average.
-// With 256 columns throughout, 512 x 1024 x 1024 took 10.8 us (64: 7.7), 1024 x 1024 from 4096 rows with fp32
-// accumulation 36 (64: 21), 2048 x 1024 x 2816 21.6 (128: 16.6); 8192 x 4096 x 4096 takes 194 (128: 244).
-inline int choose_bn(int tiles_m, int n, int num_kb, bool addend32) {
-  const int width[3] = {256, 128, 64}, kb_clk[3] = {790, 487, 312};
-  const int epi_clk = addend32 ? 815 : 690;
-  constexpr int tile_clk = 380;
-  int best = 0;
-  long long best_clk = 0;
-  for (int i = 0; i < 3; ++i) {
-    const long long tiles = static_cast<long long>(tiles_m) * ((n + width[i] - 1) / width[i]);
-    const long long waves = (tiles + sm_count() - 1) / sm_count();
-    const long long main = static_cast<long long>(num_kb) * kb_clk[i], epi = width[i] / 32 * epi_clk;
-    const long long clk = waves * ((main > epi ? main : epi) + tile_clk) + epi;
-    if (i == 0 || clk < best_clk) {
-      best = width[i];
-      best_clk = clk;
+// The form of a product of M rows, n columns (of the accumulator) and num_kb k-blocks: tiles of 128 rows on one CTA or of 256 on a pair, 64, 128
+// or 256 columns wide; the one with the shortest estimated time. Wide tiles and pairs move the fewest bytes per column, which decides once
+// every SM has several of them; below that a launch takes as long as one SM's tiles, and narrower ones spread over more SMs and have a
+// shorter epilogue; a pair costs a launch about 1 us and works for nothing on the second half of its rows where M ends in the first.
+// Nanoseconds per k-block, per 32 columns of epilogue (plain, with an addend, SwiGLU) and per tile and launch were fitted to 295 products
+// with 128 to 8192 rows timed on B200 in every form, K-major and MN-major: the choice is the fastest of the five within 9 %, within
+// 0.2 % on average, where the best of the three one-CTA widths takes 5 % longer on average and 43 % at worst. us, one CTA 256 / 128 / 64 columns, pair
+// 256 / 128, * the choice:
+//   8192 x 8192 x 8192 852 / 1172 / 1802, 750* / 894        4096 x 4096 x 4096, bf16 addend 143 / 165 / 299, 103* / 115
+//   22016 x 4096 x 4096, fp32 sums 604 / 737 / 1294, 529* / 636     2048 x 4096 x 4096 60 / 88 / 121, 49* / 61
+//   512 x 4096 x 11008 76 / 51 / 84, 61 / 45*               300 x 11008 x 2048 17.5* / 22.1 / 34.3, 27.3 / 26.5
+//   512 x 1536 x 512 10.1 / 7.4 / 6.2*, 11.2 / 8.2          1024 x 512 x 512 8.2 / 6.3 / 5.7*, 9.1 / 7.2
+struct Form {
+  int pair, width;
+  int kb, epi[3], tile, fixed;
+};
+constexpr Form kForms[] = {
+    {0, 256, 319, {337, 946, 480}, 4080, 0},
+    {0, 128, 287, {472, 946, 251}, 1612, 1040},
+    {0, 64, 220, {847, 1308, 1}, 83, 2393},
+    {1, 256, 316, {493, 866, 64}, 3126, 0},
+    {1, 128, 202, {955, 1150, 273}, 1505, 216},
+};
+inline const Form& choose_form(int M, int n, int num_kb, bool addend, bool swiglu) {
+  const Form* best = nullptr;
+  long long best_ns = 0;
+  for (const Form& f : kForms) {
+    const int rows = f.pair ? 2 * BM : BM, units = f.pair ? sm_count() / 2 : sm_count();
+    const long long tiles = static_cast<long long>((M + rows - 1) / rows) * ((n + f.width - 1) / f.width);
+    const long long waves = (tiles + units - 1) / units;
+    const long long main = static_cast<long long>(num_kb) * f.kb, epi = f.width / 32 * f.epi[swiglu ? 2 : (addend ? 1 : 0)];
+    const long long ns = f.fixed + waves * ((main > epi ? main : epi) + f.tile) + epi;
+    if (!best || ns < best_ns) {
+      best = &f;
+      best_ns = ns;
     }
   }
-  return best;
+  return *best;
 }
 
 // The operands' bases and leading dimensions in elements; launch_bn makes their tensor maps, whose boxes depend on the tile's width.
@@ -76,11 +93,39 @@ int launch_bn(const Operands& o, const Params& p, cudaStream_t stream) {
   return check_launch("gemm_bf16_kernel");
 }
 
+template <int A_MN, int B_MN, int BN_>
+int launch_pair(const Operands& o, const Params& p, cudaStream_t stream) {
+  using T = PairTile<BN_>;
+  CUtensorMap ta, tb;
+  int rc;
+  uint64_t dims[2], str[1];
+  uint32_t box[2];
+  if (A_MN) { dims[0] = p.M; dims[1] = p.K; box[0] = 64; box[1] = BK; }
+  else      { dims[0] = p.K; dims[1] = p.M; box[0] = BK; box[1] = BM; }
+  str[0] = static_cast<uint64_t>(o.lda) * 2;
+  if ((rc = make_tmap_bf16_sw128(&ta, o.a, 2, dims, str, box)) != 0) return rc;
+  if (B_MN) { dims[0] = p.N; dims[1] = p.K; box[0] = 64; box[1] = BK; }
+  else      { dims[0] = p.K; dims[1] = p.N; box[0] = BK; box[1] = BN_ / 2; }
+  str[0] = static_cast<uint64_t>(o.ldb) * 2;
+  if ((rc = make_tmap_bf16_sw128(&tb, o.b, 2, dims, str, box)) != 0) return rc;
+  auto kern = gemm_pair_kernel<A_MN, B_MN, BN_>;
+  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, T::SMEM_BYTES) != cudaSuccess) {
+    set_error("gemm: cudaFuncSetAttribute(MaxDynamicSharedMemorySize) failed");
+    return kHostLaunchFail;
+  }
+  const int tiles_n = p.swiglu_F ? (p.swiglu_F + BN_ / 2 - 1) / (BN_ / 2) : (p.N + BN_ - 1) / BN_;
+  const int tiles = ((p.M + 2 * BM - 1) / (2 * BM)) * tiles_n, pairs = sm_count() / 2;
+  kern<<<2 * (tiles < pairs ? tiles : pairs), PAIR_THREADS, T::SMEM_BYTES, stream>>>(ta, tb, p);
+  return check_launch("gemm_pair_kernel");
+}
+
 template <int A_MN, int B_MN>
 int launch(const Operands& o, const Params& p, cudaStream_t stream) {
-  const int bn = choose_bn((p.M + BM - 1) / BM, p.N, (p.K + BK - 1) / BK, (p.c_fp32 || p.r_fp32) && p.R);
-  if (bn == 256) return launch_bn<A_MN, B_MN, 256>(o, p, stream);
-  if (bn == 128) return launch_bn<A_MN, B_MN, 128>(o, p, stream);
+  const Form& f = choose_form(p.M, p.N, (p.K + BK - 1) / BK, p.R != nullptr, p.swiglu_F != 0);
+  if (f.pair)
+    return f.width == 256 ? launch_pair<A_MN, B_MN, 256>(o, p, stream) : launch_pair<A_MN, B_MN, 128>(o, p, stream);
+  if (f.width == 256) return launch_bn<A_MN, B_MN, 256>(o, p, stream);
+  if (f.width == 128) return launch_bn<A_MN, B_MN, 128>(o, p, stream);
   return launch_bn<A_MN, B_MN, 64>(o, p, stream);
 }
 

@@ -116,3 +116,35 @@ def test_gemm_fp32_addend_bf16_result(M, N, Kd, a_mn, b_mn):
     want = a.double() @ b.double().t() + r.double()
     slack = 2e-6 * (a.double().abs() @ b.double().abs().t() + r.double().abs())
     assert ((got.double() - want).abs() <= slack + 2**-8 * want.abs()).all()
+
+
+@pytest.mark.parametrize("a_mn,b_mn", [(False, False), (False, True), (True, False), (True, True)])
+@pytest.mark.parametrize("M,N,Kd", [(512, 4104, 2056), (520, 2056, 2056), (1030, 4104, 2056), (1000, 4104, 1000), (1030, 6000, 2056), (3900, 4104, 1000)])
+def test_gemm_on_cta_pairs(M, N, Kd, a_mn, b_mn):
+    """Products that get pairs of CTAs at both widths: an odd number of 128-row tiles, rows that end in either CTA's half, ragged columns
+    and K, a strided result, and results in bf16, bf16 with an addend and accumulated in fp32. Tolerances as above."""
+    from ringattention_b200.ops import _lib, kernels as K
+
+    M = (M + 7) // 8 * 8 if a_mn else M
+    g = torch.Generator(device="cuda").manual_seed(M + N)
+    a = torch.randn(M, Kd, device="cuda", generator=g).bfloat16()
+    b = torch.randn(N, Kd, device="cuda", generator=g).bfloat16()
+    A, B = (a.t().contiguous() if a_mn else a), (b.t().contiguous() if b_mn else b)
+    want = a.double() @ b.double().t()
+    slack = 2e-6 * (a.double().abs() @ b.double().abs().t())
+    wide = torch.full((M + 1, N + 24), 3.0, device="cuda")
+    acc = wide[:M, :N]
+    K.gemm(A, B, a_mn=a_mn, b_mn=b_mn, out=acc, residual=acc)
+    assert ((acc.double() - 3.0 - want).abs() <= slack + 1e-6).all() and (wide[:, N:] == 3.0).all() and (wide[M:] == 3.0).all()
+    c = K.gemm(A, B, a_mn=a_mn, b_mn=b_mn)
+    assert ((c.double() - want).abs() <= slack + 2**-8 * want.abs()).all()
+    r = torch.randn(M, N, device="cuda", generator=g).bfloat16()
+    c = K.gemm(A, B, a_mn=a_mn, b_mn=b_mn, residual=r)
+    assert ((c.double() - want - r.double()).abs() <= slack + 2e-6 * r.double().abs() + 2**-8 * (want + r.double()).abs()).all()
+    _lib.check_status()
+
+
+@pytest.mark.parametrize("M,F,Kd", [(520, 2816, 1000), (1030, 5000, 1000), (2048, 2816, 512)])
+def test_swiglu_epilogue_on_cta_pairs(M, F, Kd):
+    """One CTA of a pair holds the gate's columns, the other the matching ones of up. Tolerance as above."""
+    test_swiglu_epilogue_at_every_tile_width(M, F, Kd)
