@@ -2,8 +2,8 @@
 //
 // One CTA owns 256 query rows (two 128-row tiles) of one (batch, head) and walks the visible
 // 128-row KV tiles:
-//   warps 0-3   producer group (registers trimmed): warp 0 TMA (Q once, K/V through a 2-stage
-//               ring each), warp 1 tcgen05.mma issuer: S_w = Q_w K^T (SS), O_w += P_w V (P in TMEM)
+//   warps 0-3   producer group (registers trimmed): warp 0 TMA (Q once, K through a 2-stage ring), warp 2 TMA (V through
+//               another), warp 1 tcgen05.mma issuer: S_w = Q_w K^T (SS), O_w += P_w V (P in TMEM)
 //   warps 4-7   softmax group for tile 0, warps 8-11 for tile 1 (registers raised): tcgen05.ld S,
 //               mask, online softmax with lazy rescale of O in TMEM, P written back over S as bf16
 // TMEM: S0 | S1 | O0 | O1 (4 x 128 columns). While one group runs its softmax the tensor core
@@ -188,7 +188,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constant
     }
     for (int w = 0; w < 2; ++w) {
       mbar_init(&s_full[w], 1);
-      mbar_init(&p_full[w], 128);
+      mbar_init(&p_full[w], 4);
       mbar_init(&o_done[w], 1);
     }
     *abort_flag = 0;
@@ -240,13 +240,6 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constant
       fill_visibility(sVis + w * VIS_WORDS, nk, static_cast<int>(threadIdx.x), FWD_THREADS,
                       [&](int j) { return visible(w, j) && (!mk.bias || ((sLive[j >> 5] >> (j & 31)) & 1u)); });
   }
-  // next kv tile at or after j that q tile w sees, or nk
-  auto next_vis = [&](int w, int j) -> int {
-    if (use_vis) return vis_next(sVis + w * VIS_WORDS, j, nk);
-    for (; j < nk; ++j)
-      if (visible(w, j)) break;
-    return j;
-  };
   if (HALVES && p.splits > 1) {  // keep this split's share of the visible tiles (the launcher sees to use_vis)
     __syncthreads();
     if (threadIdx.x == 0) {
@@ -277,43 +270,70 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constant
   const uint32_t tS[2] = {tmem_base, tmem_base + 128};
   const uint32_t tO[2] = {tmem_base + 256, tmem_base + 384};
 
+  // next kv tile of a walk that any of this CTA's query tiles (`next_any`) or query tile w (`next_of`) sees, or nk
+  auto next_any = [&](VisWalk<NT>& wk, bool& s0, bool& s1) -> int {
+    if (use_vis) return wk.next(s0, s1);
+    for (; wk.at < nk; ++wk.at) {
+      s0 = visible(0, wk.at);
+      s1 = NT == 2 && visible(1, wk.at);
+      if (s0 || s1) return wk.at++;
+    }
+    return nk;
+  };
+  auto next_of = [&](VisWalk<1>& wk, int w) -> int {
+    bool s0, s1;
+    if (use_vis) return wk.next(s0, s1);
+    for (; wk.at < nk; ++wk.at)
+      if (visible(w, wk.at)) return wk.at++;
+    return nk;
+  };
+
   if (warp < 4) setmaxnreg_dec<FWD_REGS_PRODUCER>();
-  if (warp == 0) {
-    // ================================================================ TMA producer
+  if (warp == 0 || warp == 2) {
+    // ================================================================ TMA producers: Q and K (warp 0), V (warp 2)
+    // Scores are issued up to two tiles ahead of the product with V, so a stage of K comes free earlier than the stage of V that a common walk
+    // would have to fill first.
     if (lane == 0) {
-      mbar_arrive_expect_tx(q_full, NT * SM::Q_TILE_BYTES);
+      if (warp == 0) {
+        mbar_arrive_expect_tx(q_full, NT * SM::Q_TILE_BYTES);
 #pragma unroll
-      for (int w = 0; w < NT; ++w)
+        for (int w = 0; w < NT; ++w)
 #pragma unroll
-        for (int s = 0; s < NSLAB; ++s)
-          tma_load_4d(sQ + w * SM::Q_TILE_BYTES + s * SM::SLAB_BYTES, s < NQ ? &tma_q : &tma_q2, q_full,
-                      (s < NQ ? s : s - NQ) * 64, h, q0 + w * 128, b);
+          for (int s = 0; s < NSLAB; ++s)
+            tma_load_4d(sQ + w * SM::Q_TILE_BYTES + s * SM::SLAB_BYTES, s < NQ ? &tma_q : &tma_q2, q_full,
+                        (s < NQ ? s : s - NQ) * 64, h, q0 + w * 128, b);
+      }
       int it = 0;
-      auto next_any = [&](int j) { return HALVES ? next_vis(0, j) : min(next_vis(0, j), next_vis(1, j)); };
-      for (int j = next_any(0); j < nk; j = next_any(j + 1)) {
-        const int k0 = j * 128;
-        const int st = it & 1;
-        const uint32_t ph = (it >> 1) & 1;
-        const int kst = it % K_STAGES;
-        const uint32_t kph = (it / K_STAGES) & 1;
-        if (!mbar_wait_relaxed(&k_empty[kst], kph ^ 1u, wc, kTimeoutSmemEmpty)) break;
-        mbar_arrive_expect_tx(&k_full[kst], SM::K_TILE_BYTES);
+      VisWalk<NT> walk(sVis, use_vis ? nk : 0);
+      bool s0, s1;
+      for (int j = next_any(walk, s0, s1); j < nk; j = next_any(walk, s0, s1)) {
+        const int row = kv_row(j * 128);
+        if (warp == 0) {
+          const int st = it % K_STAGES;
+          if (!mbar_wait_relaxed(&k_empty[st], ((it / K_STAGES) & 1) ^ 1u, wc, kTimeoutSmemEmpty)) break;
+          mbar_arrive_expect_tx(&k_full[st], SM::K_TILE_BYTES);
 #pragma unroll
-        for (int s = 0; s < NSLAB; ++s)
-          tma_load_4d(sK + kst * SM::K_TILE_BYTES + s * SM::SLAB_BYTES, s < NQ ? &tma_k : &tma_k2, &k_full[kst],
-                      (s < NQ ? s : s - NQ) * 64, s < NQ ? h_kv : 0, kv_row(k0), b);
-        if (!mbar_wait_relaxed(&v_empty[st], ph ^ 1u, wc, kTimeoutSmemEmpty)) break;
-        mbar_arrive_expect_tx(&v_full[st], SM::V_TILE_BYTES);
+          for (int s = 0; s < NSLAB; ++s)
+            tma_load_4d(sK + st * SM::K_TILE_BYTES + s * SM::SLAB_BYTES, s < NQ ? &tma_k : &tma_k2, &k_full[st],
+                        (s < NQ ? s : s - NQ) * 64, s < NQ ? h_kv : 0, row, b);
+        } else {
+          const int st = it & 1;
+          if (!mbar_wait_relaxed(&v_empty[st], ((it >> 1) & 1) ^ 1u, wc, kTimeoutSmemEmpty)) break;
+          mbar_arrive_expect_tx(&v_full[st], SM::V_TILE_BYTES);
 #pragma unroll
-        for (int s = 0; s < VSLAB; ++s)
-          tma_load_4d(sV + st * SM::V_TILE_BYTES + s * SM::SLAB_BYTES, &tma_v, &v_full[st], s * 64,
-                      h_kv, kv_row(k0), b);
+          for (int s = 0; s < VSLAB; ++s)
+            tma_load_4d(sV + st * SM::V_TILE_BYTES + s * SM::SLAB_BYTES, &tma_v, &v_full[st], s * 64, h_kv, row, b);
+        }
         ++it;
       }
     }
     __syncwarp();
   } else if (warp == 1) {
     // ================================================================ MMA issuer (warp-uniform flow)
+    // One warp for both groups: it keeps them half a period apart, so that one group's exponentials run beside the other's products. (With
+    // a warp for each they fall into step, fight for the same unit and then wait for the same one: 4790 cycles a pair of tiles instead of 3890.)
+    // Nothing but the wait for a group's probabilities may stand between its products: a look at a barrier that has long completed takes
+    // some 200 cycles beside a busy tensor core, so the stages of K and V are waited for ahead of it.
     {
       const bool leader = elect_one();
       constexpr uint32_t idesc_s = make_idesc_bf16(128, 128, 0, 0);
@@ -344,97 +364,90 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constant
         }
         if (leader) umma_commit(&o_done[w]);
       };
+      VisWalk<NT> walk(sVis, use_vis ? nk : 0);
+      bool ok = mbar_wait(q_full, 0, wc, kTimeoutSmemFull);
+      bool n0, n1;
       if constexpr (HALVES) {
         // tile `it` of the walk belongs to group it & 1; its scores are issued two tiles ahead, behind the product of
         // the probabilities they overwrite
-        bool ok = mbar_wait(q_full, 0, wc, kTimeoutSmemFull);
-        int js = next_vis(0, 0);  // next tile whose scores are to be issued
-        int n_s = 0;
-        auto next_scores = [&]() {
-          const int st = n_s % K_STAGES;
-          if (!mbar_wait(&k_full[st], (n_s / K_STAGES) & 1, wc, kTimeoutSmemFull)) return false;
+        int n_s = 0;  // tiles whose scores are issued
+        bool more = ok && next_any(walk, n0, n1) < nk;
+        for (int i = 0; i < 2 && more; ++i) {
+          more = mbar_wait(&k_full[n_s % K_STAGES], (n_s / K_STAGES) & 1, wc, kTimeoutSmemFull);
+          if (!(ok = more)) break;
           tc_fence_after();
-          issue_s(n_s & 1, st);
-          if (leader) umma_commit(&k_empty[st]);
+          issue_s(n_s & 1, n_s % K_STAGES);
+          if (leader) umma_commit(&k_empty[n_s % K_STAGES]);
           ++n_s;
-          js = next_vis(0, js + 1);
-          return true;
-        };
-        if (ok && js < nk) ok = next_scores();
-        if (ok && js < nk) ok = next_scores();
+          more = next_any(walk, n0, n1) < nk;
+        }
         for (int it = 0; ok && it < n_s; ++it) {
           const int w = it & 1, st = it & 1;
           const uint32_t ph = (it >> 1) & 1;
           if (!mbar_wait(&v_full[st], ph, wc, kTimeoutSmemFull)) break;
+          if (more && !mbar_wait(&k_full[n_s % K_STAGES], (n_s / K_STAGES) & 1, wc, kTimeoutSmemFull)) break;
           if (!mbar_wait(&p_full[w], ph, wc, kTimeoutTmemFull)) break;
           tc_fence_after();
           issue_pv(w, st, it > 1);
           if (leader) umma_commit(&v_empty[st]);
-          if (js < nk) ok = next_scores();
+          if (more) {
+            issue_s(n_s & 1, n_s % K_STAGES);
+            if (leader) umma_commit(&k_empty[n_s % K_STAGES]);
+            ++n_s;
+            more = next_any(walk, n0, n1) < nk;
+          }
         }
       } else {
-      auto next_visible = [&](int j, bool& v0, bool& v1) {
-        const int a = next_vis(0, j), c = next_vis(1, j);
-        const int jj = min(a, c);
-        v0 = a == jj && jj < nk;
-        v1 = c == jj && jj < nk;
-        return jj;
-      };
-      bool ok = mbar_wait(q_full, 0, wc, kTimeoutSmemFull);
-      bool v0, v1;
-      int j = next_visible(0, v0, v1);
-      int it = 0;
-      int cnt[2] = {0, 0};
-      if (ok && j < nk) {
-        ok = mbar_wait(&k_full[0], 0, wc, kTimeoutSmemFull);
-        if (ok) {
-          tc_fence_after();
-          if (v0) issue_s(0, 0);
-          if (v1) issue_s(1, 0);
-          if (leader) umma_commit(&k_empty[0]);
-        }
-      }
-      while (ok && j < nk) {
-        bool n0, n1;
-        const int jn = next_visible(j + 1, n0, n1);
-        const int st = it & 1;
-        const uint32_t ph = (it >> 1) & 1;
-        const int stn = (it + 1) % K_STAGES;  // K stage of the next tile
-        const uint32_t phn = ((it + 1) / K_STAGES) & 1;
-        if (!mbar_wait(&v_full[st], ph, wc, kTimeoutSmemFull)) break;
-        bool k_ready = false;
-        if (v0) {
-          if (!mbar_wait(&p_full[0], cnt[0] & 1, wc, kTimeoutTmemFull)) break;
-          tc_fence_after();
-          issue_pv(0, st, cnt[0] != 0);
-          ++cnt[0];
-        }
-        if (jn < nk && n0) {
-          if (!mbar_wait(&k_full[stn], phn, wc, kTimeoutSmemFull)) break;
-          k_ready = true;
-          tc_fence_after();
-          issue_s(0, stn);
-        }
-        if (v1) {
-          if (!mbar_wait(&p_full[1], cnt[1] & 1, wc, kTimeoutTmemFull)) break;
-          tc_fence_after();
-          issue_pv(1, st, cnt[1] != 0);
-          ++cnt[1];
-        }
-        if (leader) umma_commit(&v_empty[st]);
-        if (jn < nk) {
-          if (n1) {
-            if (!k_ready && !mbar_wait(&k_full[stn], phn, wc, kTimeoutSmemFull)) break;
+        bool v0 = false, v1 = false;
+        int it = 0;
+        int cnt[2] = {0, 0};
+        bool have = ok && next_any(walk, v0, v1) < nk;
+        if (have) {
+          ok = mbar_wait(&k_full[0], 0, wc, kTimeoutSmemFull);
+          if (ok) {
             tc_fence_after();
-            issue_s(1, stn);
+            if (v0) issue_s(0, 0);
+            if (v1) issue_s(1, 0);
+            if (leader) umma_commit(&k_empty[0]);
           }
-          if (leader) umma_commit(&k_empty[stn]);
         }
-        j = jn;
-        v0 = n0;
-        v1 = n1;
-        ++it;
-      }
+        while (ok && have) {
+          n0 = n1 = false;
+          const bool more = next_any(walk, n0, n1) < nk;
+          const int st = it & 1;
+          const uint32_t ph = (it >> 1) & 1;
+          const int stn = (it + 1) % K_STAGES;  // K stage of the next tile
+          const uint32_t phn = ((it + 1) / K_STAGES) & 1;
+          if (!mbar_wait(&v_full[st], ph, wc, kTimeoutSmemFull)) break;
+          // (a single stage of K is filled behind the scores of this tile: waited for where it is needed)
+          if (K_STAGES > 1 && more && !mbar_wait(&k_full[stn], phn, wc, kTimeoutSmemFull)) break;
+          if (v0) {
+            if (!mbar_wait(&p_full[0], cnt[0] & 1, wc, kTimeoutTmemFull)) break;
+            tc_fence_after();
+            issue_pv(0, st, cnt[0] != 0);
+            ++cnt[0];
+          }
+          if (more && n0) {
+            if (K_STAGES == 1 && !mbar_wait(&k_full[stn], phn, wc, kTimeoutSmemFull)) break;
+            issue_s(0, stn);
+          }
+          if (v1) {
+            if (!mbar_wait(&p_full[1], cnt[1] & 1, wc, kTimeoutTmemFull)) break;
+            tc_fence_after();
+            issue_pv(1, st, cnt[1] != 0);
+            ++cnt[1];
+          }
+          if (leader) umma_commit(&v_empty[st]);
+          if (more) {
+            if (K_STAGES == 1 && !mbar_wait(&k_full[stn], phn, wc, kTimeoutSmemFull)) break;
+            if (n1) issue_s(1, stn);
+            if (leader) umma_commit(&k_empty[stn]);
+          }
+          have = more;
+          v0 = n0;
+          v1 = n1;
+          ++it;
+        }
       }
     }
     __syncwarp();
@@ -458,6 +471,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constant
     float l = 0.f;
     int cnt = 0;
     bool alive = true;
+    bool settled = false;  // every row of the warp has a reference
+    constexpr float kGrown = 32768.f;  // 128 * 2^8: a sum above it has a summand above 2^8, for which the accumulator is rescaled
 
     // Kinds of this query tile's bitmap tiles; without them every tile's bits are looked at, if there are any. A pointer for the whole
     // walk: asked for per tile out of the launch's parameters they cost every launch, those without a bitmap too (2 x 32 heads x 512, not
@@ -467,13 +482,13 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constant
                                     : nullptr;
     const bool bits = mk.drop_threshold || mk.keep;
     // every role walks the same visibility mask, so skips stay consistent
-    auto next_mine = [&](int j) {
-      j = next_vis(wv, j);
-      return HALVES && j < nk ? next_vis(wv, j + 1) : j;  // the other group takes the one between
+    VisWalk<1> walk(sVis + wv * VIS_WORDS, use_vis ? nk : 0);
+    auto next_mine = [&]() {
+      int j = next_of(walk, wv);
+      if (HALVES && (w == 1 || cnt > 0) && j < nk) j = next_of(walk, wv);  // the other group takes the one between
+      return j;
     };
-    int j = next_vis(wv, 0);
-    if (HALVES && w == 1 && j < nk) j = next_vis(wv, j + 1);
-    for (; j < nk && alive; j = next_mine(j + 1)) {
+    for (int j = next_mine(); j < nk && alive; j = next_mine()) {
       const int k0 = j * 128;
       const int kind = tile_mask(mk, b, tile_kinds ? tile_kinds[j] != 1 : bits, qi0, k0) | (EXT && !tile_window_plain(mk, p.window, qi0, k0) ? kMaskEdge : 0);
       const bool biased = mk.bias && (!use_vis || ((sAdd[j >> 5] >> (j & 31)) & 1u));
@@ -489,154 +504,159 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constant
         named_bar_sync(1 + w, 128);
       }
       // A wait that gives up must end the loop for the whole warp (the TMEM loads and stores are
-      // warp-collective). The lanes agree on that in the vote of the rescale check below, which exists
+      // warp-collective). The lanes agree on that in the vote behind the exponentials, which exists
       // anyway; until then every lane carries on (a lane that gave up merely loads a stale tile).
       const bool s_ok = mbar_wait(&s_full[w], cnt & 1, wc, kTimeoutTmemFull);
       tc_fence_after();
-      uint32_t sr[128];
+      uint32_t pk[64];
+      float sum;
+      // The scores of a tile are scaled by the reference of the tiles before it, without a look at their maximum, as long as no row's
+      // sum shows that it has grown out of it: p is at most kGrown then, and bf16, l and the accumulator are as exact at any scale. Otherwise
+      // (also as long as some row of the warp has seen no key) the tile is taken again from TMEM, with the maximum. The 64 three-way
+      // maxima ahead of the first exponential took 490 of a tile's 3900 cycles.
+      for (;;) {
+        uint32_t sr[128];
 #pragma unroll
-      for (int c = 0; c < 4; ++c) tmem_ld_x32(tS[w] + lane_base + c * 32, sr + c * 32);
-      tmem_ld_wait();
+        for (int c = 0; c < 4; ++c) tmem_ld_x32(tS[w] + lane_base + c * 32, sr + c * 32);
+        tmem_ld_wait();
 
-      float sc = p.scale_log2;  // multiplier still to be applied to sr[] inside the exp
-      // Masked tiles differ from plain ones only in this block: what hides an entry is gathered into four words of bits per
-      // row first (segment ids by warp votes), a bias is added by a loop of its own, and only words with a hole are walked
-      // column by column. One loop over 128 columns that tested bits, ids and bias for each took 8.9 us a tile (D = 64) where a plain
-      // tile takes 1.2: far more instructions than the caches hold, refetched every time.
-      if (kind != 0 || biased) {
-        uint32_t keep[4] = {0xffffffffu, 0xffffffffu, 0xffffffffu, 0xffffffffu};
-        if (kind & kMaskEdge) {
-          const int limit = causal_col_limit(mk, qpos, k0);
+        float sc = p.scale_log2;  // multiplier still to be applied to sr[] inside the exp
+        // Masked tiles differ from plain ones only in this block: what hides an entry is gathered into four words of bits per
+        // row first (segment ids by warp votes), a bias is added by a loop of its own, and only words with a hole are walked
+        // column by column. One loop over 128 columns that tested bits, ids and bias for each took 8.9 us a tile (D = 64) where a plain
+        // tile takes 1.2: far more instructions than the caches hold, refetched every time.
+        if (kind != 0 || biased) {
+          uint32_t keep[4] = {0xffffffffu, 0xffffffffu, 0xffffffffu, 0xffffffffu};
+          if (kind & kMaskEdge) {
+            const int limit = causal_col_limit(mk, qpos, k0);
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+              const int n = limit - 32 * c;
+              keep[c] = n >= 32 ? 0xffffffffu : (n <= 0 ? 0u : ((1u << n) - 1u));
+            }
+            if (EXT && p.window) {
+              const int first = qpos - p.window + 1 - mk.kmap(k0);  // columns before it are too far away
+#pragma unroll
+              for (int c = 0; c < 4; ++c) {
+                const int n = first - 32 * c;
+                keep[c] &= n >= 32 ? 0u : (n <= 0 ? 0xffffffffu : ~((1u << n) - 1u));
+              }
+            }
+          }
+          if (kind & kMaskBits) {
+            if (mk.keep) {
+              uint4 kb = make_uint4(0u, 0u, 0u, 0u);
+              if (RA_IN_BOUNDS((k0 >> 5), 4, mk.keep_sr, kTagAttnMaskBits))
+                kb = *reinterpret_cast<const uint4*>(
+                  mk.keep + b * mk.keep_sb + h * mk.keep_sh + static_cast<long long>(row_valid ? qi : mk.Sq - 1) * mk.keep_sr +
+                  (k0 >> 5));
+              keep[0] &= kb.x;
+              keep[1] &= kb.y;
+              keep[2] &= kb.z;
+              keep[3] &= kb.w;
+            }
+            if (mk.drop_threshold) {
+              const unsigned int kpos0 = static_cast<unsigned int>(mk.kmap(k0));
+#pragma unroll
+              for (int c = 0; c < 4; ++c) {
+                uint32_t drop = 0;
+#pragma unroll 1
+                for (int i = 0; i < 32; ++i)
+                  drop |= static_cast<uint32_t>(dropout_hash(mk.seed_lo, mk.seed_hi, bh_u, static_cast<unsigned int>(qpos),
+                                                             kpos0 + c * 32 + i) < mk.drop_threshold)
+                          << i;
+                keep[c] &= ~drop;
+              }
+            }
+          }
+          if (kind & kMaskSeg) keep_segment<4>(keep, sSeg + (w * 2 + buf) * 128, my_seg, lane);
+          if (biased) {
+            const float4* bias4 = reinterpret_cast<const float4*>(sBias + (w * 2 + buf) * 128);
+#pragma unroll
+            for (int g = 0; g < 32; ++g) {
+              const float4 bs = bias4[g];
+              sr[4 * g] = __float_as_uint(fmaf(__uint_as_float(sr[4 * g]), sc, bs.x));
+              sr[4 * g + 1] = __float_as_uint(fmaf(__uint_as_float(sr[4 * g + 1]), sc, bs.y));
+              sr[4 * g + 2] = __float_as_uint(fmaf(__uint_as_float(sr[4 * g + 2]), sc, bs.z));
+              sr[4 * g + 3] = __float_as_uint(fmaf(__uint_as_float(sr[4 * g + 3]), sc, bs.w));
+            }
+            sc = 1.0f;
+          }
 #pragma unroll
           for (int c = 0; c < 4; ++c) {
-            const int n = limit - 32 * c;
-            keep[c] = n >= 32 ? 0xffffffffu : (n <= 0 ? 0u : ((1u << n) - 1u));
-          }
-          if (EXT && p.window) {
-            const int first = qpos - p.window + 1 - mk.kmap(k0);  // columns before it are too far away
+            if (__all_sync(0xffffffffu, keep[c] == 0xffffffffu)) continue;
 #pragma unroll
-            for (int c = 0; c < 4; ++c) {
-              const int n = first - 32 * c;
-              keep[c] &= n >= 32 ? 0u : (n <= 0 ? 0xffffffffu : ~((1u << n) - 1u));
+            for (int i = 0; i < 32; ++i)
+              if (!((keep[c] >> i) & 1u)) sr[32 * c + i] = 0xff800000u;  // -inf
+          }
+        }
+        if (!settled) {  // online softmax with lazy rescale of the accumulator
+          float mc[4];
+#pragma unroll
+          for (int c = 0; c < 4; ++c) mc[c] = fmaxf(__uint_as_float(sr[32 * c]), __uint_as_float(sr[32 * c + 1]));
+#pragma unroll
+          for (int i = 2; i < 32; i += 2) {
+#pragma unroll
+            for (int c = 0; c < 4; ++c)
+              mc[c] = max3(mc[c], __uint_as_float(sr[32 * c + i]), __uint_as_float(sr[32 * c + i + 1]));
+          }
+          const float m_new = fmaxf(m_ref, fmaxf(fmaxf(mc[0], mc[1]), fmaxf(mc[2], mc[3])) * sc);
+          // also true when m_ref is -inf and m_new is finite
+          const bool need = cnt != 0 && m_new > m_ref + 8.0f;
+          if (cnt == 0) {
+            m_ref = m_new;
+          } else if (__any_sync(0xffffffffu, need)) {
+            if (!__all_sync(0xffffffffu, mbar_wait(&o_done[w], (cnt - 1) & 1, wc, kTimeoutTmemFull))) {
+              alive = false;
+              break;
             }
-          }
-        }
-        if (kind & kMaskBits) {
-          if (mk.keep) {
-            uint4 kb = make_uint4(0u, 0u, 0u, 0u);
-            if (RA_IN_BOUNDS((k0 >> 5), 4, mk.keep_sr, kTagAttnMaskBits))
-              kb = *reinterpret_cast<const uint4*>(
-                mk.keep + b * mk.keep_sb + h * mk.keep_sh + static_cast<long long>(row_valid ? qi : mk.Sq - 1) * mk.keep_sr +
-                (k0 >> 5));
-            keep[0] &= kb.x;
-            keep[1] &= kb.y;
-            keep[2] &= kb.z;
-            keep[3] &= kb.w;
-          }
-          if (mk.drop_threshold) {
-            const unsigned int kpos0 = static_cast<unsigned int>(mk.kmap(k0));
-#pragma unroll
-            for (int c = 0; c < 4; ++c) {
-              uint32_t drop = 0;
+            tc_fence_after();
+            const float alpha = (m_new == -INFINITY) ? 1.0f : exp2_approx(m_ref - m_new);
 #pragma unroll 1
-              for (int i = 0; i < 32; ++i)
-                drop |= static_cast<uint32_t>(dropout_hash(mk.seed_lo, mk.seed_hi, bh_u, static_cast<unsigned int>(qpos),
-                                                           kpos0 + c * 32 + i) < mk.drop_threshold)
-                        << i;
-              keep[c] &= ~drop;
+            for (int c = 0; c < DV / 32; ++c) {
+              uint32_t o[32];
+              tmem_ld_x32(tO[w] + lane_base + c * 32, o);
+              tmem_ld_wait();
+#pragma unroll
+              for (int i = 0; i < 32; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
+              tmem_st_x32(tO[w] + lane_base + c * 32, o);
             }
+            tmem_st_wait();
+            l *= alpha;
+            m_ref = m_new;
           }
         }
-        if (kind & kMaskSeg) keep_segment<4>(keep, sSeg + (w * 2 + buf) * 128, my_seg, lane);
-        if (biased) {
-          const float4* bias4 = reinterpret_cast<const float4*>(sBias + (w * 2 + buf) * 128);
+        const float m_use = (m_ref == -INFINITY) ? 0.f : m_ref;
+        const uint64_t neg_m2 = f2_pack(-m_use, -m_use);
+        const uint64_t sc2 = f2_pack(sc, sc);
+        uint64_t sum2 = f2_pack(0.f, 0.f);
 #pragma unroll
-          for (int g = 0; g < 32; ++g) {
-            const float4 bs = bias4[g];
-            sr[4 * g] = __float_as_uint(fmaf(__uint_as_float(sr[4 * g]), sc, bs.x));
-            sr[4 * g + 1] = __float_as_uint(fmaf(__uint_as_float(sr[4 * g + 1]), sc, bs.y));
-            sr[4 * g + 2] = __float_as_uint(fmaf(__uint_as_float(sr[4 * g + 2]), sc, bs.z));
-            sr[4 * g + 3] = __float_as_uint(fmaf(__uint_as_float(sr[4 * g + 3]), sc, bs.w));
-          }
-          sc = 1.0f;
+        for (int i = 0; i < 64; ++i) {
+          float x0, x1;
+          f2_unpack(f2_fma(f2_pack_u(sr[2 * i], sr[2 * i + 1]), sc2, neg_m2), x0, x1);
+          const float p0 = exp2_approx(x0), p1 = exp2_approx(x1);
+          sum2 = f2_add(sum2, f2_pack(p0, p1));
+          pk[i] = pack_bf16x2(p0, p1);
         }
-#pragma unroll
-        for (int c = 0; c < 4; ++c) {
-          if (__all_sync(0xffffffffu, keep[c] == 0xffffffffu)) continue;
-#pragma unroll
-          for (int i = 0; i < 32; ++i)
-            if (!((keep[c] >> i) & 1u)) sr[32 * c + i] = 0xff800000u;  // -inf
+        float sum_hi;
+        f2_unpack(sum2, sum, sum_hi);
+        sum += sum_hi;
+        const bool again = settled && !(sum <= kGrown);  // (NaN too)
+        if (!__any_sync(0xffffffffu, again || !s_ok)) break;
+        if (__any_sync(0xffffffffu, !s_ok)) {
+          alive = false;
+          break;
         }
+        settled = false;
       }
-      float mx;
-      {
-        float mc[4];
-#pragma unroll
-        for (int c = 0; c < 4; ++c) mc[c] = fmaxf(__uint_as_float(sr[32 * c]), __uint_as_float(sr[32 * c + 1]));
-#pragma unroll
-        for (int i = 2; i < 32; i += 2) {
-#pragma unroll
-          for (int c = 0; c < 4; ++c)
-            mc[c] = max3(mc[c], __uint_as_float(sr[32 * c + i]), __uint_as_float(sr[32 * c + i + 1]));
-        }
-        mx = fmaxf(fmaxf(mc[0], mc[1]), fmaxf(mc[2], mc[3])) * sc;
-      }
-
-      // ---- online softmax with lazy rescale of the accumulator
-      const float m_new = fmaxf(m_ref, mx);
-      // also true when m_ref is -inf and m_new is finite
-      const bool need = cnt != 0 && m_new > m_ref + 8.0f;
-      const bool rare = __any_sync(0xffffffffu, need || !s_ok);
-      if (rare && __any_sync(0xffffffffu, !s_ok)) {
-        alive = false;
-        break;
-      }
-      if (cnt == 0) {
-        m_ref = m_new;
-      } else {
-        if (rare) {
-          if (!__all_sync(0xffffffffu, mbar_wait(&o_done[w], (cnt - 1) & 1, wc, kTimeoutTmemFull))) {
-            alive = false;
-            break;
-          }
-          tc_fence_after();
-          const float alpha = (m_new == -INFINITY) ? 1.0f : exp2_approx(m_ref - m_new);
-#pragma unroll 1
-          for (int c = 0; c < DV / 32; ++c) {
-            uint32_t o[32];
-            tmem_ld_x32(tO[w] + lane_base + c * 32, o);
-            tmem_ld_wait();
-#pragma unroll
-            for (int i = 0; i < 32; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
-            tmem_st_x32(tO[w] + lane_base + c * 32, o);
-          }
-          tmem_st_wait();
-          l *= alpha;
-          m_ref = m_new;
-        }
-      }
-      const float m_use = (m_ref == -INFINITY) ? 0.f : m_ref;
-      const uint64_t neg_m2 = f2_pack(-m_use, -m_use);
-      const uint64_t sc2 = f2_pack(sc, sc);
-      uint64_t sum2 = f2_pack(0.f, 0.f);
-      uint32_t pk[64];
-#pragma unroll
-      for (int i = 0; i < 64; ++i) {
-        float x0, x1;
-        f2_unpack(f2_fma(f2_pack_u(sr[2 * i], sr[2 * i + 1]), sc2, neg_m2), x0, x1);
-        const float p0 = exp2_approx(x0), p1 = exp2_approx(x1);
-        sum2 = f2_add(sum2, f2_pack(p0, p1));
-        pk[i] = pack_bf16x2(p0, p1);
-      }
-      float sum, sum_hi;
-      f2_unpack(sum2, sum, sum_hi);
-      sum += sum_hi;
+      if (!alive) break;
+      if (!settled) settled = __all_sync(0xffffffffu, m_ref != -INFINITY);
       l += sum;
       tmem_st_x32(tS[w] + lane_base, pk);
       tmem_st_x32(tS[w] + lane_base + 32, pk + 32);
       tmem_st_wait();
       tc_fence_before();
-      mbar_arrive(&p_full[w]);
+      mbar_arrive_warp(&p_full[w]);
       ++cnt;
     }
 

@@ -317,3 +317,35 @@ def test_what_is_no_number_passes_through_a_launch_split_over_the_keys(where, ma
         dense = torch.einsum("bhqk,bkhd->bqhd", torch.softmax(x / D ** 0.5, -1), v.double())
         assert torch.equal(out.isnan(), dense.isnan()) and torch.equal(out.isinf(), dense.isinf())
         assert not torch.isfinite(out).all()
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("Sq,Sk,H", [(256, 1600, 2), (2048, 1600, 19), (130, 8000, 2)])  # one query tile a CTA, two, keys split
+@pytest.mark.parametrize("first", ["seen", "hidden"])
+def test_rows_that_outgrow_their_reference(first, Sq, Sk, H, D):
+    """Scores of a tile are scaled by the reference of the tiles before it as long as no row's sum has grown out of it. Here the logits of a row
+    step up by 2 to 800 from tile to tile, or down, or stay, by rows of all kinds side by side in a warp; `hidden`: many rows see no key
+    of the first tiles. Against dense attention in 64 bits on the same bf16 numbers: 1e-2 of the largest entry (P and the result are rounded
+    once each), the log-sum-exp within 2e-5 of the largest logit (fp32 sums of D products) plus 1e-3."""
+    from ringattention_b200.ops import _lib, flash
+
+    g = torch.Generator(device="cuda").manual_seed(Sq + D)
+    q = torch.randn(1, Sq, H, D, device="cuda", generator=g)
+    k, v = (torch.randn(1, Sk, H, D, device="cuda", generator=g) for _ in range(2))
+    q[..., 0] = torch.tensor([1.0, -1.0, 0.0, 0.25, 2.0], device="cuda")[torch.randint(0, 5, (1, Sq, H), device="cuda", generator=g)]
+    steps = torch.tensor([0.0, 2.0, 7.0, 7.0, 19.0, 60.0, 30.0, -80.0, 400.0, 390.0, 800.0], device="cuda")
+    k[..., 0] = (steps[(torch.arange(Sk, device="cuda") // 128) % steps.numel()] * D ** 0.5)[None, :, None]
+    q, k, v = q.bfloat16(), k.bfloat16(), v.bfloat16()
+    ms = flash.MaskSpec(causal_block_size=0, q_pos=flash.Positions(0), k_pos=flash.Positions(0))
+    m = torch.ones(1, 1, Sq, Sk, dtype=torch.bool, device="cuda")
+    if first == "hidden":
+        m[0, 0, 1::3, :300] = False
+        m[0, 0, 5::7, :1200] = False
+        ms.keep_q, ms.keep_k, ms.keep_tiles = flash.mask_bitmaps(m)
+    out, lse = flash.flash_fwd(q, k, v, ms)
+    _lib.check_status()
+    for h in range(H):
+        x = (q[0, :, h].double() @ k[0, :, h].double().t() / D ** 0.5).masked_fill(~m[0, 0], -float("inf"))
+        want = torch.softmax(x, -1) @ v[0, :, h].double()
+        assert (out[0, :, h].double() - want).abs().max() <= 0.01 * want.abs().max()
+        assert (lse[0, h].double() - torch.logsumexp(x, -1)).abs().max() <= 2e-5 * x[torch.isfinite(x)].abs().max() + 1e-3
