@@ -145,10 +145,10 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constant
   uint64_t* do_empty = bars + 6;
   uint64_t* s_full = bars + 7;
   uint64_t* dp_full = bars + 8;
-  uint64_t* p_ready = bars + 9;    // one arrival a warp: 8
-  uint64_t* ds_ready = bars + 10;  // one arrival a warp: 8
+  uint64_t* p_ready = bars + 9;    // 256 arrivals
+  uint64_t* ds_ready = bars + 10;  // 256 arrivals
   uint64_t* dq_full = bars + 11;
-  uint64_t* dq_empty = bars + 12;  // 4 arrivals
+  uint64_t* dq_empty = bars + 12;  // 128 arrivals
   uint64_t* acc_full = bars + 13;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 16);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
@@ -177,10 +177,10 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constant
     mbar_init(do_empty, 1);
     mbar_init(s_full, 1);
     mbar_init(dp_full, 1);
-    mbar_init(p_ready, 8);
-    mbar_init(ds_ready, 8);
+    mbar_init(p_ready, 256);
+    mbar_init(ds_ready, 256);
     mbar_init(dq_full, 1);
-    mbar_init(dq_empty, 4);
+    mbar_init(dq_empty, 128);
     mbar_init(acc_full, 1);
     *abort_flag = 0;
     fence_mbar_init();
@@ -476,7 +476,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constant
       }
       tmem_st_wait();
       tc_fence_before();
-      mbar_arrive_warp(p_ready);
+      mbar_arrive(p_ready);
       trace_event(p.trace, tr && sm_tid == 0, 1, it, 1);
 
       if (!__all_sync(0xffffffffu, mbar_wait(dp_full, par, wc, kTimeoutTmemFull))) { alive = false; break; }
@@ -521,7 +521,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constant
       tmem_st_wait();
       tc_fence_before();
       fence_proxy_async_smem();
-      mbar_arrive_warp(ds_ready);
+      mbar_arrive(ds_ready);
       trace_event(p.trace, tr && sm_tid == 0, 1, it, 3);
       ++it;
     }
@@ -595,7 +595,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constant
       for (int c = 0; c < D / 32; ++c) tmem_ld_x32(tDP + lane_base + c * 32, r + c * 32);
       tmem_ld_wait();
       tc_fence_before();
-      mbar_arrive_warp(dq_empty);
+      mbar_arrive(dq_empty);
       trace_event(p.trace, tr && warp == 12 && lane == 0, 2, it, 1);
       uint8_t* dq_row = sDQ + row * 128;
       const int swz = row & 7;
