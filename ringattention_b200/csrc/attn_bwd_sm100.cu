@@ -873,3 +873,5 @@ extern "C" int ra_attn_bwd_prep(const void* o, long long o_sb, long long o_ss, l
       lse, lse2, delta, dq_acc, B, H, Sq, Sq_pad, heads_log2);
   return check_launch("attn_bwd_prep_kernel");
 }
+
+RA_PACKED(ra_attn_bwd_prep)

@@ -1834,3 +1834,14 @@ extern "C" int ra_rope_append(void* qkv, void* k_cache, void* v_cache, long long
                                              stripe_rank, stripe_base, stripe_len0);
   return check_launch("rope_append_kernel");
 }
+
+RA_PACKED(ra_decode_merge)
+RA_PACKED(ra_kv_append)
+RA_PACKED(ra_decode_advance)
+RA_PACKED(ra_small_m_linear)
+RA_PACKED(ra_row_norm_gated)
+RA_PACKED(ra_small_m_linear_fused)
+RA_PACKED(ra_small_m_linear_mma)
+RA_PACKED(ra_small_m_linear_segments)
+RA_PACKED(ra_small_m_linear_gated)
+RA_PACKED(ra_rope_append)

@@ -836,3 +836,19 @@ extern "C" int ra_segment_tiles(const int* src, long long ld, int off0, int off1
                                                                                                    dst, mm);
   return check_launch("segment_tiles");
 }
+
+RA_PACKED(ra_rmsnorm_fwd)
+RA_PACKED(ra_rmsnorm_bwd)
+RA_PACKED(ra_rope)
+RA_PACKED(ra_rope_at)
+RA_PACKED(ra_swiglu_fwd)
+RA_PACKED(ra_swiglu_bwd)
+RA_PACKED(ra_embedding_fwd)
+RA_PACKED(ra_embedding_bwd)
+RA_PACKED(ra_xent_fwd_bwd)
+RA_PACKED(ra_sumsq)
+RA_PACKED(ra_adamw)
+RA_PACKED(ra_cast_f32_bf16)
+RA_PACKED(ra_cast_bf16_f32)
+RA_PACKED(ra_pack_mask)
+RA_PACKED(ra_segment_tiles)

@@ -197,3 +197,7 @@ extern "C" int ra_gemm_bf16_ex(const void* A, const void* B, void* C, const void
                  bias, alpha};
   return gemm::launch<0, 0>(gemm::Operands{A, B, lda, ldb}, p, static_cast<cudaStream_t>(stream));
 }
+
+RA_PACKED(ra_gemm_bf16)
+RA_PACKED(ra_gemm_bf16_swiglu)
+RA_PACKED(ra_gemm_bf16_ex)

@@ -94,3 +94,5 @@ extern "C" int ra_linear_f32(const float* A, const float* B, float* C, const flo
   lin32::linear_f32_kernel<<<grid, lin32::THREADS, 0, static_cast<cudaStream_t>(stream)>>>(p);
   return check_launch("linear_f32_kernel");
 }
+
+RA_PACKED(ra_linear_f32)

@@ -183,3 +183,8 @@ extern "C" int ra_gated_act_f32(const float* gu, float* y, long long ldy, int ro
   resid::gated_act_kernel<<<rows, 256, 0, static_cast<cudaStream_t>(stream)>>>(gu, y, ldy, F);
   return check_launch("gated_act_kernel");
 }
+
+RA_PACKED(ra_embed_f32)
+RA_PACKED(ra_norm_f32)
+RA_PACKED(ra_stream_pair)
+RA_PACKED(ra_gated_act_f32)

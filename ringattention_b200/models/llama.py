@@ -25,7 +25,7 @@ from ..ops import ffn
 from ..ops import kernels as K
 from ..ops.flash import Positions
 from ..ops.reference import shard_segments
-from ..utils.tracing import phase
+from ..utils.tracing import idle, phase
 from .params import FlatParams
 
 
@@ -71,6 +71,14 @@ class _LayerFFNLinears:
 
     def gate_up_dgrad(self, dgu, out):
         return self.P.lin_dgrad(dgu, self.gu, out=out)
+
+    def weights(self):
+        P = self.P
+        return (P.w(self.gu), P.w(self.d)) if P.shard_count == 1 and idle() else None
+
+    def wgrad_targets(self):
+        d, gu = self.P.g(self.d), self.P.g(self.gu)
+        return d, d, gu, gu
 
 
 class LlamaModel:

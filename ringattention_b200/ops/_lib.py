@@ -10,6 +10,7 @@ from __future__ import annotations
 
 import ctypes
 import os
+import struct
 import threading
 from pathlib import Path
 
@@ -147,6 +148,10 @@ def ptr(t: torch.Tensor | None) -> ctypes.c_void_p:
     return ctypes.c_void_p(0 if t is None else t.data_ptr())
 
 
+def address(t: torch.Tensor | None) -> int:
+    return 0 if t is None else t.data_ptr()
+
+
 def launches() -> int:
     """Number of kernels of this library launched so far in this process."""
     return _LAUNCHES
@@ -157,13 +162,25 @@ def count_launch(n: int = 1) -> None:
     _LAUNCHES += n
 
 
+def _entry(name: str):
+    """The launcher and, where it takes its arguments as one packed block, what packs them: the library says in which
+    format. Such launchers take plain numbers (pointers as integers)."""
+    handle = lib()
+    fmt = getattr(handle, name + "_packed_format", None)
+    if fmt is None:
+        return getattr(handle, name), None
+    fmt.restype = ctypes.c_char_p
+    return getattr(handle, name + "_packed"), struct.Struct("@" + fmt().decode()).pack
+
+
 def call(name: str, *args, n_kernels: int = 1) -> None:
     """Call launcher ``name``; raise with the library's message on a non-zero return code."""
     global _LAUNCHES
-    fn = _FNS.get(name)
-    if fn is None:
-        fn = _FNS[name] = getattr(lib(), name)
-    rc = fn(*args)
+    entry = _FNS.get(name)
+    if entry is None:
+        entry = _FNS[name] = _entry(name)
+    fn, pack = entry
+    rc = fn(pack(*args)) if pack is not None else fn(*args)
     if rc != 0:
         msg = lib().ra_last_error()
         raise KernelError(f"{name} failed ({rc}): {msg.decode() if msg else ''}")

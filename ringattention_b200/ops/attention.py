@@ -21,7 +21,7 @@ from . import flash
 from . import kernels as K
 from .flash import MaskSpec, Positions
 from .reference import shard_segments
-from ..utils.tracing import phase
+from ..utils.tracing import idle, phase
 
 
 @dataclass
@@ -106,6 +106,16 @@ def ring_forward(q, k, v, plan: RingPlan, symm_ring=None, out=None):
 def ring_backward(q, k, v, out, lse, dout, plan: RingPlan, symm_ring=None, dq=None, dk=None, dv=None):
     """Returns ``(dq, dk, dv)`` bf16. ``dq/dk/dv`` may be given as (strided) destination views."""
     B, Sq, H, D = q.shape
+    if plan.world == 1 and idle() and out.shape == q.shape:
+        if dk is None:
+            dk = torch.empty_like(k)
+        if dv is None:
+            dv = torch.empty(dk.shape, device=dk.device, dtype=dk.dtype) if dk.is_contiguous() \
+                else torch.empty_strided(dk.shape, dk.stride(), device=dk.device, dtype=dk.dtype)
+        to = torch.empty_like(q) if dq is None else dq
+        if flash.dq_rows(to) is not None and to.dtype == torch.bfloat16:
+            flash.flash_bwd_run(q, k, v, out, lse, dout, plan.steps[0].mask, to, dk, dv)
+            return to, dk, dv
     with phase("attn_bwd_prep"):
         dq_acc = torch.empty(B, Sq, H, D, device=q.device, dtype=torch.float32)
         lse2, delta = flash.flash_bwd_prep(out, dout, lse, dq_acc)

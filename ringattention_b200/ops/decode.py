@@ -9,6 +9,7 @@ from __future__ import annotations
 import ctypes
 import math
 import os
+import struct
 from typing import Optional
 
 import torch
@@ -29,23 +30,9 @@ STAGES = int(os.environ.get("RINGATTN_B200_DECODE_STAGES", "3"))
 MMA_MIN_ROWS = int(os.environ.get("RINGATTN_B200_DECODE_MMA_MIN_ROWS", "2"))
 
 
-class _DecodeArgs(ctypes.Structure):
-    _fields_ = [
-        ("q", c_vp), ("k", c_vp), ("v", c_vp),
-        ("k_sb", c_ll), ("k_ss", c_ll), ("k_sh", c_ll), ("v_sb", c_ll), ("v_ss", c_ll), ("v_sh", c_ll),
-        ("o_part", c_vp), ("lse_part", c_vp),
-        ("mask", c_vp), ("m_sb", c_ll), ("m_sh", c_ll), ("m_sq", c_ll),
-        ("B", ctypes.c_int), ("H", ctypes.c_int), ("QL", ctypes.c_int), ("S", ctypes.c_int),
-        ("D", ctypes.c_int), ("splits", ctypes.c_int),
-        ("softmax_scale", ctypes.c_float),
-        ("q_pos0", c_ll), ("k_pos0", c_ll),
-        ("pos_ptr", c_vp),
-        ("stripe_n", ctypes.c_int), ("stripe_rank", ctypes.c_int),
-        ("stripe_base", c_ll), ("stripe_len0", c_ll),
-        ("stream", c_vp),
-        ("stages", ctypes.c_int),
-        ("mma", ctypes.c_int),
-    ]
+# ``RaDecodeArgs`` (decode_sm100.cu): q k v, strides of k and v, o_part lse_part, mask and its strides, B H QL S D splits, softmax_scale,
+# q_pos0 k_pos0, pos_ptr, the stripe (ranks, rank, prefilled rows per rank, prefilled positions), stream, stages, mma
+_DECODE_ARGS = struct.Struct("@3P6q 2P P3q 6i f 2q P 2i2q P 2i")
 
 
 def _pad_q(q: torch.Tensor):
@@ -93,27 +80,16 @@ def decode_partial(q, k, v, *, n_valid: Optional[int] = None, q_pos0: int = -1, 
     rows = B * H * QL
     o_part = torch.empty(rows, splits, D, device=q.device, dtype=torch.float32)
     lse_part = torch.empty(rows, splits, device=q.device, dtype=torch.float32)
-    a = _DecodeArgs()
-    a.q, a.k, a.v = q.data_ptr(), k.data_ptr(), v.data_ptr()
-    a.k_sb, a.k_ss, a.k_sh = k.stride(0), k.stride(1), k.stride(2)
-    a.v_sb, a.v_ss, a.v_sh = v.stride(0), v.stride(1), v.stride(2)
-    a.o_part, a.lse_part = o_part.data_ptr(), lse_part.data_ptr()
+    m = (0, 0, 0, 0)
     if mask is not None:
         assert mask.dtype == torch.uint8 and mask.dim() == 4 and mask.stride(3) == 1
-        a.mask = mask.data_ptr()
-        a.m_sb = mask.stride(0) if mask.shape[0] > 1 else 0
-        a.m_sh = mask.stride(1) if mask.shape[1] > 1 else 0
-        a.m_sq = mask.stride(2) if mask.shape[2] > 1 else 0
-    a.B, a.H, a.QL, a.S, a.D, a.splits = B, H, QL, S, D, splits
-    a.softmax_scale = 1.0 / math.sqrt(D)
-    a.q_pos0, a.k_pos0 = int(q_pos0), int(k_pos0)
-    a.pos_ptr = pos_ptr
+        m = (mask.data_ptr(), *(mask.stride(i) if mask.shape[i] > 1 else 0 for i in range(3)))
     # striped cache (with pos_ptr): (ranks, rank, prefilled rows per rank, prefilled positions)
-    a.stripe_n, a.stripe_rank, a.stripe_base, a.stripe_len0 = stripe if stripe is not None else (0, 0, 0, 0)
-    a.stream = _lib.stream_handle()
-    a.stages = STAGES
-    a.mma = int(QL >= MMA_MIN_ROWS)
-    _lib.call("ra_decode_splitkv", ctypes.byref(a))
+    args = _DECODE_ARGS.pack(q.data_ptr(), k.data_ptr(), v.data_ptr(), *k.stride()[:3], *v.stride()[:3], o_part.data_ptr(),
+                             lse_part.data_ptr(), *m, B, H, QL, S, D, splits, 1.0 / math.sqrt(D), int(q_pos0), int(k_pos0), pos_ptr,
+                             *(stripe if stripe is not None else (0, 0, 0, 0)), _lib.stream_handle(), STAGES,
+                             int(QL >= MMA_MIN_ROWS))
+    _lib.call("ra_decode_splitkv", args)
     return o_part, lse_part
 
 
@@ -129,14 +105,10 @@ def merge_partials(o_part, lse_part, H: int, QL: int, *, out=None, lse_out=None,
     n_ranks = my_rank = 0
     if inbox is not None:
         o_ptrs, lse_ptrs, n_ranks, my_rank = inbox
-    _lib.call("ra_decode_merge", c_vp(o_part.data_ptr()), c_vp(lse_part.data_ptr()),
-              c_ll(o_part.stride(0)), c_ll(o_part.stride(1)), c_ll(lse_part.stride(0)),
-              c_ll(lse_part.stride(1)), rows, nparts, D, H, QL,
-              c_vp(0 if out is None else out.data_ptr()),
-              0 if out is None else int(out.dtype == torch.float32),
-              c_vp(0 if lse_out is None else lse_out.data_ptr()), c_vp(o_ptrs), c_vp(lse_ptrs),
-              n_ranks, my_rank, c_vp(step_ptr), c_ll(slot_mul), c_ll(slot_add), c_ll(out_slot[0]), c_ll(out_slot[1]), c_ll(in_slot[0]),
-              c_ll(in_slot[1]), _lib.stream_ptr())
+    _lib.call("ra_decode_merge", o_part.data_ptr(), lse_part.data_ptr(), o_part.stride(0), o_part.stride(1), lse_part.stride(0),
+              lse_part.stride(1), rows, nparts, D, H, QL, 0 if out is None else out.data_ptr(),
+              0 if out is None else int(out.dtype == torch.float32), 0 if lse_out is None else lse_out.data_ptr(), o_ptrs, lse_ptrs,
+              n_ranks, my_rank, step_ptr, slot_mul, slot_add, out_slot[0], out_slot[1], in_slot[0], in_slot[1], _lib.stream_handle())
     return out
 
 

@@ -34,16 +34,20 @@ class WeightGrad:
     def __init__(self, w: torch.Tensor, parts: int):
         self.w, self.left, self.acc, self.grad = w, parts, None, None
 
-    def add(self, dy, x):
+    def target(self):
+        """Where the next product goes, and what it is added to (or None)."""
         self.left -= 1
+        before = self.acc
         if self.left == 0:
-            self.grad = K.gemm(dy, x, a_mn=True, b_mn=True, out=torch.empty(self.w.shape, device=self.w.device, dtype=self.w.dtype),
-                               residual=self.acc)
-            self.acc = None
-        elif self.acc is None:
-            self.acc = K.gemm(dy, x, a_mn=True, b_mn=True, out_dtype=torch.float32)
-        else:
-            K.linear_wgrad(dy, x, self.acc)
+            self.grad, self.acc = torch.empty(self.w.shape, device=self.w.device, dtype=self.w.dtype), None
+            return self.grad, before
+        if before is None:
+            self.acc = torch.empty(self.w.shape, device=self.w.device, dtype=torch.float32)
+        return self.acc, before
+
+    def add(self, dy, x):
+        out, before = self.target()
+        K.gemm(dy, x, a_mn=True, b_mn=True, out=out, residual=before)
 
 
 class DenseLinears:
@@ -74,6 +78,13 @@ class DenseLinears:
     def gate_up_dgrad(self, dgu, out):
         return K.linear_dgrad(dgu, self.wgu, out=out)
 
+    def weights(self):
+        """Both weights if a chunk's backward may run in one call on them (plain tensors on this device), or None."""
+        return self.wgu, self.wd
+
+    def wgrad_targets(self):
+        return (*self.dwd.target(), *self.dwgu.target())
+
 
 def ffn_forward(lin, x: torch.Tensor, chunk: int, residual: Optional[torch.Tensor] = None,
                 keep: Optional[list] = None) -> torch.Tensor:
@@ -100,6 +111,17 @@ def ffn_backward(lin, x: torch.Tensor, dy: torch.Tensor, chunk: int, kept: Optio
     M = x.shape[0]
     dx = torch.empty_like(x)
     step = min(chunk, M)
+    w = lin.weights()
+    if w is not None and all(t.is_contiguous() and t.dtype == torch.bfloat16 for t in (x, dy, *w)):
+        F = w[1].shape[1]
+        room = torch.empty(step * F * (2 if kept is not None else 4), device=x.device, dtype=x.dtype)  # act, da and the pre-activations
+        for ci, r0 in enumerate(range(0, M, step)):
+            r1 = min(M, r0 + step)
+            n = (r1 - r0) * F
+            act, da = room[:n], room[n:2 * n]
+            gu = kept[ci] if kept is not None else room[2 * n:4 * n]
+            K.ffn_bwd_run(x[r0:r1], dy[r0:r1], dx[r0:r1], *w, gu, act, da, *lin.wgrad_targets(), recompute=kept is None)
+        return dx
     for ci, r0 in enumerate(range(0, M, step)):
         r1 = min(M, r0 + step)
         gu = kept[ci] if kept is not None else lin.gate_up(x[r0:r1])

@@ -7,17 +7,14 @@ Both take ``(B, S, H, D)`` bf16 views with a contiguous last dim (``D`` in {64, 
 """
 from __future__ import annotations
 
-import ctypes
 import math
+import struct
 from dataclasses import dataclass
 from typing import Optional
 
 import torch
 
 from . import _lib
-
-c_ll = ctypes.c_longlong
-c_vp = ctypes.c_void_p
 
 
 @dataclass
@@ -97,36 +94,15 @@ def segment_shard(seg: torch.Tensor, pos: Positions, n: int):
         seg = seg.contiguous()
     ids = torch.empty(B, n, device=seg.device, dtype=torch.int32)
     mm = torch.empty(B, (n + 127) // 128, 2, device=seg.device, dtype=torch.int32)
-    _lib.call("ra_segment_tiles", c_vp(seg.data_ptr()), c_ll(seg.stride(0)), pos.off0, pos.off1, min(pos.half, 1 << 30), B, n,
-              c_vp(ids.data_ptr()), c_vp(mm.data_ptr()), _lib.stream_ptr())
+    _lib.call("ra_segment_tiles", seg.data_ptr(), seg.stride(0), pos.off0, pos.off1, min(pos.half, 1 << 30), B, n,
+              ids.data_ptr(), mm.data_ptr(), _lib.stream_handle())
     return ids, mm
 
 
-class _FwdArgs(ctypes.Structure):
-    _fields_ = [
-        ("q", c_vp), ("k", c_vp), ("v", c_vp),
-        ("q_sb", c_ll), ("q_ss", c_ll), ("q_sh", c_ll),
-        ("k_sb", c_ll), ("k_ss", c_ll), ("k_sh", c_ll),
-        ("v_sb", c_ll), ("v_ss", c_ll), ("v_sh", c_ll),
-        ("out", c_vp), ("o_sb", c_ll), ("o_ss", c_ll), ("o_sh", c_ll), ("out_fp32", ctypes.c_int),
-        ("lse_out", c_vp),
-        ("o_prev", c_vp), ("lse_prev", c_vp),
-        ("B", ctypes.c_int), ("H", ctypes.c_int), ("Sq", ctypes.c_int), ("Sk", ctypes.c_int),
-        ("D", ctypes.c_int),
-        ("softmax_scale", ctypes.c_float),
-        ("causal_block_size", ctypes.c_int),
-        ("q_off0", ctypes.c_int), ("q_off1", ctypes.c_int), ("q_half", ctypes.c_int),
-        ("k_off0", ctypes.c_int), ("k_off1", ctypes.c_int), ("k_half", ctypes.c_int),
-        ("seg_q", c_vp), ("seg_k", c_vp), ("seg_q_mm", c_vp), ("seg_k_mm", c_vp),
-        ("bias", c_vp), ("bias_sb", c_ll), ("bias_sh", c_ll),
-        ("seed", ctypes.c_ulonglong), ("drop_threshold", ctypes.c_uint),
-        ("keep", c_vp), ("keep_sb", c_ll), ("keep_sh", c_ll), ("keep_sr", c_ll),
-        ("keep_tiles", c_vp), ("keep_tiles_sb", c_ll), ("keep_tiles_sh", c_ll),
-        ("copy_src", c_vp), ("copy_dst", c_vp), ("copy_bytes", c_ll), ("copy_ctas", ctypes.c_int),
-        ("status", c_vp),
-        ("stream", c_vp),
-        ("splits", ctypes.c_int), ("ws", c_vp),
-    ]
+# ``RaAttnFwdArgs`` (attn_fwd_sm100.cu), packed as the C compiler lays it out: q k v, their strides, out and its strides, out_fp32, lse_out,
+# o_prev lse_prev, B H Sq Sk D, softmax_scale, the mask's fields (:func:`_mask_fields`), the copy job, status, stream, splits, ws. (A
+# ctypes structure of these fields takes 11 us to fill, this 3.)
+_FWD_ARGS = struct.Struct("@3P9q P3qi P 2P 5i f 7i4P P2q QI P3q P2q 2Pqi 2P iP")
 
 
 def tma_ready(t: torch.Tensor) -> bool:
@@ -159,8 +135,8 @@ def mask_bitmaps(mask: torch.Tensor, want_q: bool = True, want_k: bool = True):
     by_q = torch.empty(B, Hm, Sq, 4 * nk, device=m.device, dtype=torch.int32) if want_q else None
     by_k = torch.empty(B, Hm, Sk, 4 * nq, device=m.device, dtype=torch.int32) if want_k else None
     tiles = torch.empty(B, Hm, nq, nk, device=m.device, dtype=torch.uint8)
-    _lib.call("ra_pack_mask", c_vp(m.data_ptr()), c_ll(m.stride(0)), c_ll(m.stride(1)), c_ll(m.stride(2)),
-              c_vp(_ptr(by_q)), c_vp(_ptr(by_k)), c_vp(tiles.data_ptr()), B, Hm, Sq, Sk, _lib.stream_ptr())
+    _lib.call("ra_pack_mask", m.data_ptr(), m.stride(0), m.stride(1), m.stride(2), _ptr(by_q), _ptr(by_k), tiles.data_ptr(),
+              B, Hm, Sq, Sk, _lib.stream_handle())
     return by_q, by_k, tiles
 
 
@@ -210,45 +186,25 @@ def flash_fwd(q, k, v, mask: MaskSpec, *, o_prev=None, lse_prev=None, out_fp32=F
         lse_out = torch.empty(B, H, Sq, device=dev, dtype=torch.float32)
     if o_prev is not None:
         assert o_prev.dtype == torch.float32 and o_prev.is_contiguous() and lse_prev is not None
-    a = _FwdArgs(q.data_ptr(), k.data_ptr(), v.data_ptr(), *q.stride()[:3], *k.stride()[:3], *v.stride()[:3],
-                 out.data_ptr(), *out.stride()[:3], int(out.dtype == torch.float32), lse_out.data_ptr(),
-                 _ptr(o_prev), _ptr(lse_prev), B, H, Sq, Sk, D, 1.0 / math.sqrt(D), *_mask_fields(mask, H),
-                 copy_src, copy_dst, copy_bytes, copy_ctas, _lib.status_tensor(dev).data_ptr(), _lib.stream_handle(), 0, 0)
-    splits = _lib.lib().ra_attn_fwd_splits(ctypes.byref(a))
+    fields = (q.data_ptr(), k.data_ptr(), v.data_ptr(), *q.stride()[:3], *k.stride()[:3], *v.stride()[:3],
+              out.data_ptr(), *out.stride()[:3], int(out.dtype == torch.float32), lse_out.data_ptr(),
+              _ptr(o_prev), _ptr(lse_prev), B, H, Sq, Sk, D, 1.0 / math.sqrt(D), *_mask_fields(mask, H),
+              copy_src, copy_dst, copy_bytes, copy_ctas, _lib.status_tensor(dev).data_ptr(), _lib.stream_handle())
+    args = _FWD_ARGS.pack(*fields, 0, 0)
+    splits = _lib.lib().ra_attn_fwd_splits(args)
     if splits > 1:  # few query tiles: the keys are split over several CTAs, partial results meet in a second launch
         ws = torch.empty(splits * B * Sq * H * (D + 1), device=dev, dtype=torch.float32)
-        a.splits, a.ws = splits, ws.data_ptr()
-    _lib.call("ra_attn_fwd", ctypes.byref(a), n_kernels=2 if splits > 1 else 1)
+        args = _FWD_ARGS.pack(*fields, splits, ws.data_ptr())
+    _lib.call("ra_attn_fwd", args, n_kernels=2 if splits > 1 else 1)
     return out, lse_out
 
 
-class _BwdArgs(ctypes.Structure):
-    _fields_ = [
-        ("q", c_vp), ("k", c_vp), ("v", c_vp), ("d_o", c_vp),
-        ("q_sb", c_ll), ("q_ss", c_ll), ("q_sh", c_ll),
-        ("k_sb", c_ll), ("k_ss", c_ll), ("k_sh", c_ll),
-        ("v_sb", c_ll), ("v_ss", c_ll), ("v_sh", c_ll),
-        ("do_sb", c_ll), ("do_ss", c_ll), ("do_sh", c_ll),
-        ("lse2", c_vp), ("delta", c_vp), ("Sq_pad", ctypes.c_int),
-        ("dq_acc", c_vp),
-        ("dk", c_vp), ("dv", c_vp), ("dkv_sb", c_ll), ("dkv_ss", c_ll), ("dkv_sh", c_ll),
-        ("dkv_mode", ctypes.c_int),
-        ("B", ctypes.c_int), ("H", ctypes.c_int), ("Sq", ctypes.c_int), ("Sk", ctypes.c_int),
-        ("D", ctypes.c_int),
-        ("softmax_scale", ctypes.c_float),
-        ("causal_block_size", ctypes.c_int),
-        ("q_off0", ctypes.c_int), ("q_off1", ctypes.c_int), ("q_half", ctypes.c_int),
-        ("k_off0", ctypes.c_int), ("k_off1", ctypes.c_int), ("k_half", ctypes.c_int),
-        ("seg_q", c_vp), ("seg_k", c_vp), ("seg_q_mm", c_vp), ("seg_k_mm", c_vp),
-        ("bias", c_vp), ("bias_sb", c_ll), ("bias_sh", c_ll),
-        ("seed", ctypes.c_ulonglong), ("drop_threshold", ctypes.c_uint),
-        ("keep", c_vp), ("keep_sb", c_ll), ("keep_sh", c_ll), ("keep_sr", c_ll),
-        ("keep_tiles", c_vp), ("keep_tiles_sb", c_ll), ("keep_tiles_sh", c_ll),
-        ("copy_src", c_vp), ("copy_dst", c_vp), ("copy_bytes", c_ll), ("copy_ctas", ctypes.c_int),
-        ("status", c_vp),
-        ("stream", c_vp),
-        ("trace", c_vp),
-    ]
+# ``RaAttnBwdArgs`` (attn_api.h): q k v dO, their strides, lse2 delta Sq_pad, dq_acc, dk dv and their strides and mode, B H Sq Sk D,
+# softmax_scale, the mask's fields, the copy job, status, stream, trace
+_BWD_FORMAT = "@4P12q 2Pi P 2P3qi 5i f 7i4P P2q QI P3q P2q 2Pqi 3P"
+_BWD_ARGS = struct.Struct(_BWD_FORMAT)
+# ``RaAttnBwdRun`` (backward_runs.cu): the same, then out and its strides, lse, dq and the distance of its rows
+_BWD_RUN_ARGS = struct.Struct(_BWD_FORMAT + "P3q 2Pq")
 
 
 # Phase-timestamp buffers by device index: a backward launch on that device records into its buffer
@@ -271,10 +227,8 @@ def flash_bwd_prep(out, dout, lse, dq_acc=None):
     delta = torch.empty(B, H, sq_pad, device=out.device, dtype=torch.float32)
     assert lse.dtype == torch.float32 and lse.is_contiguous() and lse.shape == (B, H, Sq)
     assert dq_acc is None or (dq_acc.dtype == torch.float32 and dq_acc.is_contiguous() and dq_acc.shape == out.shape)
-    _lib.call("ra_attn_bwd_prep", c_vp(out.data_ptr()), c_ll(out.stride(0)), c_ll(out.stride(1)),
-              c_ll(out.stride(2)), c_vp(dout.data_ptr()), c_ll(dout.stride(0)), c_ll(dout.stride(1)),
-              c_ll(dout.stride(2)), c_vp(lse.data_ptr()), c_vp(lse2.data_ptr()),
-              c_vp(delta.data_ptr()), c_vp(_ptr(dq_acc)), B, H, Sq, sq_pad, D, _lib.stream_ptr())
+    _lib.call("ra_attn_bwd_prep", out.data_ptr(), *out.stride()[:3], dout.data_ptr(), *dout.stride()[:3], lse.data_ptr(),
+              lse2.data_ptr(), delta.data_ptr(), _ptr(dq_acc), B, H, Sq, sq_pad, D, _lib.stream_handle())
     return lse2, delta
 
 
@@ -283,18 +237,47 @@ def flash_bwd(q, k, v, dout, lse2, delta, mask: MaskSpec, dq_acc, dk, dv, dkv_mo
     """One ring step of the backward. ``dq_acc`` (fp32, contiguous, pre-zeroed by the caller before
     the first step) receives ``dQ`` by reduction; ``dk``/``dv`` are written according to
     ``dkv_mode`` (store bf16, store fp32, or fp32 reduction into possibly remote memory)."""
+    assert dq_acc.dtype == torch.float32 and dq_acc.is_contiguous() and dq_acc.shape == q.shape
+    fields = _bwd_fields(q, k, v, dout, lse2.data_ptr(), delta.data_ptr(), lse2.shape[2], mask, dq_acc.data_ptr(), dk, dv, dkv_mode,
+                         copy_src, copy_dst, copy_bytes, copy_ctas)
+    _lib.call("ra_attn_bwd", _BWD_ARGS.pack(*fields))
+
+
+def flash_bwd_run(q, k, v, out, lse, dout, mask: MaskSpec, dq, dk, dv) -> None:
+    """The whole backward on one device in one call: :func:`flash_bwd_prep`, :func:`flash_bwd` and ``dq`` in bf16. ``dq``, ``dk`` and ``dv``
+    are bf16 views; those of ``dq`` whose batch and sequence form rows of ``H * D`` values a fixed distance apart."""
+    _check_bshd(out, "out")
+    B, Sq, H, D = q.shape
+    assert out.shape == q.shape and lse.dtype == torch.float32 and lse.is_contiguous() and lse.shape == (B, H, Sq)
+    assert dq.shape == q.shape and dq.dtype == torch.bfloat16 and dq_rows(dq) is not None
+    sq_pad = (Sq + 127) // 128 * 128
+    n, rows = B * Sq * H * D, B * H * sq_pad
+    scratch = torch.empty(n + 2 * rows, device=q.device, dtype=torch.float32)  # dq_acc, lse2, delta
+    at = scratch.data_ptr()
+    fields = _bwd_fields(q, k, v, dout, at + 4 * n, at + 4 * (n + rows), sq_pad, mask, at, dk, dv, DKV_STORE_BF16, 0, 0, 0, 0)
+    _lib.call("ra_attn_bwd_run", _BWD_RUN_ARGS.pack(*fields, out.data_ptr(), *out.stride()[:3], lse.data_ptr(), dq.data_ptr(), dq_rows(dq)),
+              n_kernels=3)
+
+
+def dq_rows(dq: torch.Tensor) -> Optional[int]:
+    """Distance in elements of the rows of ``H * D`` values that batch and sequence of ``dq (B, S, H, D)`` form, or None."""
+    B, S, H, D = dq.shape
+    sb, ss, sh, sd = dq.stride()
+    return ss if sd == 1 and sh == D and sb == S * ss else None
+
+
+def _bwd_fields(q, k, v, dout, lse2: int, delta: int, sq_pad: int, mask: MaskSpec, dq_acc: int, dk, dv, dkv_mode, copy_src, copy_dst,
+                copy_bytes, copy_ctas) -> tuple:
+    """The fields of ``RaAttnBwdArgs``."""
     _check_bshd(q, "q"); _check_bshd(k, "k"); _check_bshd(v, "v"); _check_bshd(dout, "dout")
     B, Sq, H, D = q.shape
     Sk = k.shape[1]
     dev = q.device
-    assert dq_acc.dtype == torch.float32 and dq_acc.is_contiguous() and dq_acc.shape == q.shape
     assert dk.shape == k.shape and dv.shape == k.shape and dk.stride() == dv.stride()
     want = torch.bfloat16 if dkv_mode == DKV_STORE_BF16 else torch.float32
     assert dk.dtype == want and dv.dtype == want and dk.stride(3) == 1
     tb = BWD_TRACE_BUFFERS.get(dev.index if dev.index is not None else torch.cuda.current_device())
-    a = _BwdArgs(q.data_ptr(), k.data_ptr(), v.data_ptr(), dout.data_ptr(), *q.stride()[:3], *k.stride()[:3],
-                 *v.stride()[:3], *dout.stride()[:3], lse2.data_ptr(), delta.data_ptr(), lse2.shape[2],
-                 dq_acc.data_ptr(), dk.data_ptr(), dv.data_ptr(), *dk.stride()[:3], dkv_mode, B, H, Sq, Sk, D,
-                 1.0 / math.sqrt(D), *_mask_fields(mask, H, by_k=True), copy_src, copy_dst, copy_bytes, copy_ctas,
-                 _lib.status_tensor(dev).data_ptr(), _lib.stream_handle(), 0 if tb is None else tb.data_ptr())
-    _lib.call("ra_attn_bwd", ctypes.byref(a))
+    return (q.data_ptr(), k.data_ptr(), v.data_ptr(), dout.data_ptr(), *q.stride()[:3], *k.stride()[:3], *v.stride()[:3],
+            *dout.stride()[:3], lse2, delta, sq_pad, dq_acc, dk.data_ptr(), dv.data_ptr(), *dk.stride()[:3], dkv_mode, B, H, Sq, Sk, D,
+            1.0 / math.sqrt(D), *_mask_fields(mask, H, by_k=True), copy_src, copy_dst, copy_bytes, copy_ctas,
+            _lib.status_tensor(dev).data_ptr(), _lib.stream_handle(), 0 if tb is None else tb.data_ptr())

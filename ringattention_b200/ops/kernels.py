@@ -5,21 +5,17 @@ fall back to PyTorch math. Shapes follow the LLaMA driver: activations are ``(ro
 """
 from __future__ import annotations
 
-import ctypes
 import os
 from typing import Optional
 
 import torch
 
 from . import _lib
-from ._lib import ptr, stream_ptr
-
-c_ll = ctypes.c_longlong
-c_f = ctypes.c_float
+from ._lib import address, stream_handle
 
 
 def _status():
-    return ptr(_lib.status_tensor())
+    return _lib.status_tensor().data_ptr()
 
 
 # ---------------------------------------------------------------------------------------------
@@ -35,29 +31,28 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
     ``out`` itself (in-place accumulation, used for fp32 weight-gradient accumulation), or is fp32 where C is bf16.
     """
     assert a.dtype == torch.bfloat16 and b.dtype == torch.bfloat16 and a.dim() == 2 and b.dim() == 2
-    assert a.stride(1) == 1 and b.stride(1) == 1
+    (M, K), (lda, a1) = a.shape, a.stride()
+    (N, Kb), (ldb, b1) = b.shape, b.stride()
     if a_mn:
-        K, M = a.shape
-    else:
-        M, K = a.shape
+        M, K = K, M
     if b_mn:
-        Kb, N = b.shape
-    else:
-        N, Kb = b.shape
+        N, Kb = Kb, N
+    assert a1 == 1 and b1 == 1
     assert K == Kb, f"inner dims differ: {K} vs {Kb}"
     if out is None:
         out = torch.empty(M, N, device=a.device, dtype=out_dtype)
-    assert out.shape == (M, N) and out.stride(1) == 1
+    ldc, c1 = out.stride()
+    assert out.shape == (M, N) and c1 == 1
     c_fp32 = 1 if out.dtype == torch.float32 else 0
+    res = ldr = 0
     if residual is not None:
         assert residual.shape == out.shape and residual.stride(1) == 1
         assert residual.dtype == out.dtype or (residual.dtype, out.dtype) == (torch.float32, torch.bfloat16)
         if residual.dtype != out.dtype:
             c_fp32 = 2
-    _lib.call("ra_gemm_bf16", ptr(a), ptr(b), ptr(out), ptr(residual), M, N, K,
-              c_ll(a.stride(0)), c_ll(b.stride(0)), c_ll(out.stride(0)),
-              c_ll(residual.stride(0) if residual is not None else 0),
-              int(a_mn), int(b_mn), c_fp32, group_m, _status(), stream_ptr())
+        res, ldr = residual.data_ptr(), residual.stride(0)
+    _lib.call("ra_gemm_bf16", a.data_ptr(), b.data_ptr(), out.data_ptr(), res, M, N, K, lda, ldb, ldc, ldr,
+              1 if a_mn else 0, 1 if b_mn else 0, c_fp32, group_m, _status(), stream_handle())
     return out
 
 
@@ -76,8 +71,8 @@ def linear_swiglu(x, wgu, out=None, group_m: int = 8):
     if out is None:
         out = torch.empty(M, F, device=x.device, dtype=torch.bfloat16)
     assert out.shape == (M, F) and out.stride(1) == 1 and out.dtype == torch.bfloat16
-    _lib.call("ra_gemm_bf16_swiglu", ptr(x), ptr(wgu), ptr(out), M, F, Kd, c_ll(x.stride(0)),
-              c_ll(wgu.stride(0)), c_ll(out.stride(0)), group_m, _status(), stream_ptr())
+    _lib.call("ra_gemm_bf16_swiglu", address(x), address(wgu), address(out), M, F, Kd, x.stride(0),
+              wgu.stride(0), out.stride(0), group_m, _status(), stream_handle())
     return out
 
 
@@ -113,9 +108,9 @@ def linear_ex(x, w, out, *, residual=None, tail=None, n_split: Optional[int] = N
     ld2 = tail.stride(0) if tail is not None else 0
     if x.dtype == torch.float32:
         assert out.dtype == torch.float32
-        _lib.call("ra_linear_f32", ptr(x), ptr(w), ptr(out), ptr(residual), ptr(tail), M, N, Kd, c_ll(x.stride(0)),
-                  c_ll(w.stride(0)), c_ll(out.stride(0)), c_ll(ldr), c_ll(ld2), n_split, int(relu2), ptr(bias), c_f(alpha),
-                  stream_ptr())
+        _lib.call("ra_linear_f32", address(x), address(w), address(out), address(residual), address(tail), M, N, Kd, x.stride(0),
+                  w.stride(0), out.stride(0), ldr, ld2, n_split, int(relu2), address(bias), alpha,
+                  stream_handle())
         return out
     if M <= 8 and w.is_contiguous() and (residual is None or (residual.data_ptr() == out.data_ptr() and
                                                               out.dtype == torch.float32)):
@@ -124,9 +119,9 @@ def linear_ex(x, w, out, *, residual=None, tail=None, n_split: Optional[int] = N
         if relu2:
             return linear_segments(x, w, x2=x, ya=out, act_from=0)
         return linear_segments(x, w, y=out, y32=tail, n32_from=None if tail is None else n_split, bias=bias, alpha=alpha)
-    _lib.call("ra_gemm_bf16_ex", ptr(x), ptr(w), ptr(out), ptr(residual), ptr(tail), M, N, Kd, c_ll(x.stride(0)),
-              c_ll(w.stride(0)), c_ll(out.stride(0)), c_ll(ldr), c_ll(ld2), n_split, int(relu2),
-              int(out.dtype == torch.float32), ptr(bias), c_f(alpha), 8, _status(), stream_ptr())
+    _lib.call("ra_gemm_bf16_ex", address(x), address(w), address(out), address(residual), address(tail), M, N, Kd, x.stride(0),
+              w.stride(0), out.stride(0), ldr, ld2, n_split, int(relu2),
+              int(out.dtype == torch.float32), address(bias), alpha, 8, _status(), stream_handle())
     return out
 
 
@@ -138,10 +133,10 @@ def linear_gated(x, wgu, out):
     if x.dtype == torch.float32:
         gu = torch.empty(M, 2 * F, device=x.device, dtype=torch.float32)
         linear_ex(x, wgu, gu)
-        _lib.call("ra_gated_act_f32", ptr(gu), ptr(out), c_ll(out.stride(0)), M, F, stream_ptr())
+        _lib.call("ra_gated_act_f32", address(gu), address(out), out.stride(0), M, F, stream_handle())
     elif M <= 8:
-        _lib.call("ra_small_m_linear_gated", ptr(x), c_ll(x.stride(0)), ptr(wgu), ptr(out), c_ll(out.stride(0)), M, F,
-                  x.shape[1], stream_ptr())
+        _lib.call("ra_small_m_linear_gated", address(x), x.stride(0), address(wgu), address(out), out.stride(0), M, F,
+                  x.shape[1], stream_handle())
     else:
         linear_swiglu(x, wgu, out=out[:, :F])
     return out
@@ -162,10 +157,10 @@ def linear_segments(x, w, *, x2=None, y=None, y32=None, ya=None, n32_from: Optio
     assert x2 is None or (x2.shape == x.shape and x2.stride() == x.stride())
     for t, n in ((y, min(n32_from, N)), (y32, min(act_from, N) - n32_from), (ya, N - act_from)):
         assert t is None or (t.shape[0] == M and t.stride(1) == 1 and t.shape[1] >= n)
-    ld = lambda t: c_ll(0 if t is None else t.stride(0))
-    _lib.call("ra_small_m_linear_segments", ptr(x), ptr(x2), c_ll(x.stride(0)), ptr(w), ptr(y), ld(y), ptr(y32), ld(y32),
-              int(add32), ptr(ya), ld(ya), n32_from, act_from, M, N, Kd, ptr(bias), c_f(alpha),
-              stream_ptr())
+    ld = lambda t: (0 if t is None else t.stride(0))
+    _lib.call("ra_small_m_linear_segments", address(x), address(x2), x.stride(0), address(w), address(y), ld(y), address(y32), ld(y32),
+              int(add32), address(ya), ld(ya), n32_from, act_from, M, N, Kd, address(bias), alpha,
+              stream_handle())
     return y if y is not None else (y32 if y32 is not None else ya)
 
 
@@ -179,7 +174,7 @@ def rmsnorm_fwd(x, w, eps: float, out=None, rstd=None):
         out = torch.empty_like(x)
     if rstd is None:
         rstd = torch.empty(rows, device=x.device, dtype=torch.float32)
-    _lib.call("ra_rmsnorm_fwd", ptr(x), ptr(w), ptr(out), ptr(rstd), rows, d, c_f(eps), stream_ptr())
+    _lib.call("ra_rmsnorm_fwd", address(x), address(w), address(out), address(rstd), rows, d, eps, stream_handle())
     return out, rstd
 
 
@@ -191,8 +186,8 @@ def rmsnorm_bwd(dy, x, w, rstd, dw_acc, dres=None, out=None):
         out = torch.empty_like(x)
     parts = _lib.lib().ra_rmsnorm_bwd_parts(rows)
     scratch = torch.empty(parts, d, device=x.device, dtype=torch.float32)  # per-CTA partial gain gradients
-    _lib.call("ra_rmsnorm_bwd", ptr(dy), ptr(x), ptr(w), ptr(rstd), ptr(dres), ptr(out), ptr(dw_acc),
-              ptr(scratch), rows, d, stream_ptr(), n_kernels=2)
+    _lib.call("ra_rmsnorm_bwd", address(dy), address(x), address(w), address(rstd), address(dres), address(out), address(dw_acc),
+              address(scratch), rows, d, stream_handle(), n_kernels=2)
     return out
 
 
@@ -200,9 +195,9 @@ def rope_(x, positions, theta: float, inverse: bool = False):
     """Rotate a ``(B, S, H, D)`` bf16 view in place. ``positions`` is a flash.Positions map."""
     B, S, H, D = x.shape
     assert x.stride(3) == 1 and x.dtype == torch.bfloat16
-    _lib.call("ra_rope", ptr(x), c_ll(x.stride(0)), c_ll(x.stride(1)), c_ll(x.stride(2)), B, S, H, D,
-              int(positions.off0), int(positions.off1), int(min(positions.half, 1 << 30)), c_f(theta),
-              int(inverse), stream_ptr())
+    _lib.call("ra_rope", address(x), x.stride(0), x.stride(1), x.stride(2), B, S, H, D,
+              int(positions.off0), int(positions.off1), int(min(positions.half, 1 << 30)), theta,
+              int(inverse), stream_handle())
     return x
 
 
@@ -212,7 +207,7 @@ def swiglu_fwd(gu, out=None):
     assert gu.is_contiguous()
     if out is None:
         out = torch.empty(rows, F, device=gu.device, dtype=torch.bfloat16)
-    _lib.call("ra_swiglu_fwd", ptr(gu), ptr(out), c_ll(rows), F, stream_ptr())
+    _lib.call("ra_swiglu_fwd", address(gu), address(out), rows, F, stream_handle())
     return out
 
 
@@ -220,8 +215,27 @@ def swiglu_bwd_(gu, dh):
     """Overwrites ``gu`` with ``[d gate | d up]``."""
     rows, f2 = gu.shape
     assert gu.is_contiguous() and dh.is_contiguous()
-    _lib.call("ra_swiglu_bwd", ptr(gu), ptr(dh), ptr(gu), c_ll(rows), f2 // 2, stream_ptr())
+    _lib.call("ra_swiglu_bwd", address(gu), address(dh), address(gu), rows, f2 // 2, stream_handle())
     return gu
+
+
+def ffn_bwd_run(x, dy, dx, wgu, wd, gu, act, da, dwd, dwd_add, dwgu, dwgu_add, recompute: bool) -> None:
+    """The launches of one chunk of :func:`ringattention_b200.ops.ffn.ffn_backward` in one call: ``x, dy, dx (rows, d)``, weights ``(2F, d)`` and
+    ``(d, F)``, scratch ``gu`` (``2 rows F`` values: the pre-activations, made here with ``recompute``), ``act`` and ``da`` (``rows F``); all
+    bf16 and contiguous. The weight gradients go to ``dwd`` and ``dwgu`` (fp32, or bf16), added to ``*_add`` (fp32, ``None``: nothing)."""
+    rows, d = x.shape
+    F = wd.shape[1]
+    assert dy.shape == dx.shape == x.shape and wgu.shape == dwgu.shape == (2 * F, d) and wd.shape == dwd.shape == (d, F)
+    assert gu.numel() == 2 * rows * F and act.numel() == da.numel() == rows * F
+    f32 = torch.float32
+
+    def mode(out, add):  # of the gradient's product, see gemm()
+        assert out.is_contiguous() and (add is None or (add.is_contiguous() and add.dtype == f32 and add.shape == out.shape))
+        return 1 if out.dtype == f32 else (0 if add is None else 2)
+
+    _lib.call("ra_ffn_bwd_run", x.data_ptr(), dy.data_ptr(), dx.data_ptr(), wgu.data_ptr(), wd.data_ptr(), gu.data_ptr(), act.data_ptr(),
+              da.data_ptr(), dwd.data_ptr(), address(dwd_add), dwgu.data_ptr(), address(dwgu_add), rows, d, F, int(recompute),
+              mode(dwd, dwd_add), mode(dwgu, dwgu_add), _status(), stream_handle(), n_kernels=7 if recompute else 6)
 
 
 # ---------------------------------------------------------------------------------------------
@@ -230,8 +244,8 @@ def swiglu_bwd_(gu, dh):
 def embed_f32(tokens, table, d: int, out):
     """``out (rows, ld)`` fp32 <- the tokens' rows of ``table`` (bf16 or fp32); columns past ``d`` are zeroed."""
     assert tokens.dtype == torch.int32 and tokens.is_contiguous() and out.dtype == torch.float32 and out.is_contiguous()
-    _lib.call("ra_embed_f32", ptr(tokens), ptr(table), c_ll(table.stride(0)), ptr(out), c_ll(out.stride(0)),
-              tokens.numel(), d, table.shape[0], int(table.dtype == torch.float32), stream_ptr())
+    _lib.call("ra_embed_f32", address(tokens), address(table), table.stride(0), address(out), out.stride(0),
+              tokens.numel(), d, table.shape[0], int(table.dtype == torch.float32), stream_handle())
     return out
 
 
@@ -240,8 +254,8 @@ def stream_pair(tokens, table, x, d: int):
     rows, dp = x.shape
     assert tokens.dtype == torch.int32 and tokens.numel() == rows and x.dtype == torch.float32 and x.stride(1) == 1
     out = torch.empty(rows, 2 * dp, device=x.device, dtype=table.dtype)
-    _lib.call("ra_stream_pair", ptr(tokens), ptr(table), c_ll(table.stride(0)), ptr(x), c_ll(x.stride(0)), ptr(out), rows, d,
-              dp, table.shape[0], int(table.dtype == torch.float32), stream_ptr())
+    _lib.call("ra_stream_pair", address(tokens), address(table), table.stride(0), address(x), x.stride(0), address(out), rows, d,
+              dp, table.shape[0], int(table.dtype == torch.float32), stream_handle())
     return out
 
 
@@ -254,8 +268,8 @@ def norm_f32(x, d: int, eps: float, gain_offset: float, w1, w2=None, rows_idx=No
     y2 = torch.empty_like(y1) if w2 is not None else None
     assert x.dtype == torch.float32 and x.stride(1) == 1 and w1.numel() == ld and (w2 is None or w2.numel() == ld)
     assert rows_idx is None or rows_idx.dtype == torch.int32
-    _lib.call("ra_norm_f32", ptr(x), ptr(rows_idx), ptr(w1), ptr(w2), ptr(y1), ptr(y2), rows, d, ld, c_ll(ld), c_ll(ld),
-              c_f(eps), c_f(gain_offset), int(w1.dtype == torch.float32), stream_ptr())
+    _lib.call("ra_norm_f32", address(x), address(rows_idx), address(w1), address(w2), address(y1), address(y2), rows, d, ld, ld, ld,
+              eps, gain_offset, int(w1.dtype == torch.float32), stream_handle())
     return y1, y2
 
 
@@ -268,7 +282,7 @@ def embedding_fwd(tokens, table, out=None):
     assert tokens.dtype == torch.int32 and tokens.is_contiguous()
     if out is None:
         out = torch.empty(n, d, device=table.device, dtype=torch.bfloat16)
-    _lib.call("ra_embedding_fwd", ptr(tokens), ptr(table), ptr(out), c_ll(n), d, vocab, stream_ptr())
+    _lib.call("ra_embedding_fwd", address(tokens), address(table), address(out), n, d, vocab, stream_handle())
     return out
 
 
@@ -276,7 +290,7 @@ def embedding_bwd(tokens, dy, dtable_acc):
     n = tokens.numel()
     vocab, d = dtable_acc.shape
     assert dtable_acc.dtype == torch.float32 and dy.is_contiguous()
-    _lib.call("ra_embedding_bwd", ptr(tokens), ptr(dy), ptr(dtable_acc), c_ll(n), d, vocab, stream_ptr())
+    _lib.call("ra_embedding_bwd", address(tokens), address(dy), address(dtable_acc), n, d, vocab, stream_handle())
 
 
 def xent_fwd_bwd_(logits, targets, grad_scale: float, loss=None):
@@ -286,8 +300,8 @@ def xent_fwd_bwd_(logits, targets, grad_scale: float, loss=None):
     assert logits.stride(1) == 1 and targets.dtype == torch.int32
     if loss is None:
         loss = torch.empty(rows, device=logits.device, dtype=torch.float32)
-    _lib.call("ra_xent_fwd_bwd", ptr(logits), c_ll(logits.stride(0)), ptr(targets), ptr(loss),
-              c_ll(rows), V, c_f(grad_scale), stream_ptr())
+    _lib.call("ra_xent_fwd_bwd", address(logits), logits.stride(0), address(targets), address(loss),
+              rows, V, grad_scale, stream_handle())
     return loss
 
 
@@ -297,7 +311,7 @@ def xent_fwd_bwd_(logits, targets, grad_scale: float, loss=None):
 def sumsq(g, out):
     """``out[0] += sum(g**2)`` for an fp32 buffer."""
     assert g.dtype == torch.float32 and g.is_contiguous() and out.dtype == torch.float32
-    _lib.call("ra_sumsq", ptr(g), c_ll(g.numel()), ptr(out), stream_ptr())
+    _lib.call("ra_sumsq", address(g), g.numel(), address(out), stream_handle())
     return out
 
 
@@ -307,23 +321,23 @@ def adamw_(p, m, v, g, p16, *, step: int, lr: float, beta1: float, beta2: float,
     n = p.numel()
     bc1 = 1.0 - beta1 ** step
     bc2 = 1.0 - beta2 ** step
-    _lib.call("ra_adamw", ptr(p), ptr(m), ptr(v), ptr(g), ptr(p16), c_ll(n), c_ll(decay_end),
-              c_f(lr), c_f(beta1), c_f(beta2), c_f(eps), c_f(weight_decay), c_f(bc1), c_f(bc2),
-              c_f(clip), ptr(gnorm_sq), c_f(grad_mul), stream_ptr())
+    _lib.call("ra_adamw", address(p), address(m), address(v), address(g), address(p16), n, decay_end,
+              lr, beta1, beta2, eps, weight_decay, bc1, bc2,
+              clip, address(gnorm_sq), grad_mul, stream_handle())
 
 
 def cast_f32_to_bf16(src, dst):
     """``src`` ``(rows, d)`` fp32 -> ``dst`` bf16; both 2-D views, row strides allowed."""
     rows, d = src.shape
     assert src.stride(1) == 1 and dst.stride(1) == 1 and dst.shape == src.shape
-    _lib.call("ra_cast_f32_bf16", ptr(src), ptr(dst), c_ll(rows), d, c_ll(src.stride(0)),
-              c_ll(dst.stride(0)), stream_ptr())
+    _lib.call("ra_cast_f32_bf16", address(src), address(dst), rows, d, src.stride(0),
+              dst.stride(0), stream_handle())
     return dst
 
 
 def cast_bf16_to_f32(src, dst):
     assert src.is_contiguous() and dst.is_contiguous() and src.numel() == dst.numel()
-    _lib.call("ra_cast_bf16_f32", ptr(src), ptr(dst), c_ll(src.numel()), stream_ptr())
+    _lib.call("ra_cast_bf16_f32", address(src), address(dst), src.numel(), stream_handle())
     return dst
 
 
@@ -343,7 +357,7 @@ def _small_m_linear_mma(x, w, residual, out=None):
         out = torch.empty(M, N, device=x.device, dtype=torch.bfloat16)
     assert out.is_contiguous() and out.shape == (M, N) and x.is_contiguous() and w.is_contiguous()
     assert x.shape[1] == Kd and (residual is None or residual.is_contiguous())
-    _lib.call("ra_small_m_linear_mma", ptr(x), ptr(w), ptr(out), ptr(residual), M, N, Kd, stream_ptr())
+    _lib.call("ra_small_m_linear_mma", address(x), address(w), address(out), address(residual), M, N, Kd, stream_handle())
     return out
 
 
@@ -358,7 +372,7 @@ def small_m_linear(x, w, out=None, residual=None):
     assert out.is_contiguous() and (residual is None or residual.is_contiguous())
     if _mma_linear_ok(M):
         return _small_m_linear_mma(x, w, residual, out=out)
-    _lib.call("ra_small_m_linear", ptr(x), ptr(w), ptr(out), ptr(residual), M, N, Kd, stream_ptr())
+    _lib.call("ra_small_m_linear", address(x), address(w), address(out), address(residual), M, N, Kd, stream_handle())
     return out
 
 
@@ -375,8 +389,8 @@ def _small_m_linear_fused(x, w, residual, gain, eps, prologue, out=None):
     if out is None:
         out = torch.empty(M, N, device=x.device, dtype=torch.bfloat16)
     assert out.is_contiguous() and out.shape == (M, N)
-    _lib.call("ra_small_m_linear_fused", ptr(x), ptr(w), ptr(out), ptr(residual), ptr(gain), c_f(eps), prologue,
-              M, N, Kd, stream_ptr())
+    _lib.call("ra_small_m_linear_fused", address(x), address(w), address(out), address(residual), address(gain), eps, prologue,
+              M, N, Kd, stream_handle())
     return out
 
 
@@ -420,7 +434,7 @@ def norm_swiglu_linear(x, gain, eps: float, wgu, wd, residual=None):
     assert wgu.shape == (2 * F, x.shape[1])
     if _fused_small_m_ok(x, wgu) and x.shape[0] == 1 and x.shape[1] <= _lib.lib().ra_row_linear_max_k():
         h = torch.empty(1, F, device=x.device, dtype=torch.bfloat16)
-        _lib.call("ra_row_norm_gated", ptr(x), ptr(wgu), ptr(h), ptr(gain), c_f(eps), F, x.shape[1], stream_ptr())
+        _lib.call("ra_row_norm_gated", address(x), address(wgu), address(h), address(gain), eps, F, x.shape[1], stream_handle())
         return linear_auto(h, wd, residual=residual)
     return swiglu_linear(norm_linear(x, gain, eps, wgu), wd, residual=residual)
 
@@ -432,17 +446,17 @@ def rope_append(qkv, k_cache, v_cache, pos_state, theta: float, k0: int = 0, str
     assert qkv.is_contiguous() and qkv.numel() == B * 3 * H * D
     assert k_cache.stride() == v_cache.stride() and k_cache.stride(3) == 1
     sn, sr, sb, sl = stripe if stripe is not None else (0, 0, 0, 0)
-    _lib.call("ra_rope_append", ptr(qkv), ptr(k_cache), ptr(v_cache), c_ll(k_cache.stride(0)),
-              c_ll(k_cache.stride(1)), c_ll(k_cache.stride(2)), ptr(pos_state), c_f(theta), c_ll(k0), S_max, B, H, D,
-              int(sn), int(sr), c_ll(sb), c_ll(sl), stream_ptr())
+    _lib.call("ra_rope_append", address(qkv), address(k_cache), address(v_cache), k_cache.stride(0),
+              k_cache.stride(1), k_cache.stride(2), address(pos_state), theta, k0, S_max, B, H, D,
+              int(sn), int(sr), sb, sl, stream_handle())
 
 
 def rope_at_(x, pos_state, theta: float, offset: int = 0):
     """In-place RoPE of a ``(B, S, H, D)`` view whose first token sits at ``pos_state[0] + offset``,
     with the position read from device memory (decode under a CUDA graph)."""
     B, S, H, D = x.shape
-    _lib.call("ra_rope_at", ptr(x), c_ll(x.stride(0)), c_ll(x.stride(1)), c_ll(x.stride(2)), B, S, H, D,
-              int(offset), ptr(pos_state), c_f(theta), stream_ptr())
+    _lib.call("ra_rope_at", address(x), x.stride(0), x.stride(1), x.stride(2), B, S, H, D,
+              int(offset), address(pos_state), theta, stream_handle())
     return x
 
 
@@ -454,11 +468,11 @@ def kv_append(qkv, k_cache, v_cache, pos_state, k0: int = 0, stripe=None):
     B, S_max, H, D = k_cache.shape
     assert qkv.is_contiguous() and k_cache.stride() == v_cache.stride() and k_cache.stride(3) == 1
     sn, sr, sb, sl = stripe if stripe is not None else (0, 0, 0, 0)
-    _lib.call("ra_kv_append", ptr(qkv), ptr(k_cache), ptr(v_cache), c_ll(k_cache.stride(0)), c_ll(k_cache.stride(1)),
-              c_ll(k_cache.stride(2)), ptr(pos_state), c_ll(k0), S_max, B, H, D, int(sn), int(sr), c_ll(sb), c_ll(sl),
-              stream_ptr())
+    _lib.call("ra_kv_append", address(qkv), address(k_cache), address(v_cache), k_cache.stride(0), k_cache.stride(1),
+              k_cache.stride(2), address(pos_state), k0, S_max, B, H, D, int(sn), int(sr), sb, sl,
+              stream_handle())
 
 
 def decode_advance(state):
     """``state[0] += 1`` (position) and ``state[1] += 1`` (step) on the device."""
-    _lib.call("ra_decode_advance", ptr(state), stream_ptr())
+    _lib.call("ra_decode_advance", address(state), stream_handle())

@@ -64,6 +64,11 @@ def set_phase_timer(timer: "PhaseTimer | None") -> None:
     _TIMER = timer
 
 
+def idle() -> bool:
+    """Whether :func:`phase` regions are recorded by nothing (then several may share one call)."""
+    return _TIMER is None and not _ENABLED
+
+
 @contextlib.contextmanager
 def phase(name: str):
     """Marks a host-side phase of a step (attention forward, linear layers, gradient reduction, ...):

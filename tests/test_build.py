@@ -82,3 +82,25 @@ def test_wheel_is_self_contained(tmp_path):
     env = dict(os.environ, PYTHONPATH=str(site), RINGATTN_B200_NO_AUTOBUILD="1")
     r = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, env=env, cwd=str(tmp_path))
     assert r.returncode == 0 and "ok" in r.stdout, r.stdout + r.stderr
+
+
+def test_packed_launchers_say_what_they_take():
+    """A packed launcher's format has one code for each of its parameters in the source, in their order."""
+    import ctypes
+    import re
+
+    from ringattention_b200 import _build
+
+    lib = ctypes.CDLL(str(_build.build()))
+    code = {"int": "i", "unsigned int": "I", "long long": "q", "unsigned long long": "Q", "float": "f"}
+    seen = 0
+    for src in _build.sources():
+        text = src.read_text()
+        for name in re.findall(r"^RA_PACKED\((\w+)\)", text, re.M):
+            params = re.search(r'extern "C" int ' + name + r"\(([^)]*)\)\s*\{", text).group(1).split(",")
+            want = "".join("P" if "*" in p else code[re.sub(r"\s*\w+$", "", p.strip())] for p in params)
+            fmt = getattr(lib, name + "_packed_format")
+            fmt.restype = ctypes.c_char_p
+            assert fmt().decode() == want, name
+            seen += 1
+    assert seen > 30

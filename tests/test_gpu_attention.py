@@ -349,3 +349,35 @@ def test_rows_that_outgrow_their_reference(first, Sq, Sk, H, D):
         want = torch.softmax(x, -1) @ v[0, :, h].double()
         assert (out[0, :, h].double() - want).abs().max() <= 0.01 * want.abs().max()
         assert (lse[0, h].double() - torch.logsumexp(x, -1)).abs().max() <= 2e-5 * x[torch.isfinite(x)].abs().max() + 1e-3
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("B,S,H", [(1, 1, 1), (2, 130, 3), (1, 1000, 2)])
+@pytest.mark.parametrize("views", [False, True])
+def test_backward_in_one_call(B, S, H, D, views):
+    """Preparation, backward and the cast of dQ behind one call against the three one by one (which a phase timer asks for), for gradients of
+    their own and for views of one (B, S, 3, H, D) buffer: dK and dV the same bits, dQ (sums in any order) within 2^-7 of its largest entry."""
+    from ringattention_b200.ops import _lib, attention as A
+    from ringattention_b200.config import BlockwiseKwargs
+    from ringattention_b200.utils import tracing
+
+    g = torch.Generator(device="cuda").manual_seed(S)
+    buf = torch.randn(B, S, 3, H, D, device="cuda", generator=g).bfloat16()
+    q, k, v = buf.unbind(2) if views else (torch.empty(B, S, H, D, device="cuda", dtype=torch.bfloat16).copy_(t) for t in buf.unbind(2))
+    dout = torch.randn(B, S, H, D, device="cuda", generator=g).bfloat16()
+    plan = A.make_plan(0, 1, B, S, S, H, BlockwiseKwargs(causal_block_size=1, query_chunk_size=S, key_chunk_size=S), device=q.device)
+    out, lse = A.ring_forward(q, k, v, plan)
+    got, n = [], []
+    for timed in (False, True):
+        to = torch.full_like(buf, 7.0).unbind(2) if views else (None, None, None)
+        n0 = _lib.launches()
+        tracing.set_phase_timer(tracing.PhaseTimer() if timed else None)
+        try:
+            got.append(A.ring_backward(q, k, v, out, lse, dout, plan, dq=to[0], dk=to[1], dv=to[2]))
+        finally:
+            tracing.set_phase_timer(None)
+        n.append(_lib.launches() - n0)
+    _lib.check_status()
+    (dq, dk, dv), (dq2, dk2, dv2) = got
+    assert n[0] == n[1] and torch.equal(dk, dk2) and torch.equal(dv, dv2)
+    assert (dq.float() - dq2.float()).abs().max() <= 2 ** -7 * dq2.float().abs().max() + 1e-6

@@ -64,3 +64,28 @@ def test_blockwise_feedforward_still_takes_any_callable():
     x = torch.randn(2, 256, 64, device="cuda")
     y = rab.blockwise_feedforward(lambda t: torch.tanh(lin(t)), x, 64)
     assert torch.allclose(y, torch.tanh(lin(x)), atol=1e-5)
+
+
+@pytest.mark.parametrize("rows,chunk", [(1, 1), (128, 128), (300, 128), (1000, 512)])
+@pytest.mark.parametrize("keep", [False, True])
+def test_backward_in_one_call_a_chunk(rows, chunk, keep, monkeypatch):
+    """A chunk's launches behind one call against the same launches one by one: the same kernels on the same operands, so the same
+    bits (gradients of one, two and more chunks: in bf16 at once, or fp32 between them)."""
+    from ringattention_b200.ops import _lib, ffn
+
+    g = torch.Generator(device="cuda").manual_seed(rows)
+    d, F = 256, 520
+    x, dy = (torch.randn(rows, d, device="cuda", generator=g).bfloat16() for _ in range(2))
+    wgu, wd = (torch.randn(2 * F, d, device="cuda", generator=g) * 0.1).bfloat16(), (torch.randn(d, F, device="cuda", generator=g) * 0.1).bfloat16()
+    got = []
+    for one_by_one in (False, True):
+        if one_by_one:
+            monkeypatch.setattr(ffn.DenseLinears, "weights", lambda self: None)
+        lin = ffn.DenseLinears(wgu, wd, -(-rows // chunk))
+        kept = [] if keep else None
+        y = ffn.ffn_forward(lin, x, chunk, keep=kept)
+        n0 = _lib.launches()
+        dx = ffn.ffn_backward(lin, x, dy, chunk, kept=kept)
+        got.append((y, dx, lin.dwgu.grad, lin.dwd.grad, _lib.launches() - n0))
+    for a, b in zip(*got):
+        assert torch.equal(a, b) if torch.is_tensor(a) else a == b
