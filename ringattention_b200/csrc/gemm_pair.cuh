@@ -22,7 +22,7 @@ struct PairTile {
   static constexpr int A_STAGE_BYTES = BM * BK * 2;          // this CTA's rows
   static constexpr int B_STAGE_BYTES = BN_ / 2 * BK * 2;     // this CTA's half of the columns
   static constexpr int STAGE_BYTES = A_STAGE_BYTES + B_STAGE_BYTES;
-  static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 1024 /*align*/ + 256 /*barriers*/;
+  static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + PAIR_EPI_WARPS * EPI_STAGE + 1024 /*align*/ + 256 /*barriers*/;
   static constexpr int TMEM_COLS = NUM_ACC * BN_;
 };
 
@@ -35,7 +35,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
   uint8_t* sA = smem;
   uint8_t* sB = smem + STAGES * T::A_STAGE_BYTES;
-  uint64_t* full = reinterpret_cast<uint64_t*>(sB + STAGES * T::B_STAGE_BYTES);
+  uint8_t* sE = sB + STAGES * T::B_STAGE_BYTES;
+  uint64_t* full = reinterpret_cast<uint64_t*>(sE + PAIR_EPI_WARPS * EPI_STAGE);
   uint64_t* empty = full + STAGES;
   uint64_t* tfull = empty + STAGES;
   uint64_t* tempty = tfull + NUM_ACC;
@@ -178,7 +179,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
       tile_coords(tile, tiles_m, tiles_n, group_m, tm, tn);
       const uint32_t t_row = tmem_base + (static_cast<uint32_t>(quad * 32) << 16) + static_cast<uint32_t>(acc * BN);
       // a wait that gives up ends the loop for the whole warp: the TMEM loads behind it are warp-collective
-      if (!epilogue<BN>(p, t_row, (2 * tm + static_cast<int>(rank)) * BM + quad * 32 + lane, tn, half * (BN / 64), (half + 1) * (BN / 64),
+      if (!epilogue<BN>(p, t_row, (2 * tm + static_cast<int>(rank)) * BM + quad * 32, tn, half * (BN / 64), (half + 1) * (BN / 64),
+                        sE + (warp - 2) * EPI_STAGE,
                         [&] { return __all_sync(0xffffffffu, mbar_wait(&tfull[acc], acc_phase, wc, kTimeoutTmemFull)); }))
         break;
       tc_fence_before();

@@ -24,22 +24,22 @@ namespace gemm {
 // shorter epilogue; a pair costs a launch about 1 us and works for nothing on the second half of its rows where M ends in the first.
 // Nanoseconds per k-block, per 32 columns of epilogue (plain, with an addend, SwiGLU) and per tile and launch were fitted to 295 products
 // with 128 to 8192 rows timed on B200 in every form, K-major and MN-major: the choice is the fastest of the five within 9 %, within
-// 0.2 % on average, where the best of the three one-CTA widths takes 5 % longer on average and 43 % at worst. us, one CTA 256 / 128 / 64 columns, pair
+// 0.2 % on average, where the best of the three one-CTA widths takes 5 % longer on average. us, one CTA 256 / 128 / 64 columns, pair
 // 256 / 128, * the choice:
-//   8192 x 8192 x 8192 852 / 1172 / 1802, 750* / 894        4096 x 4096 x 4096, bf16 addend 143 / 165 / 299, 103* / 115
-//   22016 x 4096 x 4096, fp32 sums 604 / 737 / 1294, 529* / 636     2048 x 4096 x 4096 60 / 88 / 121, 49* / 61
-//   512 x 4096 x 11008 76 / 51 / 84, 61 / 45*               300 x 11008 x 2048 17.5* / 22.1 / 34.3, 27.3 / 26.5
-//   512 x 1536 x 512 10.1 / 7.4 / 6.2*, 11.2 / 8.2          1024 x 512 x 512 8.2 / 6.3 / 5.7*, 9.1 / 7.2
+//   8192 x 8192 x 8192 775 / 952 / 1638, 729* / 893         4096 x 4096 x 4096, bf16 addend 125 / 143 / 252, 99* / 113
+//   22016 x 4096 x 4096, fp32 sums 550 / 679 / 1190, 510* / 618     2048 x 4096 x 4096 51 / 80 / 126, 48* / 60
+//   512 x 4096 x 11008 72 / 49 / 83, 59 / 44*               300 x 11008 x 2048 15.9* / 21.3 / 34.7, 25.4 / 25.7
+//   512 x 1536 x 512 7.9 / 6.3 / 5.9*, 8.8 / 7.4            1024 x 2816 x 1024, fp32 sums 15.5 / 15.7 / 16.9, 13.7* / 14.5
 struct Form {
   int pair, width;
   int kb, epi[3], tile, fixed;
 };
 constexpr Form kForms[] = {
-    {0, 256, 319, {337, 946, 480}, 4080, 0},
-    {0, 128, 287, {472, 946, 251}, 1612, 1040},
-    {0, 64, 220, {847, 1308, 1}, 83, 2393},
-    {1, 256, 316, {493, 866, 64}, 3126, 0},
-    {1, 128, 202, {955, 1150, 273}, 1505, 216},
+    {0, 256, 318, {224, 658, 882}, 3567, 0},
+    {0, 128, 264, {374, 559, 423}, 1419, 1719},
+    {0, 64, 242, {918, 824, 1}, 733, 1458},
+    {1, 256, 306, {396, 429, 236}, 2366, 966},
+    {1, 128, 201, {555, 469, 26}, 1716, 2215},
 };
 inline const Form& choose_form(int M, int n, int num_kb, bool addend, bool swiglu) {
   const Form* best = nullptr;
