@@ -10,6 +10,8 @@ from typing import List
 
 import torch
 
+from ..ops import kernels as K
+
 # Free memory of the device below which the allocator gives its cached blocks back before a step is recorded. While a capture is under way it
 # cannot, and the private pool of a capture takes none of them: the recording would run out of memory beside gigabytes of cached blocks, or
 # leave the driver nothing to upload the graph with. A step's own buffers are megabytes (the partial results of 512 splits of 64 heads 17, the
@@ -106,7 +108,10 @@ class InferenceEngine:
 
     def _greedy_step(self) -> None:
         logits = self._decode_body(self._tok_buf)
-        self._tok_buf.copy_(self.sample(logits).to(torch.int32))
+        if self.sample is InferenceEngine.sample and logits.is_cuda and logits.dtype == torch.float32 and logits.stride(-1) == 1:
+            K.greedy(logits, self._tok_buf)  # what sample() and the cast say, in one launch
+        else:
+            self._tok_buf.copy_(self.sample(logits).to(torch.int32))
 
     def _record(self, body) -> torch.cuda.CUDAGraph:
         """Record ``body`` as ``torch.cuda.graph`` does, but leave the allocator's cached blocks alone while the device has room
@@ -167,7 +172,7 @@ class InferenceEngine:
         torch.cuda.synchronize()
         t_prefill = time.perf_counter() - t0
         out: List[torch.Tensor] = []
-        lat: List[float] = []
+        marks: List[tuple] = []
         nxt = self.first_tokens(logits)
         eager = 0 if self._graph_serves() else 2    # buffers and kernels must exist before a step is recorded
         for i in range(new_tokens):
@@ -181,6 +186,9 @@ class InferenceEngine:
             else:
                 nxt = self.sample(self.decode_step(nxt))
             e1.record()
-            torch.cuda.synchronize()
-            lat.append(e0.elapsed_time(e1))
-        return torch.stack([t.to(torch.int64) for t in out], dim=1), {"prefill_s": t_prefill, "decode_ms": lat}
+            marks.append((e0, e1))
+        # The host waits once, not for every token: between two steps the device otherwise idles for as long as the host takes to wake up
+        # and launch the next one.
+        torch.cuda.synchronize()
+        return (torch.stack([t.to(torch.int64) for t in out], dim=1),
+                {"prefill_s": t_prefill, "decode_ms": [a.elapsed_time(b) for a, b in marks]})

@@ -473,6 +473,14 @@ def kv_append(qkv, k_cache, v_cache, pos_state, k0: int = 0, stripe=None):
               stream_handle())
 
 
+def greedy(logits, out):
+    """``out (rows,)`` int32 <- ``logits (rows, n).argmax(-1)``, fp32 rows of any distance: one launch."""
+    rows, n = logits.shape
+    assert logits.dtype == torch.float32 and logits.stride(1) == 1 and out.dtype == torch.int32 and out.is_contiguous() and out.numel() == rows
+    _lib.call("ra_greedy", logits.data_ptr(), logits.stride(0), rows, n, out.data_ptr(), stream_handle())
+    return out
+
+
 def decode_advance(state):
     """``state[0] += 1`` (position) and ``state[1] += 1`` (step) on the device."""
     _lib.call("ra_decode_advance", address(state), stream_handle())

@@ -594,3 +594,23 @@ def test_recording_a_step_when_memory_is_short(monkeypatch):
         assert torch.equal(eng.generate(prompt, 6)[0], want) and len(calls) == 1 + fails
         given_back = torch.cuda.memory_reserved() < held - cached // 2
         assert given_back == (room > 0 or fails > 0)
+
+
+@pytest.mark.parametrize("rows,n", [(1, 1), (1, 3), (2, 31), (3, 1023), (8, 32000), (1, 50257), (4, 4096)])
+@pytest.mark.parametrize("kind", ["random", "ties", "nan", "hidden", "view"])
+def test_greedy_tokens(rows, n, kind):
+    """The same column as argmax: the first of equal ones (zeros of both signs among them), a NaN before any number, rows of -inf."""
+    from ringattention_b200.ops import kernels as K
+
+    g = torch.Generator(device="cuda").manual_seed(n)
+    x = torch.randn(rows, n + 5, device="cuda", generator=g)
+    x = x[:, 1:n + 1] if kind == "view" else x[:, :n].contiguous()
+    if kind == "ties":
+        x = x.round().clamp(-1, 0) * torch.tensor([1.0, -0.0], device="cuda")[torch.randint(0, 2, x.shape, device="cuda", generator=g)]
+    elif kind == "nan":
+        x[:, n // 2:][torch.rand(rows, n - n // 2, device="cuda", generator=g) < 0.1] = float("nan")
+    elif kind == "hidden":
+        x[:] = -float("inf")
+        x[0, n - 1] = -3e38
+    out = torch.full((rows,), -7, device="cuda", dtype=torch.int32)
+    assert torch.equal(K.greedy(x, out).long(), x.argmax(-1))
