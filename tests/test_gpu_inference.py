@@ -614,3 +614,35 @@ def test_greedy_tokens(rows, n, kind):
         x[0, n - 1] = -3e38
     out = torch.full((rows,), -7, device="cuda", dtype=torch.int32)
     assert torch.equal(K.greedy(x, out).long(), x.argmax(-1))
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("QL", [1, 3, 8])
+@pytest.mark.parametrize("kind", ["filled", "filled, by query", "starts late", "a hole"])
+def test_masked_decode_of_filled_ranges(kind, QL, D):
+    """Ranges of the cache that are seen up to a place are read without asking for their rows one by one: ends on both sides of words of bits
+    and of ranges, other ends for other queries (not plain then), rows hidden at the start and in the middle. What nobody sees holds NaN.
+    Within 2^-6 of the largest entry of dense attention in 64 bits (P and the result are rounded to bf16)."""
+    import ringattention_b200 as rab
+
+    ends = [1, 31, 32, 33, 127, 128, 129, 1000, 1599, 1600]
+    B, S, H = len(ends), 1600, 3
+    g = torch.Generator(device="cuda").manual_seed(QL)
+    q = torch.randn(B, QL, H, D, device="cuda", generator=g).bfloat16()
+    k, v = (torch.randn(B, S, H, D, device="cuda", generator=g).bfloat16() for _ in range(2))
+    at = torch.arange(S, device="cuda")
+    m = (at[None] < torch.tensor(ends, device="cuda")[:, None])[:, None, None].expand(B, 1, QL, S).clone()
+    if kind == "filled, by query":
+        m[:, :, -1:] &= at < 700
+    elif kind == "starts late":
+        m &= (at >= 40) | (m.sum(-1, keepdim=True) <= 40)
+    elif kind == "a hole":
+        m[..., 45:47] = False
+    else:
+        m = m[:, :, :1]
+    dead = ~m.any(2)[:, 0]
+    k[dead], v[dead] = float("nan"), float("nan")
+    got = rab.ringattention_inference(q, k, v, m).double()
+    x = torch.einsum("bqhd,bkhd->bhqk", q.double(), torch.nan_to_num(k.double())) / D ** 0.5
+    want = torch.einsum("bhqk,bkhd->bqhd", torch.softmax(x.masked_fill(~m, -float("inf")), -1), torch.nan_to_num(v.double()))
+    assert torch.isfinite(got).all() and (got - want).abs().max() <= 2 ** -6 * want.abs().max()
