@@ -124,6 +124,8 @@ __device__ __forceinline__ bool epilogue(const Params& p, uint32_t t_row, int ro
   // The addend is loaded one piece ahead, the first while the tile's products still run: with a short K the epilogue would otherwise be a
   // chain of memory round trips longer than the main loop.
   // (bf16: by rows, four pieces of 16 bytes a lane, so that it meets the accumulator before the rounding.)
+  // It has no more columns than C: those of the fp32 tail, which takes no addend, may lie behind its last row.
+  const int add_cols = p.C2 ? p.n_split : p.N;
   float4 ahead[8];
   auto load_addend = [&](int c) {
     if (add32) {
@@ -131,14 +133,15 @@ __device__ __forceinline__ bool epilogue(const Params& p, uint32_t t_row, int ro
 #pragma unroll
       for (int i = 0; i < 8; ++i) {
         const int row = row0 + 4 * i + f_row;
-        if (row < p.M && col < p.N)
+        if (row < p.M && col < add_cols && RA_IN_BOUNDS(col, 4, p.C2 ? p.ldr : p.N, kTagGemmResidual))
           ahead[i] = *reinterpret_cast<const float4*>(reinterpret_cast<const float*>(p.R) + static_cast<long long>(row) * p.ldr + col);
       }
     } else if (row0 + lane < p.M) {
       const __nv_bfloat16* src = reinterpret_cast<const __nv_bfloat16*>(p.R) + static_cast<long long>(row0 + lane) * p.ldr + n0 + c * 32;
 #pragma unroll
       for (int j = 0; j < 4; ++j)
-        if (n0 + c * 32 + j * 8 < p.N) ahead[j] = *reinterpret_cast<const float4*>(src + 8 * j);
+        if (n0 + c * 32 + j * 8 < add_cols && RA_IN_BOUNDS(n0 + c * 32 + j * 8, 8, p.C2 ? p.ldr : p.N, kTagGemmResidual))
+          ahead[j] = *reinterpret_cast<const float4*>(src + 8 * j);
     }
   };
   // a row's 32 values in bf16, and from there to C: four lanes a row, eight columns each

@@ -92,7 +92,7 @@ def linear_ex(x, w, out, *, residual=None, tail=None, n_split: Optional[int] = N
     of ``x``.
 
     ``x (M, K)`` and ``w (N, K)`` share a type; ``out`` (a row-strided view) is of that type or fp32. ``residual`` has
-    ``out``'s type and may be ``out``. ``tail``: an fp32 view that takes the columns from ``n_split`` on. ``bias``: fp32 by
+    ``out``'s type and columns (none of the tail's) and may be ``out``. ``tail``: an fp32 view that takes the columns from ``n_split`` on. ``bias``: fp32 by
     column, with entries up to a multiple of 32; ``alpha`` other than 1 needs one."""
     M, Kd = x.shape
     N = w.shape[0]
@@ -102,6 +102,7 @@ def linear_ex(x, w, out, *, residual=None, tail=None, n_split: Optional[int] = N
     assert bias is None or (bias.dtype == torch.float32 and bias.is_contiguous() and bias.numel() >= (N + 31) // 32 * 32)
     if residual is not None:
         assert residual.dtype == out.dtype and residual.stride(1) == 1 and not relu2
+        assert residual.shape[0] == M and residual.shape[1] >= n_split
     if tail is not None:
         assert tail.dtype == torch.float32 and tail.stride(1) == 1 and tail.shape[1] >= N - n_split
     ldr = residual.stride(0) if residual is not None else 0

@@ -112,6 +112,15 @@ def main():
                       ya=wide[:, 80:176], n32_from=64, act_from=96)
     K.linear_ex(torch.randn(77, 520, device=dev).to(bf), ws_[:192].contiguous(), canary((77, 64), bf),
                 tail=canary((77, 128), torch.float32), n_split=64)
+    # an addend beside a tail: it has the columns of `out` alone, from one piece of 32 columns to several tiles of them
+    for Mx, Nx, cut in ((77, 192, 64), (77, 192, 160), (300, 1000, 32), (520, 4096, 2080)):
+        xx, wx = torch.randn(Mx, 136, device=dev).to(bf), torch.randn(Nx, 136, device=dev).to(bf)
+        want = xx.float() @ wx.float().t()
+        for dt in (bf, torch.float32):
+            o, tail = canary((Mx, cut), dt, fill=torch.ones(Mx, cut, device=dev)), canary((Mx, Nx - cut), torch.float32)
+            K.linear_ex(xx, wx, o, residual=o, tail=tail, n_split=cut)
+            assert (o.float() - 1.0 - want[:, :cut]).abs().max() <= 2 ** -8 * want.abs().max() + 2 ** -8
+            assert (tail - want[:, cut:]).abs().max() <= 1e-4 * want.abs().max()
     K.linear_ex(torch.randn(77, 70, device=dev), torch.randn(51, 70, device=dev), canary((77, 51), torch.float32), relu2=True)
     K.linear_gated(xs_, ws_[:144].contiguous(), canary((3, 72), bf))
     K.linear_gated(torch.randn(77, 520, device=dev).to(bf), ws_[:144].contiguous(), canary((77, 72), bf))
