@@ -471,8 +471,10 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constant
     float l = 0.f;
     int cnt = 0;
     bool alive = true;
-    bool settled = false;  // every row of the warp has a reference
-    constexpr float kGrown = 32768.f;  // 128 * 2^8: a sum above it has a summand above 2^8, for which the accumulator is rescaled
+    bool settled = false;  // every row of the warp has a reference, and none has outgrown its own for kWatch tiles
+    int watch = 0;         // how many of those are to come
+    constexpr int kWatch = 64;
+    constexpr float kGrown = 255.f;  // no summand of a smaller sum reaches the 2^8 above which the accumulator is rescaled
 
     // Kinds of this query tile's bitmap tiles; without them every tile's bits are looked at, if there are any. A pointer for the whole
     // walk: asked for per tile out of the launch's parameters they cost every launch, those without a bitmap too (2 x 32 heads x 512, not
@@ -511,9 +513,11 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constant
       uint32_t pk[64];
       float sum;
       // The scores of a tile are scaled by the reference of the tiles before it, without a look at their maximum, as long as no row's
-      // sum shows that it has grown out of it: p is at most kGrown then, and bf16, l and the accumulator are as exact at any scale. Otherwise
-      // (also as long as some row of the warp has seen no key) the tile is taken again from TMEM, with the maximum. The 64 three-way
-      // maxima ahead of the first exponential took 490 of a tile's 3900 cycles.
+      // sum can hold a summand that asks for another reference (also as long as some row of the warp has seen no key, the maximum comes first):
+      // the 64 three-way maxima ahead of the first exponential took 490 of a tile's 3900 cycles. Otherwise the tile is taken again from
+      // TMEM, with the maximum, and the next kWatch tiles that stay below it are too: a second pass costs a tile, the maximum 2 (D 128) to
+      // 7 % (D 64) of one. References, and so results, are those of a walk that always looks. us, always / never twice in kWatch tiles / as often
+      // as it comes, 32 heads x 4096, causal, D 128, logits as in training 162 / 156 / 158; a bias that rises by 0.5 a key 240 / 256 / 338.
       for (;;) {
         uint32_t sr[128];
 #pragma unroll
@@ -611,6 +615,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constant
               break;
             }
             tc_fence_after();
+            if (__any_sync(0xffffffffu, need && m_ref != -INFINITY)) watch = kWatch + 1;
             const float alpha = (m_new == -INFINITY) ? 1.0f : exp2_approx(m_ref - m_new);
 #pragma unroll 1
             for (int c = 0; c < DV / 32; ++c) {
@@ -641,16 +646,21 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constant
         float sum_hi;
         f2_unpack(sum2, sum, sum_hi);
         sum += sum_hi;
-        const bool again = settled && !(sum <= kGrown);  // (NaN too)
-        if (!__any_sync(0xffffffffu, again || !s_ok)) break;
+        const bool grown = !(sum <= kGrown);  // (NaN too)
+        if (!__any_sync(0xffffffffu, (settled && grown) || !s_ok)) break;
         if (__any_sync(0xffffffffu, !s_ok)) {
           alive = false;
           break;
         }
         settled = false;
+        watch = kWatch + 1;
       }
       if (!alive) break;
-      if (!settled) settled = __all_sync(0xffffffffu, m_ref != -INFINITY);
+      if (!settled) {
+        const bool quiet = __all_sync(0xffffffffu, sum <= kGrown && m_ref != -INFINITY);
+        watch = quiet ? max(watch - 1, 0) : (watch > 0 ? kWatch : 0);
+        settled = quiet && watch == 0;
+      }
       l += sum;
       tmem_st_x32(tS[w] + lane_base, pk);
       tmem_st_x32(tS[w] + lane_base + 32, pk + 32);

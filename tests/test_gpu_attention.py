@@ -1,4 +1,6 @@
 """sm_100a attention kernels (one ring step) against the fp32 dense oracle, plus the public op."""
+import math
+
 import pytest
 import torch
 
@@ -323,7 +325,7 @@ def test_what_is_no_number_passes_through_a_launch_split_over_the_keys(where, ma
 @pytest.mark.parametrize("Sq,Sk,H", [(256, 1600, 2), (2048, 1600, 19), (130, 8000, 2)])  # one query tile a CTA, two, keys split
 @pytest.mark.parametrize("first", ["seen", "hidden"])
 def test_rows_that_outgrow_their_reference(first, Sq, Sk, H, D):
-    """Scores of a tile are scaled by the reference of the tiles before it as long as no row's sum has grown out of it. Here the logits of a row
+    """Scores of a tile are scaled by the reference of the tiles before it as long as no row's sum can hold an entry that outgrows it. Here the logits of a row
     step up by 2 to 800 from tile to tile, or down, or stay, by rows of all kinds side by side in a warp; `hidden`: many rows see no key
     of the first tiles. Against dense attention in 64 bits on the same bf16 numbers: 1e-2 of the largest entry (P and the result are rounded
     once each), the log-sum-exp within 2e-5 of the largest logit (fp32 sums of D products) plus 1e-3."""
@@ -349,6 +351,39 @@ def test_rows_that_outgrow_their_reference(first, Sq, Sk, H, D):
         want = torch.softmax(x, -1) @ v[0, :, h].double()
         assert (out[0, :, h].double() - want).abs().max() <= 0.01 * want.abs().max()
         assert (lse[0, h].double() - torch.logsumexp(x, -1)).abs().max() <= 2e-5 * x[torch.isfinite(x)].abs().max() + 1e-3
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("grows", [0.0, 7.5, 10.0, 14.0, 40.0])
+def test_probabilities_are_rounded_at_the_scale_of_their_row(grows, D):
+    """The rule of the reference, which fixes at what scale a probability is rounded to bf16: the first tile's maximum, then the maximum so far
+    whenever one row of the 32 of a warp exceeds its own by 2^8. One key of the third tile stands `grows` powers of two above its row.
+    Against the same rule in 64 bits: what is left are fp32 sums and roundings that fall the other way, some 3e-5; another scale for the
+    rows' probabilities gives 1e-3."""
+    from ringattention_b200.ops import _lib, flash
+
+    Sq, Sk, H = 2048, 640, 19  # two query tiles a CTA
+    g = torch.Generator(device="cuda").manual_seed(D)
+    q, k, v = (torch.randn(1, n, H, D, device="cuda", generator=g) for n in (Sq, Sk, Sk))
+    q[..., 0], k[..., 0] = 1.0, 0.0
+    k[:, 300, :, 0] = grows * math.log(2) * D ** 0.5
+    q, k, v = q.bfloat16(), k.bfloat16(), v.bfloat16()
+    ms = flash.MaskSpec(causal_block_size=0, q_pos=flash.Positions(0), k_pos=flash.Positions(0))
+    out, _ = flash.flash_fwd(q, k, v, ms, out_fp32=True)
+    _lib.check_status()
+    for h in (0, H - 1):
+        x = q[0, :, h].double() @ k[0, :, h].double().t() * (D ** -0.5 / math.log(2))
+        m, o, l = None, 0.0, 0.0
+        for j in range(0, Sk, 128):
+            new = x[:, j:j + 128].amax(1) if m is None else torch.maximum(m, x[:, j:j + 128].amax(1))
+            if m is not None:
+                new = torch.where((new > m + 8).view(-1, 32).any(1).repeat_interleave(32), new, m)
+                o, l = o * torch.exp2(m - new)[:, None], l * torch.exp2(m - new)
+            m = new
+            p = torch.exp2(x[:, j:j + 128] - m[:, None])
+            o, l = o + p.bfloat16().double() @ v[0, j:j + 128, h].double(), l + p.sum(1)
+        want = o / l[:, None]
+        assert (out[0, :, h].double() - want).norm() <= 2e-4 * want.norm()
 
 
 @pytest.mark.parametrize("D", [64, 128])
