@@ -122,6 +122,15 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
         }
       }
     }
+    // The leader's commits arrive at both CTAs' `empty`, and nothing orders one commit's arrivals before a later one's: without this wait the
+    // last of them could reach a CTA that has seen its last accumulator and left. (A stage that was never filled passes at once.)
+    for (int i = 0; i < STAGES && ok; ++i) {
+      ok = mbar_wait(&empty[stage], phase ^ 1u, wc, kTimeoutSmemEmpty);
+      if (++stage == STAGES) {
+        stage = 0;
+        phase ^= 1u;
+      }
+    }
     __syncwarp();
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer (the leader's, warp-uniform flow)

@@ -1,5 +1,7 @@
 """Model-checks the symmetric-memory schedules (KV slots, slabs, dK/dV accumulators, decode inbox)
 over every interleaving the barriers allow, and checks that the checker notices broken variants."""
+from pathlib import Path
+
 import pytest
 
 from ringattention_b200.parallel import protocol as P
@@ -66,3 +68,32 @@ def test_row_exchange_with_two_slots_is_race_free(n, rows):
 
 def test_row_exchange_with_one_slot_overwrites_unmerged_rows():
     assert "overwrites" in (P.check_row_exchange(2, 2, launches=2, slots=1) or "")
+
+
+def _arrivals_after_exit(fills, stages, tail):
+    """A CTA pair's `empty` ring as the CTA that does not issue sees it: the issuer's commits arrive at its barriers as late as they may, that
+    is when a wait asks for them. Counts those that are still under way when the CTA leaves; the waits are the kernel's, by parity."""
+    done, issued = [0] * stages, [0] * stages  # completed phases of each barrier; commits issued for it
+
+    def wait(stage, parity):  # returns once the phase of that parity is complete: the current phase has the other one
+        while done[stage] % 2 == parity:
+            assert done[stage] < issued[stage], "waits for a commit that nobody issues"
+            done[stage] += 1
+
+    stage = phase = 0
+    for f in range(fills + (stages if tail else 0)):
+        wait(stage, phase ^ 1)
+        if f < fills:
+            issued[stage] += 1  # filled, multiplied, committed
+        stage, phase = (0, phase ^ 1) if stage + 1 == stages else (stage + 1, phase)
+    return sum(issued) - sum(done)
+
+
+@pytest.mark.parametrize("stages", [6, 8])
+def test_no_commit_reaches_a_cta_of_a_pair_that_has_left(stages):
+    for fills in range(0, 4 * stages):
+        assert _arrivals_after_exit(fills, stages, tail=True) == 0
+        assert _arrivals_after_exit(fills, stages, tail=False) == min(fills, stages)
+    src = (Path(__file__).parent.parent / "ringattention_b200/csrc/gemm_pair.cuh").read_text()
+    producer = src[src.index("TMA producer"):src.index("MMA issuer (the leader's")]
+    assert producer.count("mbar_wait(&empty[stage], phase ^ 1u") == 2 and "i < STAGES && ok" in producer
