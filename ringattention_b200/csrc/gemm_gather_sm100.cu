@@ -97,6 +97,7 @@ extern "C" int ra_gemm_bf16_gather(const void* A, void* C, const void* R, int M,
     }
   }
   Params p{C, ldc, M, N, K, c_fp32, R, ldr, group_m > 0 ? group_m : 8, status};
+  p.n_split = N;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   return b_mn ? launch_gather<1>(ta, set, p, g, st) : launch_gather<0>(ta, set, p, g, st);
 }

@@ -45,7 +45,7 @@ struct Params {
   int relu2;
   float* C2;  // null = no tail
   long long ldc2;
-  int n_split;
+  int n_split;  // N without a tail
   // Plain K-major products only, before everything else in the epilogue: v = alpha * v + bias[column] (fp32, at least N
   // entries rounded up to a multiple of 32; null: neither)
   const float* bias;
@@ -124,8 +124,7 @@ __device__ __forceinline__ bool epilogue(const Params& p, uint32_t t_row, int ro
   // The addend is loaded one piece ahead, the first while the tile's products still run: with a short K the epilogue would otherwise be a
   // chain of memory round trips longer than the main loop.
   // (bf16: by rows, four pieces of 16 bytes a lane, so that it meets the accumulator before the rounding.)
-  // It has no more columns than C: those of the fp32 tail, which takes no addend, may lie behind its last row.
-  const int add_cols = p.C2 ? p.n_split : p.N;
+  // It has n_split columns, those that do not go to the fp32 tail.
   float4 ahead[8];
   auto load_addend = [&](int c) {
     if (add32) {
@@ -133,14 +132,14 @@ __device__ __forceinline__ bool epilogue(const Params& p, uint32_t t_row, int ro
 #pragma unroll
       for (int i = 0; i < 8; ++i) {
         const int row = row0 + 4 * i + f_row;
-        if (row < p.M && col < add_cols && RA_IN_BOUNDS(col, 4, p.C2 ? p.ldr : p.N, kTagGemmResidual))
+        if (row < p.M && col < p.n_split && RA_IN_BOUNDS(col, 4, p.C2 ? p.ldr : p.N, kTagGemmResidual))
           ahead[i] = *reinterpret_cast<const float4*>(reinterpret_cast<const float*>(p.R) + static_cast<long long>(row) * p.ldr + col);
       }
     } else if (row0 + lane < p.M) {
       const __nv_bfloat16* src = reinterpret_cast<const __nv_bfloat16*>(p.R) + static_cast<long long>(row0 + lane) * p.ldr + n0 + c * 32;
 #pragma unroll
       for (int j = 0; j < 4; ++j)
-        if (n0 + c * 32 + j * 8 < add_cols && RA_IN_BOUNDS(n0 + c * 32 + j * 8, 8, p.C2 ? p.ldr : p.N, kTagGemmResidual))
+        if (n0 + c * 32 + j * 8 < p.n_split && RA_IN_BOUNDS(n0 + c * 32 + j * 8, 8, p.C2 ? p.ldr : p.N, kTagGemmResidual))
           ahead[j] = *reinterpret_cast<const float4*>(src + 8 * j);
     }
   };

@@ -86,13 +86,19 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
     int stage = 0;
     uint32_t phase = 0;
     bool ok = true;
-    for (int tile = first; tile < num_tiles && ok; tile += step) {
+    // Behind the last tile it waits for every stage once more (one that was never filled passes at once): the leader's commits arrive at both
+    // CTAs' `empty`, and nothing orders one commit's arrivals before a later one's, so the last of them could otherwise reach a CTA that has
+    // seen its last accumulator and left.
+    bool more = true;
+    for (int tile = first; more && ok; tile += step) {
+      more = tile < num_tiles;
+      const int steps = more ? num_kb : STAGES;
       int tm, tn;
       tile_coords(tile, tiles_m, tiles_n, group_m, tm, tn);
       const int m0 = (2 * tm + static_cast<int>(rank)) * BM;
       // with SwiGLU the leader's columns are the gate's and the other CTA's the matching ones of up
       const int n0 = p.swiglu_F ? static_cast<int>(rank) * p.swiglu_F + tn * (BN / 2) : tn * BN + static_cast<int>(rank) * (BN / 2);
-      for (int kb = 0; kb < num_kb; ++kb) {
+      for (int kb = 0; kb < steps; ++kb) {
         const int k0 = kb * BK;
         if (!mbar_wait(&empty[stage], phase ^ 1u, wc, kTimeoutSmemEmpty)) {
           ok = false;
@@ -101,7 +107,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
         uint8_t* a_dst = sA + stage * T::A_STAGE_BYTES;
         uint8_t* b_dst = sB + stage * T::B_STAGE_BYTES;
         const uint32_t bar = cluster_map(&full[stage], 0);
-        if (elected) {
+        if (elected && more) {
           if (rank == 0) mbar_arrive_expect_tx(&full[stage], 2 * T::STAGE_BYTES);
           if (A_MN) {
 #pragma unroll
@@ -120,15 +126,6 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
           stage = 0;
           phase ^= 1u;
         }
-      }
-    }
-    // The leader's commits arrive at both CTAs' `empty`, and nothing orders one commit's arrivals before a later one's: without this wait the
-    // last of them could reach a CTA that has seen its last accumulator and left. (A stage that was never filled passes at once.)
-    for (int i = 0; i < STAGES && ok; ++i) {
-      ok = mbar_wait(&empty[stage], phase ^ 1u, wc, kTimeoutSmemEmpty);
-      if (++stage == STAGES) {
-        stage = 0;
-        phase ^= 1u;
       }
     }
     __syncwarp();

@@ -152,6 +152,7 @@ extern "C" int ra_gemm_bf16(const void* A, const void* B, void* C, const void* R
   const gemm::Operands o{A, B, lda, ldb};
   gemm::Params p{C, ldc, M, N, K, c_fp32 == 1, R, ldr, group_m > 0 ? group_m : 8, status, 0};
   p.r_fp32 = c_fp32 == 2;
+  p.n_split = N;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   if (!a_mn && !b_mn) return gemm::launch<0, 0>(o, p, s);
   if (!a_mn && b_mn) return gemm::launch<0, 1>(o, p, s);
@@ -173,6 +174,7 @@ extern "C" int ra_gemm_bf16_swiglu(const void* A, const void* W, void* Hout, int
     return kHostBadArg;
   }
   gemm::Params p{Hout, ldh, M, 2 * F, K, 0, nullptr, 0, group_m > 0 ? group_m : 8, status, F};
+  p.n_split = 2 * F;
   return gemm::launch<0, 0>(gemm::Operands{A, W, lda, ldb}, p, static_cast<cudaStream_t>(stream));
 }
 
@@ -193,7 +195,7 @@ extern "C" int ra_gemm_bf16_ex(const void* A, const void* B, void* C, const void
     set_error("ra_gemm_bf16_ex: bad shape/alignment");
     return kHostBadArg;
   }
-  gemm::Params p{C, ldc, M, N, K, c_fp32, R, ldr, group_m > 0 ? group_m : 8, status, 0, relu2, C2, ldc2, n_split,
+  gemm::Params p{C, ldc, M, N, K, c_fp32, R, ldr, group_m > 0 ? group_m : 8, status, 0, relu2, C2, ldc2, C2 ? n_split : N,
                  bias, alpha};
   return gemm::launch<0, 0>(gemm::Operands{A, B, lda, ldb}, p, static_cast<cudaStream_t>(stream));
 }
