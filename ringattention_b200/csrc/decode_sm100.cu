@@ -89,17 +89,35 @@ constexpr int DEC_UNROLL = 4;  // cache rows per thread and loop trip
 // Which rows [r0, r1) of a CTA's range each query row attends to under the mask, as bits in shared memory (seen[i][r - r0] of
 // query row i, and of any of them behind the last), so that rows nobody sees are not loaded and the loop over the rows asks no
 // global memory: a batch of unequal lengths otherwise streams its padding too (eight rows of the batch, half to all of 4000 cached
-// rows each, 32 heads: 98 us where the visible rows take 75). Ranges too long for the bits count as seen. Returns whether
-// any row is; call with all threads of the CTA. The bits share the space of the CTA's partial results: a KB more of shared memory
+// rows each, 32 heads: 98 us where the visible rows take 75). Ranges too long for the bits count as seen. Call with all
+// threads of the CTA. The bits share the space of the CTA's partial results: a KB more of shared memory
 // would leave one CTA of the tensor-core kernel per SM instead of two (65536 rows, four query rows, 32 heads: 283 instead of 190 us).
+//
+// Where every query row sees one and the same interval of the range and nothing else, as of a batch of caches that are padded on either side,
+// [r0, r1) becomes that interval (empty, if nobody sees any of it) and `plain` is set: no row has to be asked for again, in the
+// copies and in the loop; of other masks the copies' answers are kept for the loop. All lanes count the words that they hold: a branch for the one
+// that stores them took 5 us of 90. us a call on B200, D 128, half to all rows valid (padded on the right or the left) / the same with a hole every 50
+// rows: 8 x 32 heads x 4000 rows 71 / 85, four query rows 87 / 103, 16 x 32 x 1000 40 / 52.5, 16 x 32 x 300 14.2 / 21.3; asking for every row twice
+// without a look at the whole 89 / 89, 107 / 107, 54.5 / 55, 22 / 22.
 constexpr int SEEN_ROWS = 4096, SEEN_WORDS = SEEN_ROWS / 32;
 template <int MAXQ>
-__device__ __forceinline__ bool mark_seen(uint32_t* seen, const uint8_t* mask, long long m_sq, int QL, int r0, int r1) {
+__device__ __forceinline__ void mark_seen(uint32_t* seen, const uint8_t* mask, long long m_sq, int QL, int& r0, int& r1, bool& plain) {
+  __shared__ int4 part[WARPS];  // of each warp: first row, end, rows that anybody sees (once per lane that holds them), do query rows differ
   const int n = r1 - r0;
-  if (n > SEEN_ROWS) return true;
-  bool any = false;
+  if (n > SEEN_ROWS) return;
+  int first = SEEN_ROWS, end = 0, rows = 0;
+  uint32_t differ = 0;
+  auto count = [&](uint32_t w, int at) {  // a word of rows that anybody sees
+    if (w != 0u) {
+      first = min(first, at + __ffs(static_cast<int>(w)) - 1);
+      end = at + 32 - __clz(static_cast<int>(w));
+    }
+    rows += __popc(w);
+  };
   const uint8_t* m = mask + r0;
-  if (((reinterpret_cast<uintptr_t>(m) | static_cast<uintptr_t>(m_sq)) & 3) == 0) {
+  const bool by_four = ((reinterpret_cast<uintptr_t>(m) | static_cast<uintptr_t>(m_sq)) & 3) == 0;
+  const int lanes = by_four ? 8 : 32;  // that hold one word of bits
+  if (by_four) {
     // four rows a thread and load, a word of bits from eight threads (uniform trip count)
     for (int t = threadIdx.x * 4; t < ((n + 127) & ~127); t += THREADS * 4) {
       uint32_t v[MAXQ];
@@ -123,10 +141,11 @@ __device__ __forceinline__ bool mark_seen(uint32_t* seen, const uint8_t* mask, l
 #pragma unroll
         for (int o = 1; o < 8; o <<= 1) bits |= __shfl_xor_sync(0xffffffffu, bits, o);
         if ((threadIdx.x & 7) == 0) seen[i * SEEN_WORDS + (t >> 5)] = bits;
+        if (i > 0) differ |= bits ^ all;
         all |= bits;
       }
       if (MAXQ > 1 && (threadIdx.x & 7) == 0) seen[QL * SEEN_WORDS + (t >> 5)] = all;
-      any |= all != 0;
+      count(all, t & ~31);
     }
   } else {
     for (int t = threadIdx.x; t < ((n + 31) & ~31); t += THREADS) {  // a warp's 32 rows are one word
@@ -139,35 +158,34 @@ __device__ __forceinline__ bool mark_seen(uint32_t* seen, const uint8_t* mask, l
         if (i >= QL) break;
         const uint32_t bits = __ballot_sync(0xffffffffu, on[i]);
         if ((threadIdx.x & 31) == 0) seen[i * SEEN_WORDS + (t >> 5)] = bits;
+        if (i > 0) differ |= bits ^ all;
         all |= bits;
       }
       if (MAXQ > 1 && (threadIdx.x & 31) == 0) seen[QL * SEEN_WORDS + (t >> 5)] = all;
-      any |= all != 0;
+      count(all, t & ~31);
     }
   }
-  return __syncthreads_or(any) != 0;
-}
-// Whether every query row sees the same rows [r0, end) of the range and no others, as of a batch of caches that are filled up to a place of their
-// own each; r1 becomes that end. Then no row has to be asked for again, in the copies and in the loop. us a call on B200, half to all rows
-// valid, asked / plain: 8 x 32 heads x 4000 rows 88.9 / 79.9, four query rows 108 / 89.5, 16 x 32 x 1000 55.2 / 46.9, 16 x 32 x 300 23.3 / 19.1;
-// masks with holes in every range pay for the question: 89.1 / 93.8, 22.8 / 24.5. Behind mark_seen, with all threads of the CTA.
-template <int MAXQ>
-__device__ __forceinline__ bool seen_plain(const uint32_t* seen, int QL, int r0, int& r1) {
-  __shared__ int end;
-  const int n = r1 - r0, words = (n + 31) >> 5, t = threadIdx.x;
-  if (n > SEEN_ROWS) return false;
-  static_assert(SEEN_WORDS <= THREADS, "a word a thread");
-  bool ok = true;
-  if (t < words) {
-    const uint32_t* any = seen + (MAXQ > 1 ? QL : 0) * SEEN_WORDS;
-    const uint32_t w = any[t], next = t + 1 < words ? any[t + 1] : 0u;
-    ok = (w & (w + 1u)) == 0u && (w == 0xffffffffu || next == 0u);
-    for (int i = 0; MAXQ > 1 && i < QL; ++i) ok = ok && seen[i * SEEN_WORDS + t] == w;
-    if (w != 0u && next == 0u) end = 32 * t + __popc(w);  // (several such words: not plain, and not looked at)
+  first = __reduce_min_sync(0xffffffffu, first);
+  end = __reduce_max_sync(0xffffffffu, end);
+  rows = __reduce_add_sync(0xffffffffu, rows);
+  if (MAXQ > 1) differ = __any_sync(0xffffffffu, differ != 0u);
+  if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = make_int4(first, end, rows, static_cast<int>(differ));
+  __syncthreads();
+#pragma unroll
+  for (int w = 0; w < WARPS; ++w) {
+    const int4 x = part[w];
+    first = min(first, x.x);
+    end = max(end, x.y);
+    rows = w == 0 ? x.z : rows + x.z;
+    differ |= static_cast<uint32_t>(x.w);
   }
-  if (__syncthreads_and(ok) == 0) return false;
-  r1 = r0 + end;
-  return true;
+  if (rows == 0) {
+    r1 = r0;
+  } else if (rows == (end - first) * lanes && differ == 0u) {
+    plain = true;
+    r1 = r0 + end;
+    r0 += first;
+  }
 }
 __device__ __forceinline__ bool row_seen(const uint32_t* seen, int r, int r0, int r1) {
   return r1 - r0 > SEEN_ROWS || ((seen[(r - r0) >> 5] >> ((r - r0) & 31)) & 1u);
@@ -227,7 +245,7 @@ __global__ void __launch_bounds__(THREADS) decode_splitkv_kernel(const SplitPara
     rows_per_split = (S + p.splits - 1) / p.splits;
     if (rows_per_split < 1) rows_per_split = 1;
   }
-  const int r0 = split * rows_per_split;
+  int r0 = split * rows_per_split;
   int r1 = min(S, r0 + rows_per_split);
   const __nv_bfloat16* kb = p.k + b * p.k_sb + h * p.k_sh + dl * 8;
   const __nv_bfloat16* vb = p.v + b * p.v_sb + h * p.v_sh + dl * 8;
@@ -239,10 +257,7 @@ __global__ void __launch_bounds__(THREADS) decode_splitkv_kernel(const SplitPara
   const uint32_t* const seen_any = seen + (QL > 1 ? QL : 0) * SEEN_WORDS;
   const uint8_t* mask = MASKED ? p.mask + b * p.m_sb + h * p.m_sh : nullptr;
   bool plain = !MASKED;  // no row of [r0, r1) is hidden from anybody
-  if (MASKED && r0 < r1) {
-    if (!mark_seen<QL>(seen, mask, p.m_sq, QL, r0, r1)) r1 = r0;  // nothing to see here
-    else plain = seen_plain<QL>(seen, QL, r0, r1);
-  }
+  if (MASKED && r0 < r1) mark_seen<QL>(seen, mask, p.m_sq, QL, r0, r1, plain);
 
   // Two loops, so that the one without questions is the loop of a call without a mask and the other one pays nothing for the choice.
   auto walk = [&](auto plain_rows) {
@@ -250,11 +265,15 @@ __global__ void __launch_bounds__(THREADS) decode_splitkv_kernel(const SplitPara
     // The trip count is the same for every lane of a warp (the loop variable ignores `sub`), so the
     // full-mask shuffles below always see all 32 lanes; rows past the end are merely masked out.
     // stage `slot` <- the rows of the trip that starts at row base_w (of this warp)
+    // (asked: what the copies of a trip and of the ST - 1 before it asked the mask, UNROLL bits each, so that the loop need not ask again)
+    static_assert(ST * UNROLL <= 32, "a word of answers");
+    uint32_t asked = 0;
     auto issue = [&](int base_w, int slot) {
 #pragma unroll
       for (int u = 0; u < UNROLL; ++u) {
         const int r = base_w + sub + u * step;
         const bool in = r < r1 && (PLAIN || row_seen(seen_any, r, r0, r1));
+        if (!PLAIN) asked |= static_cast<uint32_t>(in) << u;
         const long long rr = in ? r : r0;  // r0 < r1 whenever the loop runs: a valid address, never read when !in
         uint4* dst = stage_buf + ((slot * UNROLL + u) * 2) * THREADS + threadIdx.x;
         cp_async16(dst, kb + rr * p.k_ss, in ? 16 : 0);
@@ -266,6 +285,7 @@ __global__ void __launch_bounds__(THREADS) decode_splitkv_kernel(const SplitPara
 #pragma unroll
       for (int i = 0; i < ST - 1; ++i) {
         if (ahead_w < r1) issue(ahead_w, slot_in);
+        asked <<= UNROLL;
         cp_async_commit();  // one group per trip, empty or not, so that the group count below is a constant
         ahead_w += step * UNROLL;
         slot_in = slot_in + 1 == ST ? 0 : slot_in + 1;
@@ -283,11 +303,12 @@ __global__ void __launch_bounds__(THREADS) decode_splitkv_kernel(const SplitPara
         cp_async_wait<(ST > 0 ? ST - 1 : 0)>();  // all but the newest ST - 1 groups are complete: this trip's rows are in
 #pragma unroll
         for (int u = 0; u < UNROLL; ++u) {
-          ok[u] = base + u * step < r1 && (PLAIN || row_seen(seen_any, base + u * step, r0, r1));
+          ok[u] = PLAIN ? base + u * step < r1 : ((asked >> (UNROLL * (ST - 1) + u)) & 1u) != 0u;
           const uint4* src = stage_buf + ((slot_out * UNROLL + u) * 2) * THREADS + threadIdx.x;
           ku[u] = src[0];
           vu[u] = src[THREADS];
         }
+        asked <<= UNROLL;
         slot_out = slot_out + 1 == ST ? 0 : slot_out + 1;
       } else {
 #pragma unroll
@@ -437,7 +458,7 @@ __global__ void __launch_bounds__(THREADS) decode_splitkv_mma_kernel(const Split
     rows_per_split = (S + p.splits - 1) / p.splits;
     if (rows_per_split < 1) rows_per_split = 1;
   }
-  const int r0 = split * rows_per_split;
+  int r0 = split * rows_per_split;
   int r1 = min(S, r0 + rows_per_split);
   __shared__ float sm_m[WARPS][8], sm_l[WARPS][8];
   __shared__ float sm_o[WARPS][8][D];
@@ -446,10 +467,7 @@ __global__ void __launch_bounds__(THREADS) decode_splitkv_mma_kernel(const Split
   const uint32_t* const seen_any = seen + QL * SEEN_WORDS;
   const uint8_t* mask = MASKED ? p.mask + b * p.m_sb + h * p.m_sh : nullptr;
   bool plain = !MASKED;
-  if (MASKED && r0 < r1) {
-    if (!mark_seen<8>(seen, mask, p.m_sq, QL, r0, r1)) r1 = r0;  // nothing to see here
-    else plain = seen_plain<8>(seen, QL, r0, r1);
-  }
+  if (MASKED && r0 < r1) mark_seen<8>(seen, mask, p.m_sq, QL, r0, r1, plain);
   const __nv_bfloat16* kb = p.k + b * p.k_sb + h * p.k_sh;
   const __nv_bfloat16* vb = p.v + b * p.v_sb + h * p.v_sh;
 

@@ -646,3 +646,28 @@ def test_masked_decode_of_filled_ranges(kind, QL, D):
     x = torch.einsum("bqhd,bkhd->bhqk", q.double(), torch.nan_to_num(k.double())) / D ** 0.5
     want = torch.einsum("bhqk,bkhd->bqhd", torch.softmax(x.masked_fill(~m, -float("inf")), -1), torch.nan_to_num(v.double()))
     assert torch.isfinite(got).all() and (got - want).abs().max() <= 2 ** -6 * want.abs().max()
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("QL", [1, 3, 8])
+@pytest.mark.parametrize("odd", [False, True])
+def test_masked_decode_of_caches_padded_on_either_side(odd, QL, D):
+    """One interval of the cache is seen, the same by every query row: it is read without asking for its rows. Its ends lie on both sides of words of
+    bits and of ranges; `odd`: rows of the mask at addresses of any alignment. What nobody sees holds NaN. Tolerance as above."""
+    import ringattention_b200 as rab
+
+    spans = [(0, 1600), (1, 1600), (31, 32), (32, 33), (33, 127), (127, 129), (128, 1000), (500, 1599), (1599, 1600), (700, 701)]
+    B, S, H = len(spans), 1600, 3
+    g = torch.Generator(device="cuda").manual_seed(QL)
+    q = torch.randn(B, QL, H, D, device="cuda", generator=g).bfloat16()
+    k, v = (torch.randn(B, S, H, D, device="cuda", generator=g).bfloat16() for _ in range(2))
+    wide = torch.zeros(B, 1, 1, S + 1, device="cuda", dtype=torch.bool)
+    m = wide[..., 1:] if odd else wide[..., :S].contiguous()
+    for b, (lo, hi) in enumerate(spans):
+        m[b, ..., lo:hi] = True
+    dead = ~m[:, 0, 0]
+    k[dead], v[dead] = float("nan"), float("nan")
+    got = rab.ringattention_inference(q, k, v, m).double()
+    x = torch.einsum("bqhd,bkhd->bhqk", q.double(), torch.nan_to_num(k.double())) / D ** 0.5
+    want = torch.einsum("bhqk,bkhd->bqhd", torch.softmax(x.masked_fill(~m, -float("inf")), -1), torch.nan_to_num(v.double()))
+    assert torch.isfinite(got).all() and (got - want).abs().max() <= 2 ** -6 * want.abs().max()
