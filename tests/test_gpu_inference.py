@@ -648,6 +648,19 @@ def test_masked_decode_of_filled_ranges(kind, QL, D):
     assert torch.isfinite(got).all() and (got - want).abs().max() <= 2 ** -6 * want.abs().max()
 
 
+def test_nothing_is_launched_first_inside_a_capture(monkeypatch):
+    """A kernel that is loaded while a step is recorded holds up a process's first prompt: the one that only recorded steps use runs before."""
+    from ringattention_b200.config import LlamaConfig
+    from ringattention_b200.models.llama_infer import LlamaInference
+    from ringattention_b200.ops import kernels as K
+
+    capturing, greedy = [], K.greedy
+    monkeypatch.setattr(K, "greedy", lambda *a: capturing.append(torch.cuda.is_current_stream_capturing()) or greedy(*a))
+    eng = LlamaInference(LlamaConfig.named("llama-tiny"), max_context=256, batch=2, device="cuda")
+    eng.generate(torch.randint(0, 100, (2, 128), device="cuda"), 5)
+    assert capturing == [False, True]
+
+
 @pytest.mark.parametrize("D", [64, 128])
 @pytest.mark.parametrize("QL", [1, 3, 8])
 @pytest.mark.parametrize("odd", [False, True])
