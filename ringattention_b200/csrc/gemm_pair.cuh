@@ -1,4 +1,4 @@
-// GEMM on pairs of CTAs (cta_group::2): 256 x BN output tiles, for products with at least two 128-row tiles.
+// GEMM on pairs of CTAs (cta_group::2): 256 x BN output tiles.
 //
 // What bounds the one-CTA kernel (gemm_kernel.cuh) is shared memory: per k-block of 64 a 128 x 256 tile writes 48 KiB by TMA and reads them
 // once for 512 cycles of tensor work, 768 cycles at 128 bytes a clock. A pair shares the B operand: each CTA stages its own 128 rows of

@@ -22,13 +22,17 @@ namespace gemm {
 // or 256 columns wide; the one with the shortest estimated time. Wide tiles and pairs move the fewest bytes per column, which decides once
 // every SM has several of them; below that a launch takes as long as one SM's tiles, and narrower ones spread over more SMs and have a
 // shorter epilogue; a pair costs a launch about 1 us and works for nothing on the second half of its rows where M ends in the first.
-// Nanoseconds per k-block, per 32 columns of epilogue (plain, with an addend, SwiGLU) and per tile and launch were fitted to 295 products
-// with 128 to 8192 rows timed on B200 in every form, K-major and MN-major: the choice is the fastest of the five within 9 %, within
-// 0.2 % on average, where the best of the three one-CTA widths takes 5 % longer on average. us, one CTA 256 / 128 / 64 columns, pair
-// 256 / 128, * the choice:
+// Nanoseconds per k-block, per 32 columns of epilogue (plain, with an addend, SwiGLU) and per tile and launch were fitted together to 295 products
+// with 128 to 8192 rows timed on B200 in every form, K-major and MN-major; a single one of them need not be the cost of what it is named for
+// (an epilogue that hides behind the products of the next tile leaves the fit little to go by), and shapes far outside have to be timed, not
+// worked out. 687 products with 9 to 8192 rows, weights out of memory: the choice takes 0.6 % longer than the fastest of the five on average,
+// 16 % at worst (32 of them more than 5 %, mostly below 256 rows). With 128 rows or fewer, where a pair's second CTA has no row,
+// the 36 products that get pairs all the same take 6 % less on average than the best one-CTA form (-3 to 22 %).
+// us, one CTA 256 / 128 / 64 columns, pair 256 / 128, * the choice:
 //   8192 x 8192 x 8192 775 / 952 / 1638, 729* / 893         4096 x 4096 x 4096, bf16 addend 125 / 143 / 252, 99* / 113
 //   22016 x 4096 x 4096, fp32 sums 550 / 679 / 1190, 510* / 618     2048 x 4096 x 4096 51 / 80 / 126, 48* / 60
 //   512 x 4096 x 11008 72 / 49 / 83, 59 / 44*               300 x 11008 x 2048 15.9* / 21.3 / 34.7, 25.4 / 25.7
+//   9 x 4096 x 4096 28.5 / 20.2 / 24.1, 24.4 / 18.8*
 //   512 x 1536 x 512 7.9 / 6.3 / 5.9*, 8.8 / 7.4            1024 x 2816 x 1024, fp32 sums 15.5 / 15.7 / 16.9, 13.7* / 14.5
 struct Form {
   int pair, width;
@@ -198,6 +202,12 @@ extern "C" int ra_gemm_bf16_ex(const void* A, const void* B, void* C, const void
   gemm::Params p{C, ldc, M, N, K, c_fp32, R, ldr, group_m > 0 ? group_m : 8, status, 0, relu2, C2, ldc2, C2 ? n_split : N,
                  bias, alpha};
   return gemm::launch<0, 0>(gemm::Operands{A, B, lda, ldb}, p, static_cast<cudaStream_t>(stream));
+}
+
+// The form that a product gets (`addend`: there is one; with SwiGLU N counts gate and up): its tiles' columns, negative on pairs of CTAs.
+extern "C" int ra_gemm_form(int M, int N, int K, int addend, int swiglu) {
+  const ra::gemm::Form& f = ra::gemm::choose_form(M, N, (K + ra::gemm::BK - 1) / ra::gemm::BK, addend != 0, swiglu != 0);
+  return f.pair ? -f.width : f.width;
 }
 
 RA_PACKED(ra_gemm_bf16)

@@ -76,6 +76,12 @@ def linear_swiglu(x, wgu, out=None, group_m: int = 8):
     return out
 
 
+def gemm_form(M: int, N: int, Kd: int, addend: bool = False, swiglu: bool = False) -> tuple:
+    """How a product is cut up: ``(CTAs that share a tile, columns of a tile)``. With ``swiglu`` ``N`` counts gate and up."""
+    w = _lib.lib().ra_gemm_form(M, N, Kd, int(addend), int(swiglu))
+    return (2, -w) if w < 0 else (1, w)
+
+
 def linear_dgrad(dy, w, out=None, residual=None):
     """``dx = dy W (+ residual)``; ``dy (M,N)``, ``w (N,K)`` read MN-major."""
     return gemm(dy, w, b_mn=True, out=out, residual=residual)

@@ -65,7 +65,7 @@ def test_linear_fwd_dgrad_wgrad_match_autograd():
 @pytest.mark.parametrize("a_mn,b_mn", [(False, False), (False, True), (True, True)])
 @pytest.mark.parametrize("M,N,Kd", [(1, 8, 8), (128, 64, 640), (100, 72, 200), (257, 200, 1000), (2048, 1024, 328), (1100, 3000, 72), (4000, 1544, 136)])
 def test_gemm_at_every_tile_width(M, N, Kd, a_mn, b_mn):
-    """Products that get tiles of 64, 128 and 256 columns, ragged in every direction, with and without an fp32 addend. The
+    """Products that get tiles of several widths (of each form: test_every_form), ragged in every direction, with and without an fp32 addend. The
     products of bf16 numbers are exact in fp32: tolerance 2e-6 of the sum of their magnitudes, plus bf16 rounding (2^-8)."""
     from ringattention_b200.ops import _lib, kernels as K
 
@@ -88,7 +88,7 @@ def test_gemm_at_every_tile_width(M, N, Kd, a_mn, b_mn):
 
 @pytest.mark.parametrize("M,F,Kd", [(5, 8, 64), (128, 72, 200), (300, 1000, 1024), (2048, 2816, 512), (2100, 5504, 136)])
 def test_swiglu_epilogue_at_every_tile_width(M, F, Kd):
-    """Gate and up columns of a tile come from two places of the weight: ragged widths at each tile width. The result equals
+    """Gate and up columns of a tile come from two places of the weight: ragged widths (at every form: test_every_form). The result equals
     the two-pass path, up to the last bit of a bf16 (2^-8) where a sum lies on a rounding border."""
     from ringattention_b200.ops import kernels as K
 
@@ -104,7 +104,7 @@ def test_swiglu_epilogue_at_every_tile_width(M, F, Kd):
 @pytest.mark.parametrize("a_mn,b_mn", [(False, False), (True, True)])
 @pytest.mark.parametrize("M,N,Kd", [(8, 8, 8), (104, 72, 200), (2048, 1024, 328), (4000, 1544, 136)])
 def test_gemm_fp32_addend_bf16_result(M, N, Kd, a_mn, b_mn):
-    """The last part of a sum kept in fp32, at tiles of 64, 128 and 256 columns: one rounding to bf16 (2^-8 of the value at most)
+    """The last part of a sum kept in fp32 (at every form: test_every_form): one rounding to bf16 (2^-8 of the value at most)
     beside 2e-6 of the sum of the magnitudes."""
     from ringattention_b200.ops import kernels as K
 
@@ -148,3 +148,86 @@ def test_gemm_on_cta_pairs(M, N, Kd, a_mn, b_mn):
 def test_swiglu_epilogue_on_cta_pairs(M, F, Kd):
     """One CTA of a pair holds the gate's columns, the other the matching ones of up. Tolerance as above."""
     test_swiglu_epilogue_at_every_tile_width(M, F, Kd)
+
+
+# (CTAs a tile, columns) -> M, N, K that get it with and without an addend and with SwiGLU on 148 SMs; M ends in either half of a pair's rows
+FORMS = {(1, 64): (104, 208, 200), (1, 128): (104, 11024, 520), (1, 256): (264, 11024, 2056), (2, 128): (648, 1552, 2056), (2, 256): (520, 16400, 520)}
+
+
+def _operands(M, N, Kd):
+    from ringattention_b200.ops import kernels as K
+
+    g = torch.Generator(device="cuda").manual_seed(M + N)
+    a, b = torch.randn(M, Kd, device="cuda", generator=g).bfloat16(), torch.randn(N, Kd, device="cuda", generator=g).bfloat16()
+    want = a.double() @ b.double().t()
+    return K, g, a, b, want, 2e-6 * (a.double().abs() @ b.double().abs().t())
+
+
+def _form_is(form, M, N, Kd, **kw):
+    from ringattention_b200.ops import kernels as K
+
+    if torch.cuda.get_device_properties(0).multi_processor_count != 148:
+        pytest.skip("the shapes are chosen for 148 SMs")
+    assert K.gemm_form(M, N, Kd, **kw) == form
+
+
+@pytest.mark.parametrize("form", FORMS)
+def test_every_form(form):
+    """Each form of the kernel by its name, with each kind of result: bf16, bf16 with an addend in bf16 or fp32, accumulated in fp32, SwiGLU. Tolerances as
+    above; SwiGLU as the two-pass path."""
+    M, N, Kd = FORMS[form]
+    K, g, a, b, want, slack = _operands(M, N, Kd)
+    _form_is(form, M, N, Kd)
+    c = K.gemm(a, b)
+    assert ((c.double() - want).abs() <= slack + 2**-8 * want.abs()).all()
+    _form_is(form, M, N, Kd, addend=True)
+    r = torch.randn(M, N + 8, device="cuda", generator=g)[:, :N]
+    for rr in (r, r.bfloat16()):
+        c = K.gemm(a, b, out=torch.empty(M, N, device="cuda", dtype=torch.bfloat16), residual=rr)
+        assert ((c.double() - want - rr.double()).abs() <= slack + 2e-6 * rr.double().abs() + 2**-8 * (want + rr.double()).abs()).all()
+    acc = r.clone()
+    K.gemm(a, b, out=acc, residual=acc)
+    assert ((acc.double() - want - r.double()).abs() <= slack + 2e-6 * r.double().abs()).all()
+    _form_is(form, M, N, Kd, swiglu=True)
+    w = (b * Kd ** -0.5).bfloat16()
+    gu = K.linear_fwd(a, w).float()
+    h = torch.nn.functional.silu(gu[:, :N // 2]) * gu[:, N // 2:]
+    assert ((K.linear_swiglu(a, w).float() - h).abs() <= 2**-7 * h.abs() + 1e-4).all()
+
+
+@pytest.mark.parametrize("form", FORMS)
+def test_layer_epilogues_at_every_form(form):
+    """Bias with a factor, the squared relu into a strided view, and an fp32 tail that begins at a tile's start and inside either half of one."""
+    from ringattention_b200.ops import _lib
+
+    M, N, Kd = FORMS[form]
+    K, g, a, b, want, slack = _operands(M, N, Kd)
+    _form_is(form, M, N, Kd)
+    bias = torch.randn((N + 31) // 32 * 32, device="cuda", generator=g)
+    c = K.linear_ex(a, b, torch.empty(M, N, device="cuda"), bias=bias, alpha=0.37)
+    assert ((c.double() - 0.37 * want - bias[:N].double()).abs() <= slack + 1e-6 * (want.abs() + 10)).all()
+    wide = torch.full((M, N + 16), 3.0, device="cuda", dtype=torch.bfloat16)
+    K.linear_ex(a, b, wide[:, 8:8 + N], relu2=True)
+    sq = want.clamp_min(0).square()
+    assert ((wide[:, 8:8 + N].double() - sq).abs() <= 2 * want.abs() * slack + slack ** 2 + 2**-8 * sq).all()
+    assert (wide[:, :8] == 3).all() and (wide[:, 8 + N:] == 3).all()
+    at = N // (2 * form[1]) * form[1]  # where a tile begins
+    for cut in {at, at + 32, at + form[1] // 2 + form[1] // 4 // 32 * 32} - {0}:
+        main, tail = torch.empty(M, cut, device="cuda", dtype=torch.bfloat16), torch.empty(M, N - cut, device="cuda")
+        K.linear_ex(a, b, main, tail=tail, n_split=cut)
+        assert ((main.double() - want[:, :cut]).abs() <= slack[:, :cut] + 2**-8 * want[:, :cut].abs()).all()
+        assert ((tail.double() - want[:, cut:]).abs() <= slack[:, cut:]).all()
+    _lib.check_status()
+
+
+@pytest.mark.parametrize("M", [16, 128])
+@pytest.mark.parametrize("addend", [False, True])
+def test_a_pair_whose_second_cta_has_no_row(M, addend):
+    N, Kd = 1032, 4104
+    K, g, a, b, want, slack = _operands(M, N, Kd)
+    _form_is((2, 128), M, N, Kd, addend=addend)
+    r = torch.randn(M, N, device="cuda", generator=g).bfloat16() if addend else torch.zeros(M, N, device="cuda", dtype=torch.bfloat16)
+    room = torch.full((M + 256, N), 3.0, device="cuda", dtype=torch.bfloat16)
+    K.gemm(a, b, out=room[:M], residual=r if addend else None)
+    want = want + r.double()
+    assert ((room[:M].double() - want).abs() <= slack + 2e-6 * r.double().abs() + 2**-8 * want.abs()).all() and (room[M:] == 3.0).all()
