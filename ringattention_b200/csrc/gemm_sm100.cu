@@ -26,7 +26,7 @@ namespace gemm {
 // with 128 to 8192 rows timed on B200 in every form, K-major and MN-major; a single one of them need not be the cost of what it is named for
 // (an epilogue that hides behind the products of the next tile leaves the fit little to go by), and shapes far outside have to be timed, not
 // worked out. 687 products with 9 to 8192 rows, weights out of memory: the choice takes 0.6 % longer than the fastest of the five on average,
-// 16 % at worst (32 of them more than 5 %, mostly below 256 rows). With 128 rows or fewer, where a pair's second CTA has no row,
+// 16 % at worst (32 of them more than 5 %). With 128 rows or fewer, where a pair's second CTA has no row,
 // the 36 products that get pairs all the same take 6 % less on average than the best one-CTA form (-3 to 22 %).
 // us, one CTA 256 / 128 / 64 columns, pair 256 / 128, * the choice:
 //   8192 x 8192 x 8192 775 / 952 / 1638, 729* / 893         4096 x 4096 x 4096, bf16 addend 125 / 143 / 252, 99* / 113
