@@ -144,10 +144,6 @@ def stream_ptr() -> ctypes.c_void_p:
     return ctypes.c_void_p(stream_handle())
 
 
-def ptr(t: torch.Tensor | None) -> ctypes.c_void_p:
-    return ctypes.c_void_p(0 if t is None else t.data_ptr())
-
-
 def address(t: torch.Tensor | None) -> int:
     return 0 if t is None else t.data_ptr()
 
@@ -162,15 +158,28 @@ def count_launch(n: int = 1) -> None:
     _LAUNCHES += n
 
 
+# what ctypes makes of a number, by the code of its field
+_AS_C = {"P": ctypes.c_void_p, "i": ctypes.c_int, "I": ctypes.c_uint, "q": ctypes.c_longlong, "Q": ctypes.c_ulonglong, "f": ctypes.c_float}
+
+
+def _pack_as_c(pack, fmt: str, args) -> bytes:
+    """Packs what the struct module refuses as ctypes takes it: a float beyond fp32's range becomes an infinity, an integer keeps its low
+    bits, None is a null pointer."""
+    if len(args) != len(fmt):
+        raise KernelError(f"{len(args)} arguments for a launcher of {len(fmt)}")
+    return pack(*(_AS_C[c](a).value or 0 for c, a in zip(fmt, args)))
+
+
 def _entry(name: str):
-    """The launcher and, where it takes its arguments as one packed block, what packs them: the library says in which
-    format. Such launchers take plain numbers (pointers as integers)."""
+    """The launcher and, where it takes its arguments as one packed block, what packs them and the format, which the library
+    says. Such launchers take plain numbers (pointers as integers)."""
     handle = lib()
     fmt = getattr(handle, name + "_packed_format", None)
     if fmt is None:
-        return getattr(handle, name), None
+        return getattr(handle, name), None, None
     fmt.restype = ctypes.c_char_p
-    return getattr(handle, name + "_packed"), struct.Struct("@" + fmt().decode()).pack
+    text = fmt().decode()
+    return getattr(handle, name + "_packed"), struct.Struct("@" + text).pack, text
 
 
 def call(name: str, *args, n_kernels: int = 1) -> None:
@@ -179,8 +188,15 @@ def call(name: str, *args, n_kernels: int = 1) -> None:
     entry = _FNS.get(name)
     if entry is None:
         entry = _FNS[name] = _entry(name)
-    fn, pack = entry
-    rc = fn(pack(*args)) if pack is not None else fn(*args)
+    fn, pack, fmt = entry
+    if pack is None:
+        rc = fn(*args)
+    else:
+        try:
+            block = pack(*args)
+        except (struct.error, OverflowError):
+            block = _pack_as_c(pack, fmt, args)
+        rc = fn(block)
     if rc != 0:
         msg = lib().ra_last_error()
         raise KernelError(f"{name} failed ({rc}): {msg.decode() if msg else ''}")

@@ -104,3 +104,25 @@ def test_packed_launchers_say_what_they_take():
             assert fmt().decode() == want, name
             seen += 1
     assert seen > 30
+
+
+def test_packed_arguments_take_what_ctypes_took(monkeypatch):
+    import struct
+
+    from ringattention_b200.ops import _lib
+
+    fmt = "PiIqQf"
+    read, got = struct.Struct(fmt), []
+    monkeypatch.setitem(_lib._FNS, "launcher", (lambda block: got.append(read.unpack(block)) or 0, read.pack, fmt))
+
+    def taken(*args):
+        _lib.call("launcher", *args, n_kernels=0)
+        return got[-1]
+
+    assert taken(16, -5, 7, -9, 11, 0.5) == (16, -5, 7, -9, 11, 0.5)
+    assert taken(None, 2**40 + 5, -1, 2**63, -1, 1e300) == (0, 5, 2**32 - 1, -2**63, 2**64 - 1, float("inf"))
+    assert taken(0, 0, 0, 0, 0, -1e39)[5] == -float("inf")
+    with pytest.raises(_lib.KernelError):
+        taken(1, 2, 3)
+    with pytest.raises(TypeError):
+        taken(0, 0, 0, 0, 0, "x")
