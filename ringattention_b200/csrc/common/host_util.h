@@ -7,6 +7,7 @@
 #include <string.h>
 
 #include <tuple>
+#include <type_traits>
 
 namespace ra {
 
@@ -36,7 +37,10 @@ void set_error(const char* msg);
 // A launcher's arguments as one block of memory, each at its natural alignment, as Python's struct module packs them: RA_PACKED(fn) adds
 // fn_packed(block) and fn_packed_format(), the block's format ('P' pointer, 'i' int, 'q' long long, 'f' float ...). ctypes converts arguments
 // one by one: 17 of them take 6.7 us, more than the launch, packed they take 1.1.
-template <typename T> constexpr char pack_code() { return 'P'; }
+template <typename T> constexpr char pack_code() {
+  static_assert(std::is_pointer<T>::value, "no code for this type");
+  return 'P';
+}
 template <> constexpr char pack_code<int>() { return 'i'; }
 template <> constexpr char pack_code<unsigned int>() { return 'I'; }
 template <> constexpr char pack_code<long long>() { return 'q'; }
@@ -44,7 +48,6 @@ template <> constexpr char pack_code<unsigned long long>() { return 'Q'; }
 template <> constexpr char pack_code<float>() { return 'f'; }
 template <typename T>
 T unpack_next(const unsigned char* block, size_t& at) {
-  static_assert(pack_code<T>() != 'P' || sizeof(T) == sizeof(void*), "no code for this type");
   at = (at + alignof(T) - 1) / alignof(T) * alignof(T);
   T v;
   memcpy(&v, block + at, sizeof(T));

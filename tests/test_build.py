@@ -106,6 +106,41 @@ def test_packed_launchers_say_what_they_take():
     assert seen > 30
 
 
+@pytest.mark.parametrize("module,packer,source,name", [
+    ("flash", "_FWD_ARGS", "attn_fwd_sm100.cu", "RaAttnFwdArgs"), ("flash", "_BWD_ARGS", "attn_api.h", "RaAttnBwdArgs"),
+    ("flash", "_BWD_RUN_ARGS", "backward_runs.cu", "RaAttnBwdRun"), ("decode", "_DECODE_ARGS", "decode_sm100.cu", "RaDecodeArgs")])
+def test_packed_structures_are_laid_out_as_declared(module, packer, source, name):
+    """The blocks that launchers read as C structures have one code for each field that the source declares, in their order, and no less bytes."""
+    import importlib
+    import re
+    import struct
+
+    from ringattention_b200 import _build
+
+    code = {"int": "i", "unsigned int": "I", "long long": "q", "unsigned long long": "Q", "float": "f"}
+
+    def fields(src, struct_name):
+        text = re.sub(r"//[^\n]*", "", (_build.CSRC / src).read_text())
+        body = re.search(r"struct " + struct_name + r"\s*\{(.*?)\};", text, re.S).group(1)
+        out = ""
+        for decl in filter(None, (d.strip() for d in body.split(";"))):
+            kind = re.match(r"(?:const\s+)?(unsigned long long|unsigned int|long long|\w+)", decl).group(1)
+            if kind == "RaAttnBwdArgs":
+                out += fields("attn_api.h", kind)
+                continue
+            for one in decl.split(","):
+                out += "P" if "*" in one else code[kind]
+        return out
+
+    def codes(fmt):
+        return "".join(c * int(n or 1) for n, c in re.findall(r"(\d*)([a-zA-Z])", fmt))
+
+    have = getattr(importlib.import_module(f"ringattention_b200.ops.{module}"), packer)
+    want = fields(source, name)
+    assert codes(have.format) == want
+    assert have.size == struct.calcsize("@" + want + "0P")  # to the structure's end, its alignment included
+
+
 def test_packed_arguments_take_what_ctypes_took(monkeypatch):
     import struct
 
