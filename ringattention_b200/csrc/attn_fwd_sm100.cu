@@ -865,25 +865,26 @@ __global__ void __launch_bounds__(256) attn_merge_kernel(const float* __restrict
 }
 
 // How a launch is cut up: two query tiles a CTA ("pairs"), one (HALVES), or one and its keys over several CTAs. The estimate is the time of
-// the launch in hundredths of a step of pairs (two 128 x 128 tiles; 1.82 us at D 128, 1.77 at D 64): a CTA takes its steps and a
+// the launch in hundredths of a step of pairs (two 128 x 128 tiles; 1.8 us at D 128, 1.6 at D 64): a CTA takes its steps and a
 // fixed cost (start-up, first loads, epilogue), and the CTAs, longest first, go to whichever SM is free: the SMs are busy for the average load at
 // least, and the k-th CTA of an SM is no shorter than the longest that starts behind k - 1 full rounds. Segment ids and bitmaps are not
 // looked at: the causal rule alone gives the lengths.
-// The constants are fitted to 120 launches of both head dims timed in every form on B200 (300 to 32768 query rows, 2 to 32 heads, causal or not, up to
-// 65536 keys): the choice is the fastest form or within 3 % of it. A step of HALVES loads K and V for one query tile only, so at D 128 it takes
-// 15 % longer; its CTA ends sooner. us, pairs / HALVES / keys over 2 / over 4 CTAs, D 128, * the choice:
-//   32 heads x 512, not causal 18.3 / 13.8* / 35.9 / -       32 x 4096, not causal 286* / 317 / - / -     32 x 4096, causal 158* / 196 / - / -
-//   4 x 4096, causal 70.6 / 42.8* / 49.2 / 70.1              16 x 2048, not causal 41.6* / 51.3 / - / -   16 x 500 on 16384 keys 256 / 158 / 96* / 113
-//   32 x 1000 on 16384 keys 261* / 320 / 369 / 399           32 x 128 on 4096 keys 62 / 44 / 33 / 26*
-// With equal steps, a fixed cost of 2.5 steps and whole rounds for launches that are not causal only, 32 heads x 4096, not causal, went to HALVES
-// and 16 x 500 causal rows on 16384 keys to three CTAs each (136 us).
+// The constants are fitted to 110 launches of both head dims timed in every form on B200 (256 to 32768 query rows, 2 to 32 heads, causal or not, up to
+// 65536 keys): the choice takes 0.2 % longer than the fastest form on average, 6 % at worst (three of them more than 3 %). A step of HALVES
+// loads K and V for one query tile only and takes as long as one of pairs all the same; its CTAs end later (the two groups' results
+// are put together). us, pairs / HALVES / keys over 2 / over 4 CTAs, D 128, * the choice:
+//   32 heads x 512, not causal 17.2 / 13.6* / 35.0 / -       32 x 4096, not causal 277* / 283 / - / -     32 x 4096, causal 153* / 182 / - / -
+//   4 x 4096, causal 68.5 / 41.4* / 48.1 / 68.0              16 x 2048, not causal 40.7* / 49.9 / 92 / 126 16 x 500 on 16384 keys 245 / 136 / 85* / 99
+//   32 x 1000 on 16384 keys 249* / 275 / 327 / 343           32 x 128 on 4096 keys 62 / 41 / 32 / 25*     2 x 12318, causal 187 / 106* / 120 / 149
+// With constants of an earlier kernel (a step of HALVES 15 % longer, its CTA 1.4 steps shorter) the last of them went to keys over two CTAs, and the
+// choice took 0.7 % longer than the fastest on average, 14 % at worst.
 struct FwdShape {
   bool halves;
   int splits;
 };
 inline FwdShape fwd_shape(int B, int H, int Sq, int Sk, int D, int cbs, long long q_off, long long k_off, bool one_run, bool may_split) {
-  const int step = D == 128 ? 115 : 96, cta = D == 128 ? 490 : 400, cta_pair = D == 128 ? 650 : 430;  // of HALVES, HALVES, pairs
-  constexpr int step_pair = 100, merge = 500;  // merge: partial results out and in again, one more launch
+  const int step = D == 128 ? 99 : 102, cta = D == 128 ? 630 : 635, cta_pair = D == 128 ? 565 : 590;  // of HALVES, HALVES, pairs
+  constexpr int step_pair = 100, merge = 425;  // merge: partial results out and in again, one more launch
   const int nk = (Sk + 127) / 128, nq = (Sq + 127) / 128, sms = sm_count();
   const long long bh = static_cast<long long>(B) * H;
   FwdShape best{false, 1};

@@ -231,6 +231,22 @@ def test_every_way_a_forward_is_cut_up(B, Sq, Sk, H, cbs, cache_idx, D):
     _check_call(B, Sq, Sk, H, D, cbs=cbs, cache_idx=cache_idx, grad=Sq * Sk * B * H < 3e8)
 
 
+@pytest.mark.parametrize("B,Sq,Sk,H,D,cbs,splits", [
+    (1, 500, 16384, 16, 128, 0, 2), (1, 128, 4096, 32, 128, 0, 4), (1, 500, 16384, 32, 128, 0, 1), (1, 4096, 4096, 4, 128, 1, 1),
+    (1, 12318, 12318, 2, 128, 1, 1), (1, 12269, 12269, 2, 64, 1, 1)])
+def test_keys_are_split_as_was_fastest(B, Sq, Sk, H, D, cbs, splits, monkeypatch):
+    """The rule's choice where every form was timed: two heads of 12318 causal rows take 106 us on whole rows, 120 with the keys over two CTAs."""
+    from ringattention_b200.ops import _lib, flash
+
+    if torch.cuda.get_device_properties(0).multi_processor_count != 148:
+        pytest.skip("timed with 148 SMs")
+    rule, chosen = _lib.lib().ra_attn_fwd_splits, []
+    monkeypatch.setattr(_lib.lib(), "ra_attn_fwd_splits", lambda a: chosen.append(rule(a)) or chosen[-1])
+    q, k = (torch.zeros(B, n, H, D, device="cuda", dtype=torch.bfloat16) for n in (Sq, Sk))
+    flash.flash_fwd(q, k, k, flash.MaskSpec(causal_block_size=cbs, q_pos=flash.Positions(Sk - Sq), k_pos=flash.Positions(0)))
+    assert chosen == [splits]
+
+
 @pytest.mark.parametrize("D", [64, 128])
 @pytest.mark.parametrize("S,H,q_pos,k_pos", [
     (512, 8, (0,), (0,)),                     # four query tiles a head: two groups on one tile
