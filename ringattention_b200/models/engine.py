@@ -118,7 +118,8 @@ class InferenceEngine:
         (:data:`RECORD_ROOM`): emptying the cache before every prompt's recording made the next prompt's prefill allocate all of
         its buffers from the driver again. A step that needs more than there was is recorded again without the cache. The buffers of
         the graph recorded before are taken over (it is dropped here)."""
-        # eager steps sample without this kernel, and loading it while a capture is under way takes 16 to 60 ms
+        # Eager steps sample without this kernel: it would be loaded while the capture is under way. The first one of a process took 19 to 76 ms so, on
+        # two machines; 19 to 20 with the kernel there.
         if self.sample is InferenceEngine.sample and self.device.type == "cuda":
             K.greedy(torch.zeros(1, 1, device=self.device), torch.empty(1, device=self.device, dtype=torch.int32))
         torch.cuda.synchronize()
