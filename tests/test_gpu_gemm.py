@@ -121,7 +121,7 @@ def test_gemm_fp32_addend_bf16_result(M, N, Kd, a_mn, b_mn):
 @pytest.mark.parametrize("a_mn,b_mn", [(False, False), (False, True), (True, False), (True, True)])
 @pytest.mark.parametrize("M,N,Kd", [(512, 4104, 2056), (520, 2056, 2056), (1030, 4104, 2056), (1000, 4104, 1000), (1030, 6000, 2056), (3900, 4104, 1000)])
 def test_gemm_on_cta_pairs(M, N, Kd, a_mn, b_mn):
-    """Products that get pairs of CTAs at both widths: an odd number of 128-row tiles, rows that end in either CTA's half, ragged columns
+    """Products that get pairs of CTAs at both widths (1000 x 4104 x 1000 with an addend only): an odd number of 128-row tiles, rows that end in either CTA's half, ragged columns
     and K, a strided result, and results in bf16, bf16 with an addend and accumulated in fp32. Tolerances as above."""
     from ringattention_b200.ops import _lib, kernels as K
 
